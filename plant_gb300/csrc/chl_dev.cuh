@@ -32,8 +32,8 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 
 // ---------------------------------------------------------------- scans
 // Exclusive prefix sum of n u32 values into u64 outputs; out[n] = total.
-// Entries at index >= *d_n (when d_n is non-null) count as zero, so the
-// launch shape depends only on the host bound n.
+// With d_n, only the first *d_n entries are read and only their prefixes and
+// out[n] are written, so the launch shape depends only on the host bound n.
 int scan_u32_excl(const uint32_t *in, uint64_t *out, uint64_t n,
                   const uint64_t *d_n, void *tmp, size_t tmp_bytes,
                   cudaStream_t s);

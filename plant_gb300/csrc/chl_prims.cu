@@ -19,6 +19,11 @@ __device__ __forceinline__ uint64_t bound_n(uint64_t n, const uint64_t *d_n) {
     return n;
 }
 
+// Tiles that hold an item.  A bound read from the device is often far below
+// the host's (a label buffer has room for a whole superstep): walking every
+// tile of the buffer cost 0.5 ms per scan of a nearly empty 120 M entry one.
+__device__ __forceinline__ uint64_t live_tiles(uint64_t m) { return (m + kScanTile - 1) / kScanTile; }
+
 // Block-wide exclusive scan of one u64 per thread; returns the block total.
 __device__ uint64_t block_excl_scan(uint64_t x, uint64_t *warp_tot) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
@@ -53,6 +58,7 @@ __global__ void scan_tile_sums(const uint32_t *in, uint64_t n, const uint64_t *d
                                uint64_t *tile_sum, uint64_t ntiles) {
     __shared__ uint64_t wt[33];
     const uint64_t m = bound_n(n, d_n);
+    ntiles = live_tiles(m);
     for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
         uint64_t base = t * kScanTile;
         uint64_t s = 0;
@@ -68,8 +74,9 @@ __global__ void scan_tile_sums(const uint32_t *in, uint64_t n, const uint64_t *d
     }
 }
 
-__global__ void scan_tile_prefix(uint64_t *tile_sum, uint64_t ntiles, uint64_t *total_out) {
+__global__ void scan_tile_prefix(uint64_t *tile_sum, uint64_t n, const uint64_t *d_n, uint64_t *total_out) {
     __shared__ uint64_t wt[33];
+    const uint64_t ntiles = live_tiles(bound_n(n, d_n));
     uint64_t carry = 0;
     for (uint64_t b = 0; b < ntiles; b += blockDim.x) {
         uint64_t i = b + threadIdx.x;
@@ -92,6 +99,7 @@ __global__ void scan_tiles(const uint32_t *in, uint64_t *out, uint64_t n,
     __shared__ uint64_t wt[33];
     __shared__ uint32_t vals[kScanTile];
     const uint64_t m = bound_n(n, d_n);
+    ntiles = live_tiles(m);
     for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
         uint64_t base = t * kScanTile;
 #pragma unroll
@@ -133,7 +141,7 @@ int scan_u32_excl(const uint32_t *in, uint64_t *out, uint64_t n, const uint64_t 
     uint64_t *tile = (uint64_t *)tmp;
     int grid = (int)std::min<uint64_t>(ntiles, (uint64_t)device_sms() * 8);
     scan_tile_sums<<<grid, kScanThreads, 0, s>>>(in, n, d_n, tile, ntiles);
-    scan_tile_prefix<<<1, 1024, 0, s>>>(tile, ntiles, out + n);
+    scan_tile_prefix<<<1, 1024, 0, s>>>(tile, n, d_n, out + n);
     scan_tiles<<<grid, kScanThreads, 0, s>>>(in, out, n, d_n, tile, ntiles);
     CHL_CUDA(cudaGetLastError());
     return CHL_OK;
@@ -175,6 +183,29 @@ __global__ void radix_hist(const uint64_t *keys, const uint64_t *d_n, uint64_t c
         hist[(uint64_t)i * gridDim.x + blockIdx.x] = h[i];
 }
 
+// Exclusive prefix of one digit's block counts, one thread block per digit
+// (the rows are independent; the 256 digit totals are summed by every scatter
+// block for itself).  One block over all 256 x 304 counts took 60-80 us of a
+// serial chain, three quarters of a small sort; this takes about 3 us.
+__global__ void __launch_bounds__(kSortThreads) radix_rows(const uint32_t *hist, uint64_t *offs, uint64_t *tot,
+                                                           int blocks) {
+    __shared__ uint64_t wt[33];
+    __shared__ uint64_t chunk;
+    const uint64_t row = (uint64_t)blockIdx.x * blocks;
+    uint64_t carry = 0;
+    for (int b = 0; b < blocks; b += blockDim.x) {
+        const int i = b + threadIdx.x;
+        const uint64_t x = i < blocks ? hist[row + i] : 0;
+        const uint64_t ex = block_excl_scan(x, wt);
+        if (i < blocks) offs[row + i] = carry + ex;
+        if (threadIdx.x == blockDim.x - 1) chunk = ex + x;
+        __syncthreads();
+        carry += chunk;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) tot[blockIdx.x] = carry;
+}
+
 // Scatter of one digit pass.  A block walks its range in tiles of kTile
 // items: warp w holds the tile's items [w * kWarpItems, (w + 1) *
 // kWarpItems) in registers, ranks them per digit (match_any per round of 32,
@@ -189,7 +220,8 @@ constexpr int kWarpItems = 32 * kTileItems;
 
 __global__ void __launch_bounds__(kSortThreads) radix_scatter(const uint64_t *kin, const uint32_t *vin, uint64_t *kout,
                                                               uint32_t *vout, const uint64_t *d_n, uint64_t cap,
-                                                              int shift, const uint64_t *offs) {
+                                                              int shift, const uint64_t *offs, const uint64_t *tot) {
+    __shared__ uint64_t wt[33];
     __shared__ uint64_t s_k[kTile];
     __shared__ uint32_t s_v[kTile];
     __shared__ uint32_t wh[kSortWarps][kRadix];   // per-warp digit counts, then their prefix over warps
@@ -197,11 +229,12 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter(const uint64_t *ki
     __shared__ uint32_t w_tot[kSortWarps];
     __shared__ uint64_t run[kRadix];              // each digit's next global slot
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-    for (int i = tid; i < kRadix; i += blockDim.x) run[i] = offs[(uint64_t)i * gridDim.x + blockIdx.x];
     uint64_t n = *d_n;
     if (n > cap) n = cap;
     uint64_t b, e;
     block_range(n, b, e);
+    if (b == e) return;   // the whole block: a short sort leaves most blocks without items
+    run[tid] = block_excl_scan(tot[tid], wt) + offs[(uint64_t)tid * gridDim.x + blockIdx.x];
     for (uint64_t base = b; base < e; base += kTile) {
         const uint32_t cnt = (uint32_t)((e - base) < (uint64_t)kTile ? (e - base) : (uint64_t)kTile);
         for (int i = tid; i < kSortWarps * kRadix; i += blockDim.x) (&wh[0][0])[i] = 0;
@@ -271,30 +304,13 @@ __global__ void __launch_bounds__(kSortThreads) radix_scatter(const uint64_t *ki
     }
 }
 
-__global__ void hist_to_u32_excl(const uint32_t *hist, uint64_t *offs, int entries) {
-    // single block exclusive scan over digit-major histogram
-    __shared__ uint64_t wt[33];
-    __shared__ uint64_t chunk;
-    uint64_t carry = 0;
-    for (int b = 0; b < entries; b += blockDim.x) {
-        int i = b + threadIdx.x;
-        uint64_t x = i < entries ? hist[i] : 0;
-        uint64_t ex = block_excl_scan(x, wt);
-        if (i < entries) offs[i] = carry + ex;
-        if (threadIdx.x == blockDim.x - 1) chunk = ex + x;
-        __syncthreads();
-        carry += chunk;
-        __syncthreads();
-    }
-}
-
 constexpr int kSortBlocksPerSM = 2;
 
 }  // namespace
 
 size_t radix_tmp_bytes() {
     size_t g = (size_t)device_sms() * kSortBlocksPerSM;
-    return g * kRadix * (sizeof(uint32_t) + sizeof(uint64_t));
+    return (g + 1) * kRadix * (sizeof(uint32_t) + sizeof(uint64_t));
 }
 
 int radix_sort_pairs(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1,
@@ -306,13 +322,14 @@ int radix_sort_pairs(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1,
     uint64_t *offs = (uint64_t *)((char *)tmp + (size_t)grid * kRadix * sizeof(uint32_t));
     // keep offs 8-byte aligned
     offs = (uint64_t *)(((uintptr_t)offs + 7) & ~(uintptr_t)7);
+    uint64_t *tot = offs + (uint64_t)grid * kRadix;
     int p = 0;
     uint64_t *ki = k0, *ko = k1;
     uint32_t *vi = v0, *vo = v1;
     for (int shift = 0; shift < bits; shift += 8) {
         radix_hist<<<grid, kSortThreads, 0, s>>>(ki, d_n, cap, shift, hist);
-        hist_to_u32_excl<<<1, 1024, 0, s>>>(hist, offs, grid * kRadix);
-        radix_scatter<<<grid, kSortThreads, 0, s>>>(ki, vi, ko, vo, d_n, cap, shift, offs);
+        radix_rows<<<kRadix, kSortThreads, 0, s>>>(hist, offs, tot, grid);
+        radix_scatter<<<grid, kSortThreads, 0, s>>>(ki, vi, ko, vo, d_n, cap, shift, offs, tot);
         std::swap(ki, ko);
         std::swap(vi, vo);
         p ^= 1;

@@ -34,3 +34,21 @@ def test_betweenness_is_a_permutation(P):
     g = P.Graph.rmat(10, 8, seed=2)
     o = P.Order.betweenness(g, 32, seed=3)
     assert sorted(o.tolist()) == list(range(g.get_n()))
+
+
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 2047, 2048, 2049, 77824, 77825, 700001])
+def test_sort_sizes(P, n):
+    """Vertex counts at the edges of the radix sort's tiles and block ranges:
+    degree descending, ties by the seeded key."""
+    rng = np.random.default_rng(n)
+    src = rng.integers(0, n, 2 * n).astype(np.uint32)
+    dst = rng.integers(0, n, 2 * n).astype(np.uint32)
+    g = P.Graph.from_arcs(n, src[src != dst], dst[src != dst], np.ones(int((src != dst).sum()), np.int32))
+    deg = g.degrees(True).astype(np.int64) + g.degrees(False)
+    with np.errstate(over="ignore"):
+        z = np.uint64(5) * np.uint64(0x9E3779B97F4A7C15) + np.arange(n, dtype=np.uint64)
+        z = z + np.uint64(0x9E3779B97F4A7C15)
+        z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+        z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+        z = z ^ (z >> np.uint64(31))
+    assert np.array_equal(P.Order.degree(g, seed=5), np.lexsort((z, -deg)))
