@@ -42,40 +42,127 @@ __device__ __forceinline__ uint64_t gmix(uint64_t z) {
     return z ^ (z >> 31);
 }
 
-// raw features: log1p deg, log1p 2-hop degree sum, sampled clustering
+// raw features: log1p deg, log1p 2-hop degree sum, sampled clustering.
+// 16 lanes per vertex: one clustering sample each, and the neighbours' degrees
+// strided over them (whole numbers: their sum is the same in any order).  A
+// hub's list is bound by the latency of its dependent loads, so each lane has
+// 8 of them in flight; one thread per vertex took 2.61 ms on a 2^15-vertex
+// RMAT graph, all of it in its few hubs.
+constexpr int kFeatLanes = kClusterSamples;
+constexpr int kFeatLoads = 8;
+static_assert(kFeatLanes == 16, "two vertices per warp");
+
 __global__ void feat_raw(uint32_t n, const uint64_t *off_out, const uint32_t *head_out, const uint64_t *off_in,
                          uint64_t seed, float *x) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    const uint32_t sub = threadIdx.x % kFeatLanes;
+    const uint32_t mask = (threadIdx.x & 16u) ? 0xFFFF0000u : 0x0000FFFFu;
+    const uint32_t groups = gridDim.x * (blockDim.x / kFeatLanes);
+    for (uint32_t v = blockIdx.x * (blockDim.x / kFeatLanes) + threadIdx.x / kFeatLanes; v < n; v += groups) {
         const uint64_t b = off_out[v], e = off_out[v + 1];
         const double deg = (double)(e - b) + (double)(off_in[v + 1] - off_in[v]);
-        double two = 0.0;
-        for (uint64_t a = b; a < e; ++a) {
-            const uint32_t u = head_out[a];
-            two += (double)(off_out[u + 1] - off_out[u]) + (double)(off_in[u + 1] - off_in[u]);
+        uint64_t sum = 0;
+        for (uint64_t a = b + sub; a < e; a += kFeatLoads * kFeatLanes) {
+            uint32_t u[kFeatLoads];
+#pragma unroll
+            for (int q = 0; q < kFeatLoads; ++q) {
+                const uint64_t at = a + (uint64_t)q * kFeatLanes;
+                u[q] = at < e ? head_out[at] : 0xFFFFFFFFu;
+            }
+#pragma unroll
+            for (int q = 0; q < kFeatLoads; ++q)
+                if (u[q] != 0xFFFFFFFFu)
+                    sum += (off_out[u[q] + 1] - off_out[u[q]]) + (off_in[u[q] + 1] - off_in[u[q]]);
         }
-        float cc = 0.f;
+#pragma unroll
+        for (int o = kFeatLanes / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(mask, sum, o);
+        uint32_t hit = 0;
         const uint64_t d = e - b;
         if (d >= 2) {
-            uint32_t hit = 0;
-            for (int k = 0; k < kClusterSamples; ++k) {
-                const uint64_t h = gmix(seed ^ ((uint64_t)v * 0x100000001B3ull + (uint64_t)k));
-                const uint64_t i = h % d;
-                uint64_t j = (h >> 32) % (d - 1);
-                if (j >= i) ++j;
-                const uint32_t a = head_out[b + i], c = head_out[b + j];
-                const uint64_t ab = off_out[a], ae = min(off_out[a + 1], ab + kClusterScan);
-                for (uint64_t q = ab; q < ae; ++q)
-                    if (head_out[q] == c) {
-                        ++hit;
-                        break;
-                    }
+            const uint64_t h = gmix(seed ^ ((uint64_t)v * 0x100000001B3ull + (uint64_t)sub));
+            const uint64_t i = h % d;
+            uint64_t j = (h >> 32) % (d - 1);
+            if (j >= i) ++j;
+            const uint32_t a = head_out[b + i], c = head_out[b + j];
+            const uint64_t ab = off_out[a], ae = min(off_out[a + 1], ab + kClusterScan);
+            for (uint64_t q = ab; q < ae && !hit; q += kFeatLoads) {
+#pragma unroll
+                for (int t = 0; t < kFeatLoads; ++t) hit |= (q + t < ae && head_out[q + t] == c) ? 1u : 0u;
             }
-            cc = (float)hit / (float)kClusterSamples;
         }
-        x[(size_t)v * NF + 0] = (float)log1p(deg);
-        x[(size_t)v * NF + 1] = (float)log1p(two);
-        x[(size_t)v * NF + 2] = cc;
+        const uint32_t hits = __popc(__ballot_sync(mask, hit != 0));
+        if (sub == 0) {
+            x[(size_t)v * NF + 0] = (float)log1p(deg);
+            x[(size_t)v * NF + 1] = (float)log1p((double)sum);
+            x[(size_t)v * NF + 2] = (float)hits / (float)kClusterSamples;
+        }
     }
+}
+
+// Standardised feature columns, (x - mean) / population sd in double: column
+// sums, then squared deviations, each as one partial per block summed in
+// block order (the same result for the same graph), then the columns in
+// place.  On the host the same three passes and the two copies were 1.6 ms of
+// a 2.6 ms prediction for 2^18 vertices.
+constexpr int kStatThreads = 256;
+constexpr int kStatBlocks = 128;   // at most
+
+__device__ void col_totals(const double *part, int blocks, double *tot) {
+    // every thread calls; tot (shared) holds NF totals afterwards
+    __syncthreads();
+    if (threadIdx.x < NF) {
+        double t = 0.0;
+        for (int b = 0; b < blocks; ++b) t += part[b * NF + threadIdx.x];
+        tot[threadIdx.x] = t;
+    }
+    __syncthreads();
+}
+
+// part[block][k] = sum over the block's vertices of x (sums == null), or of
+// (x - mean)^2 with the means of the column sums `sums`
+__global__ void __launch_bounds__(kStatThreads) feat_stats(uint32_t n, const float *x, const double *sums,
+                                                           double *part) {
+    __shared__ double tot[NF];
+    __shared__ double wsum[kStatThreads / 32][NF];
+    double mean[NF] = {0.0, 0.0, 0.0}, acc[NF] = {0.0, 0.0, 0.0};
+    if (sums) {
+        col_totals(sums, gridDim.x, tot);
+        for (int k = 0; k < NF; ++k) mean[k] = tot[k] / n;
+    }
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+#pragma unroll
+        for (int k = 0; k < NF; ++k) {
+            const double d = (double)x[(size_t)v * NF + k] - mean[k];
+            acc[k] += sums ? d * d : d;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NF; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(kFull, acc[k], o);
+        if (lane_id() == 0) wsum[threadIdx.x >> 5][k] = acc[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < NF) {
+        double t = 0.0;
+        for (int w = 0; w < kStatThreads / 32; ++w) t += wsum[w][threadIdx.x];
+        part[blockIdx.x * NF + threadIdx.x] = t;
+    }
+}
+
+__global__ void __launch_bounds__(kStatThreads) feat_scale(uint32_t n, const double *sums, const double *squares,
+                                                           int blocks, float *x) {
+    __shared__ double tot[NF], tot2[NF];
+    col_totals(sums, blocks, tot);
+    col_totals(squares, blocks, tot2);
+    double mean[NF], inv[NF];
+    for (int k = 0; k < NF; ++k) {
+        mean[k] = tot[k] / n;
+        const double sd = n > 1 ? sqrt(tot2[k] / n) : 0.0;
+        inv[k] = sd > 1e-12 ? 1.0 / sd : 0.0;
+    }
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        for (int k = 0; k < NF; ++k)
+            x[(size_t)v * NF + k] = (float)(((double)x[(size_t)v * NF + k] - mean[k]) * inv[k]);
 }
 
 // h0 = relu(x W0 + b0), one thread per (vertex, channel)
@@ -91,7 +178,13 @@ __global__ void layer0_fwd(uint32_t n, const float *x, const float *W0, const fl
     }
 }
 
-// m(v) = mean over out-neighbours of h(u); one warp per vertex, 2 channels per lane
+// m(v) = mean over out-neighbours of h(u); one warp per vertex, 2 channels per
+// lane.  The rows are added in arc order (the sum's rounding does not depend
+// on the launch); a hub's chain is the latency of its row loads, so 32 of them
+// are in flight and the next 32 heads are read meanwhile (one row at a time
+// took 547 us a layer on a 2^15-vertex RMAT graph).
+constexpr int kRows = 32;
+
 __global__ void aggregate_mean(uint32_t n, const uint64_t *off, const uint32_t *head, const __nv_bfloat16 *h,
                                __nv_bfloat16 *m) {
     const uint32_t lane = lane_id();
@@ -99,10 +192,38 @@ __global__ void aggregate_mean(uint32_t n, const uint64_t *off, const uint32_t *
     for (uint32_t v = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); v < n; v += warps) {
         const uint64_t b = off[v], e = off[v + 1];
         float s0 = 0.f, s1 = 0.f;
-        for (uint64_t a = b; a < e; ++a) {
-            const __nv_bfloat162 t = *(const __nv_bfloat162 *)(h + (size_t)head[a] * H + 2 * lane);
-            s0 += __bfloat162float(t.x);
-            s1 += __bfloat162float(t.y);
+        uint32_t next = b + lane < e ? head[b + lane] : 0u;
+        for (uint64_t a = b; a < e; a += kRows) {
+            const uint32_t cnt = e - a < kRows ? (uint32_t)(e - a) : (uint32_t)kRows;
+            const uint32_t hd = next;
+            next = a + kRows + lane < e ? head[a + kRows + lane] : 0u;
+            if (cnt == kRows) {
+                __nv_bfloat162 t[kRows];
+#pragma unroll
+                for (int q = 0; q < kRows; ++q)
+                    t[q] = *(const __nv_bfloat162 *)(h + (size_t)__shfl_sync(kFull, hd, q) * H + 2 * lane);
+#pragma unroll
+                for (int q = 0; q < kRows; ++q) {
+                    s0 += __bfloat162float(t[q].x);
+                    s1 += __bfloat162float(t[q].y);
+                }
+            } else {
+                for (uint32_t j = 0; j < cnt; j += 4) {
+                    __nv_bfloat162 t[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const uint32_t u = __shfl_sync(kFull, hd, j + q);
+                        if (j + q < cnt) t[q] = *(const __nv_bfloat162 *)(h + (size_t)u * H + 2 * lane);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (j + q < cnt) {
+                            s0 += __bfloat162float(t[q].x);
+                            s1 += __bfloat162float(t[q].y);
+                        }
+                    }
+                }
+            }
         }
         const float inv = e > b ? 1.f / (float)(e - b) : 0.f;
         __nv_bfloat162 o;
@@ -119,10 +240,6 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
         "{%0,%1,%2,%3};\n"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
-__device__ __forceinline__ uint32_t pack2(__nv_bfloat16 lo, __nv_bfloat16 hi) {
-    return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
 // Y[n x 64] = A[n x K] B[K x 64] (+ bias, relu) where A's columns are the
@@ -249,38 +366,75 @@ __global__ void head_fwd_bwd(uint32_t n, const __nv_bfloat16 *h, const float *wo
 // tensor cores: warp w of a block owns rows k in [16w, 16w+16) of dW and
 // walks the block's slice of vertices 16 at a time (the reduction axis);
 // partial tiles are added to dW atomically.  db[c] += sum_v dz[v][c].
-__global__ void grad_w_mma(uint32_t n, const __nv_bfloat16 *A0, const __nv_bfloat16 *A1,
-                           const __nv_bfloat16 *dzb, const float *dz, float *dW, float *db) {
-    const uint32_t lane = lane_id(), gid = lane >> 2, tig = lane & 3;
-    const uint32_t warp = threadIdx.x >> 5;          // 8 warps: 128 rows of dW
+// 32 vertices' rows are staged in shared memory with 16-byte loads, the next
+// 32 on their way in registers, and both operands are read transposed with
+// ldmatrix (rows padded to fall in distinct banks).  Bound by latency at
+// training sizes: two-byte loads straight from global memory took 41 us a
+// layer on 2^15 vertices.
+constexpr int kGwRows = 32;
+constexpr int kGwThreads = 256;   // 8 warps: 128 rows of dW
+constexpr int kGwA = K2 + 8, kGwD = H + 8;   // padded rows
+
+__device__ __forceinline__ void ldmatrix_t4(uint32_t (&r)[4], const __nv_bfloat16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+
+__global__ void __launch_bounds__(kGwThreads) grad_w_mma(uint32_t n, const __nv_bfloat16 *A0, const __nv_bfloat16 *A1,
+                                                         const __nv_bfloat16 *dzb, const float *dz, float *dW,
+                                                         float *db) {
+    __shared__ __align__(16) __nv_bfloat16 sA[kGwRows * kGwA];
+    __shared__ __align__(16) __nv_bfloat16 sD[kGwRows * kGwD];
+    __shared__ float sb[kGwThreads];
+    const uint32_t tid = threadIdx.x, lane = lane_id(), gid = lane >> 2, tig = lane & 3;
+    const uint32_t warp = tid >> 5;
     const uint32_t per = ((n + gridDim.x - 1) / gridDim.x + 15) & ~15u;
-    const uint32_t v0 = blockIdx.x * per, v1 = min(n, v0 + per);
+    const uint32_t v0 = min(n, blockIdx.x * per), v1 = min(n, v0 + per);
     const int krow = (int)warp * 16;
-    const __nv_bfloat16 *src = krow < H ? A0 : A1;
-    const int kc = krow % H;
-    const __nv_bfloat16 z = __float2bfloat16_rn(0.f);
     float acc[8][4];
 #pragma unroll
     for (int j = 0; j < 8; ++j)
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[j][q] = 0.f;
-    for (uint32_t vb = v0; vb < v1; vb += 16) {
-        auto av = [&](uint32_t v, int k) -> __nv_bfloat16 { return v < v1 ? src[(size_t)v * H + kc + k] : z; };
-        auto bv = [&](uint32_t v, int c) -> __nv_bfloat16 { return v < v1 ? dzb[(size_t)v * H + c] : z; };
-        // A fragment: row = k offset, col = vertex offset
-        uint32_t a[4];
-        a[0] = pack2(av(vb + 2 * tig, gid), av(vb + 2 * tig + 1, gid));
-        a[1] = pack2(av(vb + 2 * tig, gid + 8), av(vb + 2 * tig + 1, gid + 8));
-        a[2] = pack2(av(vb + 2 * tig + 8, gid), av(vb + 2 * tig + 9, gid));
-        a[3] = pack2(av(vb + 2 * tig + 8, gid + 8), av(vb + 2 * tig + 9, gid + 8));
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int c = j * 8 + gid;
-            uint32_t b[2];
-            b[0] = pack2(bv(vb + 2 * tig, c), bv(vb + 2 * tig + 1, c));
-            b[1] = pack2(bv(vb + 2 * tig + 8, c), bv(vb + 2 * tig + 9, c));
-            mma_bf16(acc[j], a, b);
+    // a row is 8 pieces of 16 bytes in each of A0, A1 and dz: thread t holds
+    // piece t % 8 of row t / 8 of all three (32 rows)
+    const uint32_t row = tid >> 3, piece = (tid & 7) * 8;
+    uint4 p0, p1, p2;
+    auto fetch = [&](uint32_t vb) {
+        p0 = p1 = p2 = make_uint4(0, 0, 0, 0);
+        if (vb + row < v1) {
+            const size_t at = (size_t)(vb + row) * H + piece;
+            p0 = *(const uint4 *)(A0 + at);
+            p1 = *(const uint4 *)(A1 + at);
+            p2 = *(const uint4 *)(dzb + at);
         }
+    };
+    fetch(v0);
+    for (uint32_t vb = v0; vb < v1; vb += kGwRows) {
+        *(uint4 *)(sA + row * kGwA + piece) = p0;
+        *(uint4 *)(sA + row * kGwA + H + piece) = p1;
+        *(uint4 *)(sD + row * kGwD + piece) = p2;
+        __syncthreads();
+        if (vb + kGwRows < v1) fetch(vb + kGwRows);
+        const uint32_t mtx = lane >> 3, mr = lane & 7;
+#pragma unroll
+        for (int s = 0; s < kGwRows; s += 16) {
+            // A fragment: row = channel of A, column = vertex; matrices
+            // (channels 0-7 | 8-15) x (vertices 0-7 | 8-15)
+            uint32_t a[4];
+            ldmatrix_t4(a, sA + (s + (mtx >> 1) * 8 + mr) * kGwA + krow + (mtx & 1) * 8);
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                // B fragments of column tiles j and j + 1: vertices 0-7 | 8-15
+                uint32_t b[4];
+                ldmatrix_t4(b, sD + (s + (mtx & 1) * 8 + mr) * kGwD + (j + (mtx >> 1)) * 8);
+                const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+                mma_bf16(acc[j], a, b0);
+                mma_bf16(acc[j + 1], a, b1);
+            }
+        }
+        __syncthreads();
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -290,17 +444,12 @@ __global__ void grad_w_mma(uint32_t n, const __nv_bfloat16 *A0, const __nv_bfloa
         atomicAdd(&dW[(size_t)(krow + gid + 8) * H + c], acc[j][2]);
         atomicAdd(&dW[(size_t)(krow + gid + 8) * H + c + 1], acc[j][3]);
     }
-    // bias gradient (fp32) from the same slice
-    for (int c = threadIdx.x; c < H; c += blockDim.x) {
-        float s = 0.f;
-        for (uint32_t v = v0; v < v1; ++v) s += dz[(size_t)v * H + c];
-        atomicAdd(&db[c], s);
-    }
-}
-
-__global__ void to_bf16(size_t tot, const float *in, __nv_bfloat16 *out) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot; i += (size_t)gridDim.x * blockDim.x)
-        out[i] = __float2bfloat16_rn(in[i]);
+    // bias gradient (fp32) from the same slice, four rows at a time
+    float s = 0.f;
+    for (uint32_t v = v0 + tid / H; v < v1; v += kGwThreads / H) s += dz[(size_t)v * H + tid % H];
+    sb[tid] = s;
+    __syncthreads();
+    if (tid < H) atomicAdd(&db[tid], (sb[tid] + sb[tid + H]) + (sb[tid + 2 * H] + sb[tid + 3 * H]));
 }
 
 // Wt0[c][k] = W[k][c], Wt1[c][k] = W[H + k][c]  (W is [2H x H] row-major)
@@ -312,63 +461,149 @@ __global__ void transpose_w(const float *W, float *Wt0, float *Wt1) {
     }
 }
 
-// dz = dh * [h > 0] (relu derivative from the stored activation)
-__global__ void relu_bwd(size_t tot, const float *dh, const __nv_bfloat16 *h, float *dz) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tot; i += (size_t)gridDim.x * blockDim.x)
-        dz[i] = __bfloat162float(h[i]) > 0.f ? dh[i] : 0.f;
+// dz = dh * [h > 0] (relu derivative from the stored activation), written by
+// the kernel that forms dh in FP32 and, for the GEMMs, in BF16
+__device__ __forceinline__ void store_dz(size_t at, float d0, float d1, const __nv_bfloat16 *h, float *dz,
+                                         __nv_bfloat16 *dzb) {
+    const __nv_bfloat162 t = *(const __nv_bfloat162 *)(h + at);
+    const float z0 = __bfloat162float(t.x) > 0.f ? d0 : 0.f, z1 = __bfloat162float(t.y) > 0.f ? d1 : 0.f;
+    *(float2 *)(dz + at) = make_float2(z0, z1);
+    __nv_bfloat162 o;
+    o.x = __float2bfloat16_rn(z0);
+    o.y = __float2bfloat16_rn(z1);
+    *(__nv_bfloat162 *)(dzb + at) = o;
 }
 
-// dh_L = ds * w_out; dw_out += sum ds h_L; db_out += sum ds
-__global__ void head_bwd(uint32_t n, const float *ds, const __nv_bfloat16 *h, const float *wout, float *dh,
-                         float *dwout, float *dbout) {
+// dh_L = ds * w_out -> dz_L; dw_out += sum ds h_L; db_out += sum ds
+__global__ void head_bwd(uint32_t n, const float *ds, const __nv_bfloat16 *h, const float *wout, float *dz,
+                         __nv_bfloat16 *dzb, float *dwout, float *dbout) {
     __shared__ float acc[H + 1];
     for (int i = threadIdx.x; i <= H; i += blockDim.x) acc[i] = 0.f;
     __syncthreads();
-    float a[H / 32 + 1] = {0.f, 0.f, 0.f};
+    float a0 = 0.f, a1 = 0.f, ad = 0.f;
     const uint32_t lane = lane_id();
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const float w0 = wout[2 * lane], w1 = wout[2 * lane + 1];
     for (uint32_t v = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); v < n; v += warps) {
         const float d = ds[v];
-        for (int c = lane; c < H; c += 32) {
-            dh[(size_t)v * H + c] = d * wout[c];
-            a[c / 32] += d * __bfloat162float(h[(size_t)v * H + c]);
-        }
-        if (lane == 0) a[H / 32] += d;
+        const size_t at = (size_t)v * H + 2 * lane;
+        const __nv_bfloat162 t = *(const __nv_bfloat162 *)(h + at);
+        a0 += d * __bfloat162float(t.x);
+        a1 += d * __bfloat162float(t.y);
+        if (lane == 0) ad += d;
+        store_dz(at, d * w0, d * w1, h, dz, dzb);
     }
-    for (int c = lane, q = 0; c < H; c += 32, ++q) atomicAdd(&acc[c], a[q]);
-    if (lane == 0) atomicAdd(&acc[H], a[H / 32]);
+    atomicAdd(&acc[2 * lane], a0);
+    atomicAdd(&acc[2 * lane + 1], a1);
+    if (lane == 0) atomicAdd(&acc[H], ad);
     __syncthreads();
     for (int i = threadIdx.x; i < H; i += blockDim.x) atomicAdd(&dwout[i], acc[i]);
     if (threadIdx.x == 0) atomicAdd(dbout, acc[H]);
 }
 
-// dh_prev(u) = dA[u, :64] + sum_{v: u in N(v)} dA[v, 64:] / deg(v)
-// gathered over u's in-arcs (the reverse of the out-neighbour mean)
-__global__ void scatter_mean_bwd(uint32_t n, const float *dA, const uint64_t *off_in, const uint32_t *head_in,
-                                 const uint64_t *off_out, float *dh) {
-    const uint32_t lane = lane_id();
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); u < n; u += warps) {
-        float s0 = dA[(size_t)u * K2 + 2 * lane], s1 = dA[(size_t)u * K2 + 2 * lane + 1];
-        for (uint64_t a = off_in[u]; a < off_in[u + 1]; ++a) {
-            const uint32_t v = head_in[a];
-            const float inv = 1.f / (float)(off_out[v + 1] - off_out[v]);
-            s0 += dA[(size_t)v * K2 + H + 2 * lane] * inv;
-            s1 += dA[(size_t)v * K2 + H + 2 * lane + 1] * inv;
-        }
-        dh[(size_t)u * H + 2 * lane] = s0;
-        dh[(size_t)u * H + 2 * lane + 1] = s1;
+// 1 / out-degree (0 without out-arcs)
+__global__ void inv_degree(uint32_t n, const uint64_t *off, float *inv) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const uint64_t d = off[v + 1] - off[v];
+        inv[v] = d ? 1.f / (float)d : 0.f;
     }
 }
 
-// dW0 += x^T dz0, db0 += sum dz0
-__global__ void grad_w0(uint32_t n, const float *x, const float *dz, float *dW0, float *db0) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (NF + 1) * H; i += gridDim.x * blockDim.x) {
-        const int k = i / H, c = i % H;
-        double a = 0.0;
-        for (uint32_t v = 0; v < n; ++v) a += (double)(k < NF ? x[(size_t)v * NF + k] : 1.f) * dz[(size_t)v * H + c];
-        if (k < NF) dW0[k * H + c] += (float)a;
-        else db0[c] += (float)a;
+// dh_prev(u) = dA[u, :64] + sum_{v: u in N(v)} dA[v, 64:] / deg(v), gathered
+// over u's in-arcs (the reverse of the out-neighbour mean) in arc order, and
+// dz_prev from it.  As in aggregate_mean, a hub's chain is the latency of its
+// row loads: 16 rows are in flight (1.87 ms a layer with one, on a
+// 2^15-vertex RMAT graph).
+constexpr int kBwdRows = 16;
+
+__global__ void scatter_mean_bwd(uint32_t n, const float *dA, const uint64_t *off_in, const uint32_t *head_in,
+                                 const float *inv_deg, const __nv_bfloat16 *h, float *dz, __nv_bfloat16 *dzb) {
+    const uint32_t lane = lane_id();
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); u < n; u += warps) {
+        const float2 own = *(const float2 *)(dA + (size_t)u * K2 + 2 * lane);
+        float s0 = own.x, s1 = own.y;
+        const uint64_t b = off_in[u], e = off_in[u + 1];
+        uint32_t next = b + lane < e ? head_in[b + lane] : 0u;
+        float inext = b + lane < e ? inv_deg[next] : 0.f;
+        for (uint64_t a = b; a < e; a += 32) {
+            const uint32_t cnt = e - a < 32 ? (uint32_t)(e - a) : 32u;
+            const uint32_t hd = next;
+            const float iv = inext;
+            next = a + 32 + lane < e ? head_in[a + 32 + lane] : 0u;
+            inext = a + 32 + lane < e ? inv_deg[next] : 0.f;
+            if (cnt == 32) {
+#pragma unroll
+                for (int j = 0; j < 32; j += kBwdRows) {
+                    float2 t[kBwdRows];
+#pragma unroll
+                    for (int q = 0; q < kBwdRows; ++q)
+                        t[q] = *(const float2 *)(dA + (size_t)__shfl_sync(kFull, hd, j + q) * K2 + H + 2 * lane);
+#pragma unroll
+                    for (int q = 0; q < kBwdRows; ++q) {
+                        const float w = __shfl_sync(kFull, iv, j + q);
+                        s0 += t[q].x * w;
+                        s1 += t[q].y * w;
+                    }
+                }
+            } else {
+                for (uint32_t j = 0; j < cnt; j += 4) {
+                    float2 t[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const uint32_t v = __shfl_sync(kFull, hd, j + q);
+                        if (j + q < cnt) t[q] = *(const float2 *)(dA + (size_t)v * K2 + H + 2 * lane);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float w = __shfl_sync(kFull, iv, j + q);
+                        if (j + q < cnt) {
+                            s0 += t[q].x * w;
+                            s1 += t[q].y * w;
+                        }
+                    }
+                }
+            }
+        }
+        store_dz((size_t)u * H + 2 * lane, s0, s1, h, dz, dzb);
+    }
+}
+
+// acc[k][c] += x^T dz0 (k < NF) and sum dz0 (k = NF), in double: a block's
+// warps walk its vertices (2 channels per lane), their sums meet in shared
+// memory, and the block adds them to acc.  One thread per (k, c) walking all
+// vertices took 5.5 ms for 2^15 of them.
+constexpr int kGw0Threads = 256;
+
+__global__ void __launch_bounds__(kGw0Threads) grad_w0(uint32_t n, const float *x, const float *dz, double *acc) {
+    __shared__ double sum[(NF + 1) * H];
+    for (int i = threadIdx.x; i < (NF + 1) * H; i += blockDim.x) sum[i] = 0.0;
+    __syncthreads();
+    const uint32_t lane = lane_id();
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    double a[NF + 1][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+    for (uint32_t v = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); v < n; v += warps) {
+        const float2 d = *(const float2 *)(dz + (size_t)v * H + 2 * lane);
+#pragma unroll
+        for (int k = 0; k <= NF; ++k) {
+            const double f = k < NF ? (double)x[(size_t)v * NF + k] : 1.0;
+            a[k][0] += f * d.x;
+            a[k][1] += f * d.y;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k <= NF; ++k) {
+        atomicAdd(&sum[k * H + 2 * lane], a[k][0]);
+        atomicAdd(&sum[k * H + 2 * lane + 1], a[k][1]);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < (NF + 1) * H; i += blockDim.x) atomicAdd(&acc[i], sum[i]);
+}
+
+__global__ void grad_w0_out(const double *acc, float *dW0, float *db0) {
+    for (int i = threadIdx.x; i < (NF + 1) * H; i += blockDim.x) {
+        if (i < NF * H) dW0[i] += (float)acc[i];
+        else db0[i - NF * H] += (float)acc[i];
     }
 }
 
@@ -416,11 +651,14 @@ struct chl_gnn {
     DevBuf p, g, m, v;             // params, grads, Adam moments
     uint64_t step = 0;
     // per-graph scratch (grown on demand)
-    DevBuf x, hb, mb, dz, dh, dA, s, ds, y, loss, wt;
+    DevBuf x, hb, mb, dz, dA, s, ds, y, loss, wt, inv, acc;
     uint32_t cached_n = 0;
 };
 
 namespace {
+
+// doubles of the column sums and squared deviations, or of dW0 and db0
+constexpr size_t kAccBytes = sizeof(double) * (2 * kStatBlocks * NF > (NF + 1) * H ? 2 * kStatBlocks * NF : (NF + 1) * H);
 
 size_t param_count(uint32_t layers) { return kP0 + (size_t)layers * kPL + H + 1; }
 
@@ -444,23 +682,18 @@ int upload_csr(const chl_graph *g, GraphDev &d) {
     return CHL_OK;
 }
 
-// standardise feature columns (host, deterministic order)
+// standardise the feature columns of M->x in place; M->acc holds the partials
 int standardise(chl_gnn *M, uint32_t n) {
-    std::vector<float> x((size_t)n * NF);
-    CHL_CUDA(cudaMemcpy(x.data(), M->x.p, x.size() * 4, cudaMemcpyDeviceToHost));
-    for (int k = 0; k < NF; ++k) {
-        double s = 0, s2 = 0;
-        for (uint32_t v = 0; v < n; ++v) s += x[(size_t)v * NF + k];
-        const double mean = n ? s / n : 0.0;
-        for (uint32_t v = 0; v < n; ++v) {
-            const double d = x[(size_t)v * NF + k] - mean;
-            s2 += d * d;
-        }
-        const double sd = n > 1 ? std::sqrt(s2 / n) : 0.0;
-        const double inv = sd > 1e-12 ? 1.0 / sd : 0.0;
-        for (uint32_t v = 0; v < n; ++v) x[(size_t)v * NF + k] = (float)((x[(size_t)v * NF + k] - mean) * inv);
-    }
-    CHL_CUDA(cudaMemcpy(M->x.p, x.data(), x.size() * 4, cudaMemcpyHostToDevice));
+    if (n == 0) return CHL_OK;
+    const int blocks = (int)std::min<uint32_t>(kStatBlocks, (n + kStatThreads - 1) / kStatThreads);
+    int rc = M->acc.ensure(kAccBytes);
+    if (rc) return rc;
+    double *sums = M->acc.as<double>(), *squares = sums + (size_t)kStatBlocks * NF;
+    feat_stats<<<blocks, kStatThreads>>>(n, M->x.as<float>(), nullptr, sums);
+    feat_stats<<<blocks, kStatThreads>>>(n, M->x.as<float>(), sums, squares);
+    feat_scale<<<std::min(device_sms() * 4, (int)((n + kStatThreads - 1) / kStatThreads)), kStatThreads>>>(
+        n, sums, squares, blocks, M->x.as<float>());
+    CHL_CUDA(cudaGetLastError());
     return CHL_OK;
 }
 
@@ -469,9 +702,9 @@ int ensure_scratch(chl_gnn *M, uint32_t n) {
     int rc;
     if ((rc = M->x.ensure((size_t)n * NF * 4)) || (rc = M->hb.ensure((size_t)(L + 1) * n * H * 2)) ||
         (rc = M->mb.ensure((size_t)(L + 1) * n * H * 2)) || (rc = M->dz.ensure((size_t)n * H * 4)) ||
-        (rc = M->dh.ensure((size_t)n * H * 4)) || (rc = M->dA.ensure((size_t)n * K2 * 4)) ||
+        (rc = M->inv.ensure((size_t)n * 4)) || (rc = M->dA.ensure((size_t)n * K2 * 4)) ||
         (rc = M->s.ensure((size_t)n * 4)) || (rc = M->ds.ensure((size_t)n * 4)) || (rc = M->y.ensure((size_t)n * 4)) ||
-        (rc = M->loss.ensure(8)) || (rc = M->wt.ensure((size_t)2 * H * H * 4)))
+        (rc = M->loss.ensure(8)) || (rc = M->acc.ensure(kAccBytes)) || (rc = M->wt.ensure((size_t)2 * H * H * 4)))
         return rc;
     return CHL_OK;
 }
@@ -516,29 +749,28 @@ int backward(chl_gnn *M, const GraphDev &G, double *loss) {
     float *gwout = Gp + kP0 + (size_t)L * kPL;
     head_fwd_bwd<<<sms * 8, 256>>>(n, hb + (size_t)L * n * H, wout, wout + H, M->y.as<float>(), M->s.as<float>(),
                                    M->ds.as<float>(), M->loss.as<double>());
-    head_bwd<<<sms * 4, 256>>>(n, M->ds.as<float>(), hb + (size_t)L * n * H, wout, M->dh.as<float>(), gwout,
-                               gwout + H);
+    // dz in BF16 goes to m_0's slot (unused after the forward pass)
+    float *dz = M->dz.as<float>();
+    head_bwd<<<sms * 4, 256>>>(n, M->ds.as<float>(), hb + (size_t)L * n * H, wout, dz, mb, gwout, gwout + H);
+    inv_degree<<<sms, 256>>>(n, G.off_out.as<uint64_t>(), M->inv.as<float>());
     for (uint32_t l = L; l >= 1; --l) {
         const float *W = P + kP0 + (size_t)(l - 1) * kPL;
         float *gW = Gp + kP0 + (size_t)(l - 1) * kPL;
-        const __nv_bfloat16 *hl = hb + (size_t)l * n * H;
         const __nv_bfloat16 *hp = hb + (size_t)(l - 1) * n * H;
         const __nv_bfloat16 *ml = mb + (size_t)l * n * H;
-        relu_bwd<<<sms * 8, 256>>>((size_t)n * H, M->dh.as<float>(), hl, M->dz.as<float>());
-        // dz -> BF16 in m_0's slot (unused after the forward pass)
-        to_bf16<<<sms * 8, 256>>>((size_t)n * H, M->dz.as<float>(), mb);
         const uint32_t gblocks = std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)sms * 2, (n + 255) / 256));
-        grad_w_mma<<<gblocks, 256>>>(n, hp, ml, mb, M->dz.as<float>(), gW, gW + (size_t)K2 * H);
+        grad_w_mma<<<gblocks, kGwThreads>>>(n, hp, ml, mb, dz, gW, gW + (size_t)K2 * H);
         // dA = dz W^T as two K = 64 GEMMs into the two column halves of dA
         transpose_w<<<16, 256>>>(W, M->wt.as<float>(), M->wt.as<float>() + H * H);
         gemm_rows<H><<<gemm_grid<H>(sms), 128>>>(n, mb, mb, M->wt.as<float>(), nullptr, 1, nullptr, M->dA.as<float>(), K2);
         gemm_rows<H><<<gemm_grid<H>(sms), 128>>>(n, mb, mb, M->wt.as<float>() + H * H, nullptr, 1, nullptr,
                                        M->dA.as<float>() + H, K2);
         scatter_mean_bwd<<<sms * 8, 256>>>(n, M->dA.as<float>(), G.off_in.as<uint64_t>(), G.head_in.as<uint32_t>(),
-                                           G.off_out.as<uint64_t>(), M->dh.as<float>());
+                                           M->inv.as<float>(), hp, dz, mb);
     }
-    relu_bwd<<<sms * 8, 256>>>((size_t)n * H, M->dh.as<float>(), hb, M->dz.as<float>());
-    grad_w0<<<((NF + 1) * H + 127) / 128, 128>>>(n, M->x.as<float>(), M->dz.as<float>(), Gp, Gp + NF * H);
+    CHL_CUDA(cudaMemset(M->acc.p, 0, kAccBytes));
+    grad_w0<<<std::max(1, std::min(sms, (int)((n + 63) / 64))), kGw0Threads>>>(n, M->x.as<float>(), dz, M->acc.as<double>());
+    grad_w0_out<<<1, 256>>>(M->acc.as<double>(), Gp, Gp + NF * H);
     CHL_CUDA(cudaGetLastError());
     CHL_CUDA(cudaMemcpy(loss, M->loss.p, 8, cudaMemcpyDeviceToHost));
     return CHL_OK;

@@ -226,3 +226,35 @@ def test_pretrained_network_orders_exactly(P, O):
     ref, _ = O.gll(O.OGraph.from_csr(n, off, head, ln), order)
     for a, b in zip(P.build(g, order).export(), ref.export(n)):
         assert np.array_equal(np.asarray(a), np.asarray(b))
+
+
+@pytest.mark.parametrize("n", [1, 2, 17, 33, 700])
+def test_hub_degrees_at_the_row_group_edges(P, n):
+    """Stars of 31 to 65 arcs (the aggregations take 32 rows at a time, the
+    gradient GEMM 32 vertices) on vertex counts off every tile size."""
+    src, dst = [0], [min(1, n - 1)]
+    for hub, deg in enumerate((31, 32, 33, 63, 64, 65, 96)):
+        if n > 100:
+            src += [hub] * deg
+            dst += [100 + (hub * 37 + j * 3) % (n - 100) for j in range(deg)]
+        elif hub < n:
+            src += [hub] * min(deg, n - 1)
+            dst += [(hub + 1 + j) % n for j in range(min(deg, n - 1))]
+    keep = [i for i in range(len(src)) if src[i] != dst[i]]
+    g = P.Graph.from_arcs(n, [src[i] for i in keep], [dst[i] for i in keep], [1] * len(keep), undirected=n != 33)
+    c = csr4(g)
+    net = P.RankNet(LAYERS, seed=1)
+    rng = np.random.default_rng(6)
+    p = R.init_params(LAYERS, seed=8)
+    p += rng.normal(0, 0.02, p.size).astype(np.float32)
+    net.set_params(p)
+    x = P.RankNet.features(g, seed=9)
+    assert np.allclose(x, R.features(c[0], c[1], c[2], seed=9), atol=2e-5, rtol=1e-5)
+    csr = R.csr_of(*c)
+    assert rel(net.predict(g, seed=9), R.forward(p, LAYERS, x, csr, emulate=True)[0]) < EMU_REL
+    y = rng.normal(0, 1, n).astype(np.float32)
+    loss, grad = net.grad(g, y, seed=9)
+    l_emu, g_emu = R.loss_and_grad(p, LAYERS, x, csr, y, emulate=True)
+    assert abs(loss - l_emu) <= 1e-4 * l_emu
+    for bname, sl in blocks(LAYERS):
+        assert np.linalg.norm(grad[sl] - g_emu[sl]) <= EMU_REL * max(np.linalg.norm(g_emu[sl]), 1e-6), bname
