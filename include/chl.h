@@ -167,7 +167,8 @@ enum chl_build_mode {
 typedef struct chl_build_opts {
     int32_t mode;         /* chl_build_mode                                  */
     double sf;            /* superstep label budget factor (hhl -s), 0 = auto
-                             (32 on heavy-tailed graphs, 1024 otherwise)  */
+                             (32 on heavy-tailed graphs; on road-like ones
+                             what the label buffer holds, 1024 in GLL mode) */
     double ps;            /* phase switch ratio tree/label (hhl -ps), 0 =
                              auto: 1024 (the reference's default) on road-
                              like graphs, 8 on heavy-tailed ones          */
@@ -179,7 +180,9 @@ typedef struct chl_build_opts {
     int32_t use_graphs;   /* 1: capture the per-superstep kernel chain in a
                              CUDA graph                                       */
     int32_t verbose;      /* 1: print the reference's summary line            */
-    uint32_t first_superstep; /* roots in the first superstep, 0 = auto       */
+    uint32_t first_superstep; /* roots in the first superstep, 0 = auto (road-
+                             like graphs: PLaNT trees without prune tests over
+                             all roots, up to the label buffer)             */
     double growth;        /* superstep growth factor, 0 = auto                */
     uint32_t max_warps;   /* cap on concurrent trees, 0 = auto                */
     uint32_t root_limit;  /* > 0: build the trees of ranks < root_limit only
@@ -198,11 +201,10 @@ typedef struct chl_build_opts {
                              tree's queue above 1024 vertices is split, about
                              256 kept near; heavy-tailed ones: off), 1 off,
                              q > 1: split above q (about q / 4 near)        */
-    uint32_t window_target; /* trees of a superstep with no committed labels
-                             (the first) are searched label-correcting in
+    uint32_t window_target; /* large trees are searched label-correcting in
                              distance windows of about this many vertices:
-                             0 auto (1024 on heavy-tailed graphs, off on
-                             road-like ones), 1 off (batched settle rounds) */
+                             0 auto (1024; 512 on road-like graphs below 2^18
+                             vertices), 1 off (batched settle rounds)       */
     uint32_t window_warps; /* warps building one such tree: 0 auto (8 on
                              heavy-tailed graphs, else 4), 1, 2, 4 or 8     */
     uint32_t reserved[1];

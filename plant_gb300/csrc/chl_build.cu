@@ -22,7 +22,10 @@
 //  * New labels are sorted by (vertex, side, hub) with a stable radix sort
 //    and merged into the committed CSR (double-buffered) in one pass; a
 //    second copy of every list, ordered by (distance, hub), is merged too.
-//  * The tree kernel (batch_kernel) settles vertices in batches by the IN
+//  * Large trees are searched by a block each (team_kernel), label-correcting
+//    in distance windows; on road-like graphs without prune tests and mostly
+//    in one superstep.
+//  * Small pruned trees are built by a warp each: batch_kernel settles vertices in batches by the IN
 //    criterion from a near/far queue and prunes with one 16-entry item of
 //    the distance-ordered lists per lane against a shared-memory hash of the
 //    root's label.
@@ -73,7 +76,7 @@ struct BuildCtl {
     unsigned int overflow;
     unsigned int err;               // 1: distance overflow, 2: workspace bound
     unsigned int max_dist;          // largest distance of a label emitted this superstep
-    unsigned int reserved_;
+    unsigned int ratio_stop;        // the superstep ended by TreeArgs::visit_ratio
     unsigned long long max_ratio_num;  // (tree, labels) of the worst root
     unsigned long long max_ratio_den;
     unsigned long long running;     // trees of the nominal root range in progress
@@ -106,12 +109,15 @@ struct TreeArgs {
     uint32_t *ws_key;               // per warp slot, n keys each (64-bit on weighted graphs)
     uint32_t *ws_vis;
     uint32_t *ws_front;             // per warp slot: queue, next queue, far pile
-    uint32_t *ws_win;               // window kernel: 6 n words per tree (block)
+    uint32_t *ws_win;               // team kernel: 6 n words per tree (block)
     BuildCtl *ctl;
     uint32_t hash_slots;            // root hash table slots (a power of two)
     uint32_t hash_shift;            // 32 - log2(hash_slots)
     uint32_t near_on;               // queue size that starts the near/far split (0: never)
     uint32_t near_target;           // near entries aimed at per refill
+    uint32_t visit_ratio;           // no new tree once more than this many vertices per
+                                    // label were settled (0: no limit)
+    unsigned long long visit_base;  // settled vertices the ratio lets pass at first
 };
 
 // Phase-timing clock: with CHL_PHASE_TIMING it is also a compiler memory
@@ -219,6 +225,11 @@ __device__ __forceinline__ uint32_t fetch_root(const TreeArgs &a, bool &nominal)
     // no new tree once the budget is spent, or once the label buffer is full
     // (the superstep's range is then re-run with a larger buffer)
     if (used >= a.budget || used >= a.out_cap) return kInf;
+    if (a.visit_ratio &&
+        *(volatile unsigned long long *)&a.ctl->visits > a.visit_base + used * (unsigned long long)a.visit_ratio) {
+        a.ctl->ratio_stop = 1;
+        return kInf;
+    }
     const unsigned long long t = atomicAdd(&a.ctl->next_root, 1ull);
     if (t & kClosed) return kInf;
     if (t < a.r_end) {
@@ -903,79 +914,88 @@ batch_kernel(TreeArgs a) {
     }
 }
 
-// ------------------------------------------------------ window kernel
+// ------------------------------------------------------ team kernel
 //
-// Trees of a superstep with no committed labels (the first one) cannot be
-// pruned by labels, so a vertex need not be final before it is expanded:
-// such trees are searched label-correcting in distance windows [t, thr), as
-// delta-stepping does.  Every member of the window is relaxed; a member whose
-// key drops is relaxed again in the next pass, until a pass changes no key
-// below thr.  Then every key below thr is final -- it is the minimum over all
-// paths, and every other queued key is at least thr -- so the window's labels
-// are emitted from the final keys, and the next window, [thr, lo + delta),
-// is taken from the far pile (lo its smallest live key; delta starts at the
-// spread of the root's neighbours' distances and is halved or doubled after
-// each window so that a window holds about near_target vertices).  Keys carry PLaNT's via flag
-// (distance * 2 + not-via), and a flag change is a key decrease, so relaxing
-// again on every decrease keeps the flags exact; PLaNT's early exit
-// (distributed_memory/akiba.hpp:95) is tested at window boundaries, where the
-// count of queued not-via keys is exact.  GLL trees (iteration_gll) skip
-// expanding and labelling vertices ranked above the root.
+// One tree per block of T threads, searched label-correcting in distance
+// windows [.., thr): every vertex whose key drops below thr is relaxed (again)
+// in the next pass until a pass drops none.  Then every key below thr is final
+// -- it is the minimum over all paths, and every other queued key is at least
+// thr -- so the window's labels are emitted from the final keys, and the next
+// window, [thr, lo + width), is taken from the far pile (lo its smallest live
+// key).  Keys carry PLaNT's via flag (distance * 2 + not-via), and a flag
+// change is a key decrease, so relaxing again on every decrease keeps the
+// flags exact; PLaNT's early exit (distributed_memory/akiba.hpp:95) is tested
+// at window ends, where the count of queued not-via keys is exact.
 //
-// A block of TW warps builds one tree: the warps split each pass's members
-// and the pile, and append to the tree's lists through shared counters (the
-// order of members and pile entries never matters).  Per tree, in the
-// window workspace (6 n words): key, touched vertices, members, the key each
-// member was last relaxed with, and the far pile double-buffered for the
-// block-parallel refill.
-constexpr int kWinBatch = 256;   // members relaxed per warp batch
+// Pruning with committed labels stays exact under tentative distances: a
+// vertex is tested at the distance d' it is relaxed with.  A witness h with
+// d(r, h) + d(h, v) <= d also holds at any d' >= d, so a pruned vertex is
+// never expanded, and one that is unpruned at its final d was tested with it
+// last.  A vertex ranked above every root of the superstep (rank < r0) always
+// has a committed witness, and GLL trees skip every vertex ranked above the
+// root (iteration_gll, shared_memory/akiba.hpp:92): neither is queued at all.
+//
+// Bound by the latency of a pass's chain (entry, key word, arcs, the head's
+// key, its atomic), so a pass holds only the vertices that changed, a thread
+// walks one vertex's arcs with four in flight, and one barrier ends a pass.
+// Warps whose vertices have more than kTeamLight arcs flatten theirs over the
+// lanes instead.  Windows are as wide as to hold about near_target vertices.
+// Per tree, in the workspace (6 n words): key and pass mark of each vertex in
+// one 64-bit word, the vertices that joined a window, and three lists that
+// change roles (queue, next queue, far pile).
+constexpr int kTeamLight = 8;
+constexpr int kTeamArcs = 4;      // arcs in flight per thread
+constexpr int kItem = 8;          // label entries per lane and step of a prune test
+#ifndef CHL_TEAM_WARPS
+#define CHL_TEAM_WARPS 48
+#endif
+// Register budget, as resident warps per SM.  The chains leave a scheduler
+// idle most of the time, so more warps pay even at the cost of registers:
+// trees of a 512-square grid 159 ms with 20 unpruned warps, 117 with 32, 95
+// with 48; pruned ones (1024-square grid, label budget 1024 n) 1.32 s with 20,
+// 1.27 with 28, 1.33 with 32.
+constexpr int team_warps_per_sm(bool prune) { return prune ? 28 : 48; }
 
-struct WinShared {
+struct TeamShared {
     uint32_t root, nominal;
-    uint32_t nm;        // members of the window
-    uint32_t npile;     // entries of the current pile
-    uint32_t npile2;    // entries written to the other pile by a refill
-    uint32_t nvis;      // touched vertices
-    uint32_t thr;       // window end (exclusive)
-    uint32_t delta;     // window width (0: choose at the first refill)
-    uint32_t lo;        // lower bound of the live far keys
+    uint32_t nn[3];     // next queue's length, one counter per pass in turn
+    uint32_t nm;        // vertices that joined a window
+    uint32_t npile;     // far pile entries (stale ones included)
+    uint32_t nkeep;     // entries a refill keeps
+    uint32_t lo;        // lower bound of the live far keys' distances
     uint32_t kmin, kmax;
-    uint32_t changed;
-    uint32_t psel;      // which pile buffer is current
     int ql;             // queued not-via keys (PLaNT)
     uint32_t dnv;       // largest distance of a not-via member so far (PLaNT)
     uint32_t t_size, t_lab;
+    uint32_t big;       // a tentative distance reached INT_MAX
     uint32_t err;
 };
 
-__host__ __device__ constexpr size_t window_smem_per_warp() {
-    return ((size_t)8 * kWinBatch + (size_t)4 * (4 * kWinBatch + 1) + 8 + (size_t)12 * kEmit + 15) & ~(size_t)15;
-}
-__host__ __device__ constexpr size_t window_smem(int tw) {
-    return ((sizeof(WinShared) + 15) & ~(size_t)15) + (size_t)tw * window_smem_per_warp();
+__host__ __device__ constexpr size_t team_head() { return (sizeof(TeamShared) + 15) & ~(size_t)15; }
+__host__ __device__ constexpr size_t team_smem_per_warp() { return (size_t)12 * kEmit + 32 * 4; }
+__host__ __device__ constexpr size_t team_smem(int t, uint32_t hash_slots) {
+    return team_head() + (size_t)8 * hash_slots + (size_t)(t / 32) * team_smem_per_warp();
 }
 
-template <bool UNIT, bool PLANT, int TW>
-__global__ void __launch_bounds__(TW * 32)
-window_kernel(TreeArgs a) {
+template <bool UNIT, bool PLANT, bool PRUNE, int T>
+__global__ void __launch_bounds__(T, team_warps_per_sm(PRUNE) * 32 / T) team_kernel(TreeArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    WinShared &sh = *(WinShared *)smem;
+    TeamShared &sh = *(TeamShared *)smem;
+    uint64_t *s_tab = (uint64_t *)(smem + team_head());   // root label hash table
     const uint32_t tid = threadIdx.x, lane = lane_id(), wib = tid >> 5;
-    unsigned char *base = smem + ((sizeof(WinShared) + 15) & ~(size_t)15) + wib * window_smem_per_warp();
-    uint64_t *s_ba = (uint64_t *)base;                 // arc begin of batch vertex
-    uint32_t *s_bv = (uint32_t *)(s_ba + kWinBatch);   // batch vertex
-    uint32_t *s_bk = s_bv + kWinBatch;                 // batch key
-    uint32_t *s_bx = s_bk + kWinBatch;                 // arc prefix (kWinBatch + 1)
-    uint32_t *s_tl = s_bx + kWinBatch + 1;             // batch index of each vertex with arcs
-    uint64_t *s_ek = (uint64_t *)(((uintptr_t)(s_tl + kWinBatch) + 7) & ~(uintptr_t)7);   // staged label keys
-    uint32_t *s_ev = (uint32_t *)(s_ek + kEmit);       // staged label distances
+    unsigned char *base = smem + team_head() + (size_t)8 * a.hash_slots + wib * team_smem_per_warp();
+    uint64_t *s_ek = (uint64_t *)base;           // staged label keys
+    uint32_t *s_ev = (uint32_t *)(s_ek + kEmit); // staged label distances
+    uint32_t *s_ow = s_ev + kEmit;               // lanes with arcs, compacted
 
-    uint32_t *key = a.ws_win + (size_t)blockIdx.x * 6 * a.n;
-    uint32_t *vis = key + a.n;
-    uint32_t *memb = vis + a.n;      // window members
-    uint32_t *mkey = memb + a.n;     // key a member was last relaxed with
-    uint32_t *piles = mkey + a.n;    // two far piles
-    unsigned long long c_vis = 0, c_arcs = 0;
+    // word of a vertex: key in the high half, (pass << 1 | not pruned) in the low
+    unsigned long long *kw = (unsigned long long *)(a.ws_win + (size_t)blockIdx.x * 6 * a.n);
+    uint32_t *memb = (uint32_t *)(kw + a.n);
+    uint32_t *list0 = memb + a.n;
+    const uint32_t n = a.n;
+    auto key_at = [&](uint32_t v) -> uint32_t * { return (uint32_t *)(kw + v) + 1; };
+    auto mark_at = [&](uint32_t v) -> uint32_t * { return (uint32_t *)(kw + v); };
+    unsigned long long c_arcs = 0, c_reads = 0;
 
     uint32_t n_emit = 0;
     uint32_t d_hi = 0;   // largest distance this lane has written
@@ -999,16 +1019,21 @@ window_kernel(TreeArgs a) {
         n_emit = 0;
         __syncwarp();
     };
-    // warp-wide append of the lanes with `take` to a list with a shared
-    // counter; returns this lane's index (only meaningful where take)
-    auto append_at = [&](bool take, uint32_t *counter) -> uint32_t {
+    // warp-wide append of x by the lanes with `take` to a list of at most n
+    auto append = [&](bool take, uint32_t x, uint32_t *list, uint32_t *counter) {
         const uint32_t m = __ballot_sync(kFull, take);
+        if (!m) return;
         uint32_t b = 0;
-        if (m && lane == 0) b = atomicAdd(counter, (uint32_t)__popc(m));
-        b = __shfl_sync(kFull, b, 0);
-        return b + __popc(m & lanemask_lt());
+        if (lane == 0) b = atomicAdd(counter, (uint32_t)__popc(m));
+        b = __shfl_sync(kFull, b, 0) + __popc(m & lanemask_lt());
+        if (take) {
+            if (b < n) list[b] = x;
+            else sh.err = 2;
+        }
     };
 
+    if (PRUNE)
+        for (uint32_t k = tid; k < a.hash_slots; k += T) s_tab[k] = kSlotEmpty;
     while (true) {
         if (tid == 0) {
             bool nom = false;
@@ -1020,234 +1045,327 @@ window_kernel(TreeArgs a) {
         __syncthreads();
         const uint32_t r = sh.root;
         if (r == kInf) break;
-        const uint32_t v = a.order[r];
+        const uint32_t v_root = a.order[r];
         for (int sd = 0; sd < a.sides; ++sd) {
             const int f = (a.sides == 1) ? 1 : sd;
             const uint64_t *goff = a.g_off[f];
             const uint4 *farc = a.g_farc[f];
             const uint2 *fhead = a.g_fhead[f];
+            const uint2 *lscan = a.l_dent;
+            // heads ranked above this are never queued; without prune tests
+            // PLaNT trees need them all: their paths set the via flags
+            const uint32_t rskip = PLANT ? (PRUNE ? a.r0 : 0u) : r;
+            RootHash rhash;
+            uint32_t R = 0;
+            if (PRUNE) {
+                const uint32_t ridx = lidx(v_root, f, a.sides);
+                const uint64_t rb = a.l_off[ridx], re = a.l_off[ridx + 1];
+                R = (uint32_t)(re - rb);
+                rhash.tab = s_tab;
+                rhash.mask = a.hash_slots - 1;
+                rhash.g = a.l_ent + rb;
+                rhash.R = R;
+                rhash.hlast = 0;
+                rhash.Th = min(R, a.hash_slots / 2);
+                for (uint32_t k = tid; k < rhash.Th; k += T) {
+                    const uint2 e = a.l_ent[rb + k];
+                    const uint64_t val = ((uint64_t)e.x << 32) | e.y;
+                    uint32_t sl = slot_of(e.x, a.hash_shift);
+                    while (atomicCAS((unsigned long long *)&s_tab[sl], (unsigned long long)kSlotEmpty,
+                                     (unsigned long long)val) != (unsigned long long)kSlotEmpty)
+                        sl = (sl + 1) & rhash.mask;
+                }
+                if (rhash.Th) rhash.hlast = a.l_ent[rb + rhash.Th - 1].x;
+            }
+            uint32_t *front = list0, *fnext = list0 + n, *pile = list0 + 2 * (size_t)n;
             if (tid == 0) {
-                __stcg(&key[v], 1u);
-                vis[0] = v;
-                memb[0] = v;
-                mkey[0] = kInf;
+                __stcg(&kw[v_root], (1ull << 32) | 1ull);
+                memb[0] = v_root;
+                front[0] = v_root;
+                sh.nn[0] = sh.nn[1] = sh.nn[2] = 0;
                 sh.nm = 1;
                 sh.npile = 0;
-                sh.nvis = 1;
-                sh.thr = 1;          // the first window holds the root alone
-                sh.delta = 0;
                 sh.lo = kInf;
-                sh.psel = 0;
                 sh.ql = 1;
                 sh.dnv = 0;
+                sh.big = 0;
                 sh.err = 0;
             }
             __syncthreads();
-            uint32_t pmin = kInf;    // per lane: lower bound of far keys set since the last refill
-            bool changed = false;
+            uint32_t thr = 1;         // the first window holds the root alone
+            uint32_t width = 0;       // 0: choose at the first refill
+            uint32_t pass = 1;        // stamps of this tree: 2 * pass, never the reset value
+            uint32_t nf = 1, wbegin = 0;
+            uint32_t lo = kInf;       // per lane: smallest far distance set since the last refill
+            int dql = 0;              // per lane: change of the queued not-via count
 
-            // Relax the warp's nb batch vertices (arcs flattened over the lanes).
-            auto relax = [&](uint32_t nb, uint32_t thr, uint32_t *pile) {
-                uint32_t total = 0, ncomp = 0;
-                for (uint32_t j0 = 0; j0 < nb; j0 += 32) {
-                    const uint32_t j = j0 + lane;
-                    uint32_t deg = 0;
-                    if (j < nb) {
-                        const uint32_t x = s_bv[j];
-                        const uint64_t ab = goff[x];
-                        deg = (uint32_t)(goff[x + 1] - ab);
-                        s_ba[j] = ab;
-                    }
-                    uint32_t incl = deg;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const uint32_t y = __shfl_up_sync(kFull, incl, o);
-                        if (lane >= (uint32_t)o) incl += y;
-                    }
-                    const uint32_t nem = __ballot_sync(kFull, deg > 0);
-                    if (deg > 0) {
-                        const uint32_t k = ncomp + __popc(nem & lanemask_lt());
-                        s_tl[k] = j;
-                        s_bx[k] = total + incl - deg;
-                    }
-                    total += __shfl_sync(kFull, incl, 31);
-                    ncomp += __popc(nem);
+            // one relaxed arc per lane: key decrease, and the lists its head joins
+            auto relax = [&](bool act, uint32_t k, uint32_t w, uint32_t len, uint32_t rk, uint32_t pre) {
+                const uint32_t dd = (k >> 1) + len;   // both below 2^31
+                const uint32_t nk = dd * 2u + ((!PLANT || ((k & 1u) && rk >= r)) ? 1u : 0u);
+                if (act && dd >= 0x7FFFFFFFu) {
+                    sh.big = 1;
+                    act = false;
                 }
-                if (lane == 0) s_bx[ncomp] = total;
-                __syncwarp();
-                c_arcs += total;
-                uint32_t cur = 0;
-                auto owner = [&](uint32_t t0) -> uint32_t {
-                    if (cur + 1 < ncomp && s_bx[cur + 1] <= t0) ++cur;
-                    uint32_t bit = 0;
-                    const uint32_t kk = cur + 1 + lane;
-                    if (kk < ncomp) {
-                        const uint32_t st = s_bx[kk];
-                        if (st < t0 + 32) bit = 1u << (st - t0);
-                    }
-                    const uint32_t starts = __reduce_or_sync(kFull, bit);
-                    const uint32_t upto = lane == 31 ? kFull : ((2u << lane) - 1u);
-                    const uint32_t own = cur + (uint32_t)__popc(starts & upto);
-                    cur += (uint32_t)__popc(starts);
-                    return own;
-                };
-                int dql = 0;
-                // WC 32-arc chunks per step: their arc loads and atomics are
-                // issued together
-                constexpr int WC = CHL_RELAX_CHUNKS;
-                for (uint32_t t0 = 0; t0 < total; t0 += 32 * WC) {
-                    uint32_t w[WC], nk[WC], old[WC], kxs[WC], len[WC], rk[WC];
-                    bool act[WC], upd[WC];
-#pragma unroll
-                    for (int c = 0; c < WC; ++c) {
-                        w[c] = 0;
-                        nk[c] = 0;
-                        old[c] = kInf;
-                        kxs[c] = 0;
-                        len[c] = 0;
-                        rk[c] = 0;
-                        act[c] = false;
-                        upd[c] = false;
-                    }
-#pragma unroll
-                    for (int c = 0; c < WC; ++c) {
-                        const uint32_t tc = t0 + 32u * c;
-                        const uint32_t own = tc < total ? owner(tc) : 0u;
-                        const uint32_t t = tc + lane;
-                        if (t < total) {
-                            const uint32_t lo = s_tl[own];
-                            const uint64_t e = s_ba[lo] + (t - s_bx[own]);
-                            if (UNIT) {
-                                const uint2 hr = fhead[e];
-                                w[c] = hr.x;
-                                rk[c] = hr.y;
-                                len[c] = 1;
-                            } else {
-                                const uint4 hl = farc[e];
-                                w[c] = hl.x;
-                                len[c] = hl.y;
-                                rk[c] = hl.z;
-                            }
-                            kxs[c] = s_bk[lo];
-                            act[c] = true;
-                        }
-                    }
-                    uint32_t pre[WC];   // the key before the atomic (keys only decrease)
-#pragma unroll
-                    for (int c = 0; c < WC; ++c) pre[c] = (CHL_RELAX_PRECHECK && act[c]) ? __ldcg(&key[w[c]]) : kInf;
-#pragma unroll
-                    for (int c = 0; c < WC; ++c) {
-                        if (!act[c]) continue;
-                        const uint32_t nv = (!PLANT || ((kxs[c] & 1u) && rk[c] >= r)) ? 1u : 0u;
-                        const uint64_t dd64 = (uint64_t)(kxs[c] >> 1) + len[c];
-                        if (dd64 < 0x7FFFFFFFull) {
-                            nk[c] = (uint32_t)dd64 * 2u + nv;
-                            old[c] = pre[c] <= nk[c] ? pre[c] : atomicMin(&key[w[c]], nk[c]);
-                            upd[c] = nk[c] < old[c];
-                        } else {
-                            a.ctl->err = 1;   // the reference asserts dd < infty
-                        }
-                    }
-#pragma unroll
-                    for (int c = 0; c < WC; ++c) {
-                        const uint32_t dk = nk[c] >> 1;
-                        const bool fresh = upd[c] && old[c] == kInf;
-                        const bool in_win = upd[c] && dk < thr;
-                        changed |= in_win;
-                        // a new member: first touched inside the window, or a far
-                        // vertex whose key drops into it (its far entry goes stale)
-                        const bool join = in_win && (old[c] == kInf || (old[c] >> 1) >= thr);
-                        const uint32_t jo = append_at(join, &sh.nm);
-                        if (join) {
-                            if (jo < a.n) {
-                                memb[jo] = w[c];
-                                mkey[jo] = kInf;
-                            } else {
-                                sh.err = 2;
-                            }
-                        }
-                        const uint32_t vo = append_at(fresh, &sh.nvis);
-                        if (fresh) {
-                            if (vo < a.n) vis[vo] = w[c];
-                            else sh.err = 2;
-                        }
-                        if (upd[c] && dk >= thr) pmin = min(pmin, dk);
-                        const bool to_far = fresh && dk >= thr;
-                        const uint32_t po = append_at(to_far, &sh.npile);
-                        if (to_far) {
-                            if (po < a.n) pile[po] = w[c];
-                            else sh.err = 2;
-                        }
-                        if (PLANT && upd[c]) dql += (int)(nk[c] & 1u) - (old[c] == kInf ? 0 : (int)(old[c] & 1u));
+                // keys only decrease: a read no larger than nk proves the atomic idle
+                act = act && rk >= rskip && nk < pre;
+                uint32_t old = 0;
+                if (act) {
+                    old = atomicMin(key_at(w), nk);
+                    act = nk < old;
+                }
+                if (!__any_sync(kFull, act)) return;
+                bool join = false, next = false, far = false;
+                if (act) {
+                    if (PLANT) dql += (int)(nk & 1u) - (old == kInf ? 0 : (int)(old & 1u));
+                    if (dd < thr) {
+                        // a far vertex whose key drops into the window leaves a stale far entry
+                        join = old == kInf || (old >> 1) >= thr;
+                        const uint32_t stamp = pass << 1 | 1u;
+                        next = (atomicExch(mark_at(w), stamp) | 1u) != stamp;
+                    } else {
+                        lo = min(lo, dd);
+                        far = old == kInf;
                     }
                 }
-                if (PLANT) {
-                    dql = __reduce_add_sync(kFull, dql);
-                    if (lane == 0 && dql) atomicAdd(&sh.ql, dql);
-                }
-                __syncwarp();
+                append(next, w, fnext, &sh.nn[pass % 3]);
+                append(join, w, memb, &sh.nm);
+                append(far, w, pile, &sh.npile);
             };
 
             while (true) {
-                // passes over the window's members until no key below thr drops
-                while (true) {
-                    const uint32_t thr = sh.thr;
-                    uint32_t *pile = piles + (size_t)sh.psel * a.n;
-                    const uint32_t pass_n = sh.nm;
-                    changed = false;
-                    uint32_t nb = 0;
-                    for (uint32_t b0 = wib * 32; b0 < pass_n; b0 += 32 * TW) {
-                        const uint32_t i = b0 + lane;
-                        bool need = false;
-                        uint32_t x = 0, k = 0;
-                        if (i < pass_n) {
-                            x = memb[i];
-                            k = __ldcg(&key[x]);
-                            if (k != mkey[i]) {
-                                mkey[i] = k;
-                                // GLL trees do not expand vertices ranked above the root
-                                need = PLANT || __ldg(&a.rank[x]) >= r;
+                // passes over the window until no key below thr drops
+                while (nf) {
+                    if (tid == 0) sh.nn[(pass + 1) % 3] = 0;   // last read two barriers ago
+                    for (uint32_t i0 = wib * 32; i0 < nf; i0 += T) {
+                        const bool valid = i0 + lane < nf;
+                        uint32_t v = 0, k = 0, deg = 0;
+                        uint64_t ab = 0;
+                        unsigned long long word = 0;
+                        bool test = false;
+                        uint64_t lb = 0;
+                        uint32_t ln = 0;
+                        if (valid) {
+                            v = __ldcg(&front[i0 + lane]);
+                            word = __ldcg(&kw[v]);
+                            ab = goff[v];
+                            deg = (uint32_t)(goff[v + 1] - ab);
+                            k = (uint32_t)(word >> 32);
+                            if (PRUNE && R > 0) {
+                                const uint32_t xu = lidx(v, 1 - f, a.sides);
+                                lb = a.l_off[xu];
+                                ln = (uint32_t)(a.l_off[xu + 1] - lb);
+                                test = ln > 0;
                             }
                         }
-                        const uint32_t bm = __ballot_sync(kFull, need);
-                        if (need) {
-                            const uint32_t at = nb + __popc(bm & lanemask_lt());
-                            s_bv[at] = x;
-                            s_bk[at] = k;
+                        if (PRUNE && R > 0) {
+                            // Prune tests: every lane owns a vertex; the lanes take
+                            // (vertex, kItem-entry chunk) items of the vertices still
+                            // under test, several consecutive chunks of each once
+                            // fewer than 32 are left.  Lists are in distance order,
+                            // so one is done at its first entry beyond d(r, u).
+                            bool hit = false;
+                            uint32_t ch = 0;                                  // next chunk of the own vertex
+                            const uint32_t nch = (uint32_t)(((lb & 1ull) + ln + kItem - 1) / kItem);
+                            uint32_t live = __ballot_sync(kFull, test);
+                            while (live) {
+                                const uint32_t t = (uint32_t)__popc(live);
+                                // lane -> (owner, chunk offset)
+                                const uint32_t vi = lane % t, co = lane / t;
+                                if (live >> lane & 1u) s_ow[__popc(live & lanemask_lt())] = lane;
+                                __syncwarp();
+                                const uint32_t ow = s_ow[vi];
+                                const uint64_t glb = __shfl_sync(kFull, lb, ow);
+                                const uint32_t gln = __shfl_sync(kFull, ln, ow);
+                                const uint32_t gd = __shfl_sync(kFull, k, ow) >> 1;
+                                const uint32_t c = __shfl_sync(kFull, ch, ow) + co;
+                                const uint32_t gnc = __shfl_sync(kFull, nch, ow);
+                                bool h = false, done = false;
+                                if (c < gnc) {
+                                    const uint64_t e0 = (glb & ~1ull) + (uint64_t)kItem * c;
+                                    const uint32_t first = e0 < glb ? 1u : 0u;   // odd start: entry 0 is the list before
+                                    const uint64_t span = glb + gln - e0;
+                                    const uint32_t last = span < kItem ? (uint32_t)span : (uint32_t)kItem;
+                                    uint4 q[kItem / 2];
+#pragma unroll
+                                    for (int u = 0; u < kItem / 2; ++u) {
+                                        q[u] = make_uint4(0, 0xFFFFFFFFu, 0, 0xFFFFFFFFu);
+                                        if (2u * u < last) q[u] = *(const uint4 *)(lscan + e0 + 2 * u);
+                                    }
+                                    c_reads += kItem;
+                                    uint64_t w[kItem];
+                                    uint32_t sl[kItem];
+                                    uint32_t pend = 0;
+#pragma unroll
+                                    for (int u = 0; u < kItem; ++u) {
+                                        const uint32_t hh = (u & 1) ? q[u >> 1].z : q[u >> 1].x;
+                                        const uint32_t dd = (u & 1) ? q[u >> 1].w : q[u >> 1].y;
+                                        const bool in = (uint32_t)u >= first && (uint32_t)u < last;
+                                        w[u] = kSlotEmpty;
+                                        sl[u] = 0;
+                                        if (in && dd > gd) done = true;
+                                        if (in && dd <= gd) {
+                                            if (hh <= rhash.hlast) {
+                                                sl[u] = slot_of(hh, a.hash_shift);
+                                                w[u] = s_tab[sl[u]];
+                                                pend |= 1u << u;
+                                            } else if (rhash.Th < R) {
+                                                // hubs past the hashed prefix
+                                                uint32_t dr;
+                                                if (rhash.find_tail(hh, dr) && dr + dd <= gd) h = true;
+                                            }
+                                        }
+                                    }
+#pragma unroll
+                                    for (int u = 0; u < kItem; ++u) {
+                                        if (!(pend >> u & 1u)) continue;
+                                        const uint32_t hh = (u & 1) ? q[u >> 1].z : q[u >> 1].x;
+                                        const uint32_t dd = (u & 1) ? q[u >> 1].w : q[u >> 1].y;
+                                        uint64_t x = w[u];
+                                        uint32_t z = sl[u];
+                                        while (x != kSlotEmpty && (uint32_t)(x >> 32) != hh) {
+                                            z = (z + 1) & rhash.mask;
+                                            x = s_tab[z];
+                                        }
+                                        if (x != kSlotEmpty && (uint32_t)x + dd <= gd) h = true;
+                                    }
+                                }
+                                const uint32_t hm = __ballot_sync(kFull, h), dm = __ballot_sync(kFull, h || done);
+                                if (live >> lane & 1u) {
+                                    // this owner's items are lanes vi0, vi0 + t, ...
+                                    uint32_t pat = 0;
+                                    for (uint32_t x = __popc(live & lanemask_lt()); x < 32; x += t) pat |= 1u << x;
+                                    hit = (hm & pat) != 0;
+                                    ch += __popc(pat);
+                                    test = !(dm & pat) && ch < nch;
+                                }
+                                live = __ballot_sync(kFull, test);
+                            }
+                            if (valid) {
+                                if (hit) {
+                                    atomicAnd(mark_at(v), ~1u);
+                                    deg = 0;
+                                } else if (!((uint32_t)word & 1u)) {
+                                    atomicOr(mark_at(v), 1u);   // was pruned at a larger distance
+                                }
+                            }
                         }
-                        nb += __popc(bm);
-                        __syncwarp();
-                        if (nb > (uint32_t)kWinBatch - 32) {
-                            relax(nb, thr, pile);
-                            nb = 0;
+                        c_arcs += deg;
+                        const uint32_t most = __reduce_max_sync(kFull, deg);
+                        if (most <= (uint32_t)kTeamLight) {
+                            for (uint32_t h = 0; h < most; h += kTeamArcs) {
+                                uint32_t w[kTeamArcs], len[kTeamArcs], rk[kTeamArcs], pre[kTeamArcs];
+#pragma unroll
+                                for (int q = 0; q < kTeamArcs; ++q) {
+                                    w[q] = v;
+                                    len[q] = 1;
+                                    rk[q] = 0;
+                                    if (h + q < deg) {
+                                        if (UNIT) {
+                                            const uint2 x = fhead[ab + h + q];
+                                            w[q] = x.x;
+                                            rk[q] = x.y;
+                                        } else {
+                                            const uint4 x = farc[ab + h + q];
+                                            w[q] = x.x;
+                                            len[q] = x.y;
+                                            rk[q] = x.z;
+                                        }
+                                    }
+                                }
+#pragma unroll
+                                for (int q = 0; q < kTeamArcs; ++q)
+                                    pre[q] = h + q < deg && rk[q] >= rskip ? __ldcg(key_at(w[q])) : 0u;
+#pragma unroll
+                                for (int q = 0; q < kTeamArcs; ++q)
+                                    relax(h + q < deg, k, w[q], len[q], rk[q], pre[q]);
+                            }
+                        } else {
+                            // arcs flattened over the lanes; owner of arc t0 + lane from
+                            // the list starts inside the 32-arc group (one OR-reduction)
+                            uint32_t incl = deg;
+#pragma unroll
+                            for (int o = 1; o < 32; o <<= 1) {
+                                const uint32_t y = __shfl_up_sync(kFull, incl, o);
+                                if (lane >= (uint32_t)o) incl += y;
+                            }
+                            const uint32_t start = incl - deg, total = __shfl_sync(kFull, incl, 31);
+                            const uint32_t nem = __ballot_sync(kFull, deg > 0);
+                            if (deg > 0) s_ow[__popc(nem & lanemask_lt())] = lane;
+                            __syncwarp();
+                            uint32_t before = 0;   // lists that start before the group
+                            constexpr int RC = CHL_RELAX_CHUNKS;
+                            for (uint32_t t0 = 0; t0 < total; t0 += 32 * RC) {
+                                uint32_t w[RC], len[RC], rk[RC], pre[RC], kk[RC];
+#pragma unroll
+                                for (int c = 0; c < RC; ++c) {
+                                    const uint32_t tc = t0 + 32u * c;
+                                    const uint32_t bit = deg > 0 && start >= tc && start < tc + 32 ? 1u << (start - tc) : 0u;
+                                    const uint32_t starts = __reduce_or_sync(kFull, bit);
+                                    const uint32_t upto = lane == 31 ? kFull : ((2u << lane) - 1u);
+                                    const uint32_t own = before + (uint32_t)__popc(starts & upto);
+                                    before += (uint32_t)__popc(starts);
+                                    const uint32_t ol = s_ow[own ? own - 1 : 0];
+                                    const uint64_t oab = __shfl_sync(kFull, ab, ol);
+                                    const uint32_t ost = __shfl_sync(kFull, start, ol);
+                                    kk[c] = __shfl_sync(kFull, k, ol);
+                                    w[c] = v;
+                                    len[c] = 1;
+                                    rk[c] = 0;
+                                    if (tc + lane < total) {
+                                        const uint64_t e = oab + (tc + lane - ost);
+                                        if (UNIT) {
+                                            const uint2 x = fhead[e];
+                                            w[c] = x.x;
+                                            rk[c] = x.y;
+                                        } else {
+                                            const uint4 x = farc[e];
+                                            w[c] = x.x;
+                                            len[c] = x.y;
+                                            rk[c] = x.z;
+                                        }
+                                    }
+                                }
+#pragma unroll
+                                for (int c = 0; c < RC; ++c)
+                                    pre[c] = t0 + 32u * c + lane < total && rk[c] >= rskip ? __ldcg(key_at(w[c])) : 0u;
+#pragma unroll
+                                for (int c = 0; c < RC; ++c)
+                                    relax(t0 + 32u * c + lane < total, kk[c], w[c], len[c], rk[c], pre[c]);
+                            }
+                            __syncwarp();
                         }
                     }
-                    if (nb) relax(nb, thr, pile);
-                    __syncthreads();   // (a) every member counter and key update is done
-                    if (tid == 0) sh.changed = 0;
                     __syncthreads();
-                    if (__any_sync(kFull, changed) && lane == 0) sh.changed = 1;
-                    __syncthreads();
-                    if (!sh.changed) break;
+                    nf = min(sh.nn[pass % 3], n);
+                    ++pass;
+                    uint32_t *t = front;
+                    front = fnext;
+                    fnext = t;
                 }
                 // the window is final: its labels, from the final keys
-                const uint32_t nm = sh.nm;
+                const uint32_t nm = min(sh.nm, n);
+                const bool big = sh.big != 0;
                 int nv_final = 0;
                 uint32_t lab = 0, dnv = 0;
-                for (uint32_t b0 = wib * 32; b0 < nm; b0 += 32 * TW) {
+                for (uint32_t b0 = wbegin + wib * 32; b0 < nm; b0 += T) {
                     const uint32_t i = b0 + lane;
                     bool emit = false;
                     uint32_t x = 0, k = 0;
                     if (i < nm) {
-                        x = memb[i];
-                        k = __ldcg(&key[x]);
+                        x = __ldcg(&memb[i]);
+                        const unsigned long long word = __ldcg(&kw[x]);
+                        k = (uint32_t)(word >> 32);
+                        const bool unpruned = !PRUNE || R == 0 || ((uint32_t)word & 1u);
                         if (PLANT) {
                             nv_final += (int)(k & 1u);
-                            emit = (k & 1u) != 0;
-                            if (emit) dnv = max(dnv, k >> 1);
-                        } else {
-                            emit = __ldg(&a.rank[x]) >= r;   // iteration_gll :92
+                            if (k & 1u) dnv = max(dnv, k >> 1);
                         }
+                        emit = unpruned && (!PLANT || (k & 1u));
+                        if (big && unpruned)
+                            for (uint64_t e = goff[x]; e < goff[x + 1]; ++e)
+                                if ((uint64_t)(k >> 1) + (UNIT ? 1u : farc[e].y) >= 0x7FFFFFFFull)
+                                    a.ctl->err = 1;   // the reference asserts dd < infty
                     }
                     const uint32_t em = __ballot_sync(kFull, emit);
                     if (em) {
@@ -1262,42 +1380,40 @@ window_kernel(TreeArgs a) {
                     }
                 }
                 if (PLANT) {
-                    nv_final = __reduce_add_sync(kFull, nv_final);
+                    nv_final = __reduce_add_sync(kFull, nv_final - dql);
                     dnv = __reduce_max_sync(kFull, dnv);
+                    dql = 0;
                 }
-                const uint32_t pmin_w = __reduce_min_sync(kFull, pmin);
-                pmin = kInf;
+                lo = __reduce_min_sync(kFull, lo);
                 if (lane == 0) {
-                    if (PLANT && nv_final) atomicAdd(&sh.ql, -nv_final);
+                    if (PLANT && nv_final) atomicSub(&sh.ql, nv_final);
                     if (PLANT && dnv) atomicMax(&sh.dnv, dnv);
                     if (lab) atomicAdd(&sh.t_lab, lab);
-                    if (pmin_w != kInf) atomicMin(&sh.lo, pmin_w);
+                    if (lo != kInf) atomicMin(&sh.lo, lo);
                 }
-                __syncthreads();   // (b) ql, lo final for this window
+                lo = kInf;
+                __syncthreads();
                 if (PLANT && sh.ql == 0) break;   // plant :95 early exit (all queued keys are via)
-                __syncthreads();   // every thread has read ql
+                uint32_t np = min(sh.npile, n), low = sh.lo;
+                if (np == 0 || sh.err) {
+                    if (tid == 0) sh.t_size += nm - wbegin;
+                    wbegin = nm;
+                    break;
+                }
+                __syncthreads();   // the window's state is read
                 if (tid == 0) {
-                    sh.t_size += nm;
-                    sh.nm = 0;
+                    sh.t_size += nm - wbegin;
                     sh.kmin = kInf;
                     sh.kmax = 0;
-                    // the width follows the size of the window just finished
-                    if (sh.delta) {
-                        if (nm > 2 * a.near_target) sh.delta = max(sh.delta / 2, 1u);
-                        else if (nm < a.near_target / 2) sh.delta = sh.delta < 0x40000000u ? 2u * sh.delta : 0x7FFFFFFFu;
-                    }
                 }
-                __syncthreads();
-                if (sh.delta == 0) {
-                    // first refill: the spread of the root's neighbours'
-                    // distances (then adapted window by window)
-                    const uint32_t np = sh.npile;
-                    const uint32_t *pile = piles + (size_t)sh.psel * a.n;
+                if (width == 0) {
+                    // the first width: the spread of the root's neighbours' distances
+                    __syncthreads();
                     uint32_t mn = kInf, mx = 0;
-                    for (uint32_t i = tid; i < np; i += 32 * TW) {
-                        const uint32_t k = __ldcg(&key[pile[i]]) >> 1;
-                        mn = min(mn, k);
-                        mx = max(mx, k);
+                    for (uint32_t i = tid; i < np; i += T) {
+                        const uint32_t d = __ldcg(key_at(__ldcg(&pile[i]))) >> 1;
+                        mn = min(mn, d);
+                        mx = max(mx, d);
                     }
                     mn = __reduce_min_sync(kFull, mn);
                     mx = __reduce_max_sync(kFull, mx);
@@ -1306,85 +1422,81 @@ window_kernel(TreeArgs a) {
                         atomicMax(&sh.kmax, mx);
                     }
                     __syncthreads();
-                    if (tid == 0 && np > 0) {
-                        sh.lo = sh.kmin;
-                        sh.delta = max(sh.kmax - min(sh.kmin, sh.kmax), 1u);
-                    }
-                    __syncthreads();
+                    low = sh.kmin;
+                    width = max(sh.kmax - min(sh.kmin, sh.kmax), 1u);
+                } else if (nm - wbegin > 2 * a.near_target) {
+                    width = max(width / 2, 1u);
+                } else if (nm - wbegin < a.near_target / 2) {
+                    width = width < 0x40000000u ? 2 * width : 0x7FFFFFFFu;
                 }
-                // next window from the far pile: entries below the old
-                // threshold are stale (they joined a window), entries below
-                // the new one join, the rest move to the other pile buffer
-                for (int pass = 0; pass < 4; ++pass) {
-                    if (sh.nm != 0 || sh.npile == 0) break;
-                    const uint32_t t_old = sh.thr;
-                    const uint32_t thr = sat_add(sh.lo, sh.delta);
-                    const uint32_t np = sh.npile;
-                    const uint32_t *src = piles + (size_t)sh.psel * a.n;
-                    uint32_t *dst = piles + (size_t)(sh.psel ^ 1u) * a.n;
-                    __syncthreads();   // (d) every thread has read the window state
+                wbegin = nm;
+                // next window from the far pile: entries below the old thr are
+                // stale (they joined a window), entries below the new one join,
+                // the rest stay.  low is exact from the second sweep on.
+                while (nf == 0 && np > 0) {
+                    const uint32_t t_old = thr;
+                    thr = sat_add(low, width);
+                    __syncthreads();
                     if (tid == 0) {
-                        sh.npile2 = 0;
-                        sh.kmin = kInf;
+                        sh.nn[0] = 0;
+                        sh.nkeep = 0;
+                        sh.lo = kInf;
                     }
                     __syncthreads();
-                    uint32_t kmin = kInf;
-                    for (uint32_t b0 = wib * 32; b0 < np; b0 += 32 * TW) {
-                        const uint32_t i = b0 + lane;
-                        const bool valid = i < np;
-                        const uint32_t x = valid ? src[i] : 0u;
-                        const uint32_t k = valid ? (__ldcg(&key[x]) >> 1) : kInf;
-                        const bool live = valid && k >= t_old;
-                        const bool nr = live && k < thr;
-                        const bool kp = live && !nr;
-                        const uint32_t mo = append_at(nr, &sh.nm);
-                        if (nr) {
-                            memb[mo] = x;
-                            mkey[mo] = kInf;
-                        }
-                        const uint32_t ko = append_at(kp, &sh.npile2);
-                        if (kp) {
-                            dst[ko] = x;
-                            kmin = min(kmin, k);
-                        }
+                    for (uint32_t i0 = wib * 32; i0 < np; i0 += T) {
+                        const uint32_t i = i0 + lane;
+                        const uint32_t x = i < np ? __ldcg(&pile[i]) : 0u;
+                        const uint32_t d = i < np ? __ldcg(key_at(x)) >> 1 : 0u;
+                        const bool live = i < np && d >= t_old;
+                        append(live && d < thr, x, front, &sh.nn[0]);
+                        append(live && d >= thr, x, fnext, &sh.nkeep);
+                        if (live && d >= thr) lo = min(lo, d);
                     }
-                    kmin = __reduce_min_sync(kFull, kmin);
-                    if (lane == 0 && kmin != kInf) atomicMin(&sh.kmin, kmin);
-                    __syncthreads();   // (e) the refill pass is complete
-                    if (tid == 0) {
-                        sh.thr = thr;
-                        sh.psel ^= 1u;
-                        sh.npile = sh.npile2;
-                        sh.lo = sh.kmin;
-                    }
+                    lo = __reduce_min_sync(kFull, lo);
+                    if (lane == 0 && lo != kInf) atomicMin(&sh.lo, lo);
+                    lo = kInf;
                     __syncthreads();
+                    nf = sh.nn[0];
+                    np = sh.nkeep;
+                    low = sh.lo;
+                    uint32_t *t = pile;   // the kept entries are the pile now
+                    pile = fnext;
+                    fnext = t;
                 }
-                if (sh.nm == 0) {
-                    if (sh.npile > 0 && tid == 0) a.ctl->err = 2;   // not reached: lo is exact from the second pass on
-                    break;
+                for (uint32_t i = tid; i < nf; i += T) memb[nm + i] = front[i];
+                __syncthreads();
+                if (tid == 0) {
+                    sh.nm = nm + nf;
+                    sh.npile = np;
+                    sh.nn[0] = sh.nn[1] = sh.nn[2] = 0;
                 }
+                __syncthreads();
+                if (nf == 0) break;   // only stale entries were left
             }
             __syncthreads();
             if (sh.err && tid == 0) a.ctl->err = 2;
-            if (PLANT && sh.nm) {
+            const uint32_t nm = min(sh.nm, n), np = min(sh.npile, n);
+            if (PLANT && wbegin < nm) {
                 // the early exit ended the tree inside this window: count its
                 // members no farther than the last not-via vertex, the ones
                 // the reference's Dijkstra pops before it stops
                 // (distributed_memory/akiba.hpp:69-95)
-                const uint32_t nm = min(sh.nm, a.n), dl = sh.dnv;
+                const uint32_t dl = sh.dnv;
                 uint32_t c = 0;
-                for (uint32_t i = tid; i < nm; i += 32 * TW) c += (__ldcg(&key[memb[i]]) >> 1) <= dl ? 1u : 0u;
+                for (uint32_t i = wbegin + tid; i < nm; i += T) c += (__ldcg(key_at(__ldcg(&memb[i]))) >> 1) <= dl ? 1u : 0u;
                 c = __reduce_add_sync(kFull, c);
                 if (lane == 0 && c) atomicAdd(&sh.t_size, c);
+                __syncthreads();
             }
-            __syncthreads();
-            const uint32_t nvis = min(sh.nvis, a.n);
-            for (uint32_t k = tid; k < nvis; k += 32 * TW) __stcg(&key[vis[k]], kInf);
+            for (uint32_t i = tid; i < nm; i += T) __stcg(&kw[__ldcg(&memb[i])], ~0ull);
+            for (uint32_t i = tid; i < np; i += T) __stcg(&kw[__ldcg(&pile[i])], ~0ull);
+            if (PRUNE)
+                for (uint32_t k = tid; k < a.hash_slots; k += T) s_tab[k] = kSlotEmpty;
             __syncthreads();
         }
         flush_labels();
         if (tid == 0) {
-            c_vis += sh.t_size;
+            atomicAdd(&a.ctl->visits, (unsigned long long)sh.t_size);   // fetch_root reads it
             a.tree_size[r - a.r0] = sh.t_size;
             a.tree_labels[r - a.r0] = sh.t_lab;
             finish_root(a, sh.nominal != 0);
@@ -1392,28 +1504,38 @@ window_kernel(TreeArgs a) {
         __syncthreads();
     }
     d_hi = __reduce_max_sync(kFull, d_hi);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        c_arcs += __shfl_xor_sync(kFull, c_arcs, o);
+        c_reads += __shfl_xor_sync(kFull, c_reads, o);
+    }
     if (lane == 0) {
-        atomicAdd(&a.ctl->visits, c_vis);
         atomicAdd(&a.ctl->arcs, c_arcs);
+        atomicAdd(&a.ctl->label_reads, c_reads);
         if (d_hi) atomicMax(&a.ctl->max_dist, d_hi);
     }
 }
 
 using TreeKernel = void (*)(TreeArgs);
 
-template <bool UNIT, bool PLANT>
-TreeKernel window_kernel_tw(uint32_t tw) {
+template <bool UNIT, bool PLANT, bool PRUNE>
+TreeKernel team_kernel_tw(uint32_t tw) {
     switch (tw) {
-    case 1: return window_kernel<UNIT, PLANT, 1>;
-    case 2: return window_kernel<UNIT, PLANT, 2>;
-    case 8: return window_kernel<UNIT, PLANT, 8>;
-    default: return window_kernel<UNIT, PLANT, 4>;
+    case 1: return team_kernel<UNIT, PLANT, PRUNE, 32>;
+    case 2: return team_kernel<UNIT, PLANT, PRUNE, 64>;
+    case 8: return team_kernel<UNIT, PLANT, PRUNE, 256>;
+    default: return team_kernel<UNIT, PLANT, PRUNE, 128>;
     }
 }
 
-TreeKernel window_kernel_for(bool unit, bool plant, uint32_t tw) {
-    if (unit) return plant ? window_kernel_tw<true, true>(tw) : window_kernel_tw<true, false>(tw);
-    return plant ? window_kernel_tw<false, true>(tw) : window_kernel_tw<false, false>(tw);
+template <bool UNIT, bool PLANT>
+TreeKernel team_kernel_pr(bool prune, uint32_t tw) {
+    return prune ? team_kernel_tw<UNIT, PLANT, true>(tw) : team_kernel_tw<UNIT, PLANT, false>(tw);
+}
+
+TreeKernel team_kernel_for(bool unit, bool plant, bool prune, uint32_t tw) {
+    if (unit) return plant ? team_kernel_pr<true, true>(prune, tw) : team_kernel_pr<true, false>(prune, tw);
+    return plant ? team_kernel_pr<false, true>(prune, tw) : team_kernel_pr<false, false>(prune, tw);
 }
 
 __global__ void fat_arcs(uint64_t m, const uint2 *arc, const uint32_t *rank, const uint32_t *win, uint4 *out) {
@@ -1769,8 +1891,8 @@ struct Build {
     uint32_t *tsize = nullptr, *tlab = nullptr;
     uint32_t *ws_all = nullptr;   // tree workspace (both kernels' layouts)
     uint32_t *ws_key = nullptr, *ws_vis = nullptr, *ws_front = nullptr;   // batch_kernel views
-    uint32_t win_trees = 0, win_tw = 4;   // window_kernel: trees (blocks) and warps per tree
-    int ws_layout = 0;   // 1: batch_kernel keys all INF, 2: window_kernel keys all INF
+    uint32_t win_trees = 0, win_tw = 4;   // team_kernel: trees (blocks) and warps per tree
+    int ws_layout = 0;   // 1: batch_kernel keys all INF, 2: team_kernel keys all INF
     BuildCtl *ctl = nullptr;
     void *tmp = nullptr;
     size_t tmp_bytes = 0;
@@ -1941,6 +2063,25 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         const double avgdeg = n ? (double)g->off[1][n] / n : 0.0;
         heavy_tail = maxdeg > 32.0 * std::max(1.0, avgdeg);
     }
+    // vertices per distance window of the team kernel (1: settle rounds by the
+    // IN criterion instead).  Grids: 512 and 1,024 within 3% of each other,
+    // smaller graphs better with 512 (the 100-square grid 1.8 against 1.9 ms),
+    // the 1024-square one with 1,024 (1.51 against 1.56 s)
+    const uint32_t win_target = opts.window_target ? opts.window_target : (heavy_tail || n >= (1u << 18) ? 1024u : 512u);
+    // Road-like graphs build whole: PLaNT trees without prune tests are exact
+    // by their via flags alone, and cost 0.14 ns a settled vertex where a
+    // pruned one costs 1 to 2 (its list and the root's).  They settle 3.5 to
+    // 8 vertices per label on grids, pruned ones 1.3 to 2.5, so supersteps
+    // with prune tests only pay where trees stay large: on heavy-tailed
+    // graphs, and once kFreeVisits vertices per label were settled (fetch_root
+    // ends the superstep).  The 1024-square grid: trees 0.81 s in one unpruned
+    // superstep, 1.09 to 1.32 s with a label budget of 1024 n.
+    const bool whole = !heavy_tail && win_target > 1 && opts.mode != CHL_MODE_GLL && opts.first_superstep == 0;
+    constexpr uint32_t kFreeVisits = 16;
+    // pruned trees of at least this many settled vertices (by the last
+    // superstep's mean) are built by the team kernel, smaller ones a warp each
+    // (the 1024-square grid within 1% between 300 and 3,000)
+    constexpr double kTeamVisits = 1000;
     // workspace: one slot per resident warp
     const int sms = device_sms();
     const bool unit = g->unit;
@@ -1993,30 +2134,34 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         const uint32_t fit_slots = (uint32_t)std::max<size_t>(kWarpsPerBlock, ws_budget / std::max<size_t>(slot_bytes, 1));
         b.slots = std::max<uint32_t>(kWarpsPerBlock, (std::min(b.slots, fit_slots) / kWarpsPerBlock) * kWarpsPerBlock);
     }
-    // window kernel (first superstep): one tree per block of win_tw warps
-    // (auto: 8 on heavy-tailed graphs, 4 otherwise), as many trees as are
-    // resident, 6 n words each
+    // team kernel: one tree per block of win_tw warps (auto: 8 on heavy-tailed
+    // graphs, 4 otherwise), as many trees as are resident, 6 n words each
     b.win_tw = opts.window_warps ? opts.window_warps : (heavy_tail ? 8 : 4);
     if (b.win_tw != 1 && b.win_tw != 2 && b.win_tw != 4 && b.win_tw != 8) {
         set_error("window_warps must be 0, 1, 2, 4 or 8");
         return CHL_ERR_INVALID;
     }
-    {
+    // root hash slots: at most 2048 per warp-built tree within CHL_SMEM_CAP_KB
+    // of shared memory per block, and 4096 per block-built one
+    auto team_blocks = [&](bool plant, bool prune, uint32_t hash_slots, int *blocks) -> int {
         // the occupancy query counts a block's dynamic shared memory only up
         // to the kernel's current limit (48 KB by default): raise it first
-        const int wsm = (int)window_smem(b.win_tw);
-        for (int p = 0; p < 2; ++p)
-            CHL_CUDA(cudaFuncSetAttribute(window_kernel_for(unit, p != 0, b.win_tw),
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, wsm));
-        int nbw = 0;
-        CHL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbw, window_kernel_for(unit, true, b.win_tw),
-                                                                 b.win_tw * 32, wsm));
+        TreeKernel k = team_kernel_for(unit, plant, prune, b.win_tw);
+        const int sm = (int)team_smem((int)b.win_tw * 32, hash_slots);
+        CHL_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+        CHL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, b.win_tw * 32, sm));
+        *blocks = std::max(*blocks, 1) * sms;
+        return CHL_OK;
+    };
+    {
+        int blocks = 0;
+        if ((rc = team_blocks(true, false, 0, &blocks))) return rc;
         const uint64_t fit_trees = std::max<uint64_t>(1, ws_budget / std::max<uint64_t>(24ull * n, 1));
-        b.win_trees = (uint32_t)std::min<uint64_t>((uint64_t)std::max(nbw, 1) * sms, fit_trees);
+        b.win_trees = (uint32_t)std::min<uint64_t>((uint64_t)blocks, fit_trees);
     }
     // one workspace for both layouts: batch_kernel's key (two words on
     // weighted graphs), vis and queue arrays per warp slot (5 or 6 n words),
-    // window_kernel's 6 n words per tree
+    // team_kernel's 6 n words per tree
     const size_t key_words = unit ? 1 : 2;
     const size_t ws_words = std::max((size_t)b.slots * (4 + key_words) * n, (size_t)b.win_trees * 6 * n);
     if ((rc = dalloc(&b.ws_all, ws_words))) return rc;
@@ -2049,9 +2194,21 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     const double sf = opts.sf > 0 ? opts.sf : (heavy_tail ? 32.0 : 1024.0);
     // label_limit = sf * N counts both sides' labels (shared_memory/hhl.cpp:65);
     // a symmetric build stores one side.
-    const unsigned long long budget_base =
+    unsigned long long budget_base =
         (unsigned long long)std::max(1.0, sf * (double)n / (b.sides == 1 ? 2.0 : 1.0));
-    if (opts.label_cap == 0) {
+    // Supersteps of unpruned trees (whole) end at the label buffer, which has
+    // room for lists of 3 sqrt(n) (grids have 0.7 to 1.5 sqrt(n)) within a
+    // quarter of the free memory; a seventh of it is left to the trees still
+    // running when the budget is spent.
+    const bool whole_budget = whole && opts.sf <= 0 && opts.label_cap == 0;
+    if (whole_budget) {
+        size_t fr = 0, tot = 0;
+        CHL_CUDA(cudaMemGetInfo(&fr, &tot));
+        const uint64_t want = (uint64_t)(3.5 * std::sqrt((double)n) * n * b.sides) + (1u << 20);
+        if ((rc = grow_new(b, std::min<uint64_t>(want, fr / 4 / 36)))) return rc;
+        budget_base = b.new_cap - b.new_cap / 7;
+    }
+    if (opts.label_cap == 0 && !whole_budget) {
         // Room for every new label of a superstep: the budget plus what the
         // trees still running when it is spent can add (at most sides * n
         // each), so that a superstep does not overflow and run twice.  At
@@ -2074,27 +2231,20 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     uint32_t max_list = 0;   // longest committed list
     float step_tree_ms = 0;
     uint32_t step_slots = 0;   // warp slots of the last tree launch
+    double mean_visits = 0;    // settled vertices per tree of the last superstep
+    bool ratio_stopped = false;
     // Superstep schedule: superstep k covers roots [r0, r0 + size) with
     // size = clamp(growth * r0, first, n) -- small while the top hubs are not
     // yet committed (their labels prune everything later), geometric after.
     // The label budget sf * n (the reference's label_limit) also ends a
     // superstep early.
-    // label-correcting windows of the first superstep's trees: about this
-    // many vertices per window (1: IN-criterion rounds instead).  Auto: on
-    // heavy-tailed graphs, whose first trees are huge BFS-like searches
-    // (RMAT scale 20: 1.4x faster builds with 8 warps per tree); off on
-    // road-like ones (the 1024-square grid: 3.81-4.1 s with windows of
-    // 256-4096 vertices against 3.83 s without)
-    const uint32_t win_target = opts.window_target ? opts.window_target : (heavy_tail ? 1024u : 1u);
-    // Schedule defaults from graph statistics (measured on RMAT scale 18/20
-    // and 512/1024-square grids): heavy-tailed degree distributions start
-    // with one root per resident window tree (RMAT scale 20: 608 roots,
-    // 2.15 s against 2.28 s with 256 and 2.34 s with 1024) and double, so the
-    // hubs commit before the bulk of the trees while the early supersteps
-    // still fill the GPU; bounded-degree (road-like) graphs start with two
-    // roots per warp of the schedule (the 1024-square grid: 1.15x faster than
-    // one) and grow by half of the committed prefix.
-    const uint32_t auto_first = heavy_tail ? (win_target > 1 ? std::max<uint32_t>(64u, b.win_trees) : 1024u)
+    // Heavy-tailed degree distributions start with two roots per SM (RMAT
+    // scale 17: 47.6 ms with 304, 55 with 152, 68 with 1,216; a directed
+    // skewed graph of 2^15 vertices 14 ms with 304, 20 with 1,216) and
+    // double, so the hubs commit before the bulk of the trees; bounded-degree
+    // graphs outside the whole rule start with two roots per warp of the
+    // schedule and grow by half of the committed prefix.
+    const uint32_t auto_first = heavy_tail ? (win_target > 1 ? std::max<uint32_t>(64u, 2u * sms) : 1024u)
                                            : std::max<uint32_t>(64u, 2 * b.warps);
     const double auto_growth = heavy_tail ? 2.0 : 0.5;
     // phase switch ratio (the reference's -ps, default 1024): auto 8 on
@@ -2107,8 +2257,11 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         const uint32_t r_begin = r0;
         const bool plant_now = do_plant;
         const unsigned long long budget = budget_base;
+        // trees without prune tests, over all roots that are left
+        const bool unpruned = whole && plant_now && !ratio_stopped;
         uint64_t size = std::max<uint64_t>(first, (uint64_t)(growth * (double)r0));
         uint32_t r_end = (uint32_t)std::min<uint64_t>(n, (uint64_t)r0 + size);
+        if (unpruned) r_end = n;
         if (opts.root_limit) r_end = std::min<uint32_t>(r_end, opts.root_limit);
         BuildCtl hc;
         bool rerun = false;
@@ -2175,16 +2328,24 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
             void (*kern)(TreeArgs);
             size_t smem_launch = smem;
             int grid = blocks, block = kWarpsPerBlock * 32;
-            const bool windowed = committed == 0 && win_target > 1;
+            const bool windowed = win_target > 1 && (committed == 0 || unpruned || mean_visits >= kTeamVisits);
+            ta.visit_ratio = unpruned && !rerun ? kFreeVisits : 0;
+            ta.visit_base = 64ull * n;
             if (windowed) {
-                // no committed labels: no tree can be pruned, so the trees
-                // are searched label-correcting in windows (window_kernel)
+                const bool prune = committed > 0 && !unpruned;
+                uint32_t slots = prune ? 64 : 0;   // no committed labels: no root label to hash
+                while (prune && slots < 2 * max_list && slots < 4096) slots *= 2;
+                ta.hash_slots = slots;
+                ta.hash_shift = 32;
+                for (uint32_t t = slots; t > 1; t >>= 1) --ta.hash_shift;
                 ta.near_target = win_target;
                 ta.ws_win = b.ws_all;
-                grid = (int)b.win_trees;
+                int fit = 0;
+                if ((rc = team_blocks(plant_now, prune, slots, &fit))) return rc;
+                grid = (int)std::min<uint32_t>((uint32_t)fit, b.win_trees);
                 block = (int)b.win_tw * 32;
-                smem_launch = window_smem(b.win_tw);
-                kern = window_kernel_for(unit, plant_now, b.win_tw);
+                smem_launch = team_smem(block, slots);
+                kern = team_kernel_for(unit, plant_now, prune, b.win_tw);
             } else if (unit) {
                 kern = plant_now ? batch_kernel<true, true> : batch_kernel<true, false>;
             } else {
@@ -2194,8 +2355,10 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
             // reads is INF (each tree resets its own keys when it ends)
             const int layout = windowed ? 2 : 1;
             if (b.ws_layout != layout) {
-                const size_t words = windowed ? (size_t)b.win_trees * 6 * n : (size_t)b.slots * (4 + key_words) * n;
-                CHL_CUDA(cudaMemsetAsync(b.ws_all, 0xFF, words * 4, b.st));
+                if (windowed)
+                    CHL_CUDA(cudaMemset2DAsync(b.ws_all, (size_t)n * 24, 0xFF, (size_t)n * 8, b.win_trees, b.st));
+                else
+                    CHL_CUDA(cudaMemsetAsync(b.ws_all, 0xFF, (size_t)b.slots * key_words * n * 4, b.st));
                 b.ws_layout = layout;
             }
             CHL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_launch));
@@ -2231,6 +2394,9 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
             break;
         }
         const uint32_t r1 = r_end;
+        mean_visits = (double)hc.visits / std::max<uint32_t>(1, r1 - r0);
+        ratio_stopped |= hc.ratio_stop != 0;
+        const bool last = r1 >= n || (opts.root_limit && r1 >= opts.root_limit);
         visits += hc.visits;
         reads += hc.label_reads;
         arcs += hc.arcs;
@@ -2258,7 +2424,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         // array is sized for every new label before the chain (the clean
         // only removes labels).
         if ((rc = ensure_ent(&b.ent_b, &b.ent_cap_b, committed + M))) return rc;
-        if ((rc = ensure_ent(&b.dent_b, &b.dent_cap_b, committed + M))) return rc;
+        if (!last && (rc = ensure_ent(&b.dent_b, &b.dent_cap_b, committed + M))) return rc;
         const bool clean_now = !plant_now && M > 0;
         // bits of the distance part of the (list, distance) sort key
         const int dist_bits = bits_for((uint64_t)hc.max_dist + 1);
@@ -2299,7 +2465,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
             copy_old_lists<<<cgrid, 256, 0, b.st>>>(b.off_a, b.ent_a, b.off_b, b.ent_b, b.nl);
             place_new<<<cgrid, 256, 0, b.st>>>(sk, sv, d_count, b.new_cap, b.hub_bits, r0, b.pre, b.off_a,
                                                b.off_b, b.ent_b);
-            {
+            if (!last) {
                 // the same labels by (list, distance, hub), merged into the
                 // distance-ordered copy (the sort is stable: equal distances
                 // keep hub order); the key holds the distance in the bits the
@@ -2318,8 +2484,8 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
             CHL_CUDA(cudaGetLastError());
             return CHL_OK;
         };
-        kernels += 3 * ((b.key_bits + 7) / 8) + (clean_now ? 9 : 0) + 8 +
-                   2 + 3 * ((b.key_bits - b.hub_bits + dist_bits + 7) / 8);
+        kernels += 3 * ((b.key_bits + 7) / 8) + (clean_now ? 9 : 0) + 8;
+        if (!last) kernels += 2 + 3 * ((b.key_bits - b.hub_bits + dist_bits + 7) / 8);
         CHL_CUDA(cudaEventRecord(ev_a, b.st));
         if (opts.use_graphs) {
             CHL_CUDA(cudaStreamBeginCapture(b.st, cudaStreamCaptureModeThreadLocal));

@@ -255,3 +255,52 @@ def test_root_limit_gives_the_label_prefix(P, mode):
             keep = full_hub[a:b] <= top
             assert np.array_equal(hub[off[i]:off[i + 1]], full_hub[a:b][keep])
             assert np.array_equal(dist[off[i]:off[i + 1]], full_dist[a:b][keep])
+
+
+def test_unpruned_supersteps_give_way_to_pruned_ones(P, O):
+    """Random sparse graphs settle far more vertices than they label: the
+    whole-graph superstep ends by its settled-vertices ratio and the rest is
+    pruned.  Small label budgets end it by the budget instead."""
+    rng = np.random.default_rng(5)
+    n = 6000
+    src = np.repeat(np.arange(n), 3)
+    dst = rng.integers(0, n, src.size)
+    keep = src != dst
+    for undirected in (True, False):
+        g = P.Graph.from_arcs(n, src[keep], dst[keep], rng.integers(1, 100, int(keep.sum())), undirected=undirected)
+        order = P.Order.degree(g, seed=3)
+        ref = None
+        for kw in ({}, {"sf": 8.0}, {"mode": MODES["plant"], "window_warps": 1}, {"window_target": 1},
+                   {"window_warps": 8, "window_target": 64}, {"mode": MODES["gll"], "window_warps": 2}):
+            got = P.build(g, order, **kw).export()
+            ref = ref or got
+            assert all(np.array_equal(x, y) for x, y in zip(got, ref)), kw
+        pairs = np.stack([np.full(n, 17), np.arange(n)], 1).astype(np.uint32)
+        off, head, ln = g.csr(True)
+        d = np.full(n, np.inf)
+        d[17] = 0
+        tail = np.repeat(np.arange(n), np.diff(off.astype(np.int64)))
+        for _ in range(n):
+            e = d.copy()
+            np.minimum.at(e, head, d[tail] + ln)
+            if np.array_equal(e, d):
+                break
+            d = e
+        L = P.build(g, order)
+        assert np.array_equal(P.query(L, pairs), np.where(np.isinf(d), P.INFTY, d).astype(np.int64))
+
+
+def test_distances_near_int_max(P):
+    """A tentative distance past INT_MAX is no error where the final ones are
+    below it; a final one is (the reference asserts it)."""
+    big = 2 ** 31
+    g = P.Graph.from_arcs(5, [0, 0, 0, 1, 2], [1, 2, 4, 2, 3], [1, big - 10, big - 5, 1, 100])
+    order = np.array([0, 1, 2, 3, 4], np.uint32)
+    for kw in ({}, {"window_target": 1}, {"mode": MODES["gll"]}, {"window_target": 100, "window_warps": 1}):
+        L = P.build(g, order, **kw)
+        assert P.query(L, [[0, 3], [0, 4], [1, 3]]).tolist() == [102, big - 5, 101], kw
+    g = P.Graph.from_arcs(3, [0, 1, 0], [1, 2, 2], [2 ** 30, 2 ** 30, 5], undirected=True)
+    for kw in ({}, {"window_target": 1}, {"mode": MODES["gll"]}):
+        with pytest.raises(P.CHLError) as e:
+            P.build(g, np.array([0, 1, 2], np.uint32), **kw)
+        assert e.value.status == P.CHL_ERR_INVALID, kw
