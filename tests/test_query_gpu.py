@@ -59,3 +59,25 @@ def test_empty_batch(P):
     c = label_case("grid12")
     L = P.Labeling.read(c["labels"])
     assert len(P.query(L, np.zeros((0, 2), np.uint32))) == 0
+
+
+@pytest.mark.parametrize("k", [1, 2, 33, 9729, 19457, 311297, 400001])
+def test_query_chunk_and_group_edges(P, O, k):
+    """Lists of lengths at the edges of 32-entry chunks, equal and disjoint
+    ranges among them, and pair counts at the edges of a warp's group."""
+    rng = np.random.default_rng(4)
+    lens = [0, 1, 2, 31, 32, 33, 63, 64, 65, 96, 97, 200]
+    lists = []
+    for i, c in enumerate(lens):
+        lists.append(np.sort(rng.choice(300, c, replace=False)))   # dense: many common hubs
+        lists.append(np.arange(c) * 7 + 1000 * (i % 2))            # one range of two, entirely before or after
+        lists.append(np.sort(rng.choice(4000, c, replace=False)))
+    n = len(lists) // 2
+    off = np.zeros(2 * n + 1, np.uint64)
+    off[1:] = np.cumsum([len(h) for h in lists])
+    hub = np.concatenate(lists).astype(np.uint32)
+    dist = rng.integers(0, 10**6, hub.size).astype(np.int32)
+    L = P.Labeling.from_csr(n, off, hub, dist)
+    ref = O.OLabels.from_csr(n, off, hub, dist)
+    pairs = rng.integers(0, n, (k, 2)).astype(np.uint32)
+    assert np.array_equal(P.query(L, pairs), ref.query(pairs))
