@@ -126,7 +126,8 @@ SIGNATURES = {
     "chl_labels_save": (C.c_int, [_P, C.c_char_p]),
     "chl_labels_load": (C.c_int, [C.c_char_p, C.POINTER(_P)]),
     "chl_labels_free": (None, [_P]),
-    "chl_query_batch": (C.c_int, [_P, _U32P, C.c_size_t, _I32P, _P]),
+    # arrays as addresses: building a typed pointer costs more than a small call
+    "chl_query_batch": (C.c_int, [_P, _P, C.c_size_t, _P, _P]),
     "chl_query_batch_noalloc": (C.c_int, [_P, _U32P, C.c_size_t, _I32P, _P]),
     "chl_query_batch_device": (C.c_int, [_P, _P, C.c_size_t, _P, _P]),
     "chl_query_bench": (C.c_int, [_P, C.c_size_t, C.c_uint64, C.c_int, C.c_uint32, C.POINTER(C.c_double), _U64P]),
@@ -134,8 +135,8 @@ SIGNATURES = {
     "chl_query_load": (C.c_int, [C.c_char_p, C.POINTER(_U32P), C.POINTER(C.c_size_t)]),
     "chl_server_opts_default": (None, [C.POINTER(ServerOpts)]),
     "chl_server_create": (C.c_int, [_P, C.POINTER(ServerOpts), C.POINTER(_P)]),
-    "chl_server_submit": (C.c_int, [_P, _U32P, C.c_size_t, _U64P]),
-    "chl_server_wait": (C.c_int, [_P, C.c_uint64, _I32P, C.c_double, C.POINTER(C.c_double)]),
+    "chl_server_submit": (C.c_int, [_P, _P, C.c_size_t, _U64P]),
+    "chl_server_wait": (C.c_int, [_P, C.c_uint64, _P, C.c_double, C.POINTER(C.c_double)]),
     "chl_server_stats": (C.c_int, [_P, _U64P, _U64P, _U64P]),
     "chl_server_blocked": (C.c_int, [_P, _U32P]),
     "chl_server_free": (None, [_P]),
@@ -186,6 +187,14 @@ def _u32(a) -> np.ndarray:
 
 def _ptr(a: np.ndarray, t):
     return a.ctypes.data_as(t)
+
+
+def _pairs(pairs) -> np.ndarray:
+    """(k, 2) pairs as a contiguous uint32 array (as they are if they are one)."""
+    if type(pairs) is np.ndarray and pairs.dtype == np.uint32 and pairs.ndim == 2 and pairs.shape[1] == 2 \
+            and pairs.flags.c_contiguous:
+        return pairs
+    return _u32(np.asarray(pairs).reshape(-1, 2))
 
 
 # ------------------------------------------------------------------ graph
@@ -485,9 +494,9 @@ def run(g: Graph, order, phase_switch: float = 1024.0, sf: float = 32.0, verbose
 
 def query(labels: Labeling, pairs) -> np.ndarray:
     """batchLocalQuery: pairs is (k, 2) of (u, v); returns d(u -> v) int32."""
-    p = _u32(np.asarray(pairs).reshape(-1, 2))
-    out = np.zeros(len(p), np.int32)
-    _check(lib().chl_query_batch(labels._h, _ptr(p, _U32P), len(p), _ptr(out, _I32P), None), "query")
+    p = _pairs(pairs)
+    out = np.empty(len(p), np.int32)
+    _check(lib().chl_query_batch(labels._h, p.ctypes.data, len(p), out.ctypes.data, None), "query")
     return out
 
 
@@ -531,16 +540,16 @@ class Server:
         _check(lib().chl_server_create(labels._h, C.byref(o), C.byref(self._h)), "server create")
 
     def submit(self, pairs) -> int:
-        p = _u32(np.asarray(pairs).reshape(-1, 2))
+        p = _pairs(pairs)
         rid = C.c_uint64()
-        _check(lib().chl_server_submit(self._h, _ptr(p, _U32P), len(p), C.byref(rid)), "submit")
+        _check(lib().chl_server_submit(self._h, p.ctypes.data, len(p), C.byref(rid)), "submit")
         self._last_k = len(p)
         return rid.value
 
     def wait(self, rid: int, k: int, timeout_ms: float = -1.0):
         out = np.zeros(k, np.int32)
         lat = C.c_double()
-        _check(lib().chl_server_wait(self._h, rid, _ptr(out, _I32P), timeout_ms, C.byref(lat)), "wait")
+        _check(lib().chl_server_wait(self._h, rid, out.ctypes.data, timeout_ms, C.byref(lat)), "wait")
         return out, lat.value
 
     def blocked(self) -> int:

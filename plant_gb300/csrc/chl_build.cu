@@ -36,6 +36,7 @@
 #include <type_traits>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 namespace chl {
@@ -1881,9 +1882,10 @@ struct Build {
     uint64_t ent_cap_a = 0, ent_cap_b = 0;
     uint2 *dent_a = nullptr, *dent_b = nullptr;   // (distance, hub)-ordered copies
     uint64_t dent_cap_a = 0, dent_cap_b = 0;
-    uint64_t *nk0 = nullptr, *nk1 = nullptr;
+    std::unique_ptr<TmpSet> mem;   // every buffer below but the committed CSR, which becomes the labels'
+    uint64_t *nk0 = nullptr, *nk1 = nullptr;   // new labels as the trees emit them, and the sort's other half
     uint32_t *nv0 = nullptr, *nv1 = nullptr;
-    uint64_t new_cap = 0;
+    uint64_t new_cap = 0, sort_cap = 0, keep_cap = 0;
     uint32_t *cnt = nullptr;
     uint64_t *pre = nullptr;
     uint32_t *keep = nullptr;
@@ -1907,32 +1909,14 @@ struct Build {
 
     ~Build() {
         if (commit_exec) cudaGraphExecDestroy(commit_exec);
-        if (farc[1] != farc[0]) cudaFree(farc[1]);
-        if (fhead[1] != fhead[0]) cudaFree(fhead[1]);
-        cudaFree(farc[0]);
-        cudaFree(fhead[0]);
+        mem.reset();
         own.release();
-        cudaFree(order);
-        cudaFree(rank);
         cudaFree(off_a);
         cudaFree(off_b);
         cudaFree(ent_a);
         cudaFree(ent_b);
         cudaFree(dent_a);
         cudaFree(dent_b);
-        cudaFree(nk0);
-        cudaFree(nk1);
-        cudaFree(nv0);
-        cudaFree(nv1);
-        cudaFree(cnt);
-        cudaFree(pre);
-        cudaFree(keep);
-        cudaFree(kpre);
-        cudaFree(tsize);
-        cudaFree(tlab);
-        cudaFree(ws_all);
-        cudaFree(ctl);
-        cudaFree(tmp);
         if (st) cudaStreamDestroy(st);
     }
 };
@@ -1942,27 +1926,42 @@ struct Build {
 // to append, so its re-run needs exactly that many: no doubling.
 int grow_new(Build &b, uint64_t need) {
     if (need <= b.new_cap) return CHL_OK;
-    const uint64_t cap = need;
-    cudaFree(b.nk0);
-    cudaFree(b.nk1);
-    cudaFree(b.nv0);
-    cudaFree(b.nv1);
-    cudaFree(b.keep);
-    cudaFree(b.kpre);
-    b.nk0 = b.nk1 = nullptr;
-    b.nv0 = b.nv1 = nullptr;
-    b.keep = nullptr;
-    b.kpre = nullptr;
+    b.mem->put(b.nk0);
+    b.mem->put(b.nv0);
+    b.new_cap = 0;
     int rc;
-    if ((rc = dalloc(&b.nk0, cap)) || (rc = dalloc(&b.nk1, cap)) || (rc = dalloc(&b.nv0, cap)) ||
-        (rc = dalloc(&b.nv1, cap)) || (rc = dalloc(&b.keep, cap)) || (rc = dalloc(&b.kpre, cap + 1)))
-        return rc;
-    b.new_cap = cap;
-    size_t need_tmp = std::max(radix_tmp_bytes(), scan_tmp_bytes(std::max<uint64_t>(cap, b.nl)));
+    if ((rc = b.mem->get(&b.nk0, need)) || (rc = b.mem->get(&b.nv0, need))) return rc;
+    b.new_cap = need;
+    return CHL_OK;
+}
+
+// The rest of the commit's buffers, for the m labels a superstep has emitted:
+// the sort's other half, the scans' temporaries and, for a clean, its flags
+// and their prefix.
+int grow_sort(Build &b, uint64_t m, bool clean) {
+    int rc;
+    if (m > b.sort_cap || !b.nk1) {
+        b.mem->put(b.nk1);
+        b.mem->put(b.nv1);
+        b.sort_cap = 0;
+        if ((rc = b.mem->get(&b.nk1, m)) || (rc = b.mem->get(&b.nv1, m))) return rc;
+        b.sort_cap = m;
+    }
+    if (clean && (m > b.keep_cap || !b.keep)) {
+        b.mem->put(b.keep);
+        b.mem->put(b.kpre);
+        b.keep_cap = 0;
+        if ((rc = b.mem->get(&b.keep, m)) || (rc = b.mem->get(&b.kpre, m + 1))) return rc;
+        b.keep_cap = m;
+    }
+    const size_t need_tmp = std::max(radix_tmp_bytes(), scan_tmp_bytes(std::max<uint64_t>(m, b.nl)));
     if (need_tmp > b.tmp_bytes) {
-        cudaFree(b.tmp);
+        char *t = (char *)b.tmp;
+        b.mem->put(t);
         b.tmp = nullptr;
-        if ((rc = dalloc((char **)&b.tmp, need_tmp))) return rc;
+        b.tmp_bytes = 0;
+        if ((rc = b.mem->get(&t, need_tmp))) return rc;
+        b.tmp = t;
         b.tmp_bytes = need_tmp;
     }
     return CHL_OK;
@@ -2015,6 +2014,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     b.key_bits = b.hub_bits + bits_for((uint64_t)b.nl + 1);
     if (b.key_bits > 64) return CHL_ERR_INVALID;
     CHL_CUDA(cudaStreamCreateWithFlags(&b.st, cudaStreamNonBlocking));
+    b.mem.reset(new TmpSet(b.st));
     cudaEvent_t ev0, ev1, ev_a, ev_b, ev_up;
     CHL_CUDA(cudaEventCreate(&ev_up));
     CHL_CUDA(cudaEventCreate(&ev0));
@@ -2036,7 +2036,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         if ((rc = upload_graph(g, b.own, b.st))) return rc;
         b.dg = &b.own;
     }
-    if ((rc = dalloc(&b.order, n)) || (rc = dalloc(&b.rank, n))) return rc;
+    if ((rc = b.mem->get(&b.order, n)) || (rc = b.mem->get(&b.rank, n))) return rc;
     CHL_CUDA(cudaMemcpyAsync(b.order, order_h, (size_t)n * 4, cudaMemcpyHostToDevice, b.st));
     CHL_CUDA(cudaMemcpyAsync(b.rank, rank_h.data(), (size_t)n * 4, cudaMemcpyHostToDevice, b.st));
     CHL_CUDA(cudaEventRecord(ev_up, b.st));
@@ -2045,13 +2045,11 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     if ((rc = dalloc(&b.off_a, (size_t)b.nl + 1)) || (rc = dalloc(&b.off_b, (size_t)b.nl + 1)))
         return rc;
     CHL_CUDA(cudaMemsetAsync(b.off_a, 0, ((size_t)b.nl + 1) * 8, b.st));
-    if ((rc = ensure_ent(&b.ent_a, &b.ent_cap_a, 1)) || (rc = ensure_ent(&b.dent_a, &b.dent_cap_a, 1))) return rc;
-    if ((rc = dalloc(&b.cnt, (size_t)b.nl + 1)) || (rc = dalloc(&b.pre, (size_t)b.nl + 2))) return rc;
+    if ((rc = b.mem->get(&b.cnt, (size_t)b.nl + 1)) || (rc = b.mem->get(&b.pre, (size_t)b.nl + 2))) return rc;
     CHL_CUDA(cudaMemsetAsync(b.cnt, 0, ((size_t)b.nl + 1) * 4, b.st));
-    if ((rc = dalloc(&b.tsize, n)) || (rc = dalloc(&b.tlab, n))) return rc;
-    if ((rc = dalloc(&b.ctl, 1))) return rc;
-    if ((rc = grow_new(b, opts.label_cap ? (uint64_t)opts.label_cap : std::max<uint64_t>(4ull * n, 1u << 20))))
-        return rc;
+    if ((rc = b.mem->get(&b.tsize, n)) || (rc = b.mem->get(&b.tlab, n))) return rc;
+    if ((rc = b.mem->get(&b.ctl, 1))) return rc;
+    if (opts.label_cap && (rc = grow_new(b, opts.label_cap))) return rc;
 
     // heavy-tailed degree distribution: the largest out-degree above 32
     // times the mean (scale-free graphs); bounded-degree (road-like)
@@ -2096,10 +2094,10 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
             const uint64_t m = g->off[src][n];
             const int grid = std::max(1, sms * 8);
             if (unit) {
-                if ((rc = dalloc(&b.fhead[s], std::max<uint64_t>(m, 1)))) return rc;
+                if ((rc = b.mem->get(&b.fhead[s], m))) return rc;
                 fat_heads<<<grid, 256, 0, b.st>>>(m, b.dg->head[s], b.rank, b.fhead[s]);
             } else {
-                if ((rc = dalloc(&b.farc[s], std::max<uint64_t>(m, 1)))) return rc;
+                if ((rc = b.mem->get(&b.farc[s], m))) return rc;
                 fat_arcs<<<grid, 256, 0, b.st>>>(m, b.dg->arc[s], b.rank, b.dg->win[s], b.farc[s]);
             }
             CHL_CUDA(cudaGetLastError());
@@ -2164,7 +2162,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     // team_kernel's 6 n words per tree
     const size_t key_words = unit ? 1 : 2;
     const size_t ws_words = std::max((size_t)b.slots * (4 + key_words) * n, (size_t)b.win_trees * 6 * n);
-    if ((rc = dalloc(&b.ws_all, ws_words))) return rc;
+    if ((rc = b.mem->get(&b.ws_all, ws_words))) return rc;
     b.ws_key = b.ws_all;
     b.ws_vis = b.ws_all + (size_t)b.slots * key_words * n;
     b.ws_front = b.ws_vis + (size_t)b.slots * n;
@@ -2219,7 +2217,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         CHL_CUDA(cudaMemGetInfo(&fr, &tot));
         const uint64_t want = (uint64_t)budget_base + (uint64_t)std::max(b.slots, b.win_trees) * b.sides * n;
         const uint64_t fit = (uint64_t)(fr / 4 / 36);
-        if ((rc = grow_new(b, std::min(want, fit)))) return rc;
+        if ((rc = grow_new(b, std::max<uint64_t>(std::min(want, fit), std::max<uint64_t>(4ull * n, 1u << 20))))) return rc;
     }
     bool do_plant = opts.mode != CHL_MODE_GLL;
     bool switch_open = opts.mode == CHL_MODE_HYBRID;
@@ -2423,16 +2421,18 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         // captured as a CUDA graph when opts.use_graphs is set.  The entry
         // array is sized for every new label before the chain (the clean
         // only removes labels).
+        const bool clean_now = !plant_now && M > 0;
+        if ((rc = grow_sort(b, M, clean_now))) return rc;
         if ((rc = ensure_ent(&b.ent_b, &b.ent_cap_b, committed + M))) return rc;
         if (!last && (rc = ensure_ent(&b.dent_b, &b.dent_cap_b, committed + M))) return rc;
-        const bool clean_now = !plant_now && M > 0;
         // bits of the distance part of the (list, distance) sort key
         const int dist_bits = bits_for((uint64_t)hc.max_dist + 1);
         auto chain = [&]() -> int {
             int rc2;
+            const uint64_t m_cap = M;   // the sort sees the count in device memory as well
             // --- sort the new labels by (list, hub)
             int parity = 0;
-            if ((rc2 = radix_sort_pairs(b.nk0, b.nv0, b.nk1, b.nv1, (const uint64_t *)&b.ctl->nlab, b.new_cap,
+            if ((rc2 = radix_sort_pairs(b.nk0, b.nv0, b.nk1, b.nv1, (const uint64_t *)&b.ctl->nlab, m_cap,
                                         b.key_bits, b.tmp, b.tmp_bytes, b.st, &parity)))
                 return rc2;
             uint64_t *sk = parity ? b.nk1 : b.nk0;
@@ -2444,14 +2444,14 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
             // --- GLL clean (drops labels covered through a higher-ranked hub)
             if (clean_now) {
                 CHL_CUDA(cudaMemsetAsync(b.cnt, 0, ((size_t)b.nl + 1) * 4, b.st));
-                count_keys<<<cgrid, 256, 0, b.st>>>(sk, d_count, b.new_cap, b.hub_bits, b.cnt);
+                count_keys<<<cgrid, 256, 0, b.st>>>(sk, d_count, m_cap, b.hub_bits, b.cnt);
                 if ((rc2 = scan_u32_excl(b.cnt, b.pre, b.nl, nullptr, b.tmp, b.tmp_bytes, b.st))) return rc2;
-                clean_mark<<<cgrid, 256, 0, b.st>>>(sk, sv, d_count, b.new_cap, b.hub_bits, r0, b.pre, b.order,
+                clean_mark<<<cgrid, 256, 0, b.st>>>(sk, sv, d_count, m_cap, b.hub_bits, r0, b.pre, b.order,
                                                     b.rank, b.sides, b.keep);
-                if ((rc2 = scan_u32_excl(b.keep, b.kpre, b.new_cap, (const uint64_t *)d_count, b.tmp,
+                if ((rc2 = scan_u32_excl(b.keep, b.kpre, m_cap, (const uint64_t *)d_count, b.tmp,
                                          b.tmp_bytes, b.st)))
                     return rc2;
-                compact_kept<<<cgrid, 256, 0, b.st>>>(sk, sv, b.keep, b.kpre, d_count, b.new_cap, ak, av,
+                compact_kept<<<cgrid, 256, 0, b.st>>>(sk, sv, b.keep, b.kpre, d_count, m_cap, ak, av,
                                                       &b.ctl->n_keep);
                 CHL_CUDA(cudaMemcpyAsync(&b.ctl->nlab, &b.ctl->n_keep, 8, cudaMemcpyDeviceToDevice, b.st));
                 std::swap(sk, ak);
@@ -2459,20 +2459,20 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
             }
             // --- commit: merge the sorted new labels into the committed CSR
             CHL_CUDA(cudaMemsetAsync(b.cnt, 0, ((size_t)b.nl + 1) * 4, b.st));
-            count_keys<<<cgrid, 256, 0, b.st>>>(sk, d_count, b.new_cap, b.hub_bits, b.cnt);
+            count_keys<<<cgrid, 256, 0, b.st>>>(sk, d_count, m_cap, b.hub_bits, b.cnt);
             if ((rc2 = scan_u32_excl(b.cnt, b.pre, b.nl, nullptr, b.tmp, b.tmp_bytes, b.st))) return rc2;
             merge_offsets<<<cgrid, 256, 0, b.st>>>(b.off_a, b.pre, b.off_b, b.nl);
             copy_old_lists<<<cgrid, 256, 0, b.st>>>(b.off_a, b.ent_a, b.off_b, b.ent_b, b.nl);
-            place_new<<<cgrid, 256, 0, b.st>>>(sk, sv, d_count, b.new_cap, b.hub_bits, r0, b.pre, b.off_a,
+            place_new<<<cgrid, 256, 0, b.st>>>(sk, sv, d_count, m_cap, b.hub_bits, r0, b.pre, b.off_a,
                                                b.off_b, b.ent_b);
             if (!last) {
                 // the same labels by (list, distance, hub), merged into the
                 // distance-ordered copy (the sort is stable: equal distances
                 // keep hub order); the key holds the distance in the bits the
                 // superstep's largest distance needs
-                dist_keys<<<cgrid, 256, 0, b.st>>>(sk, sv, d_count, b.new_cap, b.hub_bits, dist_bits, r0, ak, av);
+                dist_keys<<<cgrid, 256, 0, b.st>>>(sk, sv, d_count, m_cap, b.hub_bits, dist_bits, r0, ak, av);
                 int par2 = 0;
-                if ((rc2 = radix_sort_pairs(ak, av, sk, sv, (const uint64_t *)d_count, b.new_cap,
+                if ((rc2 = radix_sort_pairs(ak, av, sk, sv, (const uint64_t *)d_count, m_cap,
                                             b.key_bits - b.hub_bits + dist_bits, b.tmp, b.tmp_bytes, b.st, &par2)))
                     return rc2;
                 merge_dist_lists<<<cgrid, 256, 0, b.st>>>(b.off_a, b.dent_a, b.off_b, b.pre, par2 ? sk : ak,

@@ -23,6 +23,53 @@ int cuda_status(cudaError_t e, const char *what, const char *file, int line);
 // Number of SMs of the current device (cached).
 int device_sms();
 
+// Temporary device memory of one call, ordered on stream s.  Blocks of up to
+// kTmpMost bytes come from a pool of the library's own that keeps at most
+// kTmpKeep bytes between calls (a cudaMalloc and cudaFree pair costs 60 us and
+// a synchronisation, and a small call makes a dozen); larger ones are plain
+// allocations (mapping them through a pool costs more: 16 GB 35 ms against
+// 7.7).  What outlives a call (labels, graphs, networks) is never taken from
+// here.  The pool is stream-ordered, so calls on any threads and streams may
+// share it; it is emptied when an allocation fails.
+constexpr size_t kTmpMost = (size_t)512 << 20;
+constexpr size_t kTmpKeep = (size_t)1 << 30;
+int tmp_alloc(void **p, size_t bytes, cudaStream_t s);
+void tmp_free(void *p, size_t bytes, cudaStream_t s);
+
+// The temporaries of one call, freed together (or one by one) on their stream.
+class TmpSet {
+  public:
+    explicit TmpSet(cudaStream_t s = 0) : st(s) {}
+    TmpSet(const TmpSet &) = delete;
+    TmpSet &operator=(const TmpSet &) = delete;
+    ~TmpSet() {
+        for (const auto &x : held) tmp_free(x.first, x.second, st);
+    }
+    template <typename T>
+    int get(T **p, uint64_t count) {
+        void *q = nullptr;
+        const size_t bytes = (size_t)(count ? count : 1) * sizeof(T);
+        const int rc = tmp_alloc(&q, bytes, st);
+        *p = (T *)q;
+        if (rc == 0) held.emplace_back(q, bytes);
+        return rc;
+    }
+    template <typename T>
+    void put(T *&p) {
+        for (size_t i = 0; i < held.size(); ++i)
+            if (held[i].first == (void *)p) {
+                tmp_free(held[i].first, held[i].second, st);
+                held.erase(held.begin() + i);
+                break;
+            }
+        p = nullptr;
+    }
+    cudaStream_t st;
+
+  private:
+    std::vector<std::pair<void *, size_t>> held;
+};
+
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;

@@ -662,24 +662,32 @@ constexpr size_t kAccBytes = sizeof(double) * (2 * kStatBlocks * NF > (NF + 1) *
 
 size_t param_count(uint32_t layers) { return kP0 + (size_t)layers * kPL + H + 1; }
 
+// a graph's arc lists for one call (symmetric graphs: one copy for both directions)
 struct GraphDev {
-    DevBuf off_out, head_out, off_in, head_in;
+    TmpSet tmp;
+    uint64_t *off_out = nullptr, *off_in = nullptr;
+    uint32_t *head_out = nullptr, *head_in = nullptr;
     uint32_t n = 0;
 };
 
 int upload_csr(const chl_graph *g, GraphDev &d) {
     const uint32_t n = g->n;
     d.n = n;
-    const uint64_t mo = g->off[1][n], mi = g->off[0][n];
     int rc;
-    if ((rc = d.off_out.ensure(((size_t)n + 1) * 8)) || (rc = d.head_out.ensure(std::max<uint64_t>(mo, 1) * 4)) ||
-        (rc = d.off_in.ensure(((size_t)n + 1) * 8)) || (rc = d.head_in.ensure(std::max<uint64_t>(mi, 1) * 4)))
-        return rc;
-    CHL_CUDA(cudaMemcpy(d.off_out.p, g->off[1].data(), ((size_t)n + 1) * 8, cudaMemcpyHostToDevice));
-    CHL_CUDA(cudaMemcpy(d.off_in.p, g->off[0].data(), ((size_t)n + 1) * 8, cudaMemcpyHostToDevice));
-    if (mo) CHL_CUDA(cudaMemcpy(d.head_out.p, g->head[1].data(), mo * 4, cudaMemcpyHostToDevice));
-    if (mi) CHL_CUDA(cudaMemcpy(d.head_in.p, g->head[0].data(), mi * 4, cudaMemcpyHostToDevice));
-    return CHL_OK;
+    auto put = [&](int f, uint64_t **off, uint32_t **head) -> int {
+        const uint64_t m = g->off[f][n];
+        if ((rc = d.tmp.get(off, (uint64_t)n + 1)) || (rc = d.tmp.get(head, m))) return rc;
+        CHL_CUDA(cudaMemcpy(*off, g->off[f].data(), ((size_t)n + 1) * 8, cudaMemcpyHostToDevice));
+        if (m) CHL_CUDA(cudaMemcpy(*head, g->head[f].data(), m * 4, cudaMemcpyHostToDevice));
+        return CHL_OK;
+    };
+    if ((rc = put(1, &d.off_out, &d.head_out))) return rc;
+    if (g->symmetric) {
+        d.off_in = d.off_out;
+        d.head_in = d.head_out;
+        return CHL_OK;
+    }
+    return put(0, &d.off_in, &d.head_in);
 }
 
 // standardise the feature columns of M->x in place; M->acc holds the partials
@@ -713,7 +721,7 @@ int ensure_scratch(chl_gnn *M, uint32_t n) {
 int forward(chl_gnn *M, const GraphDev &G, uint64_t seed) {
     const uint32_t n = G.n;
     const int sms = device_sms();
-    feat_raw<<<sms * 4, 256>>>(n, G.off_out.as<uint64_t>(), G.head_out.as<uint32_t>(), G.off_in.as<uint64_t>(),
+    feat_raw<<<sms * 4, 256>>>(n, G.off_out, G.head_out, G.off_in,
                                seed, M->x.as<float>());
     CHL_CUDA(cudaGetLastError());
     int rc = standardise(M, n);
@@ -725,7 +733,7 @@ int forward(chl_gnn *M, const GraphDev &G, uint64_t seed) {
         const float *W = P + kP0 + (size_t)(l - 1) * kPL;
         const __nv_bfloat16 *hp = hb + (size_t)(l - 1) * n * H;
         __nv_bfloat16 *ml = mb + (size_t)l * n * H;
-        aggregate_mean<<<sms * 8, 256>>>(n, G.off_out.as<uint64_t>(), G.head_out.as<uint32_t>(), hp, ml);
+        aggregate_mean<<<sms * 8, 256>>>(n, G.off_out, G.head_out, hp, ml);
         gemm_rows<K2><<<gemm_grid<K2>(sms), 128>>>(n, hp, ml, W, W + (size_t)K2 * H, 0, hb + (size_t)l * n * H, nullptr, 0);
     }
     const float *wout = P + kP0 + (size_t)M->layers * kPL;
@@ -752,7 +760,7 @@ int backward(chl_gnn *M, const GraphDev &G, double *loss) {
     // dz in BF16 goes to m_0's slot (unused after the forward pass)
     float *dz = M->dz.as<float>();
     head_bwd<<<sms * 4, 256>>>(n, M->ds.as<float>(), hb + (size_t)L * n * H, wout, dz, mb, gwout, gwout + H);
-    inv_degree<<<sms, 256>>>(n, G.off_out.as<uint64_t>(), M->inv.as<float>());
+    inv_degree<<<sms, 256>>>(n, G.off_out, M->inv.as<float>());
     for (uint32_t l = L; l >= 1; --l) {
         const float *W = P + kP0 + (size_t)(l - 1) * kPL;
         float *gW = Gp + kP0 + (size_t)(l - 1) * kPL;
@@ -765,7 +773,7 @@ int backward(chl_gnn *M, const GraphDev &G, double *loss) {
         gemm_rows<H><<<gemm_grid<H>(sms), 128>>>(n, mb, mb, M->wt.as<float>(), nullptr, 1, nullptr, M->dA.as<float>(), K2);
         gemm_rows<H><<<gemm_grid<H>(sms), 128>>>(n, mb, mb, M->wt.as<float>() + H * H, nullptr, 1, nullptr,
                                        M->dA.as<float>() + H, K2);
-        scatter_mean_bwd<<<sms * 8, 256>>>(n, M->dA.as<float>(), G.off_in.as<uint64_t>(), G.head_in.as<uint32_t>(),
+        scatter_mean_bwd<<<sms * 8, 256>>>(n, M->dA.as<float>(), G.off_in, G.head_in,
                                            M->inv.as<float>(), hp, dz, mb);
     }
     CHL_CUDA(cudaMemset(M->acc.p, 0, kAccBytes));
@@ -828,8 +836,8 @@ extern "C" int chl_gnn_features(const chl_graph *g, uint64_t seed, float *x) {
     GraphDev G;
     int rc;
     if ((rc = upload_csr(g, G)) || (rc = tmp.x.ensure((size_t)g->n * NF * 4))) return rc;
-    feat_raw<<<device_sms() * 4, 256>>>(g->n, G.off_out.as<uint64_t>(), G.head_out.as<uint32_t>(),
-                                        G.off_in.as<uint64_t>(), seed, tmp.x.as<float>());
+    feat_raw<<<device_sms() * 4, 256>>>(g->n, G.off_out, G.head_out,
+                                        G.off_in, seed, tmp.x.as<float>());
     CHL_CUDA(cudaGetLastError());
     if ((rc = standardise(&tmp, g->n))) return rc;
     CHL_CUDA(cudaMemcpy(x, tmp.x.p, (size_t)g->n * NF * 4, cudaMemcpyDeviceToHost));

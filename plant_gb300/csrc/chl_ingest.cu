@@ -509,22 +509,8 @@ __global__ void side_place(uint64_t cnt, const uint32_t *rf, uint32_t bit, const
         }
 }
 
-// device buffers freed on every return path
-struct Pool {
-    std::vector<void *> ptrs;
-    ~Pool() {
-        for (void *p : ptrs) cudaFree(p);
-    }
-    template <typename T>
-    int get(T **p, uint64_t count) {
-        void *q = nullptr;
-        cudaError_t e = cudaMalloc(&q, std::max<uint64_t>(count, 1) * sizeof(T));
-        if (e != cudaSuccess) return cuda_status(e, "cudaMalloc", __FILE__, __LINE__);
-        ptrs.push_back(q);
-        *p = (T *)q;
-        return CHL_OK;
-    }
-};
+using FileBuf = std::vector<char, NoInitAlloc<char>>;   // not zeroed before the read
+using Pool = TmpSet;   // device buffers freed on every return path
 
 // (k, v) stable radix sort on `bits` key bits; result in (k0, v0)
 int sort_kv(uint64_t *&k0, uint32_t *&v0, uint64_t *&k1, uint32_t *&v1, const uint64_t *d_cnt, uint64_t cnt,
@@ -561,7 +547,7 @@ int sort_records(uint64_t cnt, int dir, uint32_t *&ru, uint32_t *&rh, int32_t *&
     return CHL_OK;
 }
 
-int read_file(const char *path, std::vector<char> &buf) {
+int read_file(const char *path, FileBuf &buf) {
     FILE *f = fopen(path, "rb");
     if (!f) {
         set_error(std::string("cannot open graph file ") + path);
@@ -591,7 +577,7 @@ int read_file(const char *path, std::vector<char> &buf) {
 // only when fmt's tens digit is 1.  Returns 1 with n, skip and weighted set,
 // 0 when the host must decide (a rejected header, a comment after a number,
 // more than 18 digits).
-int metis_header(const std::vector<char> &file, long long &n, int &skip, int &weighted) {
+int metis_header(const FileBuf &file, long long &n, int &skip, int &weighted) {
     size_t q = 0;
     const size_t S = file.size();
     auto space = [&](char c) { return c == ' ' || c == '\t' || c == '\n' || c == '\v' || c == '\f' || c == '\r'; };
@@ -643,7 +629,7 @@ int metis_header(const std::vector<char> &file, long long &n, int &skip, int &we
 
 // 1: the file is of format fmt by the reference's rules and the graph was
 // built; 0: defer to the host parsers; < 0: -status of an error
-int ingest_text(const std::vector<char> &file, int fmt, bool undirected, chl_graph *g) {
+int ingest_text(const FileBuf &file, int fmt, bool undirected, chl_graph *g) {
     const uint64_t S = file.size();
     Pool pool;
     int rc;
@@ -834,7 +820,7 @@ using namespace chl;
 extern "C" int chl_graph_load_gpu(const char *path, int undirected, chl_graph **out, int *parsed_on_gpu) {
     if (!path || !out) return CHL_ERR_INVALID;
     if (parsed_on_gpu) *parsed_on_gpu = 0;
-    std::vector<char> file;
+    FileBuf file;
     int rc = read_file(path, file);
     if (rc) return rc;
     chl_graph *g = new (std::nothrow) chl_graph();

@@ -22,6 +22,10 @@ int cuda_status(cudaError_t e, const char *what, const char *file, int line) {
     return CHL_ERR_CUDA;
 }
 
+// bytes of one pinned staging buffer: pinning costs about 40 us per MB, and
+// 16 MB chunks already copy at full rate
+constexpr size_t kStage = 16ull << 20;
+
 int device_sms() {
     static int sms = 0;
     static std::once_flag once;
@@ -36,11 +40,70 @@ int device_sms() {
     return sms;
 }
 
+namespace {
+
+// the pool of tmp_alloc on the current device (null: none could be made)
+cudaMemPool_t tmp_pool() {
+    static std::mutex mu;
+    static std::vector<std::pair<bool, cudaMemPool_t>> pools;   // (tried, pool) by device
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> g(mu);
+    if ((int)pools.size() <= dev) pools.resize(dev + 1, {false, nullptr});
+    if (!pools[dev].first) {
+        pools[dev].first = true;
+        cudaMemPoolProps pr;
+        std::memset(&pr, 0, sizeof(pr));
+        pr.allocType = cudaMemAllocationTypePinned;
+        pr.location.type = cudaMemLocationTypeDevice;
+        pr.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        uint64_t keep = kTmpKeep;
+        if (cudaMemPoolCreate(&pool, &pr) == cudaSuccess &&
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+            pools[dev].second = pool;
+        else
+            cudaGetLastError();
+    }
+    return pools[dev].second;
+}
+
+}  // namespace
+
+int tmp_alloc(void **p, size_t bytes, cudaStream_t s) {
+    *p = nullptr;
+    cudaMemPool_t pool = tmp_pool();
+    const bool pooled = pool && bytes <= kTmpMost;
+    cudaError_t e = pooled ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && pool) {
+        // give back what the pool keeps, then once more
+        cudaGetLastError();
+        cudaStreamSynchronize(s);
+        cudaMemPoolTrimTo(pool, 0);
+        e = pooled ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
+        return cuda_status(e, "device allocation", __FILE__, __LINE__);
+    }
+    return CHL_OK;
+}
+
+void tmp_free(void *p, size_t bytes, cudaStream_t s) {
+    if (!p) return;
+    if (bytes <= kTmpMost && tmp_pool()) cudaFreeAsync(p, s);
+    else cudaFree(p);
+}
+
 // Device -> pageable host copy through two pinned staging buffers: the DMA
 // of one chunk overlaps the (multi-threaded) copy of the previous one out
 // of pinned memory.
 int d2h_staged(void *dst, const void *src, size_t bytes) {
-    constexpr size_t kChunk = 64ull << 20;
+    constexpr size_t kChunk = kStage;
     if (bytes <= kChunk) {
         CHL_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost));
         return CHL_OK;
@@ -415,19 +478,102 @@ extern "C" int chl_labels_list_sizes(const chl_labels *l, uint32_t *sizes) {
     return CHL_OK;
 }
 
+namespace chl {
+namespace {
+
+// Device-resident labels straight into the caller's arrays: the entries come
+// through two pinned buffers and are spread to both sides' places from there,
+// without a host mirror (whose fresh pages cost more than the copy: 704 MB of
+// a 512-square grid's labels).  hoff: the nl + 1 list offsets; off: the
+// caller's 2n + 1.  Returns 1 when a list does not fit a buffer.
+int export_device(const chl_labels *l, const uint64_t *hoff, const uint64_t *off, uint32_t *hubs, int32_t *dists) {
+    constexpr uint64_t kMost = kStage / sizeof(LabelEnt);
+    const uint32_t nl = l->nl();
+    std::vector<uint32_t> cut{0};   // lists [cut[c], cut[c + 1]) fit one buffer
+    while (cut.back() < nl) {
+        const uint32_t b = cut.back();
+        const uint64_t *e = std::upper_bound(hoff + b, hoff + nl + 1, hoff[b] + kMost) - 1;
+        if (e == hoff + b) return 1;
+        cut.push_back((uint32_t)(e - hoff));
+    }
+    struct Stage {
+        void *pin[2] = {nullptr, nullptr};
+        cudaStream_t st = nullptr;
+        cudaEvent_t ev[2] = {nullptr, nullptr};
+        ~Stage() {
+            if (st) cudaStreamSynchronize(st);
+            for (auto x : ev)
+                if (x) cudaEventDestroy(x);
+            if (st) cudaStreamDestroy(st);
+            for (auto x : pin)
+                if (x) cudaFreeHost(x);
+        }
+    } sg;
+    const size_t room = std::min<uint64_t>(kMost, l->total) * sizeof(LabelEnt);
+    for (int i = 0; i < 2; ++i) {
+        CHL_CUDA(cudaHostAlloc(&sg.pin[i], room, cudaHostAllocDefault));
+        CHL_CUDA(cudaEventCreateWithFlags(&sg.ev[i], cudaEventDisableTiming));
+    }
+    CHL_CUDA(cudaStreamCreateWithFlags(&sg.st, cudaStreamNonBlocking));
+    const size_t chunks = cut.size() - 1;
+    auto issue = [&](size_t c) -> int {
+        const uint64_t b = hoff[cut[c]], e = hoff[cut[c + 1]];
+        if (e > b)
+            CHL_CUDA(cudaMemcpyAsync(sg.pin[c & 1], l->d_ent + b, (e - b) * sizeof(LabelEnt), cudaMemcpyDeviceToHost,
+                                     sg.st));
+        CHL_CUDA(cudaEventRecord(sg.ev[c & 1], sg.st));
+        return CHL_OK;
+    };
+    int rc = chunks ? issue(0) : CHL_OK;
+    for (size_t c = 0; c < chunks && rc == CHL_OK; ++c) {
+        CHL_CUDA(cudaEventSynchronize(sg.ev[c & 1]));
+        // the other buffer was read out in the last iteration
+        if (c + 1 < chunks && (rc = issue(c + 1))) break;
+        const LabelEnt *from = (const LabelEnt *)sg.pin[c & 1] - (ptrdiff_t)hoff[cut[c]];
+        const int64_t x0 = cut[c], x1 = cut[c + 1];
+#pragma omp parallel for schedule(dynamic, 64)
+        for (int64_t x = x0; x < x1; ++x) {
+            const uint64_t b = hoff[x], cnt = hoff[x + 1] - b;
+            for (int side = 0; side < (l->sym ? 2 : 1); ++side) {
+                const uint64_t to = off[l->sym ? 2 * x + side : x];
+                if (hubs)
+                    for (uint64_t k = 0; k < cnt; ++k) hubs[to + k] = from[b + k].hub;
+                if (dists)
+                    for (uint64_t k = 0; k < cnt; ++k) dists[to + k] = (int32_t)from[b + k].dist;
+            }
+        }
+    }
+    return rc;
+}
+
+}  // namespace
+}  // namespace chl
+
 extern "C" int chl_labels_export(const chl_labels *l, uint64_t *off, uint32_t *hubs,
                                  int32_t *dists) {
     if (!l || !off) return CHL_ERR_INVALID;
-    int rc = labels_fetch_host(l);
-    if (rc) return rc;
     // offsets of the 2n lists (both sides, even when stored once), then the
     // entries, copied in parallel over vertices
-    off[0] = 0;
-    for (uint32_t v = 0; v < l->n; ++v)
-        for (int side = 0; side < 2; ++side) {
-            const uint32_t x = l->list(v, side);
-            off[2 * v + side + 1] = off[2 * v + side] + (l->h_off[x + 1] - l->h_off[x]);
-        }
+    auto offsets = [&](const uint64_t *hoff) {
+        off[0] = 0;
+        for (uint32_t v = 0; v < l->n; ++v)
+            for (int side = 0; side < 2; ++side) {
+                const uint32_t x = l->list(v, side);
+                off[2 * (size_t)v + side + 1] = off[2 * (size_t)v + side] + (hoff[x + 1] - hoff[x]);
+            }
+    };
+    if (!l->host_valid && l->d_off) {
+        std::vector<uint64_t, NoInitAlloc<uint64_t>> hoff((size_t)l->nl() + 1);
+        int rc = d2h_staged(hoff.data(), l->d_off, hoff.size() * 8);
+        if (rc) return rc;
+        offsets(hoff.data());
+        if (!hubs && !dists) return CHL_OK;
+        rc = export_device(l, hoff.data(), off, hubs, dists);
+        if (rc != 1) return rc;
+    }
+    int rc = labels_fetch_host(l);
+    if (rc) return rc;
+    offsets(l->h_off.data());
     if (hubs || dists) {
         const int64_t n = l->n;
 #pragma omp parallel for schedule(dynamic, 1024)
@@ -455,17 +601,13 @@ extern "C" int chl_labels_hub_freq(const chl_labels *l, const uint32_t *order, u
     int rc = labels_ensure_device(l);
     if (rc) return rc;
     uint32_t *d_cnt = nullptr;
-    CHL_CUDA(cudaMalloc(&d_cnt, (size_t)std::max<uint32_t>(l->n, 1) * 4));
-    cudaError_t em = cudaMemset(d_cnt, 0, (size_t)l->n * 4);
-    if (em != cudaSuccess) {
-        cudaFree(d_cnt);
-        return cuda_status(em, "cudaMemset", __FILE__, __LINE__);
-    }
+    TmpSet tmp;
+    if ((rc = tmp.get(&d_cnt, l->n))) return rc;
+    CHL_CUDA(cudaMemset(d_cnt, 0, (size_t)l->n * 4));
     if (l->total)
         hub_count<<<device_sms() * 8, 256>>>((const uint2 *)l->d_ent, l->total, d_cnt);
     std::vector<uint32_t> cnt(l->n);
     cudaError_t e = cudaMemcpy(cnt.data(), d_cnt, (size_t)l->n * 4, cudaMemcpyDeviceToHost);
-    cudaFree(d_cnt);
     if (e != cudaSuccess) return cuda_status(e, "hub_freq", __FILE__, __LINE__);
     for (uint32_t h = 0; h < l->n; ++h) freq[order[h]] = cnt[h] * (l->sym ? 2u : 1u);
     return CHL_OK;
@@ -621,33 +763,121 @@ extern "C" int chl_query_batch_noalloc(const chl_labels *l, const uint32_t *pair
     return CHL_OK;
 }
 
+// Host pairs are answered through pinned slots that the kernel reads and
+// writes over the host link itself: no device staging and no copies to order,
+// one launch per slot, the host copies of one slot under the kernel of the
+// others.  (Device staging per call: 190 us for one pair, of which the kernel
+// is 8, and 330 for 65,536.)  A set of slots belongs to one call at a time;
+// at most kSetsKept idle sets are kept.
+namespace chl {
+namespace {
+
+constexpr size_t kSlotPairs = 32768;
+constexpr int kSlots = 4;
+constexpr size_t kSetsKept = 8;   // 12 MB pinned
+
+struct SlotSet {
+    int dev = 0;
+    char *mem = nullptr;   // kSlots x (pairs, answers)
+    cudaEvent_t ev[kSlots] = {nullptr, nullptr, nullptr, nullptr};
+    uint32_t *pairs(int i) const { return (uint32_t *)(mem + (size_t)i * kSlotPairs * 12); }
+    int32_t *out(int i) const { return (int32_t *)(mem + (size_t)i * kSlotPairs * 12 + kSlotPairs * 8); }
+    ~SlotSet() {
+        for (auto x : ev)
+            if (x) cudaEventDestroy(x);
+        if (mem) cudaFreeHost(mem);
+    }
+};
+
+std::mutex g_slots_mu;
+std::vector<SlotSet *> &idle_slots() {
+    static std::vector<SlotSet *> *v = new std::vector<SlotSet *>();   // not destroyed: the driver may be gone by then
+    return *v;
+}
+
+int take_slots(SlotSet **out) {
+    int dev = 0;
+    CHL_CUDA(cudaGetDevice(&dev));
+    {
+        std::lock_guard<std::mutex> g(g_slots_mu);
+        auto &v = idle_slots();
+        for (size_t i = v.size(); i-- > 0;)
+            if (v[i]->dev == dev) {
+                *out = v[i];
+                v.erase(v.begin() + i);
+                return CHL_OK;
+            }
+    }
+    SlotSet *s = new (std::nothrow) SlotSet();
+    if (!s) return CHL_ERR_OOM;
+    s->dev = dev;
+    cudaError_t e = cudaHostAlloc((void **)&s->mem, (size_t)kSlots * kSlotPairs * 12,
+                                  cudaHostAllocMapped | cudaHostAllocPortable);
+    for (int i = 0; i < kSlots && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&s->ev[i], cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+        delete s;
+        return cuda_status(e, "query slots", __FILE__, __LINE__);
+    }
+    *out = s;
+    return CHL_OK;
+}
+
+void give_slots(SlotSet *s) {
+    {
+        std::lock_guard<std::mutex> g(g_slots_mu);
+        if (idle_slots().size() < kSetsKept) {
+            idle_slots().push_back(s);
+            return;
+        }
+    }
+    delete s;
+}
+
+int query_slots(const chl_labels *l, const uint32_t *pairs, size_t k, int32_t *out, cudaStream_t st, SlotSet *s) {
+    const size_t chunks = (k + kSlotPairs - 1) / kSlotPairs;
+    auto collect = [&](size_t c) -> int {
+        CHL_CUDA(cudaEventSynchronize(s->ev[c % kSlots]));
+        const size_t at = c * kSlotPairs, cnt = std::min(kSlotPairs, k - at);
+        std::memcpy(out + at, s->out((int)(c % kSlots)), cnt * 4);
+        return CHL_OK;
+    };
+    int rc;
+    for (size_t c = 0; c < chunks; ++c) {
+        const int i = (int)(c % kSlots);
+        if (c >= (size_t)kSlots && (rc = collect(c - kSlots))) return rc;
+        const size_t at = c * kSlotPairs, cnt = std::min(kSlotPairs, k - at);
+        std::memcpy(s->pairs(i), pairs + 2 * at, cnt * 8);
+        if ((rc = query_launch(l, s->pairs(i), cnt, s->out(i), st))) return rc;
+        CHL_CUDA(cudaEventRecord(s->ev[i], st));
+    }
+    for (size_t c = chunks > (size_t)kSlots ? chunks - kSlots : 0; c < chunks; ++c)
+        if ((rc = collect(c))) return rc;
+    return CHL_OK;
+}
+
+}  // namespace
+}  // namespace chl
+
 extern "C" int chl_query_batch(const chl_labels *l, const uint32_t *pairs, size_t k, int32_t *out,
                                void *stream) {
     if (!l || (k && (!pairs || !out))) return CHL_ERR_INVALID;
-    for (size_t i = 0; i < 2 * k; ++i)
-        if (pairs[i] >= l->n) {
-            set_error("query vertex out of range");
-            return CHL_ERR_INVALID;
-        }
-    if (k == 0) return CHL_OK;
-    cudaStream_t s = (cudaStream_t)stream;
-    uint32_t *dp = nullptr;
-    int32_t *dout = nullptr;
-    CHL_CUDA(cudaMallocAsync(&dp, k * 8, s));
-    cudaError_t e = cudaMallocAsync(&dout, k * 4, s);
-    if (e != cudaSuccess) {
-        cudaFreeAsync(dp, s);
-        return cuda_status(e, "cudaMallocAsync", __FILE__, __LINE__);
+    uint32_t most = 0;   // one pass the compiler can vectorise
+    for (size_t i = 0; i < 2 * k; ++i) most = std::max(most, pairs[i]);
+    if (k && most >= l->n) {
+        set_error("query vertex out of range");
+        return CHL_ERR_INVALID;
     }
-    int rc = CHL_OK;
-    e = cudaMemcpyAsync(dp, pairs, k * 8, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) rc = query_launch(l, dp, k, dout, s);
-    if (e == cudaSuccess && rc == CHL_OK) e = cudaMemcpyAsync(out, dout, k * 4, cudaMemcpyDeviceToHost, s);
-    cudaFreeAsync(dp, s);
-    cudaFreeAsync(dout, s);
-    cudaError_t e2 = cudaStreamSynchronize(s);
+    if (k == 0) return CHL_OK;
+    SlotSet *s = nullptr;
+    int rc = take_slots(&s);
     if (rc) return rc;
-    if (e != cudaSuccess) return cuda_status(e, "query copy", __FILE__, __LINE__);
-    if (e2 != cudaSuccess) return cuda_status(e2, "query sync", __FILE__, __LINE__);
+    rc = query_slots(l, pairs, k, out, (cudaStream_t)stream, s);
+    if (rc) {
+        // launches may still be in flight: the slots are not reused before they end
+        cudaStreamSynchronize((cudaStream_t)stream);
+        delete s;
+        return rc;
+    }
+    give_slots(s);
     return CHL_OK;
 }

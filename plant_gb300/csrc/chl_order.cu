@@ -463,17 +463,20 @@ __global__ void bc_sum(uint32_t n, uint32_t count, const double *deltas, double 
     }
 }
 
-struct Buf {
+struct Buf {   // temporary of one call, on the null stream
     void *p = nullptr;
-    ~Buf() { cudaFree(p); }
+    size_t bytes = 0;
+    Buf() = default;
+    Buf(const Buf &) = delete;
+    Buf &operator=(const Buf &) = delete;
+    ~Buf() { tmp_free(p, bytes, 0); }
     template <typename T>
     T *as() const { return (T *)p; }
 };
 
 int alloc(Buf &b, size_t bytes) {
-    cudaError_t e = cudaMalloc(&b.p, bytes ? bytes : 1);
-    if (e != cudaSuccess) return cuda_status(e, "cudaMalloc", __FILE__, __LINE__);
-    return CHL_OK;
+    b.bytes = bytes ? bytes : 1;
+    return tmp_alloc(&b.p, b.bytes, 0);
 }
 
 // Sort vertices by (primary descending, tie ascending); `primary` fills key

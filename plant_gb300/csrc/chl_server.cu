@@ -14,7 +14,7 @@
 //   * batching: the server thread packs the pending pairs of many requests
 //     (splitting large ones) into one launch of up to max_batch_pairs;
 //   * overlap: kPipes batches are in flight at once, each on its own stream
-//     (copy in, kernel, copy out), so new requests are admitted and launched
+//     (one launch; pairs and answers stay in pinned host memory), so new requests are admitted and launched
 //     while earlier ones are still on the device;
 //   * completion: answers are scattered back per request; chl_server_wait
 //     returns them with the request's submit-to-completion latency.
@@ -60,8 +60,8 @@ struct Piece {
 struct Pipe {
     cudaStream_t st = nullptr;
     cudaEvent_t ev = nullptr;
-    uint32_t *h_in = nullptr, *d_in = nullptr;
-    int32_t *h_out = nullptr, *d_out = nullptr;
+    uint32_t *h_in = nullptr;    // pinned, mapped
+    int32_t *h_out = nullptr;
     std::vector<Piece> pieces;
     size_t count = 0;
     bool busy = false;
@@ -174,9 +174,8 @@ void server_loop(chl_server *s) {
         s->n_launch++;
         s->n_pairs += p.count;
         lk.unlock();
-        cudaMemcpyAsync(p.d_in, p.h_in, p.count * 8, cudaMemcpyHostToDevice, p.st);
-        int rc = chl::query_launch(s->labels, p.d_in, p.count, p.d_out, p.st);
-        cudaMemcpyAsync(p.h_out, p.d_out, p.count * 4, cudaMemcpyDeviceToHost, p.st);
+        // the kernel reads the pairs and writes the answers over the host link
+        int rc = chl::query_launch(s->labels, p.h_in, p.count, p.h_out, p.st);
         cudaEventRecord(p.ev, p.st);
         if (rc != CHL_OK) {
             std::lock_guard<std::mutex> g(s->mu);
@@ -212,10 +211,8 @@ extern "C" int chl_server_create(const chl_labels *l, const chl_server_opts *opt
     for (Pipe &p : s->pipes) {
         cudaError_t e = cudaStreamCreateWithFlags(&p.st, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&p.ev, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaMallocHost(&p.h_in, B * 8);
-        if (e == cudaSuccess) e = cudaMallocHost(&p.h_out, B * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&p.d_in, B * 8);
-        if (e == cudaSuccess) e = cudaMalloc(&p.d_out, B * 4);
+        if (e == cudaSuccess) e = cudaHostAlloc((void **)&p.h_in, B * 8, cudaHostAllocMapped);
+        if (e == cudaSuccess) e = cudaHostAlloc((void **)&p.h_out, B * 4, cudaHostAllocMapped);
         if (e != cudaSuccess) {
             int rc = chl::cuda_status(e, "server setup", __FILE__, __LINE__);
             chl_server_free(s);
@@ -331,8 +328,6 @@ extern "C" void chl_server_free(chl_server *s) {
         if (p.ev) cudaEventDestroy(p.ev);
         cudaFreeHost(p.h_in);
         cudaFreeHost(p.h_out);
-        cudaFree(p.d_in);
-        cudaFree(p.d_out);
     }
     for (auto &kv : s->table) delete kv.second;
     delete s;

@@ -81,3 +81,48 @@ def test_query_chunk_and_group_edges(P, O, k):
     ref = O.OLabels.from_csr(n, off, hub, dist)
     pairs = rng.integers(0, n, (k, 2)).astype(np.uint32)
     assert np.array_equal(P.query(L, pairs), ref.query(pairs))
+
+
+def test_query_slots_and_threads(P, O):
+    """Host batches around the slot size and count (32,768 pairs, 4 slots),
+    from several threads at once."""
+    import threading
+    g = P.Graph.rmat(10, 8, seed=2)
+    L = P.build(g, P.Order.degree(g, seed=1))
+    ref = O.OLabels.from_csr(g.get_n(), *L.export())
+    sizes = [1, 32767, 32768, 32769, 65536, 131072, 131073, 300000]
+    pairs = {k: P.generate_query(k, g.get_n(), seed=k) for k in sizes}
+    want = {k: ref.query(pairs[k]) for k in sizes}
+    bad = []
+
+    def ask(seed):
+        for k in np.random.default_rng(seed).permutation(sizes):
+            if not np.array_equal(P.query(L, pairs[int(k)]), want[int(k)]):
+                bad.append(int(k))
+
+    ts = [threading.Thread(target=ask, args=(i,)) for i in range(12)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
+
+
+def test_export_in_pieces(P):
+    """An export larger than a staging buffer (16 MB) equals the lists asked
+    one by one, offsets alone included."""
+    import ctypes as C
+    g = P.Graph.grid(140, 140, seed=4)
+    L = P.build(g, P.Order.degree(g, seed=2))
+    assert L.total() // 2 * 8 > 16 << 20
+    off, hub, dist = L.export()
+    only = np.zeros_like(off)
+    assert P.lib().chl_labels_export(L._h, only.ctypes.data_as(C.POINTER(C.c_uint64)), None, None) == 0
+    assert np.array_equal(only, off)
+    for v in (0, 1, 777, 10000, g.get_n() - 1):
+        for side in (0, 1):
+            h, d = L.label(v, side)
+            s = slice(int(off[2 * v + side]), int(off[2 * v + side + 1]))
+            assert np.array_equal(hub[s], h) and np.array_equal(dist[s], d)
+    for a, b in zip(L.export(), (off, hub, dist)):   # from the host mirror label() made
+        assert np.array_equal(a, b)
