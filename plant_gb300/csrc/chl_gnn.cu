@@ -43,59 +43,106 @@ __device__ __forceinline__ uint64_t gmix(uint64_t z) {
 }
 
 // raw features: log1p deg, log1p 2-hop degree sum, sampled clustering.
-// 16 lanes per vertex: one clustering sample each, and the neighbours' degrees
-// strided over them (whole numbers: their sum is the same in any order).  A
-// hub's list is bound by the latency of its dependent loads, so each lane has
-// 8 of them in flight; one thread per vertex took 2.61 ms on a 2^15-vertex
-// RMAT graph, all of it in its few hubs.
-constexpr int kFeatLanes = kClusterSamples;
+// A warp takes vpw vertices (32 once there are enough to fill the GPU so,
+// down to 2: a warp's vertices are walked one pair after the other).  Degree sums: a lane each while lists are short,
+// the whole warp where a list has more than kFeatLight arcs (whole numbers:
+// the sum is the same in any order).  Clustering: 16 lanes, one sample each,
+// on two vertices at a time.  The logarithms are double and the GPU's slow
+// unit, so all 32 lanes take them together.  One thread per vertex took
+// 2.61 ms on a 2^15-vertex RMAT graph (its hubs; 0.85 with them split off, the
+// others' neighbours being hubs), 16 lanes per vertex for everything 0.55 ms
+// on a 512-square grid (two lanes' logarithms at a time).
+constexpr uint32_t kFeatLight = 32;
 constexpr int kFeatLoads = 8;
-static_assert(kFeatLanes == 16, "two vertices per warp");
+static_assert(kClusterSamples == 16, "two vertices' samples fill a warp");
+
+// whether c is among the first kClusterScan out-arcs of a
+__device__ __forceinline__ bool has_arc(const uint64_t *off, const uint32_t *head, uint32_t a, uint32_t c) {
+    const uint64_t ab = off[a], ae = min(off[a + 1], ab + kClusterScan);
+    for (uint64_t q = ab; q < ae; q += 2 * kFeatLoads) {
+        bool hit = false;
+#pragma unroll
+        for (int t = 0; t < 2 * kFeatLoads; ++t) hit |= q + t < ae && head[q + t] == c;
+        if (hit) return true;
+    }
+    return false;
+}
+
+// clustering sample k of v, whose d >= 2 arcs start at b
+__device__ __forceinline__ bool closed_pair(const uint64_t *off, const uint32_t *head, uint64_t seed, uint32_t v, int k,
+                                            uint64_t b, uint32_t d) {
+    const uint64_t h = gmix(seed ^ ((uint64_t)v * 0x100000001B3ull + (uint64_t)k));
+    const uint64_t i = h % d;
+    uint64_t j = (h >> 32) % (d - 1);
+    if (j >= i) ++j;
+    return has_arc(off, head, head[b + i], head[b + j]);
+}
 
 __global__ void feat_raw(uint32_t n, const uint64_t *off_out, const uint32_t *head_out, const uint64_t *off_in,
-                         uint64_t seed, float *x) {
-    const uint32_t sub = threadIdx.x % kFeatLanes;
-    const uint32_t mask = (threadIdx.x & 16u) ? 0xFFFF0000u : 0x0000FFFFu;
-    const uint32_t groups = gridDim.x * (blockDim.x / kFeatLanes);
-    for (uint32_t v = blockIdx.x * (blockDim.x / kFeatLanes) + threadIdx.x / kFeatLanes; v < n; v += groups) {
-        const uint64_t b = off_out[v], e = off_out[v + 1];
-        const double deg = (double)(e - b) + (double)(off_in[v + 1] - off_in[v]);
-        uint64_t sum = 0;
-        for (uint64_t a = b + sub; a < e; a += kFeatLoads * kFeatLanes) {
-            uint32_t u[kFeatLoads];
-#pragma unroll
-            for (int q = 0; q < kFeatLoads; ++q) {
-                const uint64_t at = a + (uint64_t)q * kFeatLanes;
-                u[q] = at < e ? head_out[at] : 0xFFFFFFFFu;
-            }
-#pragma unroll
-            for (int q = 0; q < kFeatLoads; ++q)
-                if (u[q] != 0xFFFFFFFFu)
-                    sum += (off_out[u[q] + 1] - off_out[u[q]]) + (off_in[u[q] + 1] - off_in[u[q]]);
+                         uint64_t seed, uint32_t vpw, float *x) {
+    const uint32_t lane = lane_id();
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    for (uint64_t v0 = (uint64_t)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * vpw; v0 < n;
+         v0 += (uint64_t)warps * vpw) {
+        const uint32_t v = (uint32_t)v0 + lane;
+        uint64_t b = 0, sum = 0;
+        uint32_t d = 0, hits = 0, deg_in = 0;
+        const bool mine = lane < vpw && v < n;
+        if (mine) {
+            b = off_out[v];
+            d = (uint32_t)(off_out[v + 1] - b);
+            deg_in = (uint32_t)(off_in[v + 1] - off_in[v]);
         }
+        auto degree = [&](uint32_t u) { return (off_out[u + 1] - off_out[u]) + (off_in[u + 1] - off_in[u]); };
+        if (d <= kFeatLight) {
+            for (uint32_t a = 0; a < d; a += kFeatLoads) {
+                uint32_t u[kFeatLoads];
 #pragma unroll
-        for (int o = kFeatLanes / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(mask, sum, o);
-        uint32_t hit = 0;
-        const uint64_t d = e - b;
-        if (d >= 2) {
-            const uint64_t h = gmix(seed ^ ((uint64_t)v * 0x100000001B3ull + (uint64_t)sub));
-            const uint64_t i = h % d;
-            uint64_t j = (h >> 32) % (d - 1);
-            if (j >= i) ++j;
-            const uint32_t a = head_out[b + i], c = head_out[b + j];
-            const uint64_t ab = off_out[a], ae = min(off_out[a + 1], ab + kClusterScan);
-            for (uint64_t q = ab; q < ae && !hit; q += kFeatLoads) {
+                for (int q = 0; q < kFeatLoads; ++q) u[q] = a + q < d ? head_out[b + a + q] : 0u;
 #pragma unroll
-                for (int t = 0; t < kFeatLoads; ++t) hit |= (q + t < ae && head_out[q + t] == c) ? 1u : 0u;
+                for (int q = 0; q < kFeatLoads; ++q)
+                    if (a + q < d) sum += degree(u[q]);
             }
         }
-        const uint32_t hits = __popc(__ballot_sync(mask, hit != 0));
-        if (sub == 0) {
-            x[(size_t)v * NF + 0] = (float)log1p(deg);
+        __syncwarp();
+        for (uint32_t m = __ballot_sync(kFull, d > kFeatLight); m; m &= m - 1) {
+            const int o = __ffs(m) - 1;
+            const uint64_t ob = __shfl_sync(kFull, b, o);
+            const uint32_t od = __shfl_sync(kFull, d, o);
+            uint64_t s = 0;
+            for (uint32_t a = lane; a < od; a += 32 * kFeatLoads) {
+                uint32_t u[kFeatLoads];
+#pragma unroll
+                for (int q = 0; q < kFeatLoads; ++q) u[q] = a + 32 * q < od ? head_out[ob + a + 32 * q] : 0u;
+#pragma unroll
+                for (int q = 0; q < kFeatLoads; ++q)
+                    if (a + 32 * q < od) s += degree(u[q]);
+            }
+#pragma unroll
+            for (int w = 16; w > 0; w >>= 1) s += __shfl_xor_sync(kFull, s, w);
+            if (lane == (uint32_t)o) sum = s;
+        }
+        for (uint32_t j = 0; j < vpw; j += 2) {
+            const uint32_t o = j + (lane >> 4);
+            const uint64_t ob = __shfl_sync(kFull, b, o);
+            const uint32_t od = __shfl_sync(kFull, d, o);
+            const bool hit = od >= 2 && closed_pair(off_out, head_out, seed, (uint32_t)v0 + o, (int)(lane & 15), ob, od);
+            const uint32_t c = __ballot_sync(kFull, hit);
+            if ((lane & ~1u) == j) hits = __popc(lane & 1u ? c >> 16 : c & 0xFFFFu);
+        }
+        if (mine) {
+            x[(size_t)v * NF + 0] = (float)log1p((double)d + (double)deg_in);
             x[(size_t)v * NF + 1] = (float)log1p((double)sum);
             x[(size_t)v * NF + 2] = (float)hits / (float)kClusterSamples;
         }
     }
+}
+
+// vertices per warp of feat_raw's launch
+uint32_t feat_vpw(uint32_t n, int sms) {
+    uint32_t v = 2;
+    while (v < 32 && (uint64_t)v * sms * 4 * 8 < n) v *= 2;
+    return v;
 }
 
 // Standardised feature columns, (x - mean) / population sd in double: column
@@ -108,10 +155,22 @@ constexpr int kStatBlocks = 128;   // at most
 
 __device__ void col_totals(const double *part, int blocks, double *tot) {
     // every thread calls; tot (shared) holds NF totals afterwards
+    // (a fixed tree, so every block and every run finds the same totals)
+    __shared__ double ws[kStatBlocks / 32][NF];
+    __syncthreads();
+    if (threadIdx.x < kStatBlocks) {
+#pragma unroll
+        for (int k = 0; k < NF; ++k) {
+            double t = (int)threadIdx.x < blocks ? part[threadIdx.x * NF + k] : 0.0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+            if (lane_id() == 0) ws[threadIdx.x >> 5][k] = t;
+        }
+    }
     __syncthreads();
     if (threadIdx.x < NF) {
         double t = 0.0;
-        for (int b = 0; b < blocks; ++b) t += part[b * NF + threadIdx.x];
+        for (int w = 0; w < kStatBlocks / 32; ++w) t += ws[w][threadIdx.x];
         tot[threadIdx.x] = t;
     }
     __syncthreads();
@@ -178,58 +237,138 @@ __global__ void layer0_fwd(uint32_t n, const float *x, const float *W0, const fl
     }
 }
 
-// m(v) = mean over out-neighbours of h(u); one warp per vertex, 2 channels per
-// lane.  The rows are added in arc order (the sum's rounding does not depend
-// on the launch); a hub's chain is the latency of its row loads, so 32 of them
-// are in flight and the next 32 heads are read meanwhile (one row at a time
-// took 547 us a layer on a 2^15-vertex RMAT graph).
-constexpr int kRows = 32;
+// Vertices whose list is longer than kHubArcs are summed by a block each
+// (hub_sum below), the others by a warp each.
+constexpr uint32_t kHubArcs = 256;
+
+// the hubs of one direction: hubs[0] = their number, hubs[1..] the vertices
+__global__ void find_hubs(uint32_t n, const uint64_t *off, uint32_t *hubs) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        if (off[v + 1] - off[v] > kHubArcs) hubs[1 + atomicAdd(&hubs[0], 1u)] = v;
+}
+
+// Ordered sum of a hub's rows by one block: kHubRows rows at a time are
+// gathered into shared memory by all threads (the next ones while these are
+// added), and one thread per channel adds them in arc order -- the same
+// additions, in the same order, as one warp walking the list, whose time is
+// the latency of its row loads (a 2^15-vertex RMAT graph's hubs: 160 us a
+// layer forward with 32 rows in flight, 680 us backward with 16).
+// row(u, c): channel c of vertex u's row as a float2 pair of channels c, c + 1;
+// scale(u): the factor of its row; init(c), done(c, sum).
+constexpr int kHubThreads = 512;
+constexpr int kHubRows = 128;
+constexpr int kHubPairs = kHubRows * (H / 2) / kHubThreads;   // channel pairs per thread and step
+
+template <bool SCALED, typename Row, typename Scale>
+__device__ __forceinline__ float hub_sum(uint64_t b, uint64_t e, const uint32_t *head, float2 (*buf)[H / 2], float *fac,
+                                         uint32_t *idx, float sum, Row row, Scale scale) {
+    const uint32_t tid = threadIdx.x;
+    float2 t[kHubPairs];
+    float f = 0.f;
+    // heads of a step are read one step ahead of its rows
+    uint32_t hn = tid < kHubRows && b + tid < e ? head[b + tid] : 0u;
+    auto fetch = [&](uint64_t a) {
+        // idx holds the heads of rows [a, a + kHubRows)
+#pragma unroll
+        for (int q = 0; q < kHubPairs; ++q) {
+            const uint32_t r = (q * kHubThreads + tid) / (H / 2), c = (q * kHubThreads + tid) % (H / 2);
+            t[q] = a + r < e ? row(idx[r], 2 * c) : make_float2(0.f, 0.f);
+        }
+        if (SCALED && tid < kHubRows) f = a + tid < e ? scale(idx[tid]) : 0.f;
+    };
+    if (tid < kHubRows) idx[tid] = hn;
+    hn = tid < kHubRows && b + kHubRows + tid < e ? head[b + kHubRows + tid] : 0u;
+    __syncthreads();
+    fetch(b);
+    for (uint64_t a = b; a < e; a += kHubRows) {
+        __syncthreads();   // the rows before are added, idx is read
+#pragma unroll
+        for (int q = 0; q < kHubPairs; ++q) (&buf[0][0])[q * kHubThreads + tid] = t[q];
+        if (SCALED && tid < kHubRows) fac[tid] = f;
+        if (tid < kHubRows) idx[tid] = hn;
+        hn = tid < kHubRows && a + 2 * kHubRows + tid < e ? head[a + 2 * kHubRows + tid] : 0u;
+        __syncthreads();
+        if (a + kHubRows < e) fetch(a + kHubRows);
+        if (tid < H) {
+            const uint32_t cnt = e - a < kHubRows ? (uint32_t)(e - a) : (uint32_t)kHubRows;
+            const float *col = (const float *)&buf[0][0] + tid;
+#pragma unroll 16
+            for (uint32_t r = 0; r < cnt; ++r) {
+                if (SCALED) sum = __fmaf_rn(col[(size_t)r * H], fac[r], sum);
+                else sum = __fadd_rn(sum, col[(size_t)r * H]);
+            }
+        }
+    }
+    __syncthreads();
+    return sum;
+}
+
+// m(v) = mean over out-neighbours of h(u) of the hubs
+__global__ void __launch_bounds__(kHubThreads) hub_mean(const uint32_t *hubs, const uint64_t *off, const uint32_t *head,
+                                                        const __nv_bfloat16 *h, __nv_bfloat16 *m) {
+    __shared__ float2 buf[kHubRows][H / 2];
+    __shared__ uint32_t idx[kHubRows];
+    const uint32_t cnt = hubs[0];
+    for (uint32_t i = blockIdx.x; i < cnt; i += gridDim.x) {
+        const uint32_t v = hubs[1 + i];
+        const uint64_t b = off[v], e = off[v + 1];
+        const float s = hub_sum<false>(
+            b, e, head, buf, nullptr, idx, 0.f,
+            [&](uint32_t u, uint32_t c) {
+                const __nv_bfloat162 t = *(const __nv_bfloat162 *)(h + (size_t)u * H + c);
+                return make_float2(__bfloat162float(t.x), __bfloat162float(t.y));
+            },
+            [](uint32_t) { return 1.f; });
+        if (threadIdx.x < H) m[(size_t)v * H + threadIdx.x] = __float2bfloat16_rn(s * (1.f / (float)(e - b)));
+    }
+}
+
+// m(v) = mean over out-neighbours of h(u), hubs left out; 8 lanes per vertex,
+// 8 channels (16 bytes) each, so a warp has four vertices' rows on their way
+// and up to kRows of each.  Rows are added in arc order.  (A warp per vertex
+// with 4 bytes per lane: 89 us a layer on a 512-square grid, bound by the
+// chain offsets, heads, rows of one vertex after the other.)
+constexpr int kRows = 8;
 
 __global__ void aggregate_mean(uint32_t n, const uint64_t *off, const uint32_t *head, const __nv_bfloat16 *h,
                                __nv_bfloat16 *m) {
-    const uint32_t lane = lane_id();
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t v = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); v < n; v += warps) {
+    const uint32_t sub = threadIdx.x & 7u, gm = 0xFFu << (threadIdx.x & 24u);
+    const uint32_t groups = gridDim.x * (blockDim.x >> 3);
+    for (uint32_t v = blockIdx.x * (blockDim.x >> 3) + (threadIdx.x >> 3); v < n; v += groups) {
         const uint64_t b = off[v], e = off[v + 1];
-        float s0 = 0.f, s1 = 0.f;
-        uint32_t next = b + lane < e ? head[b + lane] : 0u;
+        if (e - b > kHubArcs) continue;
+        float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        uint32_t next = b + sub < e ? head[b + sub] : 0u;
         for (uint64_t a = b; a < e; a += kRows) {
             const uint32_t cnt = e - a < kRows ? (uint32_t)(e - a) : (uint32_t)kRows;
             const uint32_t hd = next;
-            next = a + kRows + lane < e ? head[a + kRows + lane] : 0u;
-            if (cnt == kRows) {
-                __nv_bfloat162 t[kRows];
+            next = a + kRows + sub < e ? head[a + kRows + sub] : 0u;
+            uint4 t[kRows];
 #pragma unroll
-                for (int q = 0; q < kRows; ++q)
-                    t[q] = *(const __nv_bfloat162 *)(h + (size_t)__shfl_sync(kFull, hd, q) * H + 2 * lane);
+            for (uint32_t q = 0; q < kRows; ++q) {
+                const uint32_t u = __shfl_sync(gm, hd, q, 8);
+                if (q < cnt) t[q] = *(const uint4 *)(h + (size_t)u * H + 8 * sub);
+            }
 #pragma unroll
-                for (int q = 0; q < kRows; ++q) {
-                    s0 += __bfloat162float(t[q].x);
-                    s1 += __bfloat162float(t[q].y);
-                }
-            } else {
-                for (uint32_t j = 0; j < cnt; j += 4) {
-                    __nv_bfloat162 t[4];
+            for (uint32_t q = 0; q < kRows; ++q) {
+                if (q < cnt) {
+                    const uint32_t w[4] = {t[q].x, t[q].y, t[q].z, t[q].w};
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const uint32_t u = __shfl_sync(kFull, hd, j + q);
-                        if (j + q < cnt) t[q] = *(const __nv_bfloat162 *)(h + (size_t)u * H + 2 * lane);
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        if (j + q < cnt) {
-                            s0 += __bfloat162float(t[q].x);
-                            s1 += __bfloat162float(t[q].y);
-                        }
+                    for (int c = 0; c < 4; ++c) {   // a BF16 is the high half of its FP32
+                        s[2 * c] += __uint_as_float(w[c] << 16);
+                        s[2 * c + 1] += __uint_as_float(w[c] & 0xFFFF0000u);
                     }
                 }
             }
         }
         const float inv = e > b ? 1.f / (float)(e - b) : 0.f;
-        __nv_bfloat162 o;
-        o.x = __float2bfloat16_rn(s0 * inv);
-        o.y = __float2bfloat16_rn(s1 * inv);
-        *(__nv_bfloat162 *)(m + (size_t)v * H + 2 * lane) = o;
+        uint32_t o[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const __nv_bfloat162 t = __floats2bfloat162_rn(s[2 * c] * inv, s[2 * c + 1] * inv);
+            o[c] = *(const uint32_t *)&t;
+        }
+        *(uint4 *)(m + (size_t)v * H + 8 * sub) = make_uint4(o[0], o[1], o[2], o[3]);
     }
 }
 
@@ -511,61 +650,72 @@ __global__ void inv_degree(uint32_t n, const uint64_t *off, float *inv) {
 
 // dh_prev(u) = dA[u, :64] + sum_{v: u in N(v)} dA[v, 64:] / deg(v), gathered
 // over u's in-arcs (the reverse of the out-neighbour mean) in arc order, and
-// dz_prev from it.  As in aggregate_mean, a hub's chain is the latency of its
-// row loads: 16 rows are in flight (1.87 ms a layer with one, on a
-// 2^15-vertex RMAT graph).
-constexpr int kBwdRows = 16;
+// dz_prev from it; hubs by hub_scatter.  16 lanes per vertex, 4 channels (16
+// bytes) each, 8 rows in flight.
+constexpr int kBwdRows = 8;
+
+__global__ void __launch_bounds__(kHubThreads) hub_scatter(const uint32_t *hubs, const float *dA, const uint64_t *off_in,
+                                                           const uint32_t *head_in, const float *inv_deg,
+                                                           const __nv_bfloat16 *h, float *dz, __nv_bfloat16 *dzb) {
+    __shared__ float2 buf[kHubRows][H / 2];
+    __shared__ float fac[kHubRows];
+    __shared__ uint32_t idx[kHubRows];
+    const uint32_t cnt = hubs[0];
+    for (uint32_t i = blockIdx.x; i < cnt; i += gridDim.x) {
+        const uint32_t u = hubs[1 + i], c = threadIdx.x;
+        const float own = c < H ? dA[(size_t)u * K2 + c] : 0.f;
+        const float s = hub_sum<true>(
+            off_in[u], off_in[u + 1], head_in, buf, fac, idx, own,
+            [&](uint32_t v, uint32_t k) { return *(const float2 *)(dA + (size_t)v * K2 + H + k); },
+            [&](uint32_t v) { return inv_deg[v]; });
+        if (c < H) {
+            const size_t at = (size_t)u * H + c;
+            const float z = __bfloat162float(h[at]) > 0.f ? s : 0.f;
+            dz[at] = z;
+            dzb[at] = __float2bfloat16_rn(z);
+        }
+    }
+}
 
 __global__ void scatter_mean_bwd(uint32_t n, const float *dA, const uint64_t *off_in, const uint32_t *head_in,
                                  const float *inv_deg, const __nv_bfloat16 *h, float *dz, __nv_bfloat16 *dzb) {
-    const uint32_t lane = lane_id();
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t u = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); u < n; u += warps) {
-        const float2 own = *(const float2 *)(dA + (size_t)u * K2 + 2 * lane);
-        float s0 = own.x, s1 = own.y;
+    const uint32_t sub = threadIdx.x & 15u, gm = 0xFFFFu << (threadIdx.x & 16u);
+    const uint32_t groups = gridDim.x * (blockDim.x >> 4);
+    for (uint32_t u = blockIdx.x * (blockDim.x >> 4) + (threadIdx.x >> 4); u < n; u += groups) {
         const uint64_t b = off_in[u], e = off_in[u + 1];
-        uint32_t next = b + lane < e ? head_in[b + lane] : 0u;
-        float inext = b + lane < e ? inv_deg[next] : 0.f;
-        for (uint64_t a = b; a < e; a += 32) {
-            const uint32_t cnt = e - a < 32 ? (uint32_t)(e - a) : 32u;
+        if (e - b > kHubArcs) continue;
+        float4 s = *(const float4 *)(dA + (size_t)u * K2 + 4 * sub);
+        // each lane of the group reads one of the next 16 heads and its factor
+        uint32_t next = b + sub < e ? head_in[b + sub] : 0u;
+        float inext = b + sub < e ? inv_deg[next] : 0.f;
+        for (uint64_t a = b; a < e; a += 16) {
+            const uint32_t cnt = e - a < 16 ? (uint32_t)(e - a) : 16u;
             const uint32_t hd = next;
             const float iv = inext;
-            next = a + 32 + lane < e ? head_in[a + 32 + lane] : 0u;
-            inext = a + 32 + lane < e ? inv_deg[next] : 0.f;
-            if (cnt == 32) {
+            next = a + 16 + sub < e ? head_in[a + 16 + sub] : 0u;
+            inext = a + 16 + sub < e ? inv_deg[next] : 0.f;
+            for (uint32_t j = 0; j < cnt; j += kBwdRows) {
+                float4 t[kBwdRows];
 #pragma unroll
-                for (int j = 0; j < 32; j += kBwdRows) {
-                    float2 t[kBwdRows];
-#pragma unroll
-                    for (int q = 0; q < kBwdRows; ++q)
-                        t[q] = *(const float2 *)(dA + (size_t)__shfl_sync(kFull, hd, j + q) * K2 + H + 2 * lane);
-#pragma unroll
-                    for (int q = 0; q < kBwdRows; ++q) {
-                        const float w = __shfl_sync(kFull, iv, j + q);
-                        s0 += t[q].x * w;
-                        s1 += t[q].y * w;
-                    }
+                for (uint32_t q = 0; q < kBwdRows; ++q) {
+                    const uint32_t v = __shfl_sync(gm, hd, j + q, 16);
+                    if (j + q < cnt) t[q] = *(const float4 *)(dA + (size_t)v * K2 + H + 4 * sub);
                 }
-            } else {
-                for (uint32_t j = 0; j < cnt; j += 4) {
-                    float2 t[4];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const uint32_t v = __shfl_sync(kFull, hd, j + q);
-                        if (j + q < cnt) t[q] = *(const float2 *)(dA + (size_t)v * K2 + H + 2 * lane);
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const float w = __shfl_sync(kFull, iv, j + q);
-                        if (j + q < cnt) {
-                            s0 += t[q].x * w;
-                            s1 += t[q].y * w;
-                        }
+                for (uint32_t q = 0; q < kBwdRows; ++q) {
+                    const float w = __shfl_sync(gm, iv, j + q, 16);
+                    if (j + q < cnt) {
+                        s.x = __fmaf_rn(t[q].x, w, s.x);
+                        s.y = __fmaf_rn(t[q].y, w, s.y);
+                        s.z = __fmaf_rn(t[q].z, w, s.z);
+                        s.w = __fmaf_rn(t[q].w, w, s.w);
                     }
                 }
             }
         }
-        store_dz((size_t)u * H + 2 * lane, s0, s1, h, dz, dzb);
+        const size_t at = (size_t)u * H + 4 * sub;
+        store_dz(at, s.x, s.y, h, dz, dzb);
+        store_dz(at + 2, s.z, s.w, h, dz, dzb);
     }
 }
 
@@ -667,6 +817,7 @@ struct GraphDev {
     TmpSet tmp;
     uint64_t *off_out = nullptr, *off_in = nullptr;
     uint32_t *head_out = nullptr, *head_in = nullptr;
+    uint32_t *hubs_out = nullptr, *hubs_in = nullptr;   // find_hubs of each direction
     uint32_t n = 0;
 };
 
@@ -674,20 +825,26 @@ int upload_csr(const chl_graph *g, GraphDev &d) {
     const uint32_t n = g->n;
     d.n = n;
     int rc;
-    auto put = [&](int f, uint64_t **off, uint32_t **head) -> int {
+    auto put = [&](int f, uint64_t **off, uint32_t **head, uint32_t **hubs) -> int {
         const uint64_t m = g->off[f][n];
         if ((rc = d.tmp.get(off, (uint64_t)n + 1)) || (rc = d.tmp.get(head, m))) return rc;
         CHL_CUDA(cudaMemcpy(*off, g->off[f].data(), ((size_t)n + 1) * 8, cudaMemcpyHostToDevice));
         if (m) CHL_CUDA(cudaMemcpy(*head, g->head[f].data(), m * 4, cudaMemcpyHostToDevice));
+        // at most m / kHubArcs lists are longer than kHubArcs
+        if ((rc = d.tmp.get(hubs, m / kHubArcs + 1))) return rc;
+        CHL_CUDA(cudaMemset(*hubs, 0, 4));
+        find_hubs<<<device_sms(), 256>>>(n, *off, *hubs);
+        CHL_CUDA(cudaGetLastError());
         return CHL_OK;
     };
-    if ((rc = put(1, &d.off_out, &d.head_out))) return rc;
+    if ((rc = put(1, &d.off_out, &d.head_out, &d.hubs_out))) return rc;
     if (g->symmetric) {
         d.off_in = d.off_out;
         d.head_in = d.head_out;
+        d.hubs_in = d.hubs_out;
         return CHL_OK;
     }
-    return put(0, &d.off_in, &d.head_in);
+    return put(0, &d.off_in, &d.head_in, &d.hubs_in);
 }
 
 // standardise the feature columns of M->x in place; M->acc holds the partials
@@ -722,7 +879,7 @@ int forward(chl_gnn *M, const GraphDev &G, uint64_t seed) {
     const uint32_t n = G.n;
     const int sms = device_sms();
     feat_raw<<<sms * 4, 256>>>(n, G.off_out, G.head_out, G.off_in,
-                               seed, M->x.as<float>());
+                               seed, feat_vpw(n, sms), M->x.as<float>());
     CHL_CUDA(cudaGetLastError());
     int rc = standardise(M, n);
     if (rc) return rc;
@@ -734,6 +891,7 @@ int forward(chl_gnn *M, const GraphDev &G, uint64_t seed) {
         const __nv_bfloat16 *hp = hb + (size_t)(l - 1) * n * H;
         __nv_bfloat16 *ml = mb + (size_t)l * n * H;
         aggregate_mean<<<sms * 8, 256>>>(n, G.off_out, G.head_out, hp, ml);
+        hub_mean<<<sms * 2, kHubThreads>>>(G.hubs_out, G.off_out, G.head_out, hp, ml);
         gemm_rows<K2><<<gemm_grid<K2>(sms), 128>>>(n, hp, ml, W, W + (size_t)K2 * H, 0, hb + (size_t)l * n * H, nullptr, 0);
     }
     const float *wout = P + kP0 + (size_t)M->layers * kPL;
@@ -773,8 +931,9 @@ int backward(chl_gnn *M, const GraphDev &G, double *loss) {
         gemm_rows<H><<<gemm_grid<H>(sms), 128>>>(n, mb, mb, M->wt.as<float>(), nullptr, 1, nullptr, M->dA.as<float>(), K2);
         gemm_rows<H><<<gemm_grid<H>(sms), 128>>>(n, mb, mb, M->wt.as<float>() + H * H, nullptr, 1, nullptr,
                                        M->dA.as<float>() + H, K2);
-        scatter_mean_bwd<<<sms * 8, 256>>>(n, M->dA.as<float>(), G.off_in, G.head_in,
-                                           M->inv.as<float>(), hp, dz, mb);
+        scatter_mean_bwd<<<sms * 8, 256>>>(n, M->dA.as<float>(), G.off_in, G.head_in, M->inv.as<float>(), hp, dz, mb);
+        hub_scatter<<<sms * 2, kHubThreads>>>(G.hubs_in, M->dA.as<float>(), G.off_in, G.head_in, M->inv.as<float>(),
+                                              hp, dz, mb);
     }
     CHL_CUDA(cudaMemset(M->acc.p, 0, kAccBytes));
     grad_w0<<<std::max(1, std::min(sms, (int)((n + 63) / 64))), kGw0Threads>>>(n, M->x.as<float>(), dz, M->acc.as<double>());
@@ -837,7 +996,7 @@ extern "C" int chl_gnn_features(const chl_graph *g, uint64_t seed, float *x) {
     int rc;
     if ((rc = upload_csr(g, G)) || (rc = tmp.x.ensure((size_t)g->n * NF * 4))) return rc;
     feat_raw<<<device_sms() * 4, 256>>>(g->n, G.off_out, G.head_out,
-                                        G.off_in, seed, tmp.x.as<float>());
+                                        G.off_in, seed, feat_vpw(g->n, device_sms()), tmp.x.as<float>());
     CHL_CUDA(cudaGetLastError());
     if ((rc = standardise(&tmp, g->n))) return rc;
     CHL_CUDA(cudaMemcpy(x, tmp.x.p, (size_t)g->n * NF * 4, cudaMemcpyDeviceToHost));

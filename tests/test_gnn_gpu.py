@@ -258,3 +258,35 @@ def test_hub_degrees_at_the_row_group_edges(P, n):
     assert abs(loss - l_emu) <= 1e-4 * l_emu
     for bname, sl in blocks(LAYERS):
         assert np.linalg.norm(grad[sl] - g_emu[sl]) <= EMU_REL * max(np.linalg.norm(g_emu[sl]), 1e-6), bname
+
+
+@pytest.mark.parametrize("into", [False, True])
+def test_hubs_summed_by_blocks(P, into):
+    """Lists at the edges of the hub rule (more than 256 arcs) and of a
+    block's 128-row steps, in one direction only and (symmetric) in both."""
+    n = 3000
+    src, dst = [], []
+    for hub, deg in enumerate((255, 256, 257, 383, 384, 385, 512, 1700)):
+        for j in range(deg):
+            src.append(hub)
+            dst.append(20 + (hub * 131 + j) % (n - 20))
+    if into:
+        src, dst = dst, src
+    rng = np.random.default_rng(6)
+    p = R.init_params(LAYERS, seed=8)
+    p += rng.normal(0, 0.02, p.size).astype(np.float32)
+    y = rng.normal(0, 1, n).astype(np.float32)
+    for undirected in (False, True):
+        g = P.Graph.from_arcs(n, src, dst, [1] * len(src), undirected=undirected)
+        c = csr4(g)
+        net = P.RankNet(LAYERS, seed=1)
+        net.set_params(p)
+        x = P.RankNet.features(g, seed=9)
+        assert np.allclose(x, R.features(c[0], c[1], c[2], seed=9), atol=2e-5, rtol=1e-5)
+        csr = R.csr_of(*c)
+        assert rel(net.predict(g, seed=9), R.forward(p, LAYERS, x, csr, emulate=True)[0]) < EMU_REL
+        loss, grad = net.grad(g, y, seed=9)
+        l_emu, g_emu = R.loss_and_grad(p, LAYERS, x, csr, y, emulate=True)
+        assert abs(loss - l_emu) <= 1e-4 * l_emu
+        for bname, sl in blocks(LAYERS):
+            assert rel(grad[sl], g_emu[sl]) < EMU_REL, bname
