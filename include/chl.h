@@ -167,8 +167,9 @@ enum chl_build_mode {
 typedef struct chl_build_opts {
     int32_t mode;         /* chl_build_mode                                  */
     double sf;            /* superstep label budget factor (hhl -s), 0 = auto
-                             (32 on heavy-tailed graphs; on road-like ones
-                             what the label buffer holds, 1024 in GLL mode) */
+                             (32 on heavy-tailed graphs, 512 if their lengths
+                             are all 1; on road-like ones what the label
+                             buffer holds, 1024 in GLL mode)                */
     double ps;            /* phase switch ratio tree/label (hhl -ps), 0 =
                              auto: 1024 (the reference's default) on road-
                              like graphs, 8 on heavy-tailed ones          */

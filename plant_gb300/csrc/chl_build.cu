@@ -35,6 +35,7 @@
 #include <chrono>
 #include <type_traits>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <memory>
 #include <vector>
@@ -1539,6 +1540,235 @@ TreeKernel team_kernel_for(bool unit, bool plant, bool prune, uint32_t tw) {
     return plant ? team_kernel_pr<false, true>(prune, tw) : team_kernel_pr<false, false>(prune, tw);
 }
 
+// ------------------------------------------------------ bit-parallel trees
+//
+// Unit lengths: the trees of kBitRoots roots are searched together, a level
+// at a time, one bit per root.  A vertex's row of kBitWords words holds the
+// roots that reached it in the last level, and those of them by a via path.
+// A level pulls: vertex w ORs its in-neighbours' rows, keeps the roots that
+// have not seen w, marks as via those with a via predecessor or ranked below
+// w (update_wo_prune's flag: every shortest-path predecessor is in the last
+// level), drops those with a committed witness, and emits a label for each
+// that is left and not via.  The witness test reads L(w) once for all roots:
+// an entry (h, dh) prunes the roots within d - dh of h, one row of the table
+// M[h][.] of the batch's own committed labels.  A root whose level has no
+// not-via vertex is done (plant :95).
+// Rows of 16 lanes x 16 bytes make every gather coalesced; a batch moves each
+// arc's row once per level instead of once per root and level.  RMAT scale 17:
+// the first 1,024 roots take 0.76 ms where their trees took 24, the next 2,048
+// (pruned) 2.1 where theirs took 6.
+constexpr int kBitWords = 16;
+constexpr uint32_t kBitRoots = 64 * kBitWords;
+constexpr uint32_t kBitHeavy = 512;       // longer lists are pulled by a block each
+constexpr int kBitThreads = 256;
+constexpr int kBitGroups = kBitThreads / kBitWords;
+constexpr uint32_t kBitLevels = 64;       // more levels than this: the other kernels
+constexpr uint32_t kBitDist = 32;         // largest committed distance the table takes, exclusive
+
+struct BitArgs {
+    uint32_t n;
+    int sides, f;                   // trees of side f: rows are pulled over the reverse arcs
+    const uint64_t *roff;
+    const uint2 *rhead;
+    const uint32_t *order, *rank;
+    const uint64_t *l_off;
+    const uint2 *l_ent, *l_dent;
+    uint32_t r0, rb, nb;            // superstep's first root, batch's first root and size
+    uint32_t d;                     // level
+    uint32_t K;                     // table distances 0 .. K - 1 (K - 1 the largest committed one)
+    const ulonglong2 *cur;          // (reached, via) per vertex and word
+    ulonglong2 *nxt;
+    unsigned long long *seen;
+    const uint8_t *act;             // rows of cur that are set
+    uint8_t *act_out;
+    const unsigned long long *live; // roots with a not-via vertex in the last level
+    unsigned long long *live_out;
+    unsigned long long *M;
+    const uint32_t *heavy;          // heavy[0]: number of long lists, then their vertices
+    int hub_bits;
+    uint64_t *out_key;
+    uint32_t *out_val;
+    unsigned long long out_cap;
+    BuildCtl *ctl;
+};
+
+__global__ void bit_heavy(uint32_t n, const uint64_t *off, uint32_t *heavy) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
+        if (off[v + 1] - off[v] > kBitHeavy) heavy[1 + atomicAdd(&heavy[0], 1u)] = v;
+}
+
+// labels of the bits of nv for vertex w, by 16 lanes (mask gm, lane's word wd)
+__device__ __forceinline__ void bit_emit(const BitArgs &a, uint32_t gm, uint32_t wd, uint32_t w, unsigned long long nv) {
+    const uint32_t c = (uint32_t)__popcll(nv);
+    uint32_t incl = c;
+#pragma unroll
+    for (int o = 1; o < kBitWords; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(gm, incl, o, kBitWords);
+        if (wd >= (uint32_t)o) incl += y;
+    }
+    const uint32_t total = __shfl_sync(gm, incl, kBitWords - 1, kBitWords);
+    if (total == 0) return;
+    unsigned long long b = 0;
+    if (wd == 0) b = atomicAdd(&a.ctl->nlab, (unsigned long long)total);
+    b = __shfl_sync(gm, b, 0, kBitWords) + (incl - c);
+    const uint64_t list = (uint64_t)lidx(w, 1 - a.f, a.sides) << a.hub_bits;
+    const uint32_t rel = a.rb - a.r0 + 64u * wd;
+    for (; nv; nv &= nv - 1, ++b) {
+        if (b < a.out_cap) {
+            a.out_key[b] = list | (uint64_t)(rel + (uint32_t)__ffsll((long long)nv) - 1u);
+            a.out_val[b] = a.d;
+        } else {
+            a.ctl->overflow = 1;
+        }
+    }
+}
+
+// the batch's roots at level 0, 16 lanes each
+__global__ void bit_roots(BitArgs a) {
+    const uint32_t wd = threadIdx.x % kBitWords, gm = 0xFFFFu << (threadIdx.x & 16u);
+    const uint32_t i = blockIdx.x * kBitGroups + threadIdx.x / kBitWords;
+    if (i >= a.nb) return;
+    const uint32_t v = a.order[a.rb + i];
+    const unsigned long long bit = wd == i / 64 ? 1ull << (i % 64) : 0ull;
+    a.nxt[(size_t)v * kBitWords + wd] = make_ulonglong2(bit, 0ull);
+    a.seen[(size_t)v * kBitWords + wd] = bit;
+    if (bit) atomicOr(&a.live_out[wd], bit);
+    if (wd == 0) a.act_out[v] = 1;
+    bit_emit(a, gm, wd, v, bit);
+}
+
+// M[h][k] = roots of the batch within distance k of committed hub h; a warp per root
+__global__ void bit_table(BitArgs a) {
+    const uint32_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (i >= a.nb) return;
+    const uint32_t x = lidx(a.order[a.rb + i], a.f, a.sides);
+    const unsigned long long bit = 1ull << (i % 64);
+    for (uint64_t e = a.l_off[x] + lane_id(); e < a.l_off[x + 1]; e += 32) {
+        const uint2 q = a.l_ent[e];
+        for (uint32_t k = q.y; k < a.K; ++k) atomicOr(&a.M[((size_t)q.x * a.K + k) * kBitWords + i / 64], bit);
+    }
+}
+
+// One level.  HEAVY: a block per long list, its 16 groups of 16 lanes taking
+// every 16th arc group; otherwise 16 lanes per vertex.
+template <bool HEAVY, bool PRUNE>
+__global__ void __launch_bounds__(kBitThreads) bit_level(BitArgs a) {
+    __shared__ unsigned long long s_acc[kBitGroups][kBitWords], s_via[kBitGroups][kBitWords];
+    const uint32_t wd = threadIdx.x % kBitWords, grp = threadIdx.x / kBitWords;
+    const uint32_t gm = 0xFFFFu << (threadIdx.x & 16u);
+    const uint32_t items = HEAVY ? a.heavy[0] : a.n;
+    const unsigned long long live = a.live[wd];
+    const unsigned long long valid =
+        a.nb >= 64u * wd + 64u ? ~0ull : (a.nb > 64u * wd ? (1ull << (a.nb - 64u * wd)) - 1ull : 0ull);
+    unsigned long long c_new = 0, c_reads = 0, nv_any = 0;
+    const uint32_t step = HEAVY ? gridDim.x : gridDim.x * kBitGroups;
+    for (uint32_t it = HEAVY ? blockIdx.x : blockIdx.x * kBitGroups + grp; it < items; it += step) {
+        const uint32_t w = HEAVY ? a.heavy[1 + it] : it;
+        const uint64_t b = a.roff[w], e = a.roff[w + 1];
+        if (!HEAVY && e - b > kBitHeavy) continue;
+        const uint32_t rw = a.rank[w];
+        unsigned long long acc = 0, via = 0, seen = 0;
+        // a vertex ranked above the superstep's roots always has a committed witness
+        const bool skip = PRUNE && rw < a.r0;
+        if (!skip) {
+            seen = a.seen[(size_t)w * kBitWords + wd];
+            // roots ranked below w reach it by a via path
+            const int64_t t = (int64_t)rw - (int64_t)a.rb - 64ll * wd;
+            via = t < 0 ? ~0ull : t >= 63 ? 0ull : ~0ull << (t + 1);
+            const unsigned long long want = valid & ~seen & live;
+            // heads and their flags 16 at a time, the set rows 4 at a time; done
+            // once every wanted root has arrived by a via path
+            const uint64_t first = b + (HEAVY ? (uint64_t)grp * kBitWords : 0), stride = HEAVY ? kBitThreads : kBitWords;
+            if (__any_sync(gm, want != 0)) {
+                uint32_t hn = first + wd < e ? a.rhead[first + wd].x : 0u;
+                for (uint64_t q = first; q < e; q += stride) {
+                    const uint32_t hd = hn;
+                    const bool on = q + wd < e && a.act[hd];
+                    hn = q + stride + wd < e ? a.rhead[q + stride + wd].x : 0u;
+                    uint32_t m = __ballot_sync(gm, on) >> (threadIdx.x & 16u) & 0xFFFFu;
+                    if (!m) continue;
+                    while (m) {
+                        ulonglong2 r[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            r[u] = make_ulonglong2(0ull, 0ull);
+                            const uint32_t x = __shfl_sync(gm, hd, m ? __ffs(m) - 1 : 0, kBitWords);
+                            if (m) r[u] = a.cur[(size_t)x * kBitWords + wd];
+                            m &= m - 1;
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            acc |= r[u].x;
+                            via |= r[u].y;
+                        }
+                    }
+                    if (!__any_sync(gm, (want & ~(acc & via)) != 0)) break;
+                }
+            }
+            acc &= want;
+        }
+        if (HEAVY) {
+            s_acc[grp][wd] = acc;
+            s_via[grp][wd] = via;
+            __syncthreads();
+            if (grp == 0) {
+#pragma unroll
+                for (int g = 1; g < kBitGroups; ++g) {
+                    acc |= s_acc[g][wd];
+                    via |= s_via[g][wd];
+                }
+            }
+            __syncthreads();
+        }
+        if (!HEAVY || grp == 0) {
+            unsigned long long left = acc;
+            if (PRUNE && !skip && __any_sync(gm, left != 0)) {
+                const uint32_t x = lidx(w, 1 - a.f, a.sides);
+                const uint64_t le = a.l_off[x + 1];
+                // entries 16 at a time (their list is in distance order), 4 table rows in flight
+                for (uint64_t q = a.l_off[x]; q < le; q += kBitWords) {
+                    const uint2 en = q + wd < le ? a.l_dent[q + wd] : make_uint2(0u, 0xFFFFFFFFu);
+                    const uint32_t cnt = (uint32_t)__popc(__ballot_sync(gm, en.y <= a.d));
+                    const size_t row = ((size_t)en.x * a.K + min(a.d - min(en.y, a.d), a.K - 1)) * kBitWords;
+                    for (uint32_t j = 0; j < cnt; j += 4) {
+                        unsigned long long p[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const size_t rr = __shfl_sync(gm, row, (j + u) & (kBitWords - 1), kBitWords);
+                            p[u] = j + u < cnt ? a.M[rr + wd] : 0ull;
+                        }
+                        left &= ~(p[0] | p[1] | p[2] | p[3]);
+                    }
+                    if (wd == 0) c_reads += cnt;
+                    if (cnt < kBitWords || !__any_sync(gm, left != 0)) break;
+                }
+            }
+            c_new += (unsigned long long)__popcll(acc);
+            const bool any = __any_sync(gm, left != 0);
+            if (__any_sync(gm, acc != 0)) a.seen[(size_t)w * kBitWords + wd] = seen | acc;
+            if (wd == 0) a.act_out[w] = any ? 1 : 0;
+            if (any) {
+                a.nxt[(size_t)w * kBitWords + wd] = make_ulonglong2(left, left & via);
+                const unsigned long long nv = left & ~via;
+                nv_any |= nv;
+                bit_emit(a, gm, wd, w, nv);
+            }
+        }
+    }
+    // totals and the roots still live, one atomic per warp
+    nv_any |= __shfl_xor_sync(kFull, nv_any, 16);
+    if (lane_id() < kBitWords && (nv_any & ~*(volatile unsigned long long *)&a.live_out[wd])) atomicOr(&a.live_out[wd], nv_any);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        c_new += __shfl_xor_sync(kFull, c_new, o);
+        c_reads += __shfl_xor_sync(kFull, c_reads, o);
+    }
+    if (lane_id() == 0) {
+        if (c_new) atomicAdd(&a.ctl->visits, c_new);
+        if (c_reads) atomicAdd(&a.ctl->label_reads, c_reads);
+    }
+}
+
 __global__ void fat_arcs(uint64_t m, const uint2 *arc, const uint32_t *rank, const uint32_t *win, uint4 *out) {
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
         const uint2 a = arc[e];
@@ -2180,6 +2410,12 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         b.hash_max = t;
     }
 
+    // bit-parallel first supersteps: unit lengths and few levels (see
+    // bit_level); rows of cur, nxt and seen and two flags per vertex, in the
+    // trees' workspace
+    const size_t bit_row = (size_t)n * kBitWords;
+    bool bits_ok = unit && heavy_tail && win_target > 1 && opts.max_warps == 0 &&
+                   ws_words * 4 >= bit_row * (2 * sizeof(ulonglong2) + 8) + 2 * (size_t)n;
     // superstep loop
     // label budget per superstep (the reference's sf * N); auto: 32 on
     // heavy-tailed graphs, 1024 on road-like ones.  On road-like graphs a
@@ -2189,7 +2425,9 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     // not the budget, sets their size (measured on the 512/1024-square
     // grids: 1024 and unbounded within 1%, 128 1.27x slower; RMAT scale
     // 20: 16-64 within 3%)
-    const double sf = opts.sf > 0 ? opts.sf : (heavy_tail ? 32.0 : 1024.0);
+    // (bit-parallel supersteps have no largest tree to wait for and pay for
+    // every commit: RMAT scale 20 342 ms with 128, 309 with 512)
+    const double sf = opts.sf > 0 ? opts.sf : bits_ok ? 512.0 : heavy_tail ? 32.0 : 1024.0;
     // label_limit = sf * N counts both sides' labels (shared_memory/hhl.cpp:65);
     // a symmetric build stores one side.
     unsigned long long budget_base =
@@ -2215,10 +2453,20 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         // beyond that an overflow re-runs the superstep's root range.
         size_t fr = 0, tot = 0;
         CHL_CUDA(cudaMemGetInfo(&fr, &tot));
-        const uint64_t want = (uint64_t)budget_base + (uint64_t)std::max(b.slots, b.win_trees) * b.sides * n;
+        // Bit-parallel batches end a superstep exactly; the trees after them
+        // label a few vertices each, so room for 64 whole ones is kept.
+        const uint64_t running = bits_ok ? 64u : std::max(b.slots, b.win_trees);
+        const uint64_t want = (uint64_t)budget_base + running * b.sides * n;
         const uint64_t fit = (uint64_t)(fr / 4 / 36);
         if ((rc = grow_new(b, std::max<uint64_t>(std::min(want, fit), std::max<uint64_t>(4ull * n, 1u << 20))))) return rc;
     }
+    uint32_t *bit_long[2] = {nullptr, nullptr};   // long lists of each direction
+    unsigned long long *bit_live = nullptr;       // kBitLevels + 1 rows
+    uint32_t dist_hi = 0;                         // largest committed distance
+    uint32_t bit_hi = 0;                          // and of the superstep's labels
+    uint32_t bit_steps = 0;                       // supersteps built bit-parallel
+    double bit_mean = 0;                          // vertices a root of the last batch reached
+    constexpr double kBitShare = 10, kBitShareNext = 7;
     bool do_plant = opts.mode != CHL_MODE_GLL;
     bool switch_open = opts.mode == CHL_MODE_HYBRID;
     uint32_t r0 = 0;
@@ -2236,23 +2484,146 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     // yet committed (their labels prune everything later), geometric after.
     // The label budget sf * n (the reference's label_limit) also ends a
     // superstep early.
-    // Heavy-tailed degree distributions start with two roots per SM (RMAT
+    // Bit-parallel graphs start with two batches and treble (RMAT scale 17
+    // doubling 14.2 ms, trebling 13.2; scale 20 315 and 307).  Other
+    // heavy-tailed degree distributions start with two roots per SM (RMAT
     // scale 17: 47.6 ms with 304, 55 with 152, 68 with 1,216; a directed
     // skewed graph of 2^15 vertices 14 ms with 304, 20 with 1,216) and
     // double, so the hubs commit before the bulk of the trees; bounded-degree
     // graphs outside the whole rule start with two roots per warp of the
     // schedule and grow by half of the committed prefix.
-    const uint32_t auto_first = heavy_tail ? (win_target > 1 ? std::max<uint32_t>(64u, 2u * sms) : 1024u)
+    const uint32_t auto_first = bits_ok ? 2 * kBitRoots : heavy_tail ? (win_target > 1 ? std::max<uint32_t>(64u, 2u * sms) : 1024u)
                                            : std::max<uint32_t>(64u, 2 * b.warps);
-    const double auto_growth = heavy_tail ? 2.0 : 0.5;
+    const double auto_growth = bits_ok ? 3.0 : heavy_tail ? 2.0 : 0.5;
     // phase switch ratio (the reference's -ps, default 1024): auto 8 on
     // heavy-tailed graphs (RMAT scale 20: pruned GLL supersteps after the
     // first are faster than PLaNT trees there)
     const double ps = opts.ps > 0 ? opts.ps : (heavy_tail ? 8.0 : 1024.0);
     const uint32_t first = opts.first_superstep ? opts.first_superstep : auto_first;
     const double growth = opts.growth > 0 ? opts.growth : auto_growth;
+    // The roots [r0, r_end) by bit_level, a batch at a time until the label
+    // budget is spent; *done: the first root not taken, *deep: gave up at
+    // kBitLevels.  The host reads the live roots after each level.
+    auto bit_superstep = [&](unsigned long long budget, uint32_t r_end, uint32_t *done, bool *deep) -> int {
+        if (!bit_live) {
+            if ((rc = b.mem->get(&bit_live, (uint64_t)(kBitLevels + 1) * kBitWords))) return rc;
+            for (int f = 0; f < b.sides; ++f) {
+                const int rev = b.sides == 1 ? 1 : 1 - f;
+                const uint64_t m = g->off[g->symmetric ? 1 : rev][n];
+                if ((rc = b.mem->get(&bit_long[f], m / kBitHeavy + 1))) return rc;
+                CHL_CUDA(cudaMemsetAsync(bit_long[f], 0, 4, b.st));
+                bit_heavy<<<sms, 256, 0, b.st>>>(n, b.dg->off[rev], bit_long[f]);
+                CHL_CUDA(cudaGetLastError());
+                ++kernels;
+            }
+        }
+        b.ws_layout = 0;
+        ulonglong2 *rows[2] = {(ulonglong2 *)b.ws_all, (ulonglong2 *)b.ws_all + bit_row};
+        unsigned long long *seen = (unsigned long long *)(rows[1] + bit_row);
+        uint8_t *act[2] = {(uint8_t *)(seen + bit_row), (uint8_t *)(seen + bit_row) + n};
+        const uint32_t K = dist_hi + 1;
+        unsigned long long *M = nullptr;
+        if (r0 && (rc = b.mem->get(&M, (uint64_t)r0 * K * kBitWords))) return rc;
+        CHL_CUDA(cudaMemsetAsync(b.tsize + 0, 0, (size_t)(r_end - r0) * 4, b.st));
+        CHL_CUDA(cudaMemsetAsync(b.tlab + 0, 0, (size_t)(r_end - r0) * 4, b.st));
+        uint32_t rb = r0;
+        unsigned long long used = 0, visited = 0;
+        bit_mean = (double)n;
+        // (a re-run takes the same roots whatever they reach)
+        for (; rb < r_end && used < budget && (bit_mean * kBitShare >= n || budget == ~0ull); rb += kBitRoots) {
+            const uint32_t nb = std::min(kBitRoots, r_end - rb);
+            uint32_t last_level = 0;
+            for (int sd = 0; sd < b.sides; ++sd) {
+                const int f = b.sides == 1 ? 1 : sd, rev = b.sides == 1 ? 1 : 1 - f;
+                BitArgs a;
+                a.n = n;
+                a.sides = b.sides;
+                a.f = f;
+                a.roff = b.dg->off[rev];
+                a.rhead = b.fhead[rev];
+                a.order = b.order;
+                a.rank = b.rank;
+                a.l_off = b.off_a;
+                a.l_ent = b.ent_a;
+                a.l_dent = b.dent_a;
+                a.r0 = r0;
+                a.rb = rb;
+                a.nb = nb;
+                a.d = 0;
+                a.K = K;
+                a.seen = seen;
+                a.M = M;
+                a.heavy = bit_long[b.sides == 1 ? 0 : f];
+                a.hub_bits = b.hub_bits;
+                a.out_key = b.nk0;
+                a.out_val = b.nv0;
+                a.out_cap = b.new_cap;
+                a.ctl = b.ctl;
+                CHL_CUDA(cudaMemsetAsync(seen, 0, bit_row * 8, b.st));
+                CHL_CUDA(cudaMemsetAsync(act[0], 0, n, b.st));
+                CHL_CUDA(cudaMemsetAsync(bit_live, 0, (size_t)(kBitLevels + 1) * kBitWords * 8, b.st));
+                a.cur = rows[1];
+                a.nxt = rows[0];
+                a.act = act[1];
+                a.act_out = act[0];
+                a.live = bit_live;
+                a.live_out = bit_live;
+                bit_roots<<<(nb + kBitGroups - 1) / kBitGroups, kBitThreads, 0, b.st>>>(a);
+                if (r0) {
+                    CHL_CUDA(cudaMemsetAsync(M, 0, (size_t)r0 * K * kBitWords * 8, b.st));
+                    bit_table<<<(nb + 7) / 8, 256, 0, b.st>>>(a);
+                }
+                CHL_CUDA(cudaGetLastError());
+                kernels += r0 ? 2 : 1;
+                ++launches;
+                for (uint32_t d = 1;; ++d) {
+                    if (d > kBitLevels) {
+                        *deep = true;
+                        b.mem->put(M);
+                        return CHL_OK;
+                    }
+                    a.d = d;
+                    a.cur = rows[(d - 1) & 1];
+                    a.nxt = rows[d & 1];
+                    a.act = act[(d - 1) & 1];
+                    a.act_out = act[d & 1];
+                    a.live = bit_live + (size_t)(d - 1) * kBitWords;
+                    a.live_out = bit_live + (size_t)d * kBitWords;
+                    if (r0) {
+                        bit_level<true, true><<<sms * 4, kBitThreads, 0, b.st>>>(a);
+                        bit_level<false, true><<<sms * 8, kBitThreads, 0, b.st>>>(a);
+                    } else {
+                        bit_level<true, false><<<sms * 4, kBitThreads, 0, b.st>>>(a);
+                        bit_level<false, false><<<sms * 8, kBitThreads, 0, b.st>>>(a);
+                    }
+                    CHL_CUDA(cudaGetLastError());
+                    kernels += 2;
+                    unsigned long long live[kBitWords], any = 0;
+                    CHL_CUDA(cudaMemcpyAsync(live, a.live_out, sizeof(live), cudaMemcpyDeviceToHost, b.st));
+                    CHL_CUDA(cudaStreamSynchronize(b.st));
+                    for (unsigned long long x : live) any |= x;
+                    last_level = std::max(last_level, any ? d : d - 1);
+                    if (!any) break;
+                }
+            }
+            // labels reach the last level with a not-via vertex
+            unsigned long long tot[2] = {0, 0};
+            static_assert(offsetof(BuildCtl, visits) == offsetof(BuildCtl, nlab) + 8, "read together");
+            CHL_CUDA(cudaMemcpyAsync(tot, &b.ctl->nlab, 16, cudaMemcpyDeviceToHost, b.st));
+            CHL_CUDA(cudaStreamSynchronize(b.st));
+            used = tot[0];
+            bit_mean = (double)(tot[1] - visited) / nb;
+            visited = tot[1];
+            bit_hi = std::max(bit_hi, last_level);
+            CHL_CUDA(cudaMemcpyAsync(&b.ctl->max_dist, &bit_hi, 4, cudaMemcpyHostToDevice, b.st));
+        }
+        *done = std::min(rb, r_end);
+        b.mem->put(M);
+        return CHL_OK;
+    };
     while (r0 < n && (opts.root_limit == 0 || r0 < opts.root_limit)) {
         const uint32_t r_begin = r0;
+        bit_hi = 0;
         const bool plant_now = do_plant;
         const unsigned long long budget = budget_base;
         // trees without prune tests, over all roots that are left
@@ -2270,10 +2641,45 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         uint32_t hash_slots = 64;
         while (hash_slots < 2 * std::max<uint32_t>(max_list, 32) && 2 * hash_slots <= b.hash_max) hash_slots *= 2;
         const size_t smem = kWarpsPerBlock * batch_smem_per_warp(hash_slots);
+        // A batch costs its sweeps over all rows however few vertices its
+        // roots still reach, so a superstep ends with the first batch whose
+        // roots reach less than a tenth of the graph, and the next one is
+        // built by trees unless the last batch reached a seventh (more
+        // committed labels: RMAT scale 17 12% in roots 1,024-3,071, 1% in the
+        // next superstep, where batches would take twice the trees' 2.9 ms;
+        // scale 20 20% and then 7%, 68 ms for 6,144 roots in batches against
+        // 146 in trees)
+        bool bits_now = bits_ok && dist_hi < kBitDist && (r0 == 0 || (bit_steps == supersteps && bit_mean * kBitShareNext >= n));
         while (true) {
             std::memset(&hc, 0, sizeof(hc));
             hc.next_root = r0;
             CHL_CUDA(cudaMemcpyAsync(b.ctl, &hc, sizeof(hc), cudaMemcpyHostToDevice, b.st));
+            if (bits_now) {
+                uint32_t done = r0;
+                bool deep = false;
+                CHL_CUDA(cudaEventRecord(ev_a, b.st));
+                if ((rc = bit_superstep(rerun ? ~0ull : budget, r_end, &done, &deep))) return rc;
+                CHL_CUDA(cudaEventRecord(ev_b, b.st));
+                CHL_CUDA(cudaMemcpyAsync(&hc, b.ctl, sizeof(hc), cudaMemcpyDeviceToHost, b.st));
+                CHL_CUDA(cudaStreamSynchronize(b.st));
+                float ms = 0;
+                CHL_CUDA(cudaEventElapsedTime(&ms, ev_a, ev_b));
+                tree_ms += ms;
+                step_tree_ms = ms;
+                if (deep) {   // too many levels: the same roots by the other kernels
+                    bits_ok = bits_now = false;
+                    continue;
+                }
+                if (hc.overflow || hc.nlab > b.new_cap) {
+                    ++step_reruns;
+                    if ((rc = grow_new(b, hc.nlab + hc.nlab / 4 + 1024))) return rc;
+                    r_end = done;
+                    rerun = true;
+                    continue;
+                }
+                r_end = done;
+                break;
+            }
             TreeArgs ta;
             ta.n = n;
             ta.sides = b.sides;
@@ -2394,6 +2800,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         const uint32_t r1 = r_end;
         mean_visits = (double)hc.visits / std::max<uint32_t>(1, r1 - r0);
         ratio_stopped |= hc.ratio_stop != 0;
+        dist_hi = std::max<uint32_t>(dist_hi, hc.max_dist);
         const bool last = r1 >= n || (opts.root_limit && r1 >= opts.root_limit);
         visits += hc.visits;
         reads += hc.label_reads;
@@ -2401,7 +2808,13 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         if (plant_now) plant_roots += r1 - r0;
         unsigned long long M = hc.nlab;
         // hybrid switch (distributed_memory/akiba.hpp:297-303, 362-376)
-        if (plant_now && switch_open) {
+        // (heavy-tailed graphs switch after their bit-parallel supersteps, which
+        // measure no tree sizes: their first trees are 10 times their labels)
+        bit_steps += bits_now ? 1 : 0;
+        if (bits_now && switch_open && opts.ps <= 0) {
+            do_plant = false;
+            switch_open = false;
+        } else if (plant_now && switch_open && !bits_now) {
             unsigned long long zero = 0;
             CHL_CUDA(cudaMemcpyAsync(&b.ctl->max_ratio_num, &zero, 8, cudaMemcpyHostToDevice, b.st));
             ratio_max<<<std::max(1, sms), 256, 0, b.st>>>(b.tsize, b.tlab, &b.ctl->next_root, r0, r1, b.ctl);
@@ -2421,7 +2834,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         // captured as a CUDA graph when opts.use_graphs is set.  The entry
         // array is sized for every new label before the chain (the clean
         // only removes labels).
-        const bool clean_now = !plant_now && M > 0;
+        const bool clean_now = !plant_now && !bits_now && M > 0;   // bit-parallel labels are canonical
         if ((rc = grow_sort(b, M, clean_now))) return rc;
         if ((rc = ensure_ent(&b.ent_b, &b.ent_cap_b, committed + M))) return rc;
         if (!last && (rc = ensure_ent(&b.dent_b, &b.dent_cap_b, committed + M))) return rc;

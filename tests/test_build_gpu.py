@@ -304,3 +304,44 @@ def test_distances_near_int_max(P):
         with pytest.raises(P.CHLError) as e:
             P.build(g, np.array([0, 1, 2], np.uint32), **kw)
         assert e.value.status == P.CHL_ERR_INVALID, kw
+
+
+@pytest.mark.parametrize("kind", ["rmat", "directed", "star_path", "star_long_path"])
+def test_bit_parallel_supersteps(P, O, kind, tmp_path):
+    """Unit lengths and heavy tails: batches of 1,024 roots a bit each (part
+    batches, several per superstep, lists above 512 arcs), then the other
+    kernels; a graph deeper than 64 levels falls back to them."""
+    rng = np.random.default_rng(12)
+    if kind == "rmat":
+        g = P.Graph.rmat(13, 12, seed=9)
+        n = g.get_n()
+        off, head, ln = g.csr(True)
+        og = O.OGraph.from_csr(n, off, head, ln)
+    else:
+        if kind == "directed":
+            n = 5000
+            z = np.minimum((rng.pareto(0.9, 40000) * 3).astype(np.int64), n - 1)
+            src, dst = z, rng.integers(0, n, 40000)
+            flip = rng.random(40000) < 0.5
+            src, dst = np.where(flip, src, dst), np.where(flip, dst, src)
+        else:
+            tail = 40 if kind == "star_path" else 150
+            n = 2500
+            src = np.concatenate([np.zeros(2000, np.int64), np.arange(2000, 2000 + tail)])
+            dst = np.concatenate([np.arange(1, 2001), np.arange(2001, 2001 + tail)])
+        keep = src != dst
+        g = P.Graph.from_arcs(n, src[keep], dst[keep], np.ones(int(keep.sum()), np.int32),
+                              undirected=kind != "directed")
+        p = str(tmp_path / "g.gr")
+        g.write(p)
+        if kind == "directed":
+            og = O.OGraph.read_dimacs(p)
+        else:
+            off, head, ln = g.csr(True)
+            og = O.OGraph.from_csr(n, off, head, ln)
+    order = P.Order.degree(g, seed=4)
+    ref, _ = O.gll(og, order)
+    for kw in ({}, {"mode": MODES["gll"]}, {"mode": MODES["plant"]}, {"first_superstep": 100}, {"first_superstep": 1025},
+               {"first_superstep": 1500, "growth": 1.0}, {"sf": 0.5}, {"label_cap": 3000}, {"root_limit": n},
+               {"first_superstep": 3, "growth": 0.5}, {"window_target": 1}, {"use_graphs": 0}):
+        assert same_labels(P.build(g, order, **kw), ref, n), kw
