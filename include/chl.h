@@ -192,7 +192,7 @@ typedef struct chl_build_opts {
     int32_t superstep_extend; /* while a superstep's trees run, idle warps
                              take up to this many times its nominal roots
                              (0 auto: 4 on road-like graphs, off on heavy-
-                             tailed ones; 1 off)                            */
+                             tailed ones and in GLL mode; 1 off)            */
     uint32_t label_cap;   /* new-label buffer entries per superstep: 0 auto
                              (the label budget plus sides * n per tree still
                              running when it is spent, within a quarter of
@@ -206,8 +206,9 @@ typedef struct chl_build_opts {
                              distance windows of about this many vertices:
                              0 auto (1024; 512 on road-like graphs below 2^18
                              vertices), 1 off (batched settle rounds)       */
-    uint32_t window_warps; /* warps building one such tree: 0 auto (8 on
-                             heavy-tailed graphs, else 4), 1, 2, 4 or 8     */
+    uint32_t window_warps; /* warps building one such tree: 0 auto (32 in
+                             supersteps of at most two roots per SM, else 8 on
+                             heavy-tailed graphs and 4 on others), 1, 2, 4, 8 */
     uint32_t reserved[1];
 } chl_build_opts;
 

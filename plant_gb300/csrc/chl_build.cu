@@ -1533,6 +1533,7 @@ TreeKernel team_kernel_tw(uint32_t tw) {
     case 1: return team_kernel<UNIT, PLANT, PRUNE, 32>;
     case 2: return team_kernel<UNIT, PLANT, PRUNE, 64>;
     case 8: return team_kernel<UNIT, PLANT, PRUNE, 256>;
+    case 32: return team_kernel<UNIT, PLANT, PRUNE, 1024>;
     default: return team_kernel<UNIT, PLANT, PRUNE, 128>;
     }
 }
@@ -2376,21 +2377,29 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         set_error("window_warps must be 0, 1, 2, 4 or 8");
         return CHL_ERR_INVALID;
     }
+    // Warps per tree of a superstep: where at most two roots per SM start
+    // (unpruned first supersteps), as many as a block holds; a tree of 29,000
+    // vertices on a directed skewed graph of 2^15 is one of 152 then (build
+    // 14.6 ms with 8 warps, 8.6 with 32; weighted RMAT scale 17 in GLL mode
+    // 62 and 43).  Pruned trees keep win_tw (38.5 there with 8, 43 with 32).
+    auto team_warps = [&](bool prune, uint32_t roots) -> uint32_t {
+        return opts.window_warps == 0 && !prune && roots <= 2u * sms ? 32u : b.win_tw;
+    };
     // root hash slots: at most 2048 per warp-built tree within CHL_SMEM_CAP_KB
     // of shared memory per block, and 4096 per block-built one
-    auto team_blocks = [&](bool plant, bool prune, uint32_t hash_slots, int *blocks) -> int {
+    auto team_blocks = [&](bool plant, bool prune, uint32_t tw, uint32_t hash_slots, int *blocks) -> int {
         // the occupancy query counts a block's dynamic shared memory only up
         // to the kernel's current limit (48 KB by default): raise it first
-        TreeKernel k = team_kernel_for(unit, plant, prune, b.win_tw);
-        const int sm = (int)team_smem((int)b.win_tw * 32, hash_slots);
+        TreeKernel k = team_kernel_for(unit, plant, prune, tw);
+        const int sm = (int)team_smem((int)tw * 32, hash_slots);
         CHL_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-        CHL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, b.win_tw * 32, sm));
+        CHL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, tw * 32, sm));
         *blocks = std::max(*blocks, 1) * sms;
         return CHL_OK;
     };
     {
         int blocks = 0;
-        if ((rc = team_blocks(true, false, 0, &blocks))) return rc;
+        if ((rc = team_blocks(true, false, b.win_tw, 0, &blocks))) return rc;
         const uint64_t fit_trees = std::max<uint64_t>(1, ws_budget / std::max<uint64_t>(24ull * n, 1));
         b.win_trees = (uint32_t)std::min<uint64_t>((uint64_t)blocks, fit_trees);
     }
@@ -2440,14 +2449,14 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     unsigned long long budget_base =
         (unsigned long long)std::max(1.0, sf * (double)n / (b.sides == 1 ? 2.0 : 1.0));
     // Supersteps of unpruned trees (whole) end at the label buffer, which has
-    // room for lists of 3 sqrt(n) (grids have 0.7 to 1.5 sqrt(n)) within a
+    // room for lists of 1.7 sqrt(n) (grids have 0.7 to 1.5 sqrt(n)) within a
     // quarter of the free memory; a seventh of it is left to the trees still
     // running when the budget is spent.
     const bool whole_budget = whole && opts.sf <= 0 && opts.label_cap == 0;
     if (whole_budget) {
         size_t fr = 0, tot = 0;
         CHL_CUDA(cudaMemGetInfo(&fr, &tot));
-        const uint64_t want = (uint64_t)(3.5 * std::sqrt((double)n) * n * b.sides) + (1u << 20);
+        const uint64_t want = (uint64_t)(2.0 * std::sqrt((double)n) * n * b.sides) + (1u << 20);
         if ((rc = grow_new(b, std::min<uint64_t>(want, fr / 4 / 36)))) return rc;
         budget_base = b.new_cap - b.new_cap / 7;
     }
@@ -2493,15 +2502,22 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     // superstep early.
     // Bit-parallel graphs start with two batches and treble (RMAT scale 17
     // doubling 14.2 ms, trebling 13.2; scale 20 315 and 307).  Other
-    // heavy-tailed degree distributions start with two roots per SM (RMAT
-    // scale 17: 47.6 ms with 304, 55 with 152, 68 with 1,216; a directed
-    // skewed graph of 2^15 vertices 14 ms with 304, 20 with 1,216) and
-    // double, so the hubs commit before the bulk of the trees; bounded-degree
-    // graphs outside the whole rule start with two roots per warp of the
-    // schedule and grow by half of the committed prefix.
-    const uint32_t auto_first = bits_ok ? 2 * kBitRoots : heavy_tail ? (win_target > 1 ? std::max<uint32_t>(64u, 2u * sms) : 1024u)
-                                           : std::max<uint32_t>(64u, 2 * b.warps);
-    const double auto_growth = bits_ok ? 3.0 : heavy_tail ? 2.0 : 0.5;
+    // heavy-tailed degree distributions start with one root per SM and grow
+    // eightfold: their commits cost more than the pruning of small trees
+    // saves (a directed skewed graph of 2^15 vertices 10.0 ms growing twofold,
+    // 8.9 eightfold; weighted RMAT scale 17 74 and 70).  GLL trees emit a
+    // superset that grows with the unpruned superstep, so road-like graphs in
+    // GLL mode start with one root per SM as well and treble, without
+    // extending (the 256-square grid 67 ms; 217 with 14,592 roots, of which
+    // the clean took 176).  Bounded-degree graphs with an option that keeps
+    // them from the whole rule start with two roots per warp of the schedule
+    // and grow by half of the committed prefix.
+    const bool gll_auto = !heavy_tail && opts.mode == CHL_MODE_GLL && win_target > 1 && opts.first_superstep == 0;
+    const uint32_t auto_first = bits_ok ? 2 * kBitRoots
+                                : win_target > 1 && (heavy_tail || gll_auto) ? std::max<uint32_t>(64u, sms)
+                                : heavy_tail ? 1024u
+                                             : std::max<uint32_t>(64u, 2 * b.warps);
+    const double auto_growth = bits_ok ? 3.0 : heavy_tail ? 8.0 : gll_auto ? 2.0 : 0.5;
     // phase switch ratio (the reference's -ps, default 1024): auto 8 on
     // heavy-tailed graphs (RMAT scale 20: pruned GLL supersteps after the
     // first are faster than PLaNT trees there)
@@ -2704,7 +2720,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
             ta.r_end = r_end;
             // work-conserving extension: up to ext x the nominal size while
             // nominal trees run; none on a rerun
-            uint32_t ext = opts.superstep_extend == 0 ? (heavy_tail ? 1u : 4u)
+            uint32_t ext = opts.superstep_extend == 0 ? (heavy_tail || gll_auto ? 1u : 4u)
                                                       : (uint32_t)std::max(1, opts.superstep_extend);
             if (rerun) ext = 1;
             ta.r_hard = (uint32_t)std::min<uint64_t>(n, (uint64_t)r0 + (uint64_t)ext * (r_end - r0));
@@ -2752,11 +2768,12 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
                 ta.near_target = win_target;
                 ta.ws_win = b.ws_all;
                 int fit = 0;
-                if ((rc = team_blocks(plant_now, prune, slots, &fit))) return rc;
+                const uint32_t tw = team_warps(prune, r_end - r0);
+                if ((rc = team_blocks(plant_now, prune, tw, slots, &fit))) return rc;
                 grid = (int)std::min<uint32_t>((uint32_t)fit, b.win_trees);
-                block = (int)b.win_tw * 32;
+                block = (int)tw * 32;
                 smem_launch = team_smem(block, slots);
-                kern = team_kernel_for(unit, plant_now, prune, b.win_tw);
+                kern = team_kernel_for(unit, plant_now, prune, tw);
             } else if (unit) {
                 kern = plant_now ? batch_kernel<true, true> : batch_kernel<true, false>;
             } else {
