@@ -170,6 +170,19 @@ __device__ __forceinline__ bool snap_header(const char *p, const char *e, long l
 
 // One line per thread.  DIMACS: `p` fills the header fields; SNAP: the
 // `# Nodes:` line does.  Arcs go to unordered slots (init_arcs sorts them).
+// (one atomic per warp and line kind: a counter bumped line by line took most
+// of the 0.69 ms of a million lines)
+__device__ __forceinline__ unsigned long long take_slot(ParseOut *po, uint64_t k, bool first) {
+    const uint32_t m = __activemask(), lead = (uint32_t)__ffs(m) - 1u;
+    unsigned long long b = 0;
+    if (lane_id() == lead) {
+        b = atomicAdd(&po->arcs, (unsigned long long)__popc(m));
+        // lanes hold ascending lines: the leader's is the warp's first
+        if (first && k < *(volatile unsigned long long *)&po->first_a) atomicMin(&po->first_a, (unsigned long long)k);
+    }
+    return __shfl_sync(m, b, lead) + __popc(m & lanemask_lt());
+}
+
 __global__ void parse_lines(const char *buf, uint64_t S, const uint64_t *nl, uint64_t nnl, uint64_t lines,
                             int fmt, ParseOut *po, int64_t *au, int64_t *av, int64_t *aw) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -215,8 +228,7 @@ __global__ void parse_lines(const char *buf, uint64_t S, const uint64_t *nl, uin
                 atomicOr(&po->status, kFailFormat);
                 continue;
             }
-            const unsigned long long slot = atomicAdd(&po->arcs, 1ull);
-            atomicMin(&po->first_a, (unsigned long long)k);
+            const unsigned long long slot = take_slot(po, k, true);
             au[slot] = u;
             av[slot] = v;
             aw[slot] = 1;
@@ -238,7 +250,7 @@ __global__ void parse_lines(const char *buf, uint64_t S, const uint64_t *nl, uin
                 atomicOr(&po->status, kFailFormat);
                 continue;
             }
-            const unsigned long long slot = atomicAdd(&po->arcs, 1ull);
+            const unsigned long long slot = take_slot(po, k, false);
             au[slot] = u;
             av[slot] = v;
             aw[slot] = w;
@@ -281,8 +293,7 @@ __global__ void parse_lines(const char *buf, uint64_t S, const uint64_t *nl, uin
                 atomicOr(&po->status, kFailFormat);
                 continue;
             }
-            const unsigned long long slot = atomicAdd(&po->arcs, 1ull);
-            atomicMin(&po->first_a, (unsigned long long)k);
+            const unsigned long long slot = take_slot(po, k, true);
             au[slot] = u;
             av[slot] = v;
             aw[slot] = w;
@@ -398,10 +409,14 @@ __global__ void count_distinct(uint64_t cnt, const uint64_t *key, unsigned long 
 // add_tmp_arc: bounds check of the 32-bit vertex values (ids minus `base`:
 // 1 for DIMACS, 0 for SNAP) against n, then the two records
 // (u, v, w, fwd, und) and (v, u, w, und, rev)
+__device__ __forceinline__ uint32_t len_key(int32_t l) { return (uint32_t)l ^ 0x80000000u; }
+
+// status[0]: failures; status[1], status[2]: smallest and largest length key
 __global__ void make_records(uint64_t arcs, const int64_t *au, const int64_t *av, const int64_t *aw, long long n,
                              int base, int undirected, uint32_t *ru, uint32_t *rh, int32_t *rl, uint32_t *rf,
                              unsigned *status) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    uint32_t lo = 0xFFFFFFFFu, hi = 0;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < arcs; i += stride) {
         const uint32_t u = (uint32_t)(au[i] - base), v = (uint32_t)(av[i] - base);
         if ((long long)u >= n || (long long)v >= n) atomicOr(status, kFailFormat);
@@ -415,41 +430,73 @@ __global__ void make_records(uint64_t arcs, const int64_t *au, const int64_t *av
         rh[2 * i + 1] = u;
         rl[2 * i + 1] = w;
         rf[2 * i + 1] = (undirected ? 1u : 0u) | 2u;
+        lo = min(lo, len_key(w));
+        hi = max(hi, len_key(w));
+    }
+    lo = __reduce_min_sync(kFull, lo);
+    hi = __reduce_max_sync(kFull, hi);
+    if (lane_id() == 0 && lo <= hi) {
+        atomicMin(&status[1], lo);
+        atomicMax(&status[2], hi);
     }
 }
 
-__device__ __forceinline__ uint64_t len_key(int32_t l) { return (uint64_t)((uint32_t)l ^ 0x80000000u); }
+// Bits of a record's sort key: vertices take vb, the length above its smallest
+// lb.  Ordering by (major, length) is one sort where that fits 64 bits: digit
+// passes are what a sort costs, and most of the 12 that fixed 30-bit vertices
+// and 32-bit lengths need hold zeros (18 instead of 36 passes for a 512-square
+// grid's three sorts).
+struct KeyBits {
+    int vb, lb;
+    uint32_t len0;   // smallest length key
+};
 
-// key of cmp_by_direction without the length: u, reverse first, non-forward
-// first, head
-__device__ __forceinline__ uint64_t dir_key(uint32_t u, uint32_t h, uint32_t f) {
+// key of cmp_by_direction without the length (u, reverse first, non-forward
+// first, head), or cmp_by_head's (u, head)
+__device__ __forceinline__ uint64_t major_key(uint32_t u, uint32_t h, uint32_t f, int dir, int vb) {
+    if (!dir) return ((uint64_t)u << vb) | h;
     const uint64_t rev_last = (f & 2u) ? 0 : 1, fwd = f & 1u;
-    return ((uint64_t)u << 32) | (rev_last << 31) | (fwd << 30) | (uint64_t)h;
+    return ((uint64_t)u << (vb + 2)) | (rev_last << (vb + 1)) | (fwd << vb) | (uint64_t)h;
 }
 
-__global__ void keys_len(uint64_t cnt, const int32_t *rl, uint64_t *key, uint32_t *val) {
+__global__ void keys_whole(uint64_t cnt, const uint32_t *ru, const uint32_t *rh, const int32_t *rl, const uint32_t *rf,
+                           int dir, KeyBits kb, uint64_t *key, uint32_t *val) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < cnt; i += stride) {
-        key[i] = len_key(rl[i]);
+        key[i] = major_key(ru[i], rh[i], rf[i], dir, kb.vb) << kb.lb | (len_key(rl[i]) - kb.len0);
         val[i] = (uint32_t)i;
     }
 }
 
-// second LSD pass: key of record val[i] (dir: cmp_by_direction, else
-// cmp_by_head's (u, head))
-__global__ void keys_major(uint64_t cnt, const uint32_t *val, const uint32_t *ru, const uint32_t *rh,
-                           const uint32_t *rf, int dir, uint64_t *key) {
+__global__ void keys_len(uint64_t cnt, const int32_t *rl, uint32_t len0, uint64_t *key, uint32_t *val) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < cnt; i += stride) {
-        const uint32_t r = val[i];
-        key[i] = dir ? dir_key(ru[r], rh[r], rf[r]) : (((uint64_t)ru[r] << 30) | rh[r]);
+        key[i] = len_key(rl[i]) - len0;
+        val[i] = (uint32_t)i;
     }
 }
 
-template <typename T>
-__global__ void gather(uint64_t cnt, const uint32_t *idx, const T *in, T *out) {
+// second LSD pass where the two do not fit one key: major key of record val[i]
+__global__ void keys_major(uint64_t cnt, const uint32_t *val, const uint32_t *ru, const uint32_t *rh,
+                           const uint32_t *rf, int dir, int vb, uint64_t *key) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < cnt; i += stride) out[i] = in[idx[i]];
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < cnt; i += stride) {
+        const uint32_t r = val[i];
+        key[i] = major_key(ru[r], rh[r], rf[r], dir, vb);
+    }
+}
+
+__global__ void gather_records(uint64_t cnt, const uint32_t *idx, const uint32_t *ru, const uint32_t *rh,
+                               const int32_t *rl, const uint32_t *rf, uint32_t *tu, uint32_t *th, int32_t *tl,
+                               uint32_t *tf) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < cnt; i += stride) {
+        const uint32_t r = idx[i];
+        tu[i] = ru[r];
+        th[i] = rh[r];
+        tl[i] = rl[r];
+        tf[i] = rf[r];
+    }
 }
 
 // mode 0: keep the first of each (u, head, fwd, rev) run (records sorted by
@@ -526,19 +573,22 @@ int sort_kv(uint64_t *&k0, uint32_t *&v0, uint64_t *&k1, uint32_t *&v1, const ui
 }
 
 // Records sorted by (major key, length): permutation into v, records gathered.
-int sort_records(uint64_t cnt, int dir, uint32_t *&ru, uint32_t *&rh, int32_t *&rl, uint32_t *&rf, uint32_t *&tu,
-                 uint32_t *&th, int32_t *&tl, uint32_t *&tf, uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1,
-                 const uint64_t *d_cnt, void *tmp, size_t tmp_bytes) {
+int sort_records(uint64_t cnt, int dir, const KeyBits &kb, uint32_t *&ru, uint32_t *&rh, int32_t *&rl, uint32_t *&rf,
+                 uint32_t *&tu, uint32_t *&th, int32_t *&tl, uint32_t *&tf, uint64_t *k0, uint32_t *v0, uint64_t *k1,
+                 uint32_t *v1, const uint64_t *d_cnt, void *tmp, size_t tmp_bytes) {
     const int grid = device_sms() * 8;
-    keys_len<<<grid, 256>>>(cnt, rl, k0, v0);
-    int rc = sort_kv(k0, v0, k1, v1, d_cnt, cnt, 32, tmp, tmp_bytes);
-    if (rc) return rc;
-    keys_major<<<grid, 256>>>(cnt, v0, ru, rh, rf, dir, k0);
-    if ((rc = sort_kv(k0, v0, k1, v1, d_cnt, cnt, dir ? 62 : 60, tmp, tmp_bytes))) return rc;
-    gather<uint32_t><<<grid, 256>>>(cnt, v0, ru, tu);
-    gather<uint32_t><<<grid, 256>>>(cnt, v0, rh, th);
-    gather<int32_t><<<grid, 256>>>(cnt, v0, rl, tl);
-    gather<uint32_t><<<grid, 256>>>(cnt, v0, rf, tf);
+    const int major = 2 * kb.vb + (dir ? 2 : 0);
+    int rc;
+    if (major + kb.lb <= 64) {
+        keys_whole<<<grid, 256>>>(cnt, ru, rh, rl, rf, dir, kb, k0, v0);
+        if ((rc = sort_kv(k0, v0, k1, v1, d_cnt, cnt, major + kb.lb, tmp, tmp_bytes))) return rc;
+    } else {
+        keys_len<<<grid, 256>>>(cnt, rl, kb.len0, k0, v0);
+        if ((rc = sort_kv(k0, v0, k1, v1, d_cnt, cnt, kb.lb, tmp, tmp_bytes))) return rc;
+        keys_major<<<grid, 256>>>(cnt, v0, ru, rh, rf, dir, kb.vb, k0);
+        if ((rc = sort_kv(k0, v0, k1, v1, d_cnt, cnt, major, tmp, tmp_bytes))) return rc;
+    }
+    gather_records<<<grid, 256>>>(cnt, v0, ru, rh, rl, rf, tu, th, tl, tf);
     CHL_CUDA(cudaGetLastError());
     std::swap(ru, tu);
     std::swap(rh, th);
@@ -725,17 +775,17 @@ int ingest_text(const FileBuf &file, int fmt, bool undirected, chl_graph *g) {
     int32_t *rl, *tl;
     if ((rc = pool.get(&ru, cnt)) || (rc = pool.get(&rh, cnt)) || (rc = pool.get(&rl, cnt)) ||
         (rc = pool.get(&rf, cnt)) || (rc = pool.get(&tu, cnt)) || (rc = pool.get(&th, cnt)) ||
-        (rc = pool.get(&tl, cnt)) || (rc = pool.get(&tf, cnt)) || (rc = pool.get(&d_status, 1)))
+        (rc = pool.get(&tl, cnt)) || (rc = pool.get(&tf, cnt)) || (rc = pool.get(&d_status, 3)))
         return -rc;
     const int grid = device_sms() * 8;
-    CHL_CUDA_NEG(cudaMemset(d_status, 0, 4));
+    unsigned st[3] = {0, 0xFFFFFFFFu, 0};   // status, smallest and largest length key
+    CHL_CUDA_NEG(cudaMemcpy(d_status, st, sizeof(st), cudaMemcpyHostToDevice));
     if (arcs)
         make_records<<<grid, 256>>>(arcs, au, av, aw, n, (fmt == kFmtDimacs || fmt == kFmtMetis) ? 1 : 0,
                                     undirected ? 1 : 0, ru, rh,
                                     rl, rf, d_status);
-    unsigned st = 0;
-    CHL_CUDA_NEG(cudaMemcpy(&st, d_status, 4, cudaMemcpyDeviceToHost));
-    if (st) return 0;   // an arc endpoint outside [0, n): not this format (the host tries the others)
+    CHL_CUDA_NEG(cudaMemcpy(st, d_status, sizeof(st), cudaMemcpyDeviceToHost));
+    if (st[0]) return 0;   // an arc endpoint outside [0, n): not this format (the host tries the others)
     g->n = (uint32_t)n;
     g->m = arcs * (undirected ? 2 : 1);
     // init_arcs
@@ -749,6 +799,12 @@ int ingest_text(const FileBuf &file, int fmt, bool undirected, chl_graph *g) {
     const size_t stmp_bytes =
         std::max(scan_tmp_bytes(std::max<uint64_t>(cnt + 1, (uint64_t)n + 1)), radix_tmp_bytes());
     if ((rc = pool.get((char **)&stmp, stmp_bytes))) return -rc;
+    auto bits = [](uint64_t most) {   // bits of the values 0 .. most
+        int b = 1;
+        while (b < 64 && most >> b) ++b;
+        return b;
+    };
+    const KeyBits kb = {bits(n > 0 ? (uint64_t)n - 1 : 0), arcs ? bits(st[2] - st[1]) : 1, arcs ? st[1] : 0u};
     uint64_t live = cnt;
     auto set_count = [&](uint64_t c) -> int {
         CHL_CUDA(cudaMemcpy(d_n, &c, 8, cudaMemcpyHostToDevice));
@@ -772,11 +828,11 @@ int ingest_text(const FileBuf &file, int fmt, bool undirected, chl_graph *g) {
     };
     if (cnt) {
         if ((rc = set_count(live)) ||
-            (rc = sort_records(live, 1, ru, rh, rl, rf, tu, th, tl, tf, k0, v0, k1, v1, d_n, stmp, stmp_bytes)) ||
+            (rc = sort_records(live, 1, kb, ru, rh, rl, rf, tu, th, tl, tf, k0, v0, k1, v1, d_n, stmp, stmp_bytes)) ||
             (rc = compact(0)) || (rc = set_count(live)) ||
-            (rc = sort_records(live, 0, ru, rh, rl, rf, tu, th, tl, tf, k0, v0, k1, v1, d_n, stmp, stmp_bytes)) ||
+            (rc = sort_records(live, 0, kb, ru, rh, rl, rf, tu, th, tl, tf, k0, v0, k1, v1, d_n, stmp, stmp_bytes)) ||
             (rc = compact(1)) || (rc = set_count(live)) ||
-            (rc = sort_records(live, 1, ru, rh, rl, rf, tu, th, tl, tf, k0, v0, k1, v1, d_n, stmp, stmp_bytes)))
+            (rc = sort_records(live, 1, kb, ru, rh, rl, rf, tu, th, tl, tf, k0, v0, k1, v1, d_n, stmp, stmp_bytes)))
             return -rc;
     }
     // the two CSRs: side 1 = forward (flag bit 0), side 0 = reverse (bit 1)

@@ -238,3 +238,22 @@ def test_fuzz_files_agree(P, tmp_path):
         p = write(tmp_path, f"z{i}.txt", data)
         for und in (False, True):
             same(P, p, und)
+
+
+@pytest.mark.parametrize("n,span", [(2, 1), (3, 2), (256, 255), (257, 256), (65536, 2 ** 31 - 1), (70000, 2 ** 32 - 1),
+                                    (300000, 2 ** 32 - 1)])
+def test_sort_key_widths(P, tmp_path, n, span):
+    """Vertex and length ranges at the edges of the sort key's fields, up to
+    where vertices and length no longer share one 64-bit key: duplicate arcs
+    with other lengths, both directions, negative lengths."""
+    rng = np.random.default_rng(n)
+    low = 1 if span < 2 ** 31 else -2 ** 31
+    u = rng.integers(1, n + 1, 400)
+    v = rng.integers(1, n + 1, 400)
+    u[:3], v[:3] = [1, n, n], [n, 1, n]
+    u, v = np.concatenate([u, u[:150], v[:100]]), np.concatenate([v, v[:150], u[:100]])
+    w = low + rng.integers(0, span, u.size)
+    w[:2] = [low, low + span - (span == 2 ** 32 - 1)]
+    text = f"p sp {n} {u.size}\n" + "".join(f"a {a} {b} {c}\n" for a, b, c in zip(u, v, w))
+    for undirected in (False, True):
+        same(P, write(tmp_path, "k.gr", text), undirected, expect_gpu=True)
