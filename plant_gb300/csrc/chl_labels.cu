@@ -248,42 +248,74 @@ namespace {
 __device__ __forceinline__ uint32_t merge_min(const uint2 *A, uint32_t na, const uint2 *B, uint32_t nb) {
     const uint32_t lane = lane_id();
     uint32_t best = 0xFFFFFFFFu;
-    uint32_t ia = 0, ib = 0;
-    auto ldA = [&]() { return ia + lane < na ? A[ia + lane] : make_uint2(0xFFFFFFFFu, 0u); };
-    auto ldB = [&]() { return ib + lane < nb ? B[ib + lane] : make_uint2(0xFFFFFFFEu, 0u); };
+    uint32_t ia = 0, ib = 0;   // first entries of the chunks held
     if (na == 0 || nb == 0) return best;
-    uint2 a = ldA(), b = ldB();
-    while (true) {
-        // lower bound of a.x in the B chunk
-        uint32_t lo = 0;
+    uint2 a, b;
+    uint32_t at, hb;           // the lane's lower bound of a.x in b, and its hub
+    // lower bound by five halvings: they reach entry 31 at most, which may
+    // still be below a.x
+    auto search = [&]() {
+        int lo = -1;
 #pragma unroll
         for (int step = 16; step > 0; step >>= 1) {
-            const uint32_t hb = __shfl_sync(kFull, b.x, lo + step - 1);
-            if (hb < a.x) lo += step;
+            const int t = lo + step;
+            if (__shfl_sync(kFull, b.x, t) < a.x) lo = t;
         }
-        // five steps reach 31 at most: entry 31 may still be below a.x
-        const uint32_t hb = __shfl_sync(kFull, b.x, lo);
-        const uint32_t db = __shfl_sync(kFull, b.y, lo);
+        at = (uint32_t)(lo + 1);
+        hb = __shfl_sync(kFull, b.x, at);
+        const uint32_t db = __shfl_sync(kFull, b.y, at);
         if (hb == a.x) best = min(best, a.y + db);
-        const uint32_t la = min(na - ia, 32u) - 1u, vb = min(nb - ib, 32u);
-        const uint32_t within = __ballot_sync(kFull, lo < vb && hb >= a.x);
-        if (within >> la & 1u) {   // A's last entry is no larger than B's
+    };
+    // full chunks of both lists: no bounds to look at
+    if (na >= 32 && nb >= 32) {
+        const uint2 *pa = A + lane, *pb = B + lane;
+        const uint32_t fa = na & ~31u, fb = nb & ~31u;
+        a = pa[0];
+        b = pb[0];
+        while (true) {
+            search();
+            if ((int)__ballot_sync(kFull, hb >= a.x) < 0) {   // A's last entry is no larger than B's
+                ia += 32;
+                if (ia == fa) break;
+                a = pa[ia];
+            } else {
+                ib += 32;
+                if (ib == fb) break;
+                b = pb[ib];
+            }
+        }
+        if (ia >= na || ib >= nb) return __reduce_min_sync(kFull, best);
+    }
+    // one list's last, partial chunk against what is left of the other
+    auto ldA = [&]() { return ia + lane < na ? A[ia + lane] : make_uint2(0xFFFFFFFFu, 0u); };
+    auto ldB = [&]() { return ib + lane < nb ? B[ib + lane] : make_uint2(0xFFFFFFFEu, 0u); };
+    a = ldA();
+    b = ldB();
+    uint32_t la = min(na - ia, 32u) - 1u, vb = min(nb - ib, 32u);   // last lane of A's chunk, entries of B's
+    while (true) {
+        search();
+        const uint32_t within = __ballot_sync(kFull, at < vb && hb >= a.x);
+        if (within >> la & 1u) {
             ia += 32;
             if (ia >= na) break;
             a = ldA();
+            la = min(na - ia, 32u) - 1u;
         } else {
             ib += 32;
             if (ib >= nb) break;
             b = ldB();
+            vb = min(nb - ib, 32u);
         }
     }
     return __reduce_min_sync(kFull, best);
 }
 
-// Bound by the L2 while the labels fit it, else by DRAM latency; both keep
-// every warp slot, so registers stay at 32.  4 M pairs of a 200-square grid's
-// labels (44 MB) 2.17 -> 1.9 ms, of a 512-square one's (1.5 GB) 13.4 -> 13.3;
-// reading ahead costs more registers than it hides (2.0 to 2.2 and 13.5 to 18).
+// Bound by issue while the labels fit the L2 (585 instructions a pair at 76%
+// of the issue slots and 19% of the L2's throughput before full chunks went
+// without bounds), else by DRAM latency; both keep every warp slot, so
+// registers stay at 32.  4 M pairs of a 200-square grid's labels (44 MB) 2.17
+// -> 1.76 ms, of a 512-square one's (1.5 GB) 13.4 -> 12.5; reading chunks ahead
+// costs more registers than it hides (2.0 to 2.2 and 13.5 to 18).
 // GROUP pairs per warp.  One: every lane reads the pair and its list offsets.
 // Several: the lanes read a pair each, so the chain of three gathers before a
 // list is paid once per group, and the answers are written together.
