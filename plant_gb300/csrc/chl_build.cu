@@ -2402,6 +2402,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         if ((rc = team_blocks(true, false, b.win_tw, 0, &blocks))) return rc;
         const uint64_t fit_trees = std::max<uint64_t>(1, ws_budget / std::max<uint64_t>(24ull * n, 1));
         b.win_trees = (uint32_t)std::min<uint64_t>((uint64_t)blocks, fit_trees);
+        if (opts.max_warps) b.win_trees = std::min(b.win_trees, opts.max_warps);   // the cap on concurrent trees
     }
     // one workspace for both layouts: batch_kernel's key (two words on
     // weighted graphs), vis and queue arrays per warp slot (5 or 6 n words),
