@@ -64,7 +64,8 @@ __global__ void pack_arcs(uint64_t m, const uint32_t *head, const int32_t *len, 
 //     the next window is taken from the far pile.  Windows are as wide as to
 //     hold about kWindow vertices (256 sources of a 1024-square grid: 123 ms
 //     with 1,024, 117 with 2,048, 115 with 4,096 and 8,192; the order as a
-//     whole, against 8 s with one lane per source).  (Settling only vertices that are final by
+//     whole, against 8 s with one lane per source), distance and queue mark
+//     falling in one 64-bit minimum (115 -> 101 ms).  (Settling only vertices that are final by
 //     the IN criterion of Crauser et al. took about 8 vertices a step on
 //     road-like graphs and 43 ms for a 256-square grid.)
 //  2. Path counts sigma in waves over the shortest-path graph: a wave holds
@@ -72,7 +73,7 @@ __global__ void pack_arcs(uint64_t m, const uint32_t *head, const int32_t *len, 
 //  3. Dependencies delta over the waves in reverse.
 // Every sum of 2 and 3 runs in adjacency order with explicitly rounded
 // operations (no contraction), matching the CPU restatement bit for bit.  On
-// the 256-square grid the kernel takes 9.3 ms, one lane per source with a
+// the 256-square grid the kernel takes 8.2 ms, one lane per source with a
 // binary heap took 308.
 // A vertex of up to kLight arcs belongs to one thread, half of its arcs in
 // flight at a time; others to one warp.
@@ -82,27 +83,31 @@ constexpr int kLight = 8;
 constexpr int kGroup = kLight / 2;
 constexpr uint32_t kWindow = 4096;
 
+constexpr uint32_t kFarMark = 0xFFFFFFFFu;   // above every pass
+
 struct OrdShared {
     uint32_t nn, npile, nkeep, heavy, lo, kmin, kmax;
 };
 
 __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const uint64_t *off_out, const uint2 *arc_out,
                                                               const uint64_t *off_in, const uint2 *arc_in,
-                                                              const uint32_t *src, uint32_t *ws_dist, uint32_t *ws_mark,
+                                                              const uint32_t *src, unsigned long long *ws_word,
                                                               uint32_t *ws_list, double *ws_sigma, double *deltas) {
     __shared__ OrdShared sh;
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     const uint32_t j = blockIdx.x;
-    uint32_t *dist = ws_dist + (size_t)j * n;
-    uint32_t *mark = ws_mark + (size_t)j * n;     // 1: last pass queued in; 2: predecessors not yet counted
+    // word of a vertex: distance in the high half; in the low one the last pass
+    // it was queued in (phase 1), the predecessors not yet counted (phase 2)
+    unsigned long long *word = ws_word + (size_t)j * n;
+    auto dist_at = [&](uint32_t v) -> uint32_t { return __ldcg((const uint32_t *)(word + v) + 1); };
+    auto mark_at = [&](uint32_t v) -> uint32_t * { return (uint32_t *)(word + v); };
     uint32_t *front = ws_list + (size_t)j * 2 * n, *fnext = front + n;
     double *sigma = ws_sigma + (size_t)j * n;
     uint32_t *pile = (uint32_t *)sigma, *pile2 = pile + n;   // phase 1 only
     double *delta = deltas + (size_t)j * n;
     const uint32_t s = src[j];
     for (uint32_t v = tid; v < n; v += kOrdThreads) {
-        __stcg(&dist[v], v == s ? 0u : kInfD);
-        __stcg(&mark[v], 0u);
+        __stcg(&word[v], (unsigned long long)(v == s ? 0u : kInfD) << 32 | kFarMark);
         __stcg(&delta[v], 0.0);
     }
     if (tid == 0) {
@@ -138,11 +143,17 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
             auto relax = [&](uint32_t w, uint32_t dd, uint32_t seen) {
                 // distances only fall: a read no larger than dd proves the atomic idle
                 if (dd >= seen) return;
-                const uint32_t old = atomicMin(&dist[w], dd);
-                if (dd >= old) return;
+                // one minimum over distance and mark: the smaller distance wins
+                // and brings its mark
+                const uint32_t stamp = dd < thr ? pass : kFarMark;
+                const unsigned long long was = atomicMin(&word[w], (unsigned long long)dd << 32 | stamp);
+                const uint32_t old = (uint32_t)(was >> 32), mark = (uint32_t)was;
+                if (dd > old || (dd == old && stamp >= mark)) return;
                 if (dd < thr) {
-                    // a vertex of the far pile whose distance falls below thr leaves a stale entry there
-                    if (atomicExch(&mark[w], pass) != pass) __stcg(&fnext[atomicAdd(&sh.nn, 1u)], w);
+                    // a vertex of the far pile whose distance falls below thr
+                    // leaves a stale entry there; an equal distance only takes
+                    // the mark of a vertex the sweep queued: queued again
+                    if (mark != pass) __stcg(&fnext[atomicAdd(&sh.nn, 1u)], w);
                 } else {
                     lo = min(lo, dd);
                     if (old == kInfD) __stcg(&pile[atomicAdd(&sh.npile, 1u)], w);
@@ -151,7 +162,7 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
             for (uint32_t i = tid; i < nf; i += kOrdThreads) {
                 const uint32_t v = __ldcg(&front[i]);
                 const uint64_t ob = off_out[v], oe = off_out[v + 1];
-                const uint32_t dv = __ldcg(&dist[v]);
+                const uint32_t dv = dist_at(v);
                 if (oe - ob > kLight) {
                     sh.heavy = 1;
                     continue;
@@ -165,7 +176,7 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
                     for (int q = 0; q < kGroup; ++q)
                         hl[q] = ob + h + q < oe ? arc_out[ob + h + q] : make_uint2(v, 1u);
 #pragma unroll
-                    for (int q = 0; q < kGroup; ++q) dw[q] = ob + h + q < oe ? __ldcg(&dist[hl[q].x]) : 0u;
+                    for (int q = 0; q < kGroup; ++q) dw[q] = ob + h + q < oe ? dist_at(hl[q].x) : 0u;
 #pragma unroll
                     for (int q = 0; q < kGroup; ++q) relax(hl[q].x, dv + hl[q].y, dw[q]);
                 }
@@ -173,10 +184,10 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
             __syncthreads();
             if (sh.heavy) {
                 for_heavy(front, nf, off_out, [&](uint32_t v) {
-                    const uint32_t dv = __ldcg(&dist[v]);
+                    const uint32_t dv = dist_at(v);
                     for (uint64_t a = off_out[v] + lane; a < off_out[v + 1]; a += 32) {
                         const uint2 hl = arc_out[a];
-                        relax(hl.x, dv + hl.y, __ldcg(&dist[hl.x]));
+                        relax(hl.x, dv + hl.y, dist_at(hl.x));
                     }
                     __syncwarp();
                 });
@@ -201,7 +212,7 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
             __syncthreads();
             uint32_t mn = kInfD, mx = 0;
             for (uint32_t i = tid; i < sh.npile; i += kOrdThreads) {
-                const uint32_t d = __ldcg(&dist[__ldcg(&pile[i])]);
+                const uint32_t d = dist_at(__ldcg(&pile[i]));
                 mn = min(mn, d);
                 mx = max(mx, d);
             }
@@ -237,7 +248,7 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
             for (uint32_t i0 = 0; i0 < np; i0 += kOrdThreads) {
                 const uint32_t i = i0 + tid;
                 const uint32_t x = i < np ? __ldcg(&pile[i]) : 0u;
-                const uint32_t d = i < np ? __ldcg(&dist[x]) : 0u;
+                const uint32_t d = i < np ? dist_at(x) : 0u;
                 const bool take = i < np && d >= t_old && d < thr, keep = i < np && d >= thr;
                 const uint32_t tm = __ballot_sync(kFull, take), km = __ballot_sync(kFull, keep);
                 uint32_t tb = 0, kb = 0;
@@ -272,7 +283,7 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
         const uint32_t v = v0 + lane;
         bool h = false;
         if (v < n) {
-            const uint32_t dv = __ldcg(&dist[v]);
+            const uint32_t dv = dist_at(v);
             const uint64_t ib = off_in[v], ie = off_in[v + 1];
             uint32_t c = 0;
             h = dv != kInfD && ie - ib > kLight;
@@ -284,21 +295,21 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
 #pragma unroll
                     for (int q = 0; q < kGroup; ++q) hl[q] = ib + g + q < ie ? arc_in[ib + g + q] : make_uint2(v, 1u);
 #pragma unroll
-                    for (int q = 0; q < kGroup; ++q) c += __ldcg(&dist[hl[q].x]) + hl[q].y == dv ? 1u : 0u;
+                    for (int q = 0; q < kGroup; ++q) c += dist_at(hl[q].x) + hl[q].y == dv ? 1u : 0u;
                 }
             }
-            if (!h) __stcg(&mark[v], c);
+            if (!h) __stcg(mark_at(v), c);
         }
         for (uint32_t m = __ballot_sync(kFull, h); m; m &= m - 1) {
             const uint32_t x = v0 + __ffs(m) - 1;
-            const uint32_t dx = __ldcg(&dist[x]);
+            const uint32_t dx = dist_at(x);
             uint32_t c = 0;
             for (uint64_t a = off_in[x] + lane; a < off_in[x + 1]; a += 32) {
                 const uint2 hl = arc_in[a];
-                c += __ldcg(&dist[hl.x]) + hl.y == dx ? 1u : 0u;
+                c += dist_at(hl.x) + hl.y == dx ? 1u : 0u;
             }
             c = __reduce_add_sync(kFull, c);
-            if (lane == 0) __stcg(&mark[x], c);
+            if (lane == 0) __stcg(mark_at(x), c);
         }
     }
     uint32_t *seq = ws_list + (size_t)j * 2 * n, *wave = seq + n;   // vertices in wave order; each wave's first
@@ -313,12 +324,12 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
         }
         __syncthreads();
         auto count_down = [&](uint32_t w, uint32_t dd, uint32_t dw) {
-            if (dd == dw && dw != kInfD && atomicSub(&mark[w], 1u) == 1u) __stcg(&seq[end + atomicAdd(&sh.nn, 1u)], w);
+            if (dd == dw && dw != kInfD && atomicSub(mark_at(w), 1u) == 1u) __stcg(&seq[end + atomicAdd(&sh.nn, 1u)], w);
         };
         for (uint32_t i = begin + tid; i < end; i += kOrdThreads) {
             const uint32_t v = __ldcg(&seq[i]);
             const uint64_t ib = off_in[v], ie = off_in[v + 1], ob = off_out[v], oe = off_out[v + 1];
-            const uint32_t dv = __ldcg(&dist[v]);
+            const uint32_t dv = dist_at(v);
             if (ie - ib > kLight || oe - ob > kLight) sh.heavy = 1;
             if (ie - ib <= kLight) {
                 double acc = 0.0;
@@ -332,7 +343,7 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
                         hl[q] = ib + h + q < ie ? arc_in[ib + h + q] : make_uint2(v, 1u);   // d(v) + 1 != d(v)
 #pragma unroll
                     for (int q = 0; q < kGroup; ++q)
-                        sp[q] = __ldcg(&dist[hl[q].x]) + hl[q].y == dv ? __ldcg(&sigma[hl[q].x]) : 0.0;
+                        sp[q] = dist_at(hl[q].x) + hl[q].y == dv ? __ldcg(&sigma[hl[q].x]) : 0.0;
 #pragma unroll
                     for (int q = 0; q < kGroup; ++q) acc = __dadd_rn(acc, sp[q]);
                 }
@@ -348,7 +359,7 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
                     for (int q = 0; q < kGroup; ++q)
                         hl[q] = ob + h + q < oe ? arc_out[ob + h + q] : make_uint2(v, 1u);
 #pragma unroll
-                    for (int q = 0; q < kGroup; ++q) dw[q] = __ldcg(&dist[hl[q].x]);
+                    for (int q = 0; q < kGroup; ++q) dw[q] = dist_at(hl[q].x);
 #pragma unroll
                     for (int q = 0; q < kGroup; ++q) count_down(hl[q].x, dv + hl[q].y, dw[q]);
                 }
@@ -357,14 +368,14 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
         __syncthreads();
         if (sh.heavy) {
             for_heavy(seq + begin, end - begin, off_in, [&](uint32_t v) {
-                const uint32_t dv = __ldcg(&dist[v]);
+                const uint32_t dv = dist_at(v);
                 const uint64_t ie = off_in[v + 1];
                 double acc = 0.0;
                 for (uint64_t a = off_in[v]; a < ie; a += 32) {
                     double sp = 0.0;
                     if (a + lane < ie) {
                         const uint2 hl = arc_in[a + lane];
-                        if (__ldcg(&dist[hl.x]) + hl.y == dv) sp = __ldcg(&sigma[hl.x]);
+                        if (dist_at(hl.x) + hl.y == dv) sp = __ldcg(&sigma[hl.x]);
                     }
                     for (uint32_t m = __ballot_sync(kFull, sp != 0.0); m; m &= m - 1)
                         acc = __dadd_rn(acc, __shfl_sync(kFull, sp, __ffs(m) - 1));
@@ -372,10 +383,10 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
                 if (lane == 0) __stcg(&sigma[v], v == s ? 1.0 : acc);
             });
             for_heavy(seq + begin, end - begin, off_out, [&](uint32_t v) {
-                const uint32_t dv = __ldcg(&dist[v]);
+                const uint32_t dv = dist_at(v);
                 for (uint64_t a = off_out[v] + lane; a < off_out[v + 1]; a += 32) {
                     const uint2 hl = arc_out[a];
-                    count_down(hl.x, dv + hl.y, __ldcg(&dist[hl.x]));
+                    count_down(hl.x, dv + hl.y, dist_at(hl.x));
                 }
                 __syncwarp();
             });
@@ -399,7 +410,7 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
                 sh.heavy = 1;
                 continue;
             }
-            const uint32_t dv = __ldcg(&dist[v]);
+            const uint32_t dv = dist_at(v);
             const double sv = __ldcg(&sigma[v]);
             double acc = 0.0;
 #pragma unroll
@@ -412,7 +423,7 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
                 for (int q = 0; q < kGroup; ++q) hl[q] = ob + h + q < oe ? arc_out[ob + h + q] : make_uint2(v, 1u);
 #pragma unroll
                 for (int q = 0; q < kGroup; ++q) {
-                    const uint32_t d = __ldcg(&dist[hl[q].x]);
+                    const uint32_t d = dist_at(hl[q].x);
                     on[q] = d != kInfD && dv + hl[q].y == d;
                 }
 #pragma unroll
@@ -430,7 +441,7 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
         if (sh.heavy) {
             for_heavy(seq + begin, end - begin, off_out, [&](uint32_t v) {
                 const uint64_t oe = off_out[v + 1];
-                const uint32_t dv = __ldcg(&dist[v]);
+                const uint32_t dv = dist_at(v);
                 const double sv = __ldcg(&sigma[v]);
                 double acc = 0.0;
                 for (uint64_t a = off_out[v]; a < oe; a += 32) {
@@ -438,7 +449,7 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
                     double t = 0.0;
                     if (a + lane < oe) {
                         const uint2 hl = arc_out[a + lane];
-                        const uint32_t d = __ldcg(&dist[hl.x]);
+                        const uint32_t d = dist_at(hl.x);
                         on = d != kInfD && dv + hl.y == d;
                         if (on)
                             t = __dmul_rn(__ddiv_rn(sv, __ldcg(&sigma[hl.x])), __dadd_rn(1.0, __ldcg(&delta[hl.x])));
@@ -595,13 +606,12 @@ extern "C" int chl_order_betweenness(const chl_graph *g, uint32_t sources, uint6
         CHL_CUDA(cudaDeviceSynchronize());
     }
     // one block per source
-    Buf wd, wm, wl, wsg;
-    if ((rc = alloc(wd, (size_t)sources * n * 4)) || (rc = alloc(wm, (size_t)sources * n * 4)) ||
-        (rc = alloc(wl, (size_t)sources * n * 8)) || (rc = alloc(wsg, (size_t)sources * n * 8)))
+    Buf ww, wl, wsg;
+    if ((rc = alloc(ww, (size_t)sources * n * 8)) || (rc = alloc(wl, (size_t)sources * n * 8)) || (rc = alloc(wsg, (size_t)sources * n * 8)))
         return rc;
     brandes_kernel<<<sources, kOrdThreads>>>(n, off_out.as<uint64_t>(), arc_out.as<uint2>(), off_in.as<uint64_t>(),
-                                             arc_in.as<uint2>(), dsrc.as<uint32_t>(), wd.as<uint32_t>(),
-                                             wm.as<uint32_t>(), wl.as<uint32_t>(), wsg.as<double>(),
+                                             arc_in.as<uint2>(), dsrc.as<uint32_t>(),
+                                             ww.as<unsigned long long>(), wl.as<uint32_t>(), wsg.as<double>(),
                                              deltas.as<double>());
     CHL_CUDA(cudaGetLastError());
     bc_sum<<<device_sms() * 4, 256>>>(n, sources, deltas.as<double>(), bc.as<double>());
