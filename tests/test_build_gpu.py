@@ -345,3 +345,27 @@ def test_bit_parallel_supersteps(P, O, kind, tmp_path):
                {"first_superstep": 1500, "growth": 1.0}, {"sf": 0.5}, {"label_cap": 3000}, {"root_limit": n},
                {"first_superstep": 3, "growth": 0.5}, {"window_target": 1}, {"use_graphs": 0}):
         assert same_labels(P.build(g, order, **kw), ref, n), kw
+
+
+@pytest.mark.parametrize("directed", [False, True])
+def test_numbered_trees(P, directed):
+    """Graphs of 2^16 vertices and more are renumbered for their unpruned
+    trees: scrambled ids, isolated vertices and directed lengths give the
+    labels of the warp-built trees."""
+    side = 270
+    n = side * side + 37
+    rng = np.random.default_rng(8)
+    i = rng.permutation(n)[:side * side].reshape(side, side)
+    u = np.concatenate([i[:, :-1].ravel(), i[:-1].ravel()])
+    v = np.concatenate([i[:, 1:].ravel(), i[1:].ravel()])
+    if directed:
+        u, v = np.concatenate([u, v]), np.concatenate([v, u])
+        keep = rng.random(u.size) < 0.97
+        u, v = u[keep], v[keep]
+    w = rng.integers(1, 1000, u.size)
+    for length in (w, np.ones_like(w)):
+        g = P.Graph.from_arcs(n, u, v, length, undirected=not directed)
+        order = P.Order.betweenness(g, 48, seed=2)
+        want = P.build(g, order, window_target=1).digest()
+        assert P.build(g, order).digest() == want
+        assert P.build(g, order, sf=20.0).digest() == want    # several unpruned supersteps
