@@ -179,9 +179,9 @@ def peaks():
 
 
 def profile_traffic():
-    """DRAM bytes per algorithmic byte of the tree kernel, from the committed
-    ncu capture of a smaller grid (scaled to this workload's launches)."""
-    p = os.path.join(ROOT, "profiles", "batch_kernel_traffic_grid512.json")
+    """DRAM bytes per algorithmic byte of the grids' tree kernel, from the
+    committed ncu capture of a smaller grid (scaled to this workload's launches)."""
+    p = os.path.join(ROOT, "profiles", "team_kernel_traffic_grid512.json")
     try:
         with open(p) as f:
             return json.load(f)
@@ -582,7 +582,9 @@ def run_ours(args, ws, rank):
     per_launch_tree = avg_tree_ms / max(1, stats[-1]["tree_launches"])
     peak, peak_kind = peaks()
     achieved = work / (avg_tree_ms / 1e3) / 1e9
-    traffic = profile_traffic()
+    # grids build in unpruned blocks, heavy-tailed unit graphs mostly bit-parallel
+    tree_kernel = "team_kernel" if args.workload == "grid" else "bit_level"
+    traffic = profile_traffic() if args.workload == "grid" else None
     # queries on the resident labels (uniform pairs, device resident)
     qk = 1 << 22
     q_ms, q_bytes = P.query_bench(L, qk, iters=20, seed=7)
@@ -624,7 +626,7 @@ def run_ours(args, ws, rank):
                                  if traffic and ("dram_per_trace_byte" in traffic or not trace) else None),
                      "traffic_note": ("bytes per launch, scaled from " + traffic["workload"] + " (ncu)"
                                       if traffic else None),
-                     "kernel": "batch_kernel", "algorithmic_bytes_per_build": work,
+                     "kernel": tree_kernel, "algorithmic_bytes_per_build": work,
                      "work_model": ("sequential PLL trace, profiles/pll_trace_" + workload_slug(args) + ".json"
                                     if trace else "labelled vertices only (closed form, lower bound)"),
                      "labelled_bytes_per_build": labelled,

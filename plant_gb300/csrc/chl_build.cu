@@ -25,10 +25,13 @@
 //  * Large trees are searched by a block each (team_kernel), label-correcting
 //    in distance windows; on road-like graphs without prune tests and mostly
 //    in one superstep.
-//  * Small pruned trees are built by a warp each: batch_kernel settles vertices in batches by the IN
-//    criterion from a near/far queue and prunes with one 16-entry item of
-//    the distance-ordered lists per lane against a shared-memory hash of the
-//    root's label.
+//  * Unit-length heavy-tailed graphs grow 32 trees per 32-bit word of a vertex,
+//    level by level and all roots at once (bit_level), up to where their trees
+//    are small.
+//  * Small pruned trees are built by a warp each (batch_kernel): vertices
+//    settle in batches by the IN criterion from a near/far queue and are
+//    pruned with one 16-entry item of the distance-ordered lists per lane
+//    against a shared-memory hash of the root's label.
 #include "chl_dev.cuh"
 
 #include <algorithm>
@@ -2090,7 +2093,7 @@ template <typename T>
 int dalloc(T **p, size_t count) {
     *p = nullptr;
     if (count == 0) count = 1;
-    cudaError_t e = cudaMalloc((void **)p, count * sizeof(T));
+    cudaError_t e = long_malloc((void **)p, count * sizeof(T));
     if (e != cudaSuccess) {
         cudaGetLastError();
         set_error(std::string("device allocation failed: ") + cudaGetErrorString(e));
@@ -2436,7 +2439,8 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     // with prune tests only pay where trees stay large: on heavy-tailed
     // graphs, and once kFreeVisits vertices per label were settled (fetch_root
     // ends the superstep).  The 1024-square grid: trees 0.81 s in one unpruned
-    // superstep, 1.09 to 1.32 s with a label budget of 1024 n.
+    // superstep, 1.09 to 1.32 s with a label budget of 1024 n (0.70 in one
+    // since the trees have a numbering of their own, see number_by_cells).
     const bool whole = !heavy_tail && win_target > 1 && opts.mode != CHL_MODE_GLL && opts.first_superstep == 0;
     constexpr uint32_t kFreeVisits = 16;
     // pruned trees of at least this many settled vertices (by the last
@@ -3234,6 +3238,7 @@ extern "C" int chl_graph_to_device(chl_graph *g) {
 extern "C" int chl_graph_release_device(chl_graph *g) {
     if (!g) return CHL_ERR_INVALID;
     chl::graph_release_device(g);
+    chl::tmp_trim();
     return CHL_OK;
 }
 

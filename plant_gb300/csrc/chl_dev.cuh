@@ -30,11 +30,20 @@ int device_sms();
 // allocations (mapping them through a pool costs more: 16 GB 35 ms against
 // 7.7).  What outlives a call (labels, graphs, networks) is never taken from
 // here.  The pool is stream-ordered, so calls on any threads and streams may
-// share it; it is emptied when an allocation fails.
+// share it; it is emptied when an allocation fails (a tmp_alloc or a
+// long_malloc) and when a graph's device copy is released.
 constexpr size_t kTmpMost = (size_t)512 << 20;
 constexpr size_t kTmpKeep = (size_t)1 << 30;
 int tmp_alloc(void **p, size_t bytes, cudaStream_t s);
 void tmp_free(void *p, size_t bytes, cudaStream_t s);
+void tmp_trim();
+// cudaMalloc for what outlives a call: once more without the pool's idle
+// memory if there is no room.
+cudaError_t long_malloc(void **p, size_t bytes);
+template <typename T>
+cudaError_t long_malloc(T **p, size_t bytes) {
+    return long_malloc((void **)p, bytes);
+}
 
 // The temporaries of one call, freed together (or one by one) on their stream.
 class TmpSet {
@@ -47,11 +56,16 @@ class TmpSet {
     }
     template <typename T>
     int get(T **p, uint64_t count) {
-        void *q = nullptr;
         const size_t bytes = (size_t)(count ? count : 1) * sizeof(T);
-        const int rc = tmp_alloc(&q, bytes, st);
-        *p = (T *)q;
-        if (rc == 0) held.emplace_back(q, bytes);
+        *p = nullptr;
+        try {
+            held.emplace_back(nullptr, bytes);
+        } catch (...) {   // callers are C entries
+            return CHL_ERR_OOM;
+        }
+        const int rc = tmp_alloc(&held.back().first, bytes, st);
+        *p = (T *)held.back().first;
+        if (rc) held.pop_back();
         return rc;
     }
     template <typename T>

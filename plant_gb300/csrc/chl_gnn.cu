@@ -780,7 +780,7 @@ struct DevBuf {
         cudaFree(p);
         p = nullptr;
         bytes = 0;
-        cudaError_t e = cudaMalloc(&p, b ? b : 1);
+        cudaError_t e = long_malloc(&p, b ? b : 1);
         if (e != cudaSuccess) return cuda_status(e, "cudaMalloc", __FILE__, __LINE__);
         bytes = b;
         return CHL_OK;

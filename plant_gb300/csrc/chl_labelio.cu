@@ -175,9 +175,9 @@ int write_labels_text_device(const chl_labels *l, const char *path) {
     const int sms = device_sms();
     DevMem d_len, d_loff, d_tmp, d_buf[2];
     const size_t tmp_bytes = scan_tmp_bytes(lines);
-    CHL_CUDA(cudaMalloc(&d_len.p, std::max<uint64_t>(lines, 1) * 4));
-    CHL_CUDA(cudaMalloc(&d_loff.p, (lines + 1) * 8));
-    CHL_CUDA(cudaMalloc(&d_tmp.p, std::max<size_t>(tmp_bytes, 16)));
+    CHL_CUDA(long_malloc(&d_len.p, std::max<uint64_t>(lines, 1) * 4));
+    CHL_CUDA(long_malloc(&d_loff.p, (lines + 1) * 8));
+    CHL_CUDA(long_malloc(&d_tmp.p, std::max<size_t>(tmp_bytes, 16)));
     Stream st[2];
     for (auto &s : st) {
         CHL_CUDA(cudaStreamCreateWithFlags(&s.s, cudaStreamNonBlocking));
@@ -208,7 +208,7 @@ int write_labels_text_device(const chl_labels *l, const char *path) {
     Pinned hbuf[2];
     const uint64_t bufsz = std::min<uint64_t>(cap, std::max<uint64_t>(loff[lines], 1));
     for (int i = 0; i < 2; ++i) {
-        CHL_CUDA(cudaMalloc(&d_buf[i].p, bufsz));
+        CHL_CUDA(long_malloc(&d_buf[i].p, bufsz));
         CHL_CUDA(cudaHostAlloc(&hbuf[i].p, bufsz, cudaHostAllocDefault));
     }
     FILE *f = fopen(path, "wb");
@@ -355,9 +355,9 @@ extern "C" int chl_labels_load(const char *path, chl_labels **out) {
             return CHL_ERR_FORMAT;
         }
     DevMem d_off, d_ent, d_bad;
-    CHL_CUDA(cudaMalloc(&d_off.p, (nl + 1) * 8));
-    CHL_CUDA(cudaMalloc(&d_ent.p, std::max<uint64_t>(total, 1) * sizeof(LabelEnt)));
-    CHL_CUDA(cudaMalloc(&d_bad.p, 4));
+    CHL_CUDA(long_malloc(&d_off.p, (nl + 1) * 8));
+    CHL_CUDA(long_malloc(&d_ent.p, std::max<uint64_t>(total, 1) * sizeof(LabelEnt)));
+    CHL_CUDA(long_malloc(&d_bad.p, 4));
     CHL_CUDA(cudaMemcpy(d_off.p, off.data(), (nl + 1) * 8, cudaMemcpyHostToDevice));
     if (total) {
         Pinned hb;

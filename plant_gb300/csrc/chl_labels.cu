@@ -45,16 +45,20 @@ namespace {
 // the pool of tmp_alloc on the current device (null: none could be made)
 cudaMemPool_t tmp_pool() {
     static std::mutex mu;
-    static std::vector<std::pair<bool, cudaMemPool_t>> pools;   // (tried, pool) by device
+    constexpr int kDevs = 64;
+    static struct {
+        bool tried;
+        cudaMemPool_t pool;
+    } pools[kDevs];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
+    if (dev >= kDevs) return nullptr;
     std::lock_guard<std::mutex> g(mu);
-    if ((int)pools.size() <= dev) pools.resize(dev + 1, {false, nullptr});
-    if (!pools[dev].first) {
-        pools[dev].first = true;
+    if (!pools[dev].tried) {
+        pools[dev].tried = true;
         cudaMemPoolProps pr;
         std::memset(&pr, 0, sizeof(pr));
         pr.allocType = cudaMemAllocationTypePinned;
@@ -64,11 +68,11 @@ cudaMemPool_t tmp_pool() {
         uint64_t keep = kTmpKeep;
         if (cudaMemPoolCreate(&pool, &pr) == cudaSuccess &&
             cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
-            pools[dev].second = pool;
+            pools[dev].pool = pool;
         else
             cudaGetLastError();
     }
-    return pools[dev].second;
+    return pools[dev].pool;
 }
 
 }  // namespace
@@ -97,6 +101,22 @@ void tmp_free(void *p, size_t bytes, cudaStream_t s) {
     if (!p) return;
     if (bytes <= kTmpMost && tmp_pool()) cudaFreeAsync(p, s);
     else cudaFree(p);
+}
+
+void tmp_trim() {
+    if (cudaMemPool_t pool = tmp_pool()) cudaMemPoolTrimTo(pool, 0);
+}
+
+cudaError_t long_malloc(void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        // what was freed on a stream goes back to the pool at a synchronise
+        cudaGetLastError();
+        cudaDeviceSynchronize();
+        tmp_trim();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
 }
 
 // Device -> pageable host copy through two pinned staging buffers: the DMA
@@ -169,8 +189,8 @@ int labels_fetch_host(const chl_labels *l) {
 int labels_ensure_device(const chl_labels *L) {
     if (L->d_off) return CHL_OK;
     const uint32_t nl = L->nl();
-    cudaError_t e = cudaMalloc(&L->d_off, ((size_t)nl + 1) * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&L->d_ent, std::max<uint64_t>(L->total, 1) * sizeof(LabelEnt));
+    cudaError_t e = long_malloc(&L->d_off, ((size_t)nl + 1) * 8);
+    if (e == cudaSuccess) e = long_malloc(&L->d_ent, std::max<uint64_t>(L->total, 1) * sizeof(LabelEnt));
     if (e == cudaSuccess)
         e = cudaMemcpy(L->d_off, L->h_off.data(), ((size_t)nl + 1) * 8, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && L->total)
@@ -581,12 +601,7 @@ int export_device(const chl_labels *l, const uint64_t *hoff, const uint64_t *off
     return rc;
 }
 
-}  // namespace
-}  // namespace chl
-
-extern "C" int chl_labels_export(const chl_labels *l, uint64_t *off, uint32_t *hubs,
-                                 int32_t *dists) {
-    if (!l || !off) return CHL_ERR_INVALID;
+int labels_export(const chl_labels *l, uint64_t *off, uint32_t *hubs, int32_t *dists) {
     // offsets of the 2n lists (both sides, even when stored once), then the
     // entries, copied in parallel over vertices
     auto offsets = [&](const uint64_t *hoff) {
@@ -625,6 +640,20 @@ extern "C" int chl_labels_export(const chl_labels *l, uint64_t *off, uint32_t *h
     return CHL_OK;
 }
 
+}  // namespace
+}  // namespace chl
+
+extern "C" int chl_labels_export(const chl_labels *l, uint64_t *off, uint32_t *hubs,
+                                 int32_t *dists) {
+    if (!l || !off) return CHL_ERR_INVALID;
+    try {
+        return labels_export(l, off, hubs, dists);
+    } catch (...) {
+        set_error("host allocation failed during export");
+        return CHL_ERR_OOM;
+    }
+}
+
 extern "C" int chl_labels_import(uint32_t n, const uint64_t *off, const uint32_t *hubs,
                                  const int32_t *dists, chl_labels **out) {
     if (!off || !out || (off[2ull * n] && (!hubs || !dists))) return CHL_ERR_INVALID;
@@ -653,7 +682,7 @@ extern "C" int chl_labels_digest(const chl_labels *l, uint64_t *digest) {
     int rc = labels_ensure_device(l);
     if (rc) return rc;
     unsigned long long *d_acc = nullptr;
-    CHL_CUDA(cudaMalloc(&d_acc, sizeof(unsigned long long)));
+    CHL_CUDA(long_malloc(&d_acc, sizeof(unsigned long long)));
     unsigned long long acc = 0;
     cudaError_t e = cudaMemset(d_acc, 0, sizeof(acc));
     if (e == cudaSuccess && l->n) {
@@ -690,9 +719,9 @@ extern "C" int chl_query_bench(const chl_labels *l, size_t k, uint64_t seed, int
     unsigned long long *dbytes = nullptr;
     cudaStream_t st = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
-    cudaError_t e = cudaMalloc(&dp, k * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&dout, k * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&dbytes, 8);
+    cudaError_t e = long_malloc(&dp, k * 8);
+    if (e == cudaSuccess) e = long_malloc(&dout, k * 4);
+    if (e == cudaSuccess) e = long_malloc(&dbytes, 8);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&e0);
     if (e == cudaSuccess) e = cudaEventCreate(&e1);
@@ -825,21 +854,18 @@ struct SlotSet {
 };
 
 std::mutex g_slots_mu;
-std::vector<SlotSet *> &idle_slots() {
-    static std::vector<SlotSet *> *v = new std::vector<SlotSet *>();   // not destroyed: the driver may be gone by then
-    return *v;
-}
+SlotSet *g_idle[kSetsKept];   // plain pointers: not destroyed at exit, when the driver may be gone
+size_t g_idle_n = 0;
 
 int take_slots(SlotSet **out) {
     int dev = 0;
     CHL_CUDA(cudaGetDevice(&dev));
     {
         std::lock_guard<std::mutex> g(g_slots_mu);
-        auto &v = idle_slots();
-        for (size_t i = v.size(); i-- > 0;)
-            if (v[i]->dev == dev) {
-                *out = v[i];
-                v.erase(v.begin() + i);
+        for (size_t i = g_idle_n; i-- > 0;)
+            if (g_idle[i]->dev == dev) {
+                *out = g_idle[i];
+                g_idle[i] = g_idle[--g_idle_n];
                 return CHL_OK;
             }
     }
@@ -860,8 +886,8 @@ int take_slots(SlotSet **out) {
 void give_slots(SlotSet *s) {
     {
         std::lock_guard<std::mutex> g(g_slots_mu);
-        if (idle_slots().size() < kSetsKept) {
-            idle_slots().push_back(s);
+        if (g_idle_n < kSetsKept) {
+            g_idle[g_idle_n++] = s;
             return;
         }
     }
