@@ -8,6 +8,7 @@
 #include <memory>
 #include <utility>
 #include <vector>
+#include <atomic>
 
 #include "../../include/chl.h"
 
@@ -110,6 +111,7 @@ struct chl_labels {
     mutable std::vector<uint64_t> h_off;
     mutable std::vector<LabelEnt, NoInitAlloc<LabelEnt>> h_ent;
     mutable bool host_valid = false;
+    mutable std::atomic<bool> exported{false};   // an export went past the mirror
     chl_build_stats stats{};
     uint32_t nl() const { return sym ? n : 2 * n; }
     uint32_t list(uint32_t v, int side) const { return sym ? v : 2 * v + (uint32_t)side; }

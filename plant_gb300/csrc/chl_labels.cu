@@ -539,10 +539,9 @@ namespace {
 // a 512-square grid's labels).  hoff: the nl + 1 list offsets; off: the
 // caller's 2n + 1.  Returns 1 when a list does not fit a buffer.
 int export_device(const chl_labels *l, const uint64_t *hoff, const uint64_t *off, uint32_t *hubs, int32_t *dists) {
-    // pieces of an eighth, at least 1 MB: pinning 2 x 12 MB took 1 ms of a
-    // 10,000-vertex grid's 1.6 ms export
+    // pieces of an eighth: pinning 2 x 16 MB takes 1.5 ms of the 3 that 21 MB of labels take
     const uint64_t kMost =
-        std::min<uint64_t>(kStage, std::max<uint64_t>(l->total * sizeof(LabelEnt) / 8, 1u << 20)) / sizeof(LabelEnt);
+        std::min<uint64_t>(kStage, l->total * sizeof(LabelEnt) / 8) / sizeof(LabelEnt);
     const uint32_t nl = l->nl();
     std::vector<uint32_t> cut{0};   // lists [cut[c], cut[c + 1]) fit one buffer
     while (cut.back() < nl) {
@@ -612,12 +611,19 @@ int labels_export(const chl_labels *l, uint64_t *off, uint32_t *hubs, int32_t *d
                 off[2 * (size_t)v + side + 1] = off[2 * (size_t)v + side] + (hoff[x + 1] - hoff[x]);
             }
     };
-    if (!l->host_valid && l->d_off) {
+    // Labels of one staging buffer at most are fetched whole and kept: 0.76 ms
+    // for a 100-square grid's 7.6 MB against 0.92 through pinned pieces.  Larger
+    // ones (62 MB: 4.7 against 3.3 ms, 855 MB: 39 against 25) come in pieces the
+    // first time; a second export makes the mirror, from which the ones after
+    // it are faster still (2.5 and 21 ms).
+    const bool entries = hubs || dists;
+    if (!l->host_valid && l->d_off &&
+        (!entries || (l->total * sizeof(LabelEnt) > kStage && !l->exported.exchange(true)))) {
         std::vector<uint64_t, NoInitAlloc<uint64_t>> hoff((size_t)l->nl() + 1);
         int rc = d2h_staged(hoff.data(), l->d_off, hoff.size() * 8);
         if (rc) return rc;
         offsets(hoff.data());
-        if (!hubs && !dists) return CHL_OK;
+        if (!entries) return CHL_OK;
         rc = export_device(l, hoff.data(), off, hubs, dists);
         if (rc != 1) return rc;
     }
@@ -838,6 +844,7 @@ namespace {
 
 constexpr size_t kSlotPairs = 32768;
 constexpr int kSlots = 4;
+constexpr size_t kManyPairs = 1u << 19;
 constexpr size_t kSetsKept = 8;   // 12 MB pinned
 
 struct SlotSet {
@@ -894,6 +901,12 @@ void give_slots(SlotSet *s) {
     delete s;
 }
 
+uint32_t largest(const uint32_t *x, size_t cnt) {
+    uint32_t m = 0;
+    for (size_t i = 0; i < cnt; ++i) m = std::max(m, x[i]);
+    return m;
+}
+
 int query_slots(const chl_labels *l, const uint32_t *pairs, size_t k, int32_t *out, cudaStream_t st, SlotSet *s) {
     const size_t chunks = (k + kSlotPairs - 1) / kSlotPairs;
     auto collect = [&](size_t c) -> int {
@@ -922,8 +935,19 @@ int query_slots(const chl_labels *l, const uint32_t *pairs, size_t k, int32_t *o
 extern "C" int chl_query_batch(const chl_labels *l, const uint32_t *pairs, size_t k, int32_t *out,
                                void *stream) {
     if (!l || (k && (!pairs || !out))) return CHL_ERR_INVALID;
-    uint32_t most = 0;   // one pass the compiler can vectorise
-    for (size_t i = 0; i < 2 * k; ++i) most = std::max(most, pairs[i]);
+    // one pass the compiler can vectorise, shared by the cores where it is long
+    // (2 M pairs: the call 1.57 ms, 2.44 on one core)
+    uint32_t most = 0;
+    if (k < kManyPairs) {
+        most = largest(pairs, 2 * k);
+    } else {
+        constexpr int64_t kParts = 64;
+#pragma omp parallel for reduction(max : most)
+        for (int64_t q = 0; q < kParts; ++q) {
+            const size_t b = 2 * k / kParts * q, e = q + 1 < kParts ? 2 * k / kParts * (q + 1) : 2 * k;
+            most = std::max(most, largest(pairs + b, e - b));
+        }
+    }
     if (k && most >= l->n) {
         set_error("query vertex out of range");
         return CHL_ERR_INVALID;

@@ -126,3 +126,20 @@ def test_export_in_pieces(P):
             assert np.array_equal(hub[s], h) and np.array_equal(dist[s], d)
     for a, b in zip(L.export(), (off, hub, dist)):   # from the host mirror label() made
         assert np.array_equal(a, b)
+
+
+def test_export_again(P):
+    """A second export (through the host mirror it makes) and later ones equal
+    the first (in pieces); many pairs with one out of range are refused."""
+    g = P.Graph.grid(140, 140, seed=4)
+    L = P.build(g, P.Order.degree(g, seed=2))
+    first = L.export()
+    for _ in range(2):
+        for a, b in zip(L.export(), first):
+            assert np.array_equal(a, b)
+    pairs = P.generate_query(700_001, g.get_n(), seed=1)
+    want = P.query(L, pairs)
+    assert np.array_equal(want[-1000:], P.query(L, pairs[-1000:]))
+    pairs[654_321, 1] = g.get_n()
+    with pytest.raises(P.CHLError):
+        P.query(L, pairs)
