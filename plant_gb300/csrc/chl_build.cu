@@ -2430,8 +2430,14 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     // vertices per distance window of the team kernel (1: settle rounds by the
     // IN criterion instead).  Grids: 512 and 1,024 within 3% of each other,
     // smaller graphs better with 512 (the 100-square grid 1.8 against 1.9 ms),
-    // the 1024-square one with 1,024 (1.51 against 1.56 s)
-    const uint32_t win_target = opts.window_target ? opts.window_target : (heavy_tail || n >= (1u << 18) ? 1024u : 512u);
+    // large ones with wider windows (512-square trees 94.6, 90.3, 93.3 ms with
+    // 512, 1,024, 2,048; 768-square 330.8 and 328.6 with 1,024 and 2,048;
+    // 1024-square 887 and 863; 1448-square 1,330 and 1,297)
+    const uint32_t win_target = opts.window_target ? opts.window_target
+                                : heavy_tail       ? 1024u
+                                : n < (1u << 18)   ? 512u
+                                : n < (1u << 19)   ? 1024u
+                                                   : 2048u;
     // Road-like graphs build whole: PLaNT trees without prune tests are exact
     // by their via flags alone, and cost 0.14 ns a settled vertex where a
     // pruned one costs 1 to 2 (its list and the root's).  They settle 3.5 to

@@ -671,13 +671,17 @@ extern "C" int chl_labels_hub_freq(const chl_labels *l, const uint32_t *order, u
     int rc = labels_ensure_device(l);
     if (rc) return rc;
     uint32_t *d_cnt = nullptr;
-    TmpSet tmp;
-    if ((rc = tmp.get(&d_cnt, l->n))) return rc;
-    CHL_CUDA(cudaMemset(d_cnt, 0, (size_t)l->n * 4));
+    CHL_CUDA(long_malloc(&d_cnt, (size_t)std::max<uint32_t>(l->n, 1) * 4));
+    cudaError_t em = cudaMemset(d_cnt, 0, (size_t)l->n * 4);
+    if (em != cudaSuccess) {
+        cudaFree(d_cnt);
+        return cuda_status(em, "cudaMemset", __FILE__, __LINE__);
+    }
     if (l->total)
         hub_count<<<device_sms() * 8, 256>>>((const uint2 *)l->d_ent, l->total, d_cnt);
     std::vector<uint32_t> cnt(l->n);
     cudaError_t e = cudaMemcpy(cnt.data(), d_cnt, (size_t)l->n * 4, cudaMemcpyDeviceToHost);
+    cudaFree(d_cnt);
     if (e != cudaSuccess) return cuda_status(e, "hub_freq", __FILE__, __LINE__);
     for (uint32_t h = 0; h < l->n; ++h) freq[order[h]] = cnt[h] * (l->sym ? 2u : 1u);
     return CHL_OK;
