@@ -631,6 +631,9 @@ def run_ours(args, ws, rank):
                                     if trace else "labelled vertices only (closed form, lower bound)"),
                      "labelled_bytes_per_build": labelled,
                      "pll_scanned_bytes_per_build": (float(trace["scanned_bytes"]) if trace else None),
+                     "work_note": ("sequential PLL's bytes over our tree time; unpruned trees do not read the label "
+                                   "lists counted there, so the ratio may pass 1" if tree_kernel == "team_kernel"
+                                   else None),
                      "tree_ms_per_build": avg_tree_ms, "tree_launches": stats[-1]["tree_launches"],
                      "ms_per_launch": per_launch_tree},
         "build": {"build_s": ms_step / 1e3, "avg_label": stats[-1]["avg_label"], "labels": labels,

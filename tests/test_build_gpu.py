@@ -369,3 +369,31 @@ def test_numbered_trees(P, directed):
         want = P.build(g, order, window_target=1).digest()
         assert P.build(g, order).digest() == want
         assert P.build(g, order, sf=20.0).digest() == want    # several unpruned supersteps
+
+
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("n", [40, 700, 1500])
+def test_rows_of_arcs(P, O, directed, n, tmp_path):
+    """Weighted trees read a vertex's first four arcs as a row: degrees around
+    4, 8 and 32, lists past the row, vertices without arcs, every number of
+    warps per tree (32 by default on few roots)."""
+    rng = np.random.default_rng(n)
+    # few lists pass their row (an eighth at most): their arcs meet in a few heads
+    deg = np.resize([0, 1, 2, 1], n)
+    over = rng.permutation(n)[:n // 16]
+    deg[over] = np.minimum(np.resize([5, 8, 9, 31, 32, 33, 36, 37, 300], over.size), n - 1)
+    src = np.repeat(np.arange(n), deg)
+    dst = np.where(deg[src] > 2, over[rng.integers(0, over.size, src.size)], (src + rng.integers(1, n, src.size)) % n)
+    src, dst = src[src != dst], dst[src != dst]
+    g = P.Graph.from_arcs(n, src, dst, rng.integers(1, 20, src.size), undirected=not directed)
+    p = str(tmp_path / "g.gr")
+    g.write(p)
+    if directed:
+        og = O.OGraph.read_dimacs(p)
+    else:
+        og = O.OGraph.from_csr(n, *g.csr(True))
+    order = P.Order.degree(g, seed=4)
+    ref, _ = O.gll(og, order)
+    for kw in ({}, {"mode": MODES["gll"]}, {"mode": MODES["plant"]}, {"window_warps": 1}, {"window_warps": 2},
+               {"window_warps": 4}, {"window_warps": 8, "window_target": 16}, {"first_superstep": 30}):
+        assert same_labels(P.build(g, order, **kw), ref, n), kw
