@@ -1007,8 +1007,7 @@ __global__ void __launch_bounds__(T, team_warps_per_sm(PRUNE) * 32 / T) team_ker
     uint32_t *list0 = memb + a.n;
     const uint32_t n = a.n;
     static_assert(!ROWS || (!UNIT && !PRUNE), "rows hold lengths and are not tested");
-    auto key_at = [&](uint32_t v) -> uint32_t * { return (uint32_t *)(kw + v) + 1; };
-    auto mark_at = [&](uint32_t v) -> uint32_t * { return (uint32_t *)(kw + v); };
+    auto key_at = [&](uint32_t v) -> const uint32_t * { return (const uint32_t *)(kw + v) + 1; };   // read only
     unsigned long long c_arcs = 0, c_reads = 0;
 
     uint32_t n_emit = 0;
@@ -1378,11 +1377,14 @@ __global__ void __launch_bounds__(T, team_warps_per_sm(PRUNE) * 32 / T) team_ker
                                 live = __ballot_sync(kFull, test);
                             }
                             if (valid) {
+                                // 64 bits wide like the minimum that other warps lower
+                                // the word with: atomics of different widths on the
+                                // same bytes are not atomic to each other
                                 if (hit) {
-                                    atomicAnd(mark_at(v), ~1u);
+                                    atomicAnd(kw + v, ~1ull);
                                     deg = 0;
                                 } else if (!((uint32_t)word & 1u)) {
-                                    atomicOr(mark_at(v), 1u);   // was pruned at a larger distance
+                                    atomicOr(kw + v, 1ull);   // was pruned at a larger distance
                                 }
                             }
                         }

@@ -1,0 +1,32 @@
+"""Rules of the kernels that no run can show broken: a violation works on the
+hardware at hand or depends on how a warp happens to be scheduled, so the
+sources are looked at instead."""
+import os
+import re
+
+from conftest import ROOT
+
+
+def body(path, start):
+    """Source of the function whose definition contains `start`, without comments."""
+    src = open(os.path.join(ROOT, "plant_gb300", "csrc", path)).read()
+    src = re.sub(r"//[^\n]*", "", src)
+    at = src.index(start)
+    i = src.index("{", src.index(")", at))
+    depth = 0
+    for j in range(i, len(src)):
+        depth += {"{": 1, "}": -1}.get(src[j], 0)
+        if depth == 0:
+            return src[at:j + 1]
+    raise AssertionError("unbalanced braces")
+
+
+def test_key_words_see_atomics_of_one_width():
+    """The block trees lower a vertex's 64-bit word (key and pass mark) with
+    atomicMin while other warps set and clear its prune bit: every atomic on
+    the word has to be as wide, or they are not atomic to each other."""
+    src = body("chl_build.cu", "team_kernel(TreeArgs a)")
+    on_word = re.findall(r"atomic\w+\(\s*(?:kw|key_at|mark_at|\(uint32_t \*\))[^;]*;", src)
+    assert len(on_word) >= 3
+    for call in on_word:
+        assert re.match(r"atomic\w+\(\s*kw \+ ", call), call
