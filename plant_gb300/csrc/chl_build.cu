@@ -2788,9 +2788,10 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     const uint32_t first = opts.first_superstep ? opts.first_superstep : auto_first;
     const double growth = opts.growth > 0 ? opts.growth : auto_growth;
     // The roots [r0, r_end) by bit_level, a batch at a time until the label
-    // budget is spent; *done: the first root not taken, *deep: gave up at
-    // kBitLevels.  The host reads the live roots after each level.
-    auto bit_superstep = [&](unsigned long long budget, uint32_t r_end, uint32_t *done, bool *deep) -> int {
+    // budget is spent; *done: the first root not taken, *off: gave up, at
+    // kBitLevels or for want of room for the table (up to 4 KB per committed
+    // root).  The host reads the live roots after each level.
+    auto bit_superstep = [&](unsigned long long budget, uint32_t r_end, uint32_t *done, bool *off) -> int {
         if (!bit_live) {
             if ((rc = b.mem->get(&bit_live, (uint64_t)(kBitLevels + 1) * kBitWords))) return rc;
             for (int f = 0; f < b.sides; ++f) {
@@ -2809,7 +2810,10 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         uint8_t *act[2] = {(uint8_t *)(seen + bit_row), (uint8_t *)(seen + bit_row) + n};
         const uint32_t K = dist_hi + 1;
         unsigned long long *M = nullptr;
-        if (r0 && (rc = b.mem->get(&M, (uint64_t)r0 * K * kBitWords))) return rc;
+        if (r0 && (rc = b.mem->get(&M, (uint64_t)r0 * K * kBitWords))) {
+            *off = rc == CHL_ERR_OOM;
+            return *off ? CHL_OK : rc;
+        }
         CHL_CUDA(cudaMemsetAsync(b.tsize + 0, 0, (size_t)(r_end - r0) * 4, b.st));
         CHL_CUDA(cudaMemsetAsync(b.tlab + 0, 0, (size_t)(r_end - r0) * 4, b.st));
         uint32_t rb = r0;
@@ -2864,7 +2868,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
                 ++launches;
                 for (uint32_t d = 1;; ++d) {
                     if (d > kBitLevels) {
-                        *deep = true;
+                        *off = true;
                         b.mem->put(M);
                         return CHL_OK;
                     }
@@ -2942,9 +2946,9 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
             CHL_CUDA(cudaMemcpyAsync(b.ctl, &hc, sizeof(hc), cudaMemcpyHostToDevice, b.st));
             if (bits_now) {
                 uint32_t done = r0;
-                bool deep = false;
+                bool off = false;
                 CHL_CUDA(cudaEventRecord(ev_a, b.st));
-                if ((rc = bit_superstep(rerun ? ~0ull : budget, r_end, &done, &deep))) return rc;
+                if ((rc = bit_superstep(rerun ? ~0ull : budget, r_end, &done, &off))) return rc;
                 CHL_CUDA(cudaEventRecord(ev_b, b.st));
                 CHL_CUDA(cudaMemcpyAsync(&hc, b.ctl, sizeof(hc), cudaMemcpyDeviceToHost, b.st));
                 CHL_CUDA(cudaStreamSynchronize(b.st));
@@ -2952,7 +2956,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
                 CHL_CUDA(cudaEventElapsedTime(&ms, ev_a, ev_b));
                 tree_ms += ms;
                 step_tree_ms = ms;
-                if (deep) {   // too many levels: the same roots by the other kernels
+                if (off) {   // the same roots by the other kernels
                     bits_ok = bits_now = false;
                     continue;
                 }

@@ -1,0 +1,82 @@
+"""Builds on a device with little memory (fake_device_memory.c refuses the
+allocations, on the host): what is only there for speed gives way."""
+import json
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+pytestmark = pytest.mark.gpu
+
+CHILD = r"""
+import ctypes as C, json, os, sys
+import numpy as np
+import plant_gb300 as P
+
+fake = C.CDLL(os.environ["LD_PRELOAD"])
+fake.fake_device_set.argtypes = [C.c_size_t]
+fake.fake_device_live.restype = C.c_size_t
+spec = json.loads(sys.argv[1])
+n = spec["n"]
+if spec["kind"] == "spider":
+    # legs of 31 unit arcs around a centre, vertices nearer to it ranked higher:
+    # every tree reaches all legs by via paths and labels little more than its own
+    leg = 1 + np.arange(n - 1).reshape(-1, 31)
+    src = np.concatenate([np.zeros(len(leg), np.int64), leg[:, :-1].ravel()])
+    dst = np.concatenate([leg[:, 0], leg[:, 1:].ravel()])
+    order = np.concatenate([[0], leg.T.ravel()]).astype(np.uint32)
+    g = P.Graph.from_arcs(n, src, dst, np.ones(src.size, np.int32), undirected=True)
+else:
+    # disjoint pairs: next to no labels, so the graph's copies weigh most
+    src = np.arange(0, n, 2)
+    src, dst = np.concatenate([src, src + 1]), np.concatenate([src + 1, src])
+    g = P.Graph.from_arcs(n, src, dst, 3 + (src & 1))
+    order = np.random.default_rng(1).permutation(n).astype(np.uint32)
+want = P.build(g, order, **spec["kw"])
+got = []
+for limit in spec["limits"]:
+    fake.fake_device_set(limit + fake.fake_device_live())
+    try:
+        L = P.build(g, order, **spec["kw"])
+        got.append([limit, "ok" if L.digest() == want.digest() else "wrong labels"])
+        del L
+    except P.CHLError as e:
+        got.append([limit, "status %d" % e.status])
+    fake.fake_device_set(C.c_size_t(-1).value)
+held = fake.fake_device_live()
+del want
+print(json.dumps({"got": got, "held": held, "left": fake.fake_device_live()}))
+"""
+
+
+@pytest.fixture(scope="module")
+def fake_lib(tmp_path_factory):
+    if shutil.which("gcc") is None:
+        pytest.skip("no C compiler")
+    so = str(tmp_path_factory.mktemp("fake") / "fake_device_memory.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", os.path.join(ROOT, "tests", "fake_device_memory.c"), "-o", so,
+                    "-ldl"], check=True)
+    return so
+
+
+def builds(fake_lib, kind, n, limits, **kw):
+    """Outcome of a build for each number of bytes the device has left."""
+    spec = {"kind": kind, "n": n, "kw": kw, "limits": limits}
+    r = subprocess.run([sys.executable, "-c", CHILD, json.dumps(spec)], cwd=ROOT, capture_output=True, text=True,
+                       timeout=300, env={**os.environ, "LD_PRELOAD": fake_lib})
+    assert r.returncode == 0, r.stderr
+    out = json.loads(r.stdout.splitlines()[-1])
+    assert out["left"] == 0   # a failed build gives back what it took
+    return [x for _, x in out["got"]]
+
+
+def test_bit_parallel_table_that_finds_no_room(P, fake_lib):
+    """The second bit-parallel superstep's table (5,500 committed roots, 32
+    distances: 22.5 MB) does not fit: the trees, which need none, go on."""
+    n = 1 + 500 * 31
+    assert builds(fake_lib, "spider", n, [44 << 20, 52 << 20, 1 << 30], first_superstep=5500) == ["ok"] * 3
+    assert builds(fake_lib, "spider", n, [16 << 20], first_superstep=5500) == ["status 3"]
