@@ -2449,6 +2449,29 @@ int fill_rows(Build &b, TreeArgs &ta, int sms, unsigned long long &kernels) {
     return CHL_OK;
 }
 
+// Gives back the copies of the graph that are there for speed alone: the
+// numbering (its arcs in it) and the rows.  False if there were none.
+bool drop_copies(Build &b) {
+    if (!b.newid && !b.row[0]) return false;
+    b.mem->put(b.newid);
+    b.mem->put(b.orig);
+    for (int s = 0; s < 2; ++s) {   // side 1 may be side 0's: put knows what is held
+        b.mem->put(b.off_n[s]);
+        b.mem->put(b.farc_n[s]);
+        b.mem->put(b.fhead_n[s]);
+        b.mem->put(b.row[s]);
+    }
+    return true;
+}
+
+// What get() allocates, without those copies if there is no room beside them.
+template <typename Get>
+int with_room(Build &b, Get get) {
+    int rc = get();
+    if (rc == CHL_ERR_OOM && drop_copies(b)) rc = get();
+    return rc;
+}
+
 int ensure_ent(uint2 **p, uint64_t *cap, uint64_t need) {
     if (need <= *cap) return CHL_OK;
     uint64_t c = std::max<uint64_t>(need, *cap + *cap / 2);
@@ -2607,7 +2630,12 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
             b.fhead[1] = b.fhead[0];
         }
     }
-    if (whole && n >= kNumberedFrom && (rc = number_by_cells(b, g, sms, prep_kernels))) return rc;
+    // (the numbering and the rows are for speed alone: without room the trees
+    // walk the caller's lists, and what is needed later takes their place)
+    if (whole && n >= kNumberedFrom && (rc = number_by_cells(b, g, sms, prep_kernels))) {
+        if (rc != CHL_ERR_OOM) return rc;
+        drop_copies(b);
+    }
     // key, vis and three queue arrays per warp slot (the 32-bit-key size
     // sets the schedule's warp count; the slots below use the real one)
     const size_t per_slot = (size_t)n * 20;
@@ -2671,7 +2699,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     // team_kernel's 6 n words per tree
     const size_t key_words = unit ? 1 : 2;
     const size_t ws_words = std::max((size_t)b.slots * (4 + key_words) * n, (size_t)b.win_trees * 6 * n);
-    if ((rc = b.mem->get(&b.ws_all, ws_words))) return rc;
+    if ((rc = with_room(b, [&] { return b.mem->get(&b.ws_all, ws_words); }))) return rc;
     b.ws_key = b.ws_all;
     b.ws_vis = b.ws_all + (size_t)b.slots * key_words * n;
     b.ws_front = b.ws_vis + (size_t)b.slots * n;
@@ -2720,7 +2748,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         size_t fr = 0, tot = 0;
         CHL_CUDA(cudaMemGetInfo(&fr, &tot));
         const uint64_t want = (uint64_t)(2.0 * std::sqrt((double)n) * n * b.sides) + (1u << 20);
-        if ((rc = grow_new(b, std::min<uint64_t>(want, fr / 4 / 36)))) return rc;
+        if ((rc = with_room(b, [&] { return grow_new(b, std::min<uint64_t>(want, fr / 4 / 36)); }))) return rc;
         budget_base = b.new_cap - b.new_cap / 7;
     }
     if (opts.label_cap == 0 && !whole_budget) {
@@ -2737,7 +2765,8 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         const uint64_t running = bits_ok ? 64u : std::max(b.slots, b.win_trees);
         const uint64_t want = (uint64_t)budget_base + running * b.sides * n;
         const uint64_t fit = (uint64_t)(fr / 4 / 36);
-        if ((rc = grow_new(b, std::max<uint64_t>(std::min(want, fit), std::max<uint64_t>(4ull * n, 1u << 20))))) return rc;
+        const uint64_t cap = std::max<uint64_t>(std::min(want, fit), std::max<uint64_t>(4ull * n, 1u << 20));
+        if ((rc = with_room(b, [&] { return grow_new(b, cap); }))) return rc;
     }
     uint32_t *bit_long[2] = {nullptr, nullptr};   // long lists of each direction
     unsigned long long *bit_live = nullptr;       // kBitLevels + 1 rows
@@ -2962,7 +2991,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
                 }
                 if (hc.overflow || hc.nlab > b.new_cap) {
                     ++step_reruns;
-                    if ((rc = grow_new(b, hc.nlab + hc.nlab / 4 + 1024))) return rc;
+                    if ((rc = with_room(b, [&] { return grow_new(b, hc.nlab + hc.nlab / 4 + 1024); }))) return rc;
                     r_end = done;
                     rerun = true;
                     continue;
@@ -3045,7 +3074,11 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
                         ta.g_fhead[s] = b.fhead_n[s];
                     }
                 }
-                if (rows && !prune && (rc = fill_rows(b, ta, sms, kernels))) return rc;
+                if (rows && !prune && (rc = fill_rows(b, ta, sms, kernels))) {
+                    if (rc != CHL_ERR_OOM) return rc;
+                    for (auto &r : b.row) b.mem->put(r);
+                    rows = false;
+                }
                 int fit = 0;
                 const uint32_t tw = team_warps(prune, r_end - r0);
                 if ((rc = team_blocks(plant_now, prune, tw, slots, &fit))) return rc;
@@ -3092,7 +3125,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
             if (hc.overflow || hc.nlab > b.new_cap) {
                 ++step_reruns;
                 // re-run the same root range with room for every label
-                if ((rc = grow_new(b, hc.nlab + hc.nlab / 4 + 1024))) return rc;
+                if ((rc = with_room(b, [&] { return grow_new(b, hc.nlab + hc.nlab / 4 + 1024); }))) return rc;
                 r_end = r1;
                 rerun = true;
                 continue;
@@ -3138,9 +3171,12 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         // array is sized for every new label before the chain (the clean
         // only removes labels).
         const bool clean_now = !plant_now && !bits_now && M > 0;   // bit-parallel labels are canonical
-        if ((rc = grow_sort(b, M, clean_now))) return rc;
-        if ((rc = ensure_ent(&b.ent_b, &b.ent_cap_b, committed + M))) return rc;
-        if (!last && (rc = ensure_ent(&b.dent_b, &b.dent_cap_b, committed + M))) return rc;
+        auto commit_room = [&]() -> int {
+            if ((rc = grow_sort(b, M, clean_now))) return rc;
+            if ((rc = ensure_ent(&b.ent_b, &b.ent_cap_b, committed + M))) return rc;
+            return last ? CHL_OK : ensure_ent(&b.dent_b, &b.dent_cap_b, committed + M);
+        };
+        if ((rc = with_room(b, commit_room))) return rc;
         // bits of the distance part of the (list, distance) sort key
         const int dist_bits = bits_for((uint64_t)hc.max_dist + 1);
         auto chain = [&]() -> int {

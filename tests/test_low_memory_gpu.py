@@ -80,3 +80,10 @@ def test_bit_parallel_table_that_finds_no_room(P, fake_lib):
     n = 1 + 500 * 31
     assert builds(fake_lib, "spider", n, [44 << 20, 52 << 20, 1 << 30], first_superstep=5500) == ["ok"] * 3
     assert builds(fake_lib, "spider", n, [16 << 20], first_superstep=5500) == ["status 3"]
+
+
+@pytest.mark.parametrize("n,limits", [(1 << 17, [62 << 20, 72 << 20, 1 << 30]), (60000, [27 << 20, 31 << 20, 1 << 30])])
+def test_graph_copies_that_find_no_room(P, fake_lib, n, limits):
+    """The numbering (from 2^16 vertices) and the rows of arcs, or what is
+    allocated after them, do not fit: the build goes on without them."""
+    assert builds(fake_lib, "pairs", n, limits) == ["ok"] * 3
