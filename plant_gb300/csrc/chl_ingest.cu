@@ -168,24 +168,23 @@ __device__ __forceinline__ bool snap_header(const char *p, const char *e, long l
     return full;
 }
 
-// One line per thread.  DIMACS: `p` fills the header fields; SNAP: the
-// `# Nodes:` line does.  Arcs go to unordered slots (init_arcs sorts them).
-// (one atomic per warp and line kind: a counter bumped line by line took most
-// of the 0.69 ms of a million lines)
-__device__ __forceinline__ unsigned long long take_slot(ParseOut *po, uint64_t k, bool first) {
+// An arc slot for each lane that is here, by one atomic for all of them (a
+// counter bumped line by line took most of the 0.69 ms of a million lines).
+// Lanes may meet here from different turns of the caller's loop: nothing
+// follows from the mask but their number.
+__device__ __forceinline__ unsigned long long take_slot(ParseOut *po) {
     const uint32_t m = __activemask(), lead = (uint32_t)__ffs(m) - 1u;
     unsigned long long b = 0;
-    if (lane_id() == lead) {
-        b = atomicAdd(&po->arcs, (unsigned long long)__popc(m));
-        // lanes hold ascending lines: the leader's is the warp's first
-        if (first && k < *(volatile unsigned long long *)&po->first_a) atomicMin(&po->first_a, (unsigned long long)k);
-    }
+    if (lane_id() == lead) b = atomicAdd(&po->arcs, (unsigned long long)__popc(m));
     return __shfl_sync(m, b, lead) + __popc(m & lanemask_lt());
 }
 
+// One line per thread.  DIMACS: `p` fills the header fields; SNAP: the
+// `# Nodes:` line does.  Arcs go to unordered slots (init_arcs sorts them).
 __global__ void parse_lines(const char *buf, uint64_t S, const uint64_t *nl, uint64_t nnl, uint64_t lines,
                             int fmt, ParseOut *po, int64_t *au, int64_t *av, int64_t *aw) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    unsigned long long first_a = ~0ull;   // this thread's first arc line
     for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < lines; k += stride) {
         const uint64_t start = k == 0 ? 0 : nl[k - 1] + 1;
         const bool has_nl = k < nnl;
@@ -228,7 +227,8 @@ __global__ void parse_lines(const char *buf, uint64_t S, const uint64_t *nl, uin
                 atomicOr(&po->status, kFailFormat);
                 continue;
             }
-            const unsigned long long slot = take_slot(po, k, true);
+            const unsigned long long slot = take_slot(po);
+            first_a = min(first_a, (unsigned long long)k);
             au[slot] = u;
             av[slot] = v;
             aw[slot] = 1;
@@ -250,7 +250,7 @@ __global__ void parse_lines(const char *buf, uint64_t S, const uint64_t *nl, uin
                 atomicOr(&po->status, kFailFormat);
                 continue;
             }
-            const unsigned long long slot = take_slot(po, k, false);
+            const unsigned long long slot = take_slot(po);
             au[slot] = u;
             av[slot] = v;
             aw[slot] = w;
@@ -293,7 +293,8 @@ __global__ void parse_lines(const char *buf, uint64_t S, const uint64_t *nl, uin
                 atomicOr(&po->status, kFailFormat);
                 continue;
             }
-            const unsigned long long slot = take_slot(po, k, true);
+            const unsigned long long slot = take_slot(po);
+            first_a = min(first_a, (unsigned long long)k);
             au[slot] = u;
             av[slot] = v;
             aw[slot] = w;
@@ -301,6 +302,9 @@ __global__ void parse_lines(const char *buf, uint64_t S, const uint64_t *nl, uin
         }
         atomicOr(&po->status, kFailFormat);
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) first_a = min(first_a, __shfl_xor_sync(kFull, first_a, o));
+    if (lane_id() == 0 && first_a != ~0ull) atomicMin(&po->first_a, first_a);
 }
 
 // ---- METIS (shared_memory/graph.hpp:211-256) on the device

@@ -257,3 +257,16 @@ def test_sort_key_widths(P, tmp_path, n, span):
     text = f"p sp {n} {u.size}\n" + "".join(f"a {a} {b} {c}\n" for a, b, c in zip(u, v, w))
     for undirected in (False, True):
         same(P, write(tmp_path, "k.gr", text), undirected, expect_gpu=True)
+
+
+@pytest.mark.parametrize("before", [False, True])
+def test_header_line_among_several_turns(P, tmp_path, before):
+    """More lines than threads, the header after 400,000 comments of many
+    lengths: one arc on a line before it rejects the file, none does not."""
+    rng = np.random.default_rng(6)
+    pad = ["c" + "x" * int(k) for k in rng.integers(0, 40, 400_000)]
+    arcs = [f"a {u} {v} {w}" if w else "c" for u, v, w in rng.integers(0, 50, (300_000, 3)) + [1, 1, 0]]
+    if before:
+        pad[399_990] = "a 1 2 3"
+    p = write(tmp_path, "h.gr", "\n".join(pad + ["p sp 50 300000"] + arcs) + "\n")
+    same(P, p, expect_gpu=not before)

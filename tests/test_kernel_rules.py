@@ -30,3 +30,16 @@ def test_key_words_see_atomics_of_one_width():
     assert len(on_word) >= 3
     for call in on_word:
         assert re.match(r"atomic\w+\(\s*kw \+ ", call), call
+
+
+def test_line_order_is_not_read_from_a_lane_mask():
+    """Lanes that __activemask() finds together in the line parser may be in
+    different turns of its loop, so the lowest of them need not hold the
+    smallest line: the first arc's line comes from every thread's own."""
+    src = open(os.path.join(ROOT, "plant_gb300", "csrc", "chl_ingest.cu")).read()
+    assert "__activemask()" in body("chl_ingest.cu", "take_slot(")
+    assert "first_a" not in body("chl_ingest.cu", "take_slot(")
+    assert src.count("atomicMin(&po->first_a") == 1
+    parse = body("chl_ingest.cu", "parse_lines(")
+    tail = parse[parse.rindex("kFailFormat"):]
+    assert "__shfl_xor_sync(kFull, first_a" in tail and "atomicMin(&po->first_a, first_a)" in tail
