@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 namespace chl {
@@ -72,11 +73,14 @@ __global__ void pack_arcs(uint64_t m, const uint32_t *head, const int32_t *len, 
 //     the vertices whose predecessors are all counted.
 //  3. Dependencies delta over the waves in reverse.
 // Every sum of 2 and 3 runs in adjacency order with explicitly rounded
-// operations (no contraction), matching the CPU restatement bit for bit.  On
-// the 256-square grid the kernel takes 8.2 ms, one lane per source with a
-// binary heap took 308.
+// operations (no contraction), matching the CPU restatement bit for bit.  The
+// order of a 256-square grid by 256 sources takes 7.5 ms, 308 with one lane
+// per source and a binary heap.
 // A vertex of up to kLight arcs belongs to one thread, half of its arcs in
-// flight at a time; others to one warp.
+// flight at a time; others to one warp.  Which arcs of a short list lie on
+// shortest paths is found once and kept as two bytes beside the vertex's
+// distance: phases 2 and 3 gather no distances, a trip less in either chain
+// (9.0 -> 7.5 ms).
 constexpr int kOrdThreads = 512;
 constexpr uint32_t kOrdWarps = kOrdThreads / 32;
 constexpr int kLight = 8;
@@ -84,9 +88,29 @@ constexpr int kGroup = kLight / 2;
 constexpr uint32_t kWindow = 4096;
 
 constexpr uint32_t kFarMark = 0xFFFFFFFFu;   // above every pass
+constexpr uint32_t kShort = 0x80000000u;     // both lists have at most kLight arcs, see the words below
+static_assert(kLight == 8, "a byte of a word says which arcs of a list count");
+
+// Passes and waves of at most kNarrow vertices (a lane each), none with a long
+// list, are run by warp 0 alone, one after the other, while the block waits at
+// one barrier.  Such steps cost their barriers and dependent accesses (an L2
+// atomic takes 500 cycles, a load 300), and graphs one or two vertices wide
+// consist of them: the queue stays in shared memory with what the next step
+// wants to know of its vertices, two arcs at a time keep the loops short, a
+// lone vertex needs no atomics, and phase 3 reads ahead for all waves among
+// the next 32 vertices.  16 sources of a path of 3,000 vertices 13.6 -> 4.7 ms
+// (6.1 with a lane per source, whose heap and lists one thread's L1 serves), a
+// ladder of 3,000 rungs 18.1 -> 9.6 (13.9), a directed cycle of 5,000 24.2 ->
+// 7.6 (8.1).
+constexpr uint32_t kNarrow = 32;
+constexpr std::integral_constant<int, 2> kTwo{};
+constexpr std::integral_constant<int, 4> kFour{};
 
 struct OrdShared {
     uint32_t nn, npile, nkeep, heavy, lo, kmin, kmax;
+    uint32_t a, b, c;   // state that warp 0 hands back
+    uint32_t stale;     // a queued vertex's distance fell again in the same pass
+    uint32_t q[kNarrow * kLight], qx[kNarrow * kLight];   // vertices; their distances or marks
 };
 
 __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const uint64_t *off_out, const uint2 *arc_out,
@@ -97,7 +121,9 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     const uint32_t j = blockIdx.x;
     // word of a vertex: distance in the high half; in the low one the last pass
-    // it was queued in (phase 1), the predecessors not yet counted (phase 2)
+    // it was queued in (phase 1), then (phases 2 and 3) the predecessors not yet
+    // counted and, where both its lists are short, which of their arcs lie on
+    // shortest paths: kShort | out-arcs << 16 | in-arcs << 8 | predecessors
     unsigned long long *word = ws_word + (size_t)j * n;
     auto dist_at = [&](uint32_t v) -> uint32_t { return __ldcg((const uint32_t *)(word + v) + 1); };
     auto mark_at = [&](uint32_t v) -> uint32_t * { return (uint32_t *)(word + v); };
@@ -115,14 +141,15 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
         sh.npile = 0;
         sh.lo = kInfD;
     }
-    // run body(v) by whole warps for the listed vertices with more than kLight arcs
-    auto for_heavy = [&](const uint32_t *list, uint32_t cnt, const uint64_t *off, auto body) {
+    __syncthreads();
+    // run body(v) by whole warps for the listed vertices that are long(v)
+    auto for_heavy = [&](const uint32_t *list, uint32_t cnt, auto is_long, auto body) {
         for (uint32_t i0 = warp * 32; i0 < cnt; i0 += kOrdThreads) {
             uint32_t v = 0;
             bool h = false;
             if (i0 + lane < cnt) {
                 v = __ldcg(&list[i0 + lane]);
-                h = off[v + 1] - off[v] > kLight;
+                h = is_long(v);
             }
             for (uint32_t m = __ballot_sync(kFull, h); m; m &= m - 1) body(__shfl_sync(kFull, v, __ffs(m) - 1));
         }
@@ -132,32 +159,100 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
     uint32_t nf = 1, thr = 1, width = 0, pass = 0, members = 0;
     while (true) {
         // passes over the window until no distance below thr falls
+        uint32_t lo = kInfD;   // smallest distance at or past thr this thread has set
+        // one minimum over distance and mark: the smaller distance wins and
+        // brings its mark
+        // (alone: no other thread of the block is at work)
+        auto lower = [&](uint32_t w, uint32_t dd, bool alone) {
+            const unsigned long long now = (unsigned long long)dd << 32 | (dd < thr ? pass : kFarMark);
+            if (!alone) return atomicMin(&word[w], now);
+            const unsigned long long was = word[w];
+            if (now < was) word[w] = now;
+            return was;
+        };
+        // the lists that w joins, whose word was `was` before
+        auto settle = [&](uint32_t w, uint32_t dd, unsigned long long was, auto push) {
+            const uint32_t stamp = dd < thr ? pass : kFarMark;
+            const uint32_t old = (uint32_t)(was >> 32), mark = (uint32_t)was;
+            if (dd > old || (dd == old && stamp >= mark)) return;
+            if (dd < thr) {
+                // a vertex of the far pile whose distance falls below thr
+                // leaves a stale entry there; an equal distance only takes
+                // the mark of a vertex the sweep queued: queued again
+                if (mark != pass) push(atomicAdd(&sh.nn, 1u), w);
+                else sh.stale = 1;
+            } else {
+                lo = min(lo, dd);
+                if (old == kInfD) __stcg(&pile[atomicAdd(&sh.npile, 1u)], w);
+            }
+        };
         while (nf) {
+            if (nf <= kNarrow) {
+                if (warp == 0) {
+                    uint32_t cnt = nf, v = lane < cnt ? __ldcg(&front[lane]) : s, dv = dist_at(v);
+                    bool heavy;
+                    while (true) {
+                        const bool on = lane < cnt;
+                        const uint64_t ob = on ? off_out[v] : 0, oe = on ? off_out[v + 1] : 0;
+                        heavy = __any_sync(kFull, oe - ob > kLight);
+                        if (heavy) break;
+                        ++pass;
+                        if (lane == 0) sh.nn = sh.stale = 0;
+                        __syncwarp();
+                        // no read first, and two minima on their way together
+#pragma unroll 1
+                        for (uint64_t e = ob; e < oe; e += 2) {
+                            const uint2 x = arc_out[e], y = e + 1 < oe ? arc_out[e + 1] : make_uint2(v, kInfD);
+                            const uint32_t dx = dv + x.y, dy = dv + y.y;
+                            const unsigned long long wx = dx < kInfD ? lower(x.x, dx, cnt == 1) : 0ull;
+                            const unsigned long long wy = dy < kInfD ? lower(y.x, dy, cnt == 1) : 0ull;
+                            auto queue = [&](uint32_t w, uint32_t dd, unsigned long long was) {
+                                if (dd < kInfD)
+                                    settle(w, dd, was, [&](uint32_t i, uint32_t) {
+                                        sh.q[i] = w;
+                                        sh.qx[i] = dd;
+                                    });
+                            };
+                            queue(x.x, dx, wx);
+                            queue(y.x, dy, wy);
+                        }
+                        __syncwarp();
+                        members += cnt;
+                        cnt = sh.nn;
+                        if (cnt == 0 || cnt > kNarrow) break;
+                        v = lane < cnt ? sh.q[lane] : s;
+                        dv = sh.stale ? dist_at(v) : sh.qx[lane];
+                        __syncwarp();   // the queue is read before the next pass writes it
+                    }
+                    if (heavy) {
+                        if (lane < cnt) __stcg(&front[lane], v);
+                    } else {
+                        for (uint32_t i = lane; i < cnt; i += 32) __stcg(&front[i], sh.q[i]);
+                    }
+                    if (lane == 0) {
+                        sh.a = cnt;
+                        sh.b = pass;
+                        sh.c = members;
+                        sh.heavy = heavy ? 1u : 0u;
+                    }
+                }
+                __syncthreads();
+                nf = sh.a;
+                pass = sh.b;
+                members = sh.c;
+                const bool heavy = sh.heavy != 0;
+                __syncthreads();   // the state is read before it changes
+                if (!heavy) continue;
+            }
             ++pass;
             if (tid == 0) {
                 sh.nn = 0;
                 sh.heavy = 0;
             }
             __syncthreads();
-            uint32_t lo = kInfD;   // smallest distance at or past thr this thread has set
             auto relax = [&](uint32_t w, uint32_t dd, uint32_t seen) {
                 // distances only fall: a read no larger than dd proves the atomic idle
-                if (dd >= seen) return;
-                // one minimum over distance and mark: the smaller distance wins
-                // and brings its mark
-                const uint32_t stamp = dd < thr ? pass : kFarMark;
-                const unsigned long long was = atomicMin(&word[w], (unsigned long long)dd << 32 | stamp);
-                const uint32_t old = (uint32_t)(was >> 32), mark = (uint32_t)was;
-                if (dd > old || (dd == old && stamp >= mark)) return;
-                if (dd < thr) {
-                    // a vertex of the far pile whose distance falls below thr
-                    // leaves a stale entry there; an equal distance only takes
-                    // the mark of a vertex the sweep queued: queued again
-                    if (mark != pass) __stcg(&fnext[atomicAdd(&sh.nn, 1u)], w);
-                } else {
-                    lo = min(lo, dd);
-                    if (old == kInfD) __stcg(&pile[atomicAdd(&sh.npile, 1u)], w);
-                }
+                if (dd < seen) settle(w, dd, lower(w, dd, false), [&](uint32_t i, uint32_t x) { __stcg(&fnext[i], x); });
             };
             for (uint32_t i = tid; i < nf; i += kOrdThreads) {
                 const uint32_t v = __ldcg(&front[i]);
@@ -183,7 +278,7 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
             }
             __syncthreads();
             if (sh.heavy) {
-                for_heavy(front, nf, off_out, [&](uint32_t v) {
+                for_heavy(front, nf, [&](uint32_t v) { return off_out[v + 1] - off_out[v] > kLight; }, [&](uint32_t v) {
                     const uint32_t dv = dist_at(v);
                     for (uint64_t a = off_out[v] + lane; a < off_out[v + 1]; a += 32) {
                         const uint2 hl = arc_out[a];
@@ -192,8 +287,6 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
                     __syncwarp();
                 });
             }
-            lo = __reduce_min_sync(kFull, lo);
-            if (lane == 0 && lo != kInfD) atomicMin(&sh.lo, lo);
             __syncthreads();
             members += nf;
             nf = sh.nn;
@@ -202,6 +295,9 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
             fnext = t;
             __syncthreads();   // the counters are read before the next pass clears them
         }
+        lo = __reduce_min_sync(kFull, lo);
+        if (lane == 0 && lo != kInfD) atomicMin(&sh.lo, lo);
+        __syncthreads();
         if (sh.npile == 0) break;
         if (width == 0) {
             // the first width: the spread of the source's neighbours
@@ -278,27 +374,35 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
     }
     __syncthreads();
 
-    // ---- phase 2: tight in-arcs of every reached vertex, then the waves
+    // ---- phase 2: tight arcs of every reached vertex, then the waves
     for (uint32_t v0 = warp * 32; v0 < n; v0 += kOrdThreads) {
         const uint32_t v = v0 + lane;
         bool h = false;
         if (v < n) {
             const uint32_t dv = dist_at(v);
-            const uint64_t ib = off_in[v], ie = off_in[v + 1];
-            uint32_t c = 0;
-            h = dv != kInfD && ie - ib > kLight;
-            if (dv != kInfD && !h) {
+            uint32_t mark = 0;
+            if (dv != kInfD) {
+                const uint64_t ib = off_in[v], ie = off_in[v + 1], ob = off_out[v], oe = off_out[v + 1];
+                h = ie - ib > kLight || oe - ob > kLight;
 #pragma unroll
                 for (int g = 0; g < kLight; g += kGroup) {
-                    if (ib + g >= ie) break;
-                    uint2 hl[kGroup];
+                    if (h || (ib + g >= ie && ob + g >= oe)) break;
+                    uint2 hi[kGroup], ho[kGroup];   // past an end: d(v) + 1 != d(v)
 #pragma unroll
-                    for (int q = 0; q < kGroup; ++q) hl[q] = ib + g + q < ie ? arc_in[ib + g + q] : make_uint2(v, 1u);
+                    for (int q = 0; q < kGroup; ++q) {
+                        hi[q] = ib + g + q < ie ? arc_in[ib + g + q] : make_uint2(v, 1u);
+                        ho[q] = ob + g + q < oe ? arc_out[ob + g + q] : make_uint2(v, 1u);
+                    }
 #pragma unroll
-                    for (int q = 0; q < kGroup; ++q) c += dist_at(hl[q].x) + hl[q].y == dv ? 1u : 0u;
+                    for (int q = 0; q < kGroup; ++q) {
+                        const uint32_t dw = dist_at(ho[q].x);
+                        if (dist_at(hi[q].x) + hi[q].y == dv) mark += 1u | 1u << (8 + g + q);
+                        if (dw != kInfD && dv + ho[q].y == dw) mark |= 1u << (16 + g + q);
+                    }
                 }
+                mark |= kShort;
             }
-            if (!h) __stcg(mark_at(v), c);
+            if (!h) __stcg(mark_at(v), mark);
         }
         for (uint32_t m = __ballot_sync(kFull, h); m; m &= m - 1) {
             const uint32_t x = v0 + __ffs(m) - 1;
@@ -316,58 +420,111 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
     if (tid == 0) __stcg(&seq[0], s);
     uint32_t begin = 0, end = 1, waves = 0;
     __syncthreads();
+    auto is_long = [&](uint32_t v) { return !(__ldcg(mark_at(v)) & kShort); };
+    // one predecessor of w is counted: the next wave takes w after its last
+    // (push gets its place there and w's mark)
+    auto count_down = [&](uint32_t w, bool alone, auto push) {
+        const uint32_t mark = alone ? *mark_at(w) : atomicSub(mark_at(w), 1u);
+        if (alone) *mark_at(w) = mark - 1u;
+        if ((mark & kShort ? mark & 0xFFu : mark) == 1u) push(atomicAdd(&sh.nn, 1u), mark);
+    };
+    // the first G bits of m, taken from it: arc numbers, or kLight past the last
+    auto take = [](auto &at, uint32_t &m) {
+#pragma unroll
+        for (int &q : at) {
+            q = m ? __ffs(m) - 1 : kLight;
+            m &= m - 1;
+        }
+    };
+    // sigma(v) and the vertices it completes, for a vertex of short lists, G
+    // arcs of each at a time
+    auto count_paths = [&](auto group, uint32_t v, uint32_t mark, bool alone, auto push) {
+        constexpr int G = decltype(group)::value;
+        const uint64_t ib = off_in[v], ob = off_out[v];
+        double acc = 0.0;
+#pragma unroll 1
+        for (uint32_t im = mark >> 8 & 0xFFu, om = mark >> 16 & 0xFFu; im | om;) {
+            int ai[G], ao[G];
+            uint32_t p[G], w[G];
+            double sp[G];
+            take(ai, im);
+            take(ao, om);
+#pragma unroll
+            for (int q = 0; q < G; ++q) {
+                p[q] = ai[q] < kLight ? arc_in[ib + ai[q]].x : v;
+                w[q] = ao[q] < kLight ? arc_out[ob + ao[q]].x : v;
+            }
+#pragma unroll
+            for (int q = 0; q < G; ++q) sp[q] = ai[q] < kLight ? sigma[p[q]] : 0.0;
+#pragma unroll
+            for (int q = 0; q < G; ++q)
+                if (ao[q] < kLight) count_down(w[q], alone, [&](uint32_t i, uint32_t m) { push(i, w[q], m); });
+#pragma unroll
+            for (int q = 0; q < G; ++q)
+                if (ai[q] < kLight) acc = __dadd_rn(acc, sp[q]);
+        }
+        sigma[v] = v == s ? 1.0 : acc;
+    };
     while (begin < end) {
+        if (end - begin <= kNarrow) {
+            if (warp == 0) {
+                uint32_t cnt = end - begin, v = lane < cnt ? __ldcg(&seq[begin + lane]) : s;
+                uint32_t mark = __ldcg(mark_at(v));
+                bool heavy;
+                while (true) {
+                    heavy = __any_sync(kFull, lane < cnt && !(mark & kShort));
+                    if (heavy) break;
+                    if (lane == 0) {
+                        __stcg(&wave[waves], begin);
+                        sh.nn = 0;
+                    }
+                    __syncwarp();
+                    if (lane < cnt)
+                        count_paths(kTwo, v, mark, cnt == 1, [&](uint32_t i, uint32_t w, uint32_t m) {
+                            sh.q[i] = w;
+                            sh.qx[i] = m;
+                            __stcg(&seq[end + i], w);
+                        });
+                    __syncwarp();
+                    ++waves;
+                    begin = end;
+                    cnt = sh.nn;
+                    end += cnt;
+                    if (cnt == 0 || cnt > kNarrow) break;
+                    v = lane < cnt ? sh.q[lane] : s;
+                    mark = sh.qx[lane];
+                    __syncwarp();   // the queue is read before the next wave writes it
+                }
+                if (lane == 0) {
+                    sh.a = begin;
+                    sh.b = end;
+                    sh.c = waves;
+                    sh.heavy = heavy ? 1u : 0u;
+                }
+            }
+            __syncthreads();
+            begin = sh.a;
+            end = sh.b;
+            waves = sh.c;
+            const bool heavy = sh.heavy != 0;
+            __syncthreads();   // the state is read before it changes
+            if (!heavy) continue;
+        }
         if (tid == 0) {
             __stcg(&wave[waves], begin);
             sh.nn = 0;
             sh.heavy = 0;
         }
         __syncthreads();
-        auto count_down = [&](uint32_t w, uint32_t dd, uint32_t dw) {
-            if (dd == dw && dw != kInfD && atomicSub(mark_at(w), 1u) == 1u) __stcg(&seq[end + atomicAdd(&sh.nn, 1u)], w);
-        };
+        auto push = [&](uint32_t i, uint32_t w, uint32_t) { __stcg(&seq[end + i], w); };
         for (uint32_t i = begin + tid; i < end; i += kOrdThreads) {
-            const uint32_t v = __ldcg(&seq[i]);
-            const uint64_t ib = off_in[v], ie = off_in[v + 1], ob = off_out[v], oe = off_out[v + 1];
-            const uint32_t dv = dist_at(v);
-            if (ie - ib > kLight || oe - ob > kLight) sh.heavy = 1;
-            if (ie - ib <= kLight) {
-                double acc = 0.0;
-#pragma unroll
-                for (int h = 0; h < kLight; h += kGroup) {
-                    if (ib + h >= ie) break;
-                    uint2 hl[kGroup];
-                    double sp[kGroup];
-#pragma unroll
-                    for (int q = 0; q < kGroup; ++q)
-                        hl[q] = ib + h + q < ie ? arc_in[ib + h + q] : make_uint2(v, 1u);   // d(v) + 1 != d(v)
-#pragma unroll
-                    for (int q = 0; q < kGroup; ++q)
-                        sp[q] = dist_at(hl[q].x) + hl[q].y == dv ? __ldcg(&sigma[hl[q].x]) : 0.0;
-#pragma unroll
-                    for (int q = 0; q < kGroup; ++q) acc = __dadd_rn(acc, sp[q]);
-                }
-                __stcg(&sigma[v], v == s ? 1.0 : acc);
-            }
-            if (oe - ob <= kLight) {
-#pragma unroll
-                for (int h = 0; h < kLight; h += kGroup) {
-                    if (ob + h >= oe) break;
-                    uint2 hl[kGroup];
-                    uint32_t dw[kGroup];
-#pragma unroll
-                    for (int q = 0; q < kGroup; ++q)
-                        hl[q] = ob + h + q < oe ? arc_out[ob + h + q] : make_uint2(v, 1u);
-#pragma unroll
-                    for (int q = 0; q < kGroup; ++q) dw[q] = dist_at(hl[q].x);
-#pragma unroll
-                    for (int q = 0; q < kGroup; ++q) count_down(hl[q].x, dv + hl[q].y, dw[q]);
-                }
-            }
+            const uint32_t v = __ldcg(&seq[i]), mark = __ldcg(mark_at(v));
+            if (mark & kShort) count_paths(kFour, v, mark, false, push);
+            else sh.heavy = 1;
         }
         __syncthreads();
         if (sh.heavy) {
-            for_heavy(seq + begin, end - begin, off_in, [&](uint32_t v) {
+            for_heavy(seq + begin, end - begin, is_long, [&](uint32_t v) {
                 const uint32_t dv = dist_at(v);
                 const uint64_t ie = off_in[v + 1];
                 double acc = 0.0;
@@ -375,18 +532,17 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
                     double sp = 0.0;
                     if (a + lane < ie) {
                         const uint2 hl = arc_in[a + lane];
-                        if (dist_at(hl.x) + hl.y == dv) sp = __ldcg(&sigma[hl.x]);
+                        if (dist_at(hl.x) + hl.y == dv) sp = sigma[hl.x];
                     }
                     for (uint32_t m = __ballot_sync(kFull, sp != 0.0); m; m &= m - 1)
                         acc = __dadd_rn(acc, __shfl_sync(kFull, sp, __ffs(m) - 1));
                 }
-                if (lane == 0) __stcg(&sigma[v], v == s ? 1.0 : acc);
-            });
-            for_heavy(seq + begin, end - begin, off_out, [&](uint32_t v) {
-                const uint32_t dv = dist_at(v);
+                if (lane == 0) sigma[v] = v == s ? 1.0 : acc;
                 for (uint64_t a = off_out[v] + lane; a < off_out[v + 1]; a += 32) {
                     const uint2 hl = arc_out[a];
-                    count_down(hl.x, dv + hl.y, dist_at(hl.x));
+                    const uint32_t dw = dist_at(hl.x);
+                    if (dw != kInfD && dv + hl.y == dw)
+                        count_down(hl.x, false, [&](uint32_t i, uint32_t m) { push(i, hl.x, m); });
                 }
                 __syncwarp();
             });
@@ -399,50 +555,109 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
     }
 
     // ---- phase 3: dependencies over the waves in reverse, successors in out order
-    while (waves-- > 0) {
-        begin = __ldcg(&wave[waves]);
+    auto depend = [&](uint32_t v, uint32_t mark) {   // delta(v), short lists
+        constexpr int G = kGroup;
+        const uint64_t ob = off_out[v];
+        const double sv = sigma[v];
+        double acc = 0.0;
+#pragma unroll 1
+        for (uint32_t om = mark >> 16 & 0xFFu; om;) {
+            int ao[G];
+            uint32_t w[G];
+            double sw[G], dw[G];
+            take(ao, om);
+#pragma unroll
+            for (int q = 0; q < G; ++q) w[q] = ao[q] < kLight ? arc_out[ob + ao[q]].x : v;
+#pragma unroll
+            for (int q = 0; q < G; ++q) {
+                sw[q] = ao[q] < kLight ? sigma[w[q]] : 1.0;
+                dw[q] = ao[q] < kLight ? delta[w[q]] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < G; ++q)
+                if (ao[q] < kLight) acc = __dadd_rn(acc, __dmul_rn(__ddiv_rn(sv, sw[q]), __dadd_rn(1.0, dw[q])));
+        }
+        delta[v] = v == s ? 0.0 : acc;   // the source's own dependency is not counted
+    };
+    while (waves > 0) {
+        begin = __ldcg(&wave[waves - 1]);
+        if (end - begin <= kNarrow) {
+            if (warp == 0) {
+                // the last 32 vertices of the sequence a lane each, newest first:
+                // all that does not hang on a dependency is read for all of their
+                // waves together, then the waves follow one another
+                bool heavy = false;
+                while (waves > 0 && !heavy) {
+                    const uint32_t first = lane < waves ? end - 1 - __ldcg(&wave[waves - 1 - lane]) : 32u;
+                    // lanes that hold a wave's first vertex, up to the one with a long list
+                    uint32_t firsts = __reduce_or_sync(kFull, first < 32 ? 1u << first : 0u);
+                    const bool on = lane < end;
+                    const uint32_t v = on ? __ldcg(&seq[end - 1 - lane]) : s, mark = on ? __ldcg(mark_at(v)) : kShort;
+                    const uint32_t longs = __ballot_sync(kFull, !(mark & kShort));
+                    if (longs) firsts &= (longs & (0u - longs)) - 1u;
+                    heavy = longs && !firsts;
+                    if (!firsts) break;
+                    const uint32_t below = kFull >> __clz(firsts);   // lanes of whole waves
+                    const uint64_t ob = off_out[v];
+                    const double sv = sigma[v];
+                    uint32_t om = below >> lane & 1u ? mark >> 16 & 0xFFu : 0u;
+                    int at[2];
+                    take(at, om);
+                    uint32_t w[2];
+                    double q[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        w[i] = at[i] < kLight ? arc_out[ob + at[i]].x : v;
+                        q[i] = at[i] < kLight ? __ddiv_rn(sv, sigma[w[i]]) : 0.0;
+                    }
+                    uint32_t from = 0;
+                    for (uint32_t f = firsts; f; f &= f - 1) {
+                        const uint32_t to = (uint32_t)__ffs(f);   // lanes [from, to) are a wave
+                        if (lane >= from && lane < to) {
+                            double acc = 0.0;
+#pragma unroll
+                            for (int i = 0; i < 2; ++i)
+                                if (at[i] < kLight) acc = __dadd_rn(acc, __dmul_rn(q[i], __dadd_rn(1.0, delta[w[i]])));
+                            for (uint32_t m = om; m; m &= m - 1) {
+                                const uint32_t x = arc_out[ob + __ffs(m) - 1].x;
+                                acc = __dadd_rn(acc, __dmul_rn(__ddiv_rn(sv, sigma[x]), __dadd_rn(1.0, delta[x])));
+                            }
+                            delta[v] = v == s ? 0.0 : acc;
+                        }
+                        __syncwarp();
+                        from = to;
+                    }
+                    end -= from;
+                    waves -= (uint32_t)__popc(firsts);
+                }
+                if (lane == 0) {
+                    sh.b = end;
+                    sh.c = waves;
+                    sh.heavy = heavy ? 1u : 0u;
+                }
+            }
+            __syncthreads();
+            end = sh.b;
+            waves = sh.c;
+            const bool heavy = sh.heavy != 0;
+            __syncthreads();   // the state is read before it changes
+            if (!heavy) continue;
+            begin = __ldcg(&wave[waves - 1]);
+        }
+        --waves;
         if (tid == 0) sh.heavy = 0;
         __syncthreads();
         for (uint32_t i = begin + tid; i < end; i += kOrdThreads) {
-            const uint32_t v = __ldcg(&seq[i]);
-            const uint64_t ob = off_out[v], oe = off_out[v + 1];
-            if (oe - ob > kLight) {
-                sh.heavy = 1;
-                continue;
-            }
-            const uint32_t dv = dist_at(v);
-            const double sv = __ldcg(&sigma[v]);
-            double acc = 0.0;
-#pragma unroll
-            for (int h = 0; h < kLight; h += kGroup) {
-                if (ob + h >= oe) break;
-                uint2 hl[kGroup];
-                bool on[kGroup];
-                double sw[kGroup], dw[kGroup];
-#pragma unroll
-                for (int q = 0; q < kGroup; ++q) hl[q] = ob + h + q < oe ? arc_out[ob + h + q] : make_uint2(v, 1u);
-#pragma unroll
-                for (int q = 0; q < kGroup; ++q) {
-                    const uint32_t d = dist_at(hl[q].x);
-                    on[q] = d != kInfD && dv + hl[q].y == d;
-                }
-#pragma unroll
-                for (int q = 0; q < kGroup; ++q) {
-                    sw[q] = on[q] ? __ldcg(&sigma[hl[q].x]) : 1.0;
-                    dw[q] = on[q] ? __ldcg(&delta[hl[q].x]) : 0.0;
-                }
-#pragma unroll
-                for (int q = 0; q < kGroup; ++q)
-                    if (on[q]) acc = __dadd_rn(acc, __dmul_rn(__ddiv_rn(sv, sw[q]), __dadd_rn(1.0, dw[q])));
-            }
-            __stcg(&delta[v], v == s ? 0.0 : acc);   // the source's own dependency is not counted
+            const uint32_t v = __ldcg(&seq[i]), mark = __ldcg(mark_at(v));
+            if (mark & kShort) depend(v, mark);
+            else sh.heavy = 1;
         }
         __syncthreads();
         if (sh.heavy) {
-            for_heavy(seq + begin, end - begin, off_out, [&](uint32_t v) {
+            for_heavy(seq + begin, end - begin, is_long, [&](uint32_t v) {
                 const uint64_t oe = off_out[v + 1];
                 const uint32_t dv = dist_at(v);
-                const double sv = __ldcg(&sigma[v]);
+                const double sv = sigma[v];
                 double acc = 0.0;
                 for (uint64_t a = off_out[v]; a < oe; a += 32) {
                     bool on = false;
@@ -451,13 +666,12 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
                         const uint2 hl = arc_out[a + lane];
                         const uint32_t d = dist_at(hl.x);
                         on = d != kInfD && dv + hl.y == d;
-                        if (on)
-                            t = __dmul_rn(__ddiv_rn(sv, __ldcg(&sigma[hl.x])), __dadd_rn(1.0, __ldcg(&delta[hl.x])));
+                        if (on) t = __dmul_rn(__ddiv_rn(sv, sigma[hl.x]), __dadd_rn(1.0, delta[hl.x]));
                     }
                     for (uint32_t m = __ballot_sync(kFull, on); m; m &= m - 1)
                         acc = __dadd_rn(acc, __shfl_sync(kFull, t, __ffs(m) - 1));
                 }
-                if (lane == 0) __stcg(&delta[v], v == s ? 0.0 : acc);
+                if (lane == 0) delta[v] = v == s ? 0.0 : acc;
             });
         }
         __syncthreads();
@@ -465,7 +679,6 @@ __global__ void __launch_bounds__(kOrdThreads) brandes_kernel(uint32_t n, const 
     }
 }
 
-// bc[v] = sum over sources j (in list order) of delta_j[v]
 __global__ void bc_sum(uint32_t n, uint32_t count, const double *deltas, double *bc) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         double acc = 0.0;

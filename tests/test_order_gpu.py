@@ -92,3 +92,67 @@ def test_betweenness_shapes(P, O, kind, tmp_path):
     og = O.OGraph.read_dimacs(p) if kind == "directed" else oracle_graph(P, O, g)
     for sources in (1, 40):
         assert np.array_equal(P.Order.betweenness(g, sources, seed=7), og.betweenness_order(sources, 7))
+
+
+def thin_graph(kind):
+    rng = np.random.default_rng(8)
+    if kind in ("path", "scattered_path"):
+        n = 3000
+        src, dst = np.arange(n - 1), np.arange(1, n)
+        if kind == "scattered_path":
+            ids = rng.permutation(n)
+            src, dst = ids[src], ids[dst]
+    elif kind == "cycle":
+        n = 2000
+        src, dst = np.arange(n), (np.arange(n) + 1) % n
+    elif kind.startswith("strip"):
+        wide, n = int(kind[5:]), 40 * int(kind[5:])
+        v = np.arange(n).reshape(40, wide)
+        src, dst = np.concatenate([v[:, :-1].ravel(), v[:-1].ravel()]), np.concatenate([v[:, 1:].ravel(), v[1:].ravel()])
+    elif kind == "caterpillar":   # lists of 8, 9 and 40 arcs among short ones
+        n, spine = 1500, 400
+        src, dst = [np.arange(spine - 1)], [np.arange(1, spine)]
+        at = spine
+        for v, legs in zip(range(0, spine, 9), np.resize([6, 7, 38, 1], spine)):
+            src.append(np.full(legs, v))
+            dst.append(np.arange(at, at + legs))
+            at += legs
+        src, dst = np.concatenate(src), np.concatenate(dst)
+    else:   # "thin_tree": each vertex hangs on one of the three before it
+        n = 3000
+        src = np.arange(1, n)
+        dst = np.maximum(0, src - 1 - rng.integers(0, 3, n - 1))
+    w = np.ones(src.size, int) if kind == "strip33" else rng.integers(1, 4, src.size)
+    return n, src, dst, w
+
+
+@pytest.mark.parametrize("kind", ["path", "scattered_path", "cycle", "strip2", "strip4", "strip5", "strip31", "strip32",
+                                  "strip33", "strip70", "caterpillar", "thin_tree"])
+def test_betweenness_narrow_steps(P, O, kind, tmp_path):
+    """Passes and waves around 32 vertices (run by one warp), around one, and
+    long lists among them."""
+    n, src, dst, w = thin_graph(kind)
+    g = P.Graph.from_arcs(n, src.astype(np.uint32), dst.astype(np.uint32), w.astype(np.int32),
+                          undirected=kind != "cycle")
+    p = str(tmp_path / "g.gr")
+    g.write(p)
+    og = O.OGraph.read_dimacs(p) if kind == "cycle" else oracle_graph(P, O, g)
+    for sources in (1, 24):
+        assert np.array_equal(P.Order.betweenness(g, sources, seed=3), og.betweenness_order(sources, 3))
+
+
+@pytest.mark.parametrize("kind,most", [("path", 9.0), ("cycle", 6.0)])
+def test_betweenness_of_thin_graphs_is_no_crawl(P, kind, most):
+    """Steps of one or two vertices are not paid at a block's price: 13.6 and
+    9.8 ms with block barriers around each, 6.1 and 3.6 with a lane per source,
+    4.7 and 3.1 with a warp for them."""
+    import time
+    n, src, dst, w = thin_graph(kind)
+    g = P.Graph.from_arcs(n, src.astype(np.uint32), dst.astype(np.uint32), w.astype(np.int32),
+                          undirected=kind != "cycle")
+    best = np.inf
+    for _ in range(7):
+        t = time.perf_counter()
+        P.Order.betweenness(g, 16, seed=1)
+        best = min(best, (time.perf_counter() - t) * 1e3)
+    assert best < most
