@@ -2734,11 +2734,13 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     // 20: 16-64 within 3%)
     // (bit-parallel supersteps have no largest tree to wait for and pay for
     // every commit: RMAT scale 20 342 ms with 128, 309 with 512)
-    const double sf = opts.sf > 0 ? opts.sf : bits_ok ? 512.0 : heavy_tail ? 32.0 : 1024.0;
     // label_limit = sf * N counts both sides' labels (shared_memory/hhl.cpp:65);
     // a symmetric build stores one side.
-    unsigned long long budget_base =
-        (unsigned long long)std::max(1.0, sf * (double)n / (b.sides == 1 ? 2.0 : 1.0));
+    auto label_budget = [&]() -> unsigned long long {
+        const double sf = opts.sf > 0 ? opts.sf : bits_ok ? 512.0 : heavy_tail ? 32.0 : 1024.0;
+        return (unsigned long long)std::max(1.0, sf * (double)n / (b.sides == 1 ? 2.0 : 1.0));
+    };
+    unsigned long long budget_base = label_budget();
     // Supersteps of unpruned trees (whole) end at the label buffer, which has
     // room for lists of 1.7 sqrt(n) (grids have 0.7 to 1.5 sqrt(n)) within a
     // quarter of the free memory; a seventh of it is left to the trees still
@@ -2805,17 +2807,24 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     // them from the whole rule start with two roots per warp of the schedule
     // and grow by half of the committed prefix.
     const bool gll_auto = !heavy_tail && opts.mode == CHL_MODE_GLL && win_target > 1 && opts.first_superstep == 0;
-    const uint32_t auto_first = bits_ok ? 2 * kBitRoots
-                                : win_target > 1 && (heavy_tail || gll_auto) ? std::max<uint32_t>(64u, sms)
-                                : heavy_tail ? 1024u
-                                             : std::max<uint32_t>(64u, 2 * b.warps);
-    const double auto_growth = bits_ok ? 3.0 : heavy_tail ? 8.0 : gll_auto ? 2.0 : 0.5;
+    // (a build that leaves the bit-parallel kernel goes on by the schedule of
+    // the others: step_end and label_budget are asked again)
+    auto step_end = [&](uint32_t from) -> uint32_t {
+        const uint32_t auto_first = bits_ok ? 2 * kBitRoots
+                                    : win_target > 1 && (heavy_tail || gll_auto) ? std::max<uint32_t>(64u, sms)
+                                    : heavy_tail ? 1024u
+                                                 : std::max<uint32_t>(64u, 2 * b.warps);
+        const double auto_growth = bits_ok ? 3.0 : heavy_tail ? 8.0 : gll_auto ? 2.0 : 0.5;
+        const uint32_t first = opts.first_superstep ? opts.first_superstep : auto_first;
+        const double growth = opts.growth > 0 ? opts.growth : auto_growth;
+        const uint64_t size = std::max<uint64_t>(first, (uint64_t)(growth * (double)from));
+        const uint32_t end = (uint32_t)std::min<uint64_t>(n, (uint64_t)from + size);
+        return opts.root_limit ? std::min<uint32_t>(end, opts.root_limit) : end;
+    };
     // phase switch ratio (the reference's -ps, default 1024): auto 8 on
     // heavy-tailed graphs (RMAT scale 20: pruned GLL supersteps after the
     // first are faster than PLaNT trees there)
     const double ps = opts.ps > 0 ? opts.ps : (heavy_tail ? 8.0 : 1024.0);
-    const uint32_t first = opts.first_superstep ? opts.first_superstep : auto_first;
-    const double growth = opts.growth > 0 ? opts.growth : auto_growth;
     // The roots [r0, r_end) by bit_level, a batch at a time until the label
     // budget is spent; *done: the first root not taken, *off: gave up, at
     // kBitLevels or for want of room for the table (up to 4 KB per committed
@@ -2944,13 +2953,11 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         const uint32_t r_begin = r0;
         bit_hi = 0;
         const bool plant_now = do_plant;
-        const unsigned long long budget = budget_base;
+        unsigned long long budget = budget_base;
         // trees without prune tests, over all roots that are left
         const bool unpruned = whole && plant_now && !ratio_stopped;
-        uint64_t size = std::max<uint64_t>(first, (uint64_t)(growth * (double)r0));
-        uint32_t r_end = (uint32_t)std::min<uint64_t>(n, (uint64_t)r0 + size);
-        if (unpruned) r_end = n;
-        if (opts.root_limit) r_end = std::min<uint32_t>(r_end, opts.root_limit);
+        uint32_t r_end = step_end(r0);
+        if (unpruned) r_end = opts.root_limit ? std::min<uint32_t>(n, opts.root_limit) : n;
         BuildCtl hc;
         bool rerun = false;
         uint32_t step_reruns = 0;
@@ -2985,8 +2992,11 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
                 CHL_CUDA(cudaEventElapsedTime(&ms, ev_a, ev_b));
                 tree_ms += ms;
                 step_tree_ms = ms;
-                if (off) {   // the same roots by the other kernels
+                if (off) {   // these roots by the other kernels
                     bits_ok = bits_now = false;
+                    if (rerun) continue;   // over the same range
+                    r_end = step_end(r0);
+                    budget = budget_base = label_budget();
                     continue;
                 }
                 if (hc.overflow || hc.nlab > b.new_cap) {

@@ -397,3 +397,27 @@ def test_rows_of_arcs(P, O, directed, n, tmp_path):
     for kw in ({}, {"mode": MODES["gll"]}, {"mode": MODES["plant"]}, {"window_warps": 1}, {"window_warps": 2},
                {"window_warps": 4}, {"window_warps": 8, "window_target": 16}, {"first_superstep": 30}):
         assert same_labels(P.build(g, order, **kw), ref, n), kw
+
+
+@pytest.mark.parametrize("mode", list(MODES))
+def test_deep_unit_graphs_keep_the_trees_schedule(P, mode):
+    """A heavy-tailed unit-length graph deeper than 64 levels leaves the
+    bit-parallel kernel: its first superstep is then the trees' (one root per
+    SM), not 2,048 roots whose trees nothing prunes."""
+    g0 = P.Graph.rmat(13, 8, seed=3)
+    off, head, _ = g0.csr(True)
+    src, dst = np.repeat(np.arange(g0.get_n()), np.diff(off.astype(np.int64))), head.astype(np.int64)
+    keep = src < dst
+    n, tail = g0.get_n() + 200, np.arange(g0.get_n(), g0.get_n() + 200)
+    src = np.concatenate([src[keep], [0], tail[:-1]])
+    dst = np.concatenate([dst[keep], tail])
+    g = P.Graph.from_arcs(n, src, dst, np.ones(src.size, np.int32), undirected=True)
+    order = P.Order.degree(g, seed=1)
+    L = P.build(g, order, mode=MODES[mode])
+    assert L.digest() == P.build(g, order, window_target=1).digest()
+    assert L.stats()["visits"] < 3_000_000
+    if mode == "hybrid":
+        assert L.stats()["plant_roots"] < 1024
+    for kw in ({"first_superstep": 300}, {"label_cap": 2000}, {"sf": 0.5}, {"root_limit": 100}):
+        a, b = P.build(g, order, mode=MODES[mode], **kw), P.build(g, order, mode=MODES[mode], window_target=1, **kw)
+        assert a.digest() == b.digest(), kw
