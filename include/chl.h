@@ -225,12 +225,14 @@ typedef struct chl_build_stats {
                               labels into the committed label arrays      */
     double h2d_ms;         /* graph/order upload                            */
     uint64_t labels;       /* total label entries (both sides)              */
-    uint64_t visits;       /* vertices settled over all trees               */
+    uint64_t visits;       /* vertices settled over all trees (bit-parallel
+                              ones: whole levels)                         */
     uint64_t label_reads;  /* label entries read by prune tests             */
-    uint64_t arcs;         /* arcs relaxed                                  */
+    uint64_t arcs;         /* arcs relaxed: those of the settled vertices that
+                              were not pruned                             */
     uint32_t supersteps;
     uint32_t plant_roots;  /* roots built as un-pruned PLaNT trees          */
-    uint64_t tree_launches;
+    uint64_t tree_launches;   /* launches of the kernels that build trees  */
     uint64_t kernel_launches;
     double avg_label;
 } chl_build_stats;

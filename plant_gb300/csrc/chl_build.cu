@@ -1655,6 +1655,7 @@ struct BitArgs {
     int sides, f;                   // trees of side f: rows are pulled over the reverse arcs
     const uint64_t *roff;
     const uint2 *rhead;
+    const uint64_t *foff;           // lists of the arcs the trees follow (statistics)
     const uint32_t *order, *rank;
     const uint64_t *l_off;
     const uint2 *l_ent, *l_dent;
@@ -1718,7 +1719,11 @@ __global__ void bit_roots(BitArgs a) {
     a.nxt[(size_t)v * kBitWords + wd] = make_ulonglong2(bit, 0ull);
     a.seen[(size_t)v * kBitWords + wd] = bit;
     if (bit) atomicOr(&a.live_out[wd], bit);
-    if (wd == 0) a.act_out[v] = 1;
+    if (wd == 0) {
+        a.act_out[v] = 1;
+        atomicAdd(&a.ctl->arcs, (unsigned long long)(a.foff[v + 1] - a.foff[v]));
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.ctl->visits, (unsigned long long)a.nb);
     bit_emit(a, gm, wd, v, bit);
 }
 
@@ -1745,7 +1750,7 @@ __global__ void __launch_bounds__(kBitThreads) bit_level(BitArgs a) {
     const unsigned long long live = a.live[wd];
     const unsigned long long valid =
         a.nb >= 64u * wd + 64u ? ~0ull : (a.nb > 64u * wd ? (1ull << (a.nb - 64u * wd)) - 1ull : 0ull);
-    unsigned long long c_new = 0, c_reads = 0, nv_any = 0;
+    unsigned long long c_new = 0, c_reads = 0, c_arcs = 0, nv_any = 0;
     const uint32_t step = HEAVY ? gridDim.x : gridDim.x * kBitGroups;
     for (uint32_t it = HEAVY ? blockIdx.x : blockIdx.x * kBitGroups + grp; it < items; it += step) {
         const uint32_t w = HEAVY ? a.heavy[1 + it] : it;
@@ -1836,6 +1841,7 @@ __global__ void __launch_bounds__(kBitThreads) bit_level(BitArgs a) {
                 a.nxt[(size_t)w * kBitWords + wd] = make_ulonglong2(left, left & via);
                 const unsigned long long nv = left & ~via;
                 nv_any |= nv;
+                c_arcs += (unsigned long long)__popcll(left) * (a.foff[w + 1] - a.foff[w]);
                 bit_emit(a, gm, wd, w, nv);
             }
         }
@@ -1847,8 +1853,10 @@ __global__ void __launch_bounds__(kBitThreads) bit_level(BitArgs a) {
     for (int o = 16; o > 0; o >>= 1) {
         c_new += __shfl_xor_sync(kFull, c_new, o);
         c_reads += __shfl_xor_sync(kFull, c_reads, o);
+        c_arcs += __shfl_xor_sync(kFull, c_arcs, o);
     }
     if (lane_id() == 0) {
+        if (c_arcs) atomicAdd(&a.ctl->arcs, c_arcs);
         if (c_new) atomicAdd(&a.ctl->visits, c_new);
         if (c_reads) atomicAdd(&a.ctl->label_reads, c_reads);
     }
@@ -2869,6 +2877,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
                 a.f = f;
                 a.roff = b.dg->off[rev];
                 a.rhead = b.fhead[rev];
+                a.foff = b.dg->off[f];
                 a.order = b.order;
                 a.rank = b.rank;
                 a.l_off = b.off_a;
@@ -2903,7 +2912,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
                 }
                 CHL_CUDA(cudaGetLastError());
                 kernels += r0 ? 2 : 1;
-                ++launches;
+                launches += r0 ? 2 : 1;
                 for (uint32_t d = 1;; ++d) {
                     if (d > kBitLevels) {
                         *off = true;
@@ -2926,6 +2935,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
                     }
                     CHL_CUDA(cudaGetLastError());
                     kernels += 2;
+                    launches += 2;
                     unsigned long long live[kBitWords], any = 0;
                     CHL_CUDA(cudaMemcpyAsync(live, a.live_out, sizeof(live), cudaMemcpyDeviceToHost, b.st));
                     CHL_CUDA(cudaStreamSynchronize(b.st));

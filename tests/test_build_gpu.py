@@ -421,3 +421,42 @@ def test_deep_unit_graphs_keep_the_trees_schedule(P, mode):
     for kw in ({"first_superstep": 300}, {"label_cap": 2000}, {"sf": 0.5}, {"root_limit": 100}):
         a, b = P.build(g, order, mode=MODES[mode], **kw), P.build(g, order, mode=MODES[mode], window_target=1, **kw)
         assert a.digest() == b.digest(), kw
+
+
+def test_bit_parallel_statistics(P):
+    """Visits and arcs of bit-parallel trees, against a level-by-level search
+    of every root with PLaNT's via flags; every level's launches counted."""
+    rng = np.random.default_rng(3)
+    n = 700
+    src = np.concatenate([np.zeros(500, np.int64), rng.integers(0, n, 2500)])
+    dst = np.concatenate([rng.permutation(np.arange(1, n))[:500], rng.integers(0, n, 2500)])
+    keep = src != dst
+    g = P.Graph.from_arcs(n, src[keep], dst[keep], np.ones(int(keep.sum()), np.int32))
+    order = P.Order.degree(g, seed=2)
+    rank = np.empty(n, np.int64)
+    rank[order] = np.arange(n)
+    st = P.build(g, order, mode=MODES["plant"]).stats()
+    visits = arcs = levels = 0
+    for forward in (True, False):
+        off, head, _ = g.csr(forward)
+        deg = np.diff(off.astype(np.int64))
+        adj = np.zeros((n, n), bool)
+        adj[np.repeat(np.arange(n), deg), head] = True
+        depth = 0
+        for r in range(n):
+            seen, new, via, d = np.zeros(n, bool), np.zeros(n, bool), np.zeros(n, bool), 0
+            new[order[r]] = True
+            while True:
+                seen |= new
+                visits += int(new.sum())
+                arcs += int(deg[new].sum())
+                if not (new & ~via).any():
+                    break
+                nxt = adj[new].any(0) & ~seen
+                via = nxt & (adj[new & via].any(0) | (rank < r))
+                new = nxt
+                d += 1
+            depth = max(depth, d)
+        levels += depth
+    assert st["supersteps"] == 1 and (st["visits"], st["arcs"]) == (visits, arcs)
+    assert st["tree_launches"] == 2 + 2 * levels
