@@ -719,20 +719,22 @@ __global__ void scatter_mean_bwd(uint32_t n, const float *dA, const uint64_t *of
     }
 }
 
-// acc[k][c] += x^T dz0 (k < NF) and sum dz0 (k = NF), in double: a block's
-// warps walk its vertices (2 channels per lane), their sums meet in shared
-// memory, and the block adds them to acc.  One thread per (k, c) walking all
-// vertices took 5.5 ms for 2^15 of them.
+// part[block][k][c]: x^T dz0 (k < NF) and sum dz0 (k = NF) over the block's
+// vertices, in double.  A block's warps walk its vertices (2 channels per
+// lane) and are added up in order, as grad_w0_out adds up the blocks: the same
+// graph gives the same bits.  One thread per (k, c) walking all vertices took
+// 5.5 ms for 2^15 of them.
 constexpr int kGw0Threads = 256;
+constexpr int kGw0Blocks = 192;      // at most (one per SM)
+constexpr int kGw0 = (NF + 1) * H;   // sums
+constexpr int kGw0Parts = 32;        // threads per sum of grad_w0_out, 32 sums a block
 
-__global__ void __launch_bounds__(kGw0Threads) grad_w0(uint32_t n, const float *x, const float *dz, double *acc) {
-    __shared__ double sum[(NF + 1) * H];
-    for (int i = threadIdx.x; i < (NF + 1) * H; i += blockDim.x) sum[i] = 0.0;
-    __syncthreads();
-    const uint32_t lane = lane_id();
+__global__ void __launch_bounds__(kGw0Threads) grad_w0(uint32_t n, const float *x, const float *dz, double *part) {
+    __shared__ double sum[kGw0Threads / 32][kGw0];
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     double a[NF + 1][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-    for (uint32_t v = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); v < n; v += warps) {
+    for (uint32_t v = blockIdx.x * (blockDim.x >> 5) + warp; v < n; v += warps) {
         const float2 d = *(const float2 *)(dz + (size_t)v * H + 2 * lane);
 #pragma unroll
         for (int k = 0; k <= NF; ++k) {
@@ -743,18 +745,30 @@ __global__ void __launch_bounds__(kGw0Threads) grad_w0(uint32_t n, const float *
     }
 #pragma unroll
     for (int k = 0; k <= NF; ++k) {
-        atomicAdd(&sum[k * H + 2 * lane], a[k][0]);
-        atomicAdd(&sum[k * H + 2 * lane + 1], a[k][1]);
+        sum[warp][k * H + 2 * lane] = a[k][0];
+        sum[warp][k * H + 2 * lane + 1] = a[k][1];
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < (NF + 1) * H; i += blockDim.x) atomicAdd(&acc[i], sum[i]);
+    for (int i = threadIdx.x; i < kGw0; i += blockDim.x) {
+        double t = 0.0;
+        for (int w = 0; w < kGw0Threads / 32; ++w) t += sum[w][i];
+        part[(size_t)blockIdx.x * kGw0 + i] = t;
+    }
 }
 
-__global__ void grad_w0_out(const double *acc, float *dW0, float *db0) {
-    for (int i = threadIdx.x; i < (NF + 1) * H; i += blockDim.x) {
-        if (i < NF * H) dW0[i] += (float)acc[i];
-        else db0[i - NF * H] += (float)acc[i];
+__global__ void __launch_bounds__(32 * kGw0Parts) grad_w0_out(const double *part, int blocks, float *dW0, float *db0) {
+    __shared__ double sum[kGw0Parts][32];
+    const int i = blockIdx.x * 32 + lane_id(), q = threadIdx.x >> 5;
+    double t = 0.0;
+    for (int j = q; j < blocks; j += kGw0Parts) t += part[(size_t)j * kGw0 + i];
+    sum[q][lane_id()] = t;
+    for (int w = kGw0Parts / 2; w > 0; w >>= 1) {
+        __syncthreads();
+        if (q < w) sum[q][lane_id()] += sum[q + w][lane_id()];
     }
+    if (q) return;
+    if (i < NF * H) dW0[i] += (float)sum[0][lane_id()];
+    else db0[i - NF * H] += (float)sum[0][lane_id()];
 }
 
 __global__ void adam_step(size_t np, float *p, const float *g, float *m, float *vv, float lr, float b1, float b2,
@@ -807,8 +821,8 @@ struct chl_gnn {
 
 namespace {
 
-// doubles of the column sums and squared deviations, or of dW0 and db0
-constexpr size_t kAccBytes = sizeof(double) * (2 * kStatBlocks * NF > (NF + 1) * H ? 2 * kStatBlocks * NF : (NF + 1) * H);
+// doubles of the column sums and squared deviations, or of dW0's and db0's parts
+constexpr size_t kAccBytes = sizeof(double) * std::max(2 * kStatBlocks * NF, kGw0Blocks * kGw0);
 
 size_t param_count(uint32_t layers) { return kP0 + (size_t)layers * kPL + H + 1; }
 
@@ -976,9 +990,9 @@ int backward(chl_gnn *M, GraphDev &G, double *loss) {
         scatter_mean_bwd<<<sms * 8, 256>>>(n, M->dA.as<float>(), G.off_in, G.head_in, M->inv.as<float>(), hp, dz, mb);
         if ((rc = G.join())) return rc;
     }
-    CHL_CUDA(cudaMemset(M->acc.p, 0, kAccBytes));
-    grad_w0<<<std::max(1, std::min(sms, (int)((n + 63) / 64))), kGw0Threads>>>(n, M->x.as<float>(), dz, M->acc.as<double>());
-    grad_w0_out<<<1, 256>>>(M->acc.as<double>(), Gp, Gp + NF * H);
+    const int blocks = std::max(1, std::min({sms, kGw0Blocks, (int)((n + 63) / 64)}));
+    grad_w0<<<blocks, kGw0Threads>>>(n, M->x.as<float>(), dz, M->acc.as<double>());
+    grad_w0_out<<<kGw0 / 32, 32 * kGw0Parts>>>(M->acc.as<double>(), blocks, Gp, Gp + NF * H);
     CHL_CUDA(cudaGetLastError());
     CHL_CUDA(cudaMemcpy(loss, M->loss.p, 8, cudaMemcpyDeviceToHost));
     return CHL_OK;

@@ -290,3 +290,21 @@ def test_hubs_summed_by_blocks(P, into):
         assert abs(loss - l_emu) <= 1e-4 * l_emu
         for bname, sl in blocks(LAYERS):
             assert rel(grad[sl], g_emu[sl]) < EMU_REL, bname
+
+
+def test_first_layer_gradient_is_repeatable(P):
+    """W0's and b0's gradients are summed in a fixed order.  Two copies of a
+    grid with opposite residuals (targets 0 and twice the score) cancel to what
+    rounding leaves, where any other order shows."""
+    side = 60
+    v = np.arange(2 * side * side).reshape(2, side, side)
+    src = np.concatenate([v[:, :, :-1].ravel(), v[:, :-1].ravel()])
+    dst = np.concatenate([v[:, :, 1:].ravel(), v[:, 1:].ravel()])
+    g = P.Graph.from_arcs(v.size, src, dst, np.ones(src.size, np.int32), undirected=True)
+    net = P.RankNet(LAYERS, seed=5)
+    y = net.predict(g, seed=1) * np.repeat(np.float32([0, 2]), side * side)
+    first = slice(0, 4 * 64)
+    _, want = net.grad(g, y, seed=1)
+    assert np.any(want[first])   # not the exact cancellation, which any order gives
+    for _ in range(40):
+        assert np.array_equal(net.grad(g, y, seed=1)[1][first], want[first])
