@@ -204,8 +204,8 @@ typedef struct chl_build_opts {
                              q > 1: split above q (about q / 4 near)        */
     uint32_t window_target; /* large trees are searched label-correcting in
                              distance windows of about this many vertices:
-                             0 auto (1024; on road-like graphs 512 below 2^18
-                             vertices and 2048 from 2^19), 1 off (batched
+                             0 auto (1024; on road-like graphs 512 below
+                             3 * 2^16 vertices and 2048 from 2^19), 1 off (batched
                              settle rounds)                                 */
     uint32_t window_warps; /* warps building one such tree: 0 auto (32 in
                              supersteps of at most two roots per SM, else 8 on

@@ -2585,14 +2585,16 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         rows = past <= n / 8;
     }
     // vertices per distance window of the team kernel (1: settle rounds by the
-    // IN criterion instead).  Grids: 512 and 1,024 within 3% of each other,
-    // smaller graphs better with 512 (the 100-square grid 1.8 against 1.9 ms),
-    // large ones with wider windows (512-square trees 94.6, 90.3, 93.3 ms with
-    // 512, 1,024, 2,048; 768-square 330.8 and 328.6 with 1,024 and 2,048;
-    // 1024-square 887 and 863; 1448-square 1,330 and 1,297)
+    // IN criterion instead).  Larger graphs' trees are better with wider
+    // windows: tree ms of grids of 400 to 900 squared with 512, 1,024 and 2,048
+    //   160,000 vertices  36.0  36.2  39.1      462,000  221.0  207.1  208.2
+    //   202,500           56.7  54.8  58.1      524,000  263.3  245.5  245.7
+    //   262,000           85.7  83.2  86.7      590,000  334.3  308.4  305.5
+    //   360,000          142.1 135.2 138.4      810,000  566.1  514.4  500.7
+    // so the lines lie at 3 * 2^16 and 2^19
     const uint32_t win_target = opts.window_target ? opts.window_target
                                 : heavy_tail       ? 1024u
-                                : n < (1u << 18)   ? 512u
+                                : n < (3u << 16)   ? 512u
                                 : n < (1u << 19)   ? 1024u
                                                    : 2048u;
     // Road-like graphs build whole: PLaNT trees without prune tests are exact

@@ -460,3 +460,14 @@ def test_bit_parallel_statistics(P):
         levels += depth
     assert st["supersteps"] == 1 and (st["visits"], st["arcs"]) == (visits, arcs)
     assert st["tree_launches"] == 2 + 2 * levels
+
+
+@pytest.mark.parametrize("side", [443, 444, 724, 725])
+def test_window_widths_of_large_grids(P, side):
+    """Either side of the sizes where windows get wider (3 * 2^16 and 2^19
+    vertices): the labels of the top hubs are those of any other width."""
+    g = P.Graph.grid(side, side, seed=3)
+    order = P.Order.degree(g, seed=1)
+    want = P.build(g, order, root_limit=300, window_target=64).digest()
+    for kw in ({}, {"window_target": 512}, {"window_target": 2048, "window_warps": 4}):
+        assert P.build(g, order, root_limit=300, **kw).digest() == want, kw
