@@ -18,6 +18,11 @@
  *  - Handles are opaque and owned by the caller; free them with chl_*_free.
  *    Mutating calls on one handle must not run concurrently.
  *    chl_query_batch may run concurrently on distinct streams.
+ *  - Between calls the library keeps up to 1 GB of idle device memory per
+ *    device (its calls' temporaries) and up to 12 MB of pinned host memory.
+ *    Its own allocations take the idle device memory back when they find no
+ *    room; other allocators of the process cannot: chl_graph_release_device,
+ *    on any graph, gives it back.
  *  - The engine runs on the current CUDA device.  There is no CPU fallback:
  *    if no device is usable, GPU entry points return CHL_ERR_CUDA.
  */
@@ -114,6 +119,8 @@ int chl_graph_export(const chl_graph *g, int forward, uint64_t *off, uint32_t *h
  * with their input resident in HBM (no counterpart: the reference is CPU
  * only).  chl_graph_free releases it. */
 int chl_graph_to_device(chl_graph *g);
+/* Free that copy (none: no error), and give back to the device what the
+ * library keeps idle there between calls. */
 int chl_graph_release_device(chl_graph *g);
 void chl_graph_free(chl_graph *g);
 

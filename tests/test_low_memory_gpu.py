@@ -87,3 +87,27 @@ def test_graph_copies_that_find_no_room(P, fake_lib, n, limits):
     """The numbering (from 2^16 vertices) and the rows of arcs, or what is
     allocated after them, do not fit: the build goes on without them."""
     assert builds(fake_lib, "pairs", n, limits) == ["ok"] * 3
+
+
+def test_idle_memory_is_bounded_and_given_back(P):
+    """What the library keeps between calls stays below 1 GB and goes back to
+    the device when a graph's device copy is released."""
+    import ctypes as C
+    rt = C.CDLL("libcudart.so.13")
+
+    def free():
+        f, t = C.c_size_t(), C.c_size_t()
+        assert rt.cudaMemGetInfo(C.byref(f), C.byref(t)) == 0
+        return f.value
+
+    g = P.Graph.grid(300, 300, seed=1)
+    order = P.Order.betweenness(g, 64, seed=1)
+    P.build(g, order)
+    g.release_device()
+    at_first = free()
+    for _ in range(3):
+        P.build(g, order)
+        P.Order.betweenness(g, 64, seed=1)
+    assert at_first - free() <= (1 << 30) + (64 << 20)
+    g.release_device()
+    assert at_first - free() <= 64 << 20
