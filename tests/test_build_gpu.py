@@ -471,3 +471,24 @@ def test_window_widths_of_large_grids(P, side):
     want = P.build(g, order, root_limit=300, window_target=64).digest()
     for kw in ({}, {"window_target": 512}, {"window_target": 2048, "window_warps": 4}):
         assert P.build(g, order, root_limit=300, **kw).digest() == want, kw
+
+
+@pytest.mark.parametrize("directed", [False, True])
+def test_numbered_trees_again_and_in_part(P, directed):
+    """Renumbered graphs (2^16 vertices and more): supersteps run again after
+    an overflow, ended by a root limit, and with few trees at a time."""
+    side = 260
+    rng = np.random.default_rng(2)
+    i = rng.permutation(side * side).reshape(side, side)
+    u = np.concatenate([i[:, :-1].ravel(), i[:-1].ravel()])
+    v = np.concatenate([i[:, 1:].ravel(), i[1:].ravel()])
+    if directed:
+        u, v = np.concatenate([u, v]), np.concatenate([v, u])
+    for length in (rng.integers(1, 100, u.size), np.ones(u.size, np.int64)):
+        g = P.Graph.from_arcs(side * side, u, v, length, undirected=not directed)
+        order = P.Order.betweenness(g, 48, seed=2)
+        want = P.build(g, order, window_target=1, root_limit=3000).digest()
+        for kw in ({}, {"label_cap": 100_000}, {"max_warps": 64}, {"sf": 3.0}, {"label_cap": 3_000_000, "max_warps": 500}):
+            assert P.build(g, order, root_limit=3000, **kw).digest() == want, kw
+        whole = P.build(g, order)
+        assert P.build(g, order, label_cap=1_000_000).digest() == whole.digest()

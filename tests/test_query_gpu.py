@@ -143,3 +143,73 @@ def test_export_again(P):
     pairs[654_321, 1] = g.get_n()
     with pytest.raises(P.CHLError):
         P.query(L, pairs)
+
+
+class Device:
+    """Arrays in device memory through the CUDA runtime that the library uses."""
+
+    def __init__(self):
+        import ctypes as C
+        self.C, self.held = C, []
+        self.rt = C.CDLL("libcudart.so.13")
+        self.rt.cudaMemcpy.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
+        self.rt.cudaFree.argtypes = [C.c_void_p]
+
+    def put(self, a):
+        p = self.C.c_void_p()
+        assert self.rt.cudaMalloc(self.C.byref(p), self.C.c_size_t(a.nbytes)) == 0
+        self.held.append(p)
+        assert self.rt.cudaMemcpy(p, a.ctypes.data, a.nbytes, 1) == 0
+        return p
+
+    def get(self, p, like):
+        out = np.empty_like(like)
+        assert self.rt.cudaMemcpy(out.ctypes.data, p, out.nbytes, 2) == 0
+        return out
+
+    def free(self):
+        for p in self.held:
+            self.rt.cudaFree(p)
+
+    def sms(self):
+        v = self.C.c_int()
+        assert self.rt.cudaDeviceGetAttribute(self.C.byref(v), 16, 0) == 0   # multiprocessor count
+        return v.value
+
+
+@pytest.mark.parametrize("more", [-1, 0, 1, 2, 3, 60001])
+def test_device_query_groups(P, O, more):
+    """Device pairs around the size from which a warp takes four at a time
+    (64 * 32 per SM), remainders of a group included: lists of lengths at the
+    edges of chunks, empty ones, vertices out of range; nothing is written past
+    the last answer."""
+    rng = np.random.default_rng(4)
+    lens = [0, 1, 2, 31, 32, 33, 63, 64, 65, 96, 97, 200]
+    lists = []
+    for i, c in enumerate(lens):
+        lists.append(np.sort(rng.choice(300, c, replace=False)))
+        lists.append(np.arange(c) * 7 + 1000 * (i % 2))
+        lists.append(np.sort(rng.choice(4000, c, replace=False)))
+    n = len(lists) // 2
+    off = np.zeros(2 * n + 1, np.uint64)
+    off[1:] = np.cumsum([len(h) for h in lists])
+    hub = np.concatenate(lists).astype(np.uint32)
+    dist = rng.integers(0, 10**6, hub.size).astype(np.int32)
+    L = P.Labeling.from_csr(n, off, hub, dist)
+    ref = O.OLabels.from_csr(n, off, hub, dist)
+    dev = Device()
+    try:
+        k = dev.sms() * 64 * 32 + more
+        pairs = rng.integers(0, n, (k, 2)).astype(np.uint32)
+        out_of_range = rng.random(k) < 0.01
+        pairs[out_of_range, rng.integers(0, 2, k)[out_of_range]] = rng.choice([n, n + 1, 2**31, 2**32 - 1])
+        out = np.full(k + 64, -7, np.int32)
+        dp, do = dev.put(pairs), dev.put(out)
+        assert P.lib().chl_query_batch_device(L._h, dp, k, do, None) == P.CHL_OK
+        got = dev.get(do, out)
+    finally:
+        dev.free()
+    want = np.full(k, P.INFTY, np.int32)
+    want[~out_of_range] = ref.query(pairs[~out_of_range])
+    assert np.array_equal(got[:k], want)
+    assert (got[k:] == -7).all()
