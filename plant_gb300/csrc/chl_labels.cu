@@ -85,8 +85,7 @@ int tmp_alloc(void **p, size_t bytes, cudaStream_t s) {
     if (e == cudaErrorMemoryAllocation && pool) {
         // give back what the pool keeps, then once more
         cudaGetLastError();
-        cudaStreamSynchronize(s);
-        cudaMemPoolTrimTo(pool, 0);
+        tmp_trim();
         e = pooled ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMalloc(p, bytes);
     }
     if (e != cudaSuccess) {
@@ -103,16 +102,19 @@ void tmp_free(void *p, size_t bytes, cudaStream_t s) {
     else cudaFree(p);
 }
 
+// A trim gives back only what was freed before a synchronise, and temporaries
+// are freed on whichever stream their call ran on.
 void tmp_trim() {
-    if (cudaMemPool_t pool = tmp_pool()) cudaMemPoolTrimTo(pool, 0);
+    if (cudaMemPool_t pool = tmp_pool()) {
+        if (cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
+        cudaMemPoolTrimTo(pool, 0);
+    }
 }
 
 cudaError_t long_malloc(void **p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e == cudaErrorMemoryAllocation) {
-        // what was freed on a stream goes back to the pool at a synchronise
         cudaGetLastError();
-        cudaDeviceSynchronize();
         tmp_trim();
         e = cudaMalloc(p, bytes);
     }
