@@ -2687,12 +2687,20 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
     };
     // root hash slots: at most 2048 per warp-built tree within CHL_SMEM_CAP_KB
     // of shared memory per block, and 4096 per block-built one
+    int max_smem = 0;
+    CHL_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, 0));
+    // A kernel's limit of dynamic shared memory belongs to the process: it is
+    // always raised to the same value, so that builds of other threads never
+    // find it below what they launch with.  (The occupancy query counts a
+    // block's dynamic shared memory only up to that limit, 48 KB by default.)
+    auto allow_smem = [&](TreeKernel k) -> int {
+        CHL_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+        return CHL_OK;
+    };
     auto team_blocks = [&](bool plant, bool prune, uint32_t tw, uint32_t hash_slots, int *blocks) -> int {
-        // the occupancy query counts a block's dynamic shared memory only up
-        // to the kernel's current limit (48 KB by default): raise it first
         TreeKernel k = team_kernel_for(unit, plant, prune, rows, tw);
         const int sm = (int)team_smem((int)tw * 32, hash_slots);
-        CHL_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+        if ((rc = allow_smem(k))) return rc;
         CHL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, tw * 32, sm));
         *blocks = std::max(*blocks, 1) * sms;
         return CHL_OK;
@@ -2719,8 +2727,6 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
         // memory per block (measured on the 1024-square grid: 2048 slots at 2
         // resident blocks per SM beat 1024 slots at 3 by 1.3x -- entries past
         // half the table are searched in global memory)
-        int max_smem = 0;
-        CHL_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, 0));
         const size_t smem_cap = std::min<size_t>((size_t)max_smem, CHL_SMEM_CAP_KB * 1024);
         uint32_t t = 64;
         while (2 * t <= 2048 && kWarpsPerBlock * batch_smem_per_warp(2 * t) <= smem_cap) t *= 2;
@@ -3123,7 +3129,7 @@ int build_labels(const chl_graph *g, const uint32_t *order_h, uint32_t n,
                     CHL_CUDA(cudaMemsetAsync(b.ws_all, 0xFF, (size_t)b.slots * key_words * n * 4, b.st));
                 b.ws_layout = layout;
             }
-            CHL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_launch));
+            if ((rc = allow_smem(kern))) return rc;
             CHL_CUDA(cudaEventRecord(ev_a, b.st));
             kern<<<grid, block, smem_launch, b.st>>>(ta);
             step_slots = (uint32_t)grid * (uint32_t)block / 32;

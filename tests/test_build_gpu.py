@@ -492,3 +492,38 @@ def test_numbered_trees_again_and_in_part(P, directed):
             assert P.build(g, order, root_limit=3000, **kw).digest() == want, kw
         whole = P.build(g, order)
         assert P.build(g, order, label_cap=1_000_000).digest() == whole.digest()
+
+
+def test_builds_of_several_threads(P):
+    """Builds at once, whose kernels want different amounts of shared memory,
+    neither fail nor change each other's labels."""
+    import threading
+    rng = np.random.default_rng(1)
+    graphs = [P.Graph.rmat(12, 8, seed=1), P.Graph.grid(60, 60, seed=2)]
+    for i, (n, m) in enumerate([(300, 1200), (2000, 20000), (4000, 16000), (900, 9000)]):
+        src, dst = rng.integers(0, n, m), rng.integers(0, n, m)
+        keep = src != dst
+        graphs.append(P.Graph.from_arcs(n, src[keep], dst[keep], rng.integers(1, 100, int(keep.sum())),
+                                        undirected=bool(i % 2)))
+    orders = [P.Order.degree(g, seed=1) for g in graphs]
+    opts = [{}, {"mode": 1}, {"first_superstep": 64}, {"window_target": 1},
+            {"mode": 2, "first_superstep": 50, "window_warps": 2}]
+    want = [[P.build(g, o, **kw).digest() for kw in opts] for g, o in zip(graphs, orders)]
+    bad = []
+
+    def work(seed):
+        r = np.random.default_rng(seed)
+        for _ in range(60):
+            i, j = int(r.integers(len(graphs))), int(r.integers(len(opts)))
+            try:
+                if P.build(graphs[i], orders[i], **opts[j]).digest() != want[i][j]:
+                    bad.append((i, j, "other labels"))
+            except P.CHLError as e:
+                bad.append((i, j, str(e)))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(12)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
