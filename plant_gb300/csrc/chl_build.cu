@@ -10,8 +10,9 @@
 //
 // Design (one process, one GPU):
 //  * Roots are taken in rank order in supersteps.  A persistent kernel runs
-//    one tree per warp; warps pull roots from a device counter until the
-//    superstep's label budget (sf * n, the reference's label_limit) is spent.
+//    one tree per block or warp, or 1,024 at once (below); its blocks pull
+//    roots from a device counter until the superstep's label budget (sf * n,
+//    the reference's label_limit) is spent.
 //  * Every tree prunes only against labels committed by EARLIER supersteps
 //    (read-only during the kernel), so a superstep's output does not depend
 //    on warp scheduling.
@@ -959,14 +960,13 @@ constexpr int kTeamArcs = 4;      // arcs in flight per thread
 constexpr int kRowArcs = 4;       // arc records per row: one per lane of a group
 constexpr int kRowSteps = 3;      // steps of 8 vertices in flight per warp (512-square trees 90.4, 86.8, 85.9, 95.5 ms with 1 to 4)
 constexpr int kItem = 8;          // label entries per lane and step of a prune test
-#ifndef CHL_TEAM_WARPS
-#define CHL_TEAM_WARPS 48
-#endif
 // Register budget, as resident warps per SM.  The chains leave a scheduler
 // idle most of the time, so more warps pay even at the cost of registers:
 // trees of a 512-square grid 159 ms with 20 unpruned warps, 117 with 32, 95
 // with 48; pruned ones (1024-square grid, label budget 1024 n) 1.32 s with 20,
-// 1.27 with 28, 1.33 with 32.
+// 1.27 with 28, 1.33 with 32.  The budget costs spills: unpruned trees of 2 to
+// 8 warps have 40 registers and spill up to 16 bytes, 32 to 80 where they read
+// rows; pruned ones have 72 or 80 and spill 48 to 140.
 constexpr int team_warps_per_sm(bool prune) { return prune ? 28 : 48; }
 
 struct TeamShared {
@@ -1213,7 +1213,7 @@ __global__ void __launch_bounds__(T, team_warps_per_sm(PRUNE) * 32 / T) team_ker
             };
 
             // one pass over rows: four lanes per vertex, so that a row is one
-            // access, eight vertices per step and up to four steps in flight
+            // access, eight vertices per step and up to kRowSteps steps in flight
             auto pass_rows = [&]() {
                 const uint32_t steps = min((nf + T / 4 - 1) / (T / 4), (uint32_t)kRowSteps);
                 const uint32_t g = lane / kRowArcs, slot = lane % kRowArcs;
@@ -1604,11 +1604,12 @@ using TreeKernel = void (*)(TreeArgs);
 
 template <bool UNIT, bool PLANT, bool PRUNE, bool ROWS>
 TreeKernel team_kernel_tw(uint32_t tw) {
+    if constexpr (!PRUNE)   // pruned trees never take 32 warps
+        if (tw == 32) return team_kernel<UNIT, PLANT, PRUNE, ROWS, 1024>;
     switch (tw) {
     case 1: return team_kernel<UNIT, PLANT, PRUNE, ROWS, 32>;
     case 2: return team_kernel<UNIT, PLANT, PRUNE, ROWS, 64>;
     case 8: return team_kernel<UNIT, PLANT, PRUNE, ROWS, 256>;
-    case 32: return team_kernel<UNIT, PLANT, PRUNE, ROWS, 1024>;
     default: return team_kernel<UNIT, PLANT, PRUNE, ROWS, 128>;
     }
 }

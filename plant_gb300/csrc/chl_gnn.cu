@@ -816,7 +816,6 @@ struct chl_gnn {
     uint64_t step = 0;
     // per-graph scratch (grown on demand)
     DevBuf x, hb, mb, dz, dA, s, ds, y, loss, wt, inv, acc;
-    uint32_t cached_n = 0;
 };
 
 namespace {
