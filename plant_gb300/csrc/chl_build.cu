@@ -1842,7 +1842,7 @@ __global__ void __launch_bounds__(kBitThreads) bit_level(BitArgs a) {
                 a.nxt[(size_t)w * kBitWords + wd] = make_ulonglong2(left, left & via);
                 const unsigned long long nv = left & ~via;
                 nv_any |= nv;
-                c_arcs += (unsigned long long)__popcll(left) * (a.foff[w + 1] - a.foff[w]);
+                c_arcs += (unsigned long long)__popcll(left) * (a.sides == 1 ? e - b : a.foff[w + 1] - a.foff[w]);
                 bit_emit(a, gm, wd, w, nv);
             }
         }
