@@ -725,7 +725,7 @@ __global__ void scatter_mean_bwd(uint32_t n, const float *dA, const uint64_t *of
 // graph gives the same bits.  One thread per (k, c) walking all vertices took
 // 5.5 ms for 2^15 of them.
 constexpr int kGw0Threads = 256;
-constexpr int kGw0Blocks = 192;      // at most (one per SM)
+constexpr int kGw0Rows = 64;         // vertices per block, at least
 constexpr int kGw0 = (NF + 1) * H;   // sums
 constexpr int kGw0Parts = 32;        // threads per sum of grad_w0_out, 32 sums a block
 
@@ -820,8 +820,8 @@ struct chl_gnn {
 
 namespace {
 
-// doubles of the column sums and squared deviations, or of dW0's and db0's parts
-constexpr size_t kAccBytes = sizeof(double) * std::max(2 * kStatBlocks * NF, kGw0Blocks * kGw0);
+// the column sums and squared deviations
+constexpr size_t kAccBytes = sizeof(double) * 2 * kStatBlocks * NF;
 
 size_t param_count(uint32_t layers) { return kP0 + (size_t)layers * kPL + H + 1; }
 
@@ -916,7 +916,7 @@ int ensure_scratch(chl_gnn *M, uint32_t n) {
     int rc;
     if ((rc = M->x.ensure((size_t)n * NF * 4)) || (rc = M->hb.ensure((size_t)(L + 1) * n * H * 2)) ||
         (rc = M->mb.ensure((size_t)(L + 1) * n * H * 2)) || (rc = M->dz.ensure((size_t)n * H * 4)) ||
-        (rc = M->inv.ensure((size_t)n * 4)) || (rc = M->dA.ensure((size_t)n * K2 * 4)) ||
+        (rc = M->inv.ensure((size_t)n * 4)) || (rc = M->dA.ensure(std::max((size_t)n * K2 * 4, kGw0 * sizeof(double)))) ||
         (rc = M->s.ensure((size_t)n * 4)) || (rc = M->ds.ensure((size_t)n * 4)) || (rc = M->y.ensure((size_t)n * 4)) ||
         (rc = M->loss.ensure(8)) || (rc = M->acc.ensure(kAccBytes)) || (rc = M->wt.ensure((size_t)2 * H * H * 4)))
         return rc;
@@ -989,9 +989,11 @@ int backward(chl_gnn *M, GraphDev &G, double *loss) {
         scatter_mean_bwd<<<sms * 8, 256>>>(n, M->dA.as<float>(), G.off_in, G.head_in, M->inv.as<float>(), hp, dz, mb);
         if ((rc = G.join())) return rc;
     }
-    const int blocks = std::max(1, std::min({sms, kGw0Blocks, (int)((n + 63) / 64)}));
-    grad_w0<<<blocks, kGw0Threads>>>(n, M->x.as<float>(), dz, M->acc.as<double>());
-    grad_w0_out<<<kGw0 / 32, 32 * kGw0Parts>>>(M->acc.as<double>(), blocks, Gp, Gp + NF * H);
+    // the parts go to dA, which is done with: 512 bytes per vertex (2 KB at
+    // least, one part) against 2 KB per kGw0Rows vertices
+    const int blocks = std::max(1, std::min(sms, (int)((n + kGw0Rows - 1) / kGw0Rows)));
+    grad_w0<<<blocks, kGw0Threads>>>(n, M->x.as<float>(), dz, M->dA.as<double>());
+    grad_w0_out<<<kGw0 / 32, 32 * kGw0Parts>>>(M->dA.as<double>(), blocks, Gp, Gp + NF * H);
     CHL_CUDA(cudaGetLastError());
     CHL_CUDA(cudaMemcpy(loss, M->loss.p, 8, cudaMemcpyDeviceToHost));
     return CHL_OK;

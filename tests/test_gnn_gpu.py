@@ -308,3 +308,18 @@ def test_first_layer_gradient_is_repeatable(P):
     assert np.any(want[first])   # not the exact cancellation, which any order gives
     for _ in range(40):
         assert np.array_equal(net.grad(g, y, seed=1)[1][first], want[first])
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 63, 64, 65, 129])
+def test_gradient_of_few_vertices(P, n):
+    """Vertex counts at the edges of the first layer's blocks of 64: no residual,
+    no gradient; else finite ones, the same bits each time."""
+    src = np.arange(n - 1)
+    g = P.Graph.from_arcs(n, src, src + 1, np.ones(n - 1, np.int32), undirected=True)
+    net = P.RankNet(LAYERS, seed=3)
+    y = net.predict(g, seed=1)
+    loss, grad = net.grad(g, y, seed=1)
+    assert loss == 0 and not np.any(grad)
+    _, a = net.grad(g, y + 1, seed=1)
+    _, b = net.grad(g, y + 1, seed=1)
+    assert np.array_equal(a[:4 * 64], b[:4 * 64]) and np.all(np.isfinite(a))
