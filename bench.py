@@ -14,14 +14,16 @@ label build (all roots, canonical labels) with the graph resident in HBM.
   e2e    : labels/s through the C ABI from host buffers: graph + order
            upload, build, and the labels read back to host memory, timed on
            the host around each step
-  roofline: tree kernel, algorithmic bytes / tree-kernel time.  The bytes
-           are sequential PLL's (roots one at a time in rank order, each
-           tree pruned with the complete labels of higher-ranked hubs):
-           8 B per entry of every settled vertex's label list, per out-arc
-           of every settled vertex and per label written, counted once per
-           workload by oracle/pll_trace.py into profiles/pll_trace_*.json;
-           without such a file, the closed form over the labelled vertices
-           (a lower bound) stands in
+  roofline: the tree launch's DRAM traffic over its time.  The traffic is
+           that of a smaller grid's launch (profiles/), as a ratio to
+           sequential PLL's bytes and scaled by them.  Those bytes over the
+           trees' time stand apart as sequential_work_*: roots one at a time
+           in rank order, each tree pruned with the complete labels of
+           higher-ranked hubs, 8 B per entry of every settled vertex's label
+           list, per out-arc of every settled vertex and per label written,
+           counted once per workload by oracle/pll_trace.py into
+           profiles/pll_trace_*.json; without such a file, the closed form
+           over the labelled vertices (a lower bound) stands in
   cpu_baseline: the CPU restatement of the reference GLL (OpenMP, all host
            cores), estimated for the whole build from replays of a sample of
            its supersteps, each from its committed state (the complete labels
@@ -189,6 +191,22 @@ def profile_traffic():
         return None
 
 
+def roofline(tree_ms, launches, work, traffic_ratio, peak, peak_kind):
+    """The tree launches against the HBM: the DRAM traffic of one (measured on
+    a smaller grid, as a ratio to sequential PLL's bytes) over its time, and,
+    apart from that, the rate at which sequential PLL's bytes are disposed of
+    -- work, not traffic: unpruned and bit-parallel trees do not read the label
+    lists counted there, so it may pass the bandwidth."""
+    ms = tree_ms / max(1, launches)
+    traffic = work / max(1, launches) * traffic_ratio if traffic_ratio else None
+    gbs = traffic / (ms / 1e3) / 1e9 if traffic else None
+    rate = work / (tree_ms / 1e3) / 1e9
+    return {"bound": "hbm", "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak if gbs else None,
+            "peak_kind": peak_kind, "traffic": traffic, "ms_per_launch": ms, "tree_launches": launches,
+            "tree_ms_per_build": tree_ms, "sequential_work_bytes_per_build": work,
+            "sequential_work_gbs": rate, "sequential_work_over_peak": rate / peak}
+
+
 def profile_trace(args):
     """Sequential PLL work counts of this workload (oracle/pll_trace.py), or
     None when no trace is committed for it."""
@@ -349,7 +367,8 @@ def build_work_bytes(L, g):
 
 def schedule_used(g):
     """The tuned-schedule table line chl_build applies to g (autotune on), or
-    the built-in defaults when the table has no line for g's class."""
+    the built-in defaults when the table has no line for g's class or one that
+    leaves every option automatic."""
     cls = g.graph_class()
     path = os.environ.get("CHL_SCHEDULES") or os.path.join(ROOT, "plant_gb300", "tuned_schedules.txt")
     try:
@@ -358,8 +377,9 @@ def schedule_used(g):
                 t = line.split()
                 if t and not line.startswith("#") and t[0] == cls:
                     keys = ("first_superstep", "growth", "sf", "queue_split", "window_target", "window_warps", "ps")
-                    return {"class": cls, "source": os.path.basename(path),
-                            "table": dict(zip(keys, (float(x) for x in t[1:])))}
+                    table = dict(zip(keys, (float(x) for x in t[1:])))
+                    if any(table.values()):
+                        return {"class": cls, "source": os.path.basename(path), "table": table}
     except OSError:
         pass
     return {"class": cls, "source": "built-in defaults"}
@@ -579,9 +599,7 @@ def run_ours(args, ws, rank):
     trace = profile_trace(args)
     work = float(trace["algorithmic_bytes"]) if trace else labelled
     avg_tree_ms = float(np.mean(tree_ms))
-    per_launch_tree = avg_tree_ms / max(1, stats[-1]["tree_launches"])
     peak, peak_kind = peaks()
-    achieved = work / (avg_tree_ms / 1e3) / 1e9
     # grids build in unpruned blocks, heavy-tailed unit graphs mostly bit-parallel
     tree_kernel = "team_kernel" if args.workload == "grid" else "bit_level"
     traffic = profile_traffic() if args.workload == "grid" else None
@@ -619,23 +637,16 @@ def run_ours(args, ws, rank):
         "clocks": ck.summary(),
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
         "gpu_launches": launches,
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "peak_kind": peak_kind,
-                     "traffic": (work / max(1, stats[-1]["tree_launches"])
-                                 * traffic["dram_per_trace_byte" if trace else "dram_per_labelled_byte"]
-                                 if traffic and ("dram_per_trace_byte" in traffic or not trace) else None),
+        "roofline": {**roofline(avg_tree_ms, stats[-1]["tree_launches"], work,
+                                traffic.get("dram_per_trace_byte" if trace else "dram_per_labelled_byte")
+                                if traffic else None, peak, peak_kind),
                      "traffic_note": ("bytes per launch, scaled from " + traffic["workload"] + " (ncu)"
-                                      if traffic else None),
-                     "kernel": tree_kernel, "algorithmic_bytes_per_build": work,
+                                      if traffic else "no capture of this workload's kernel"),
+                     "kernel": tree_kernel,
                      "work_model": ("sequential PLL trace, profiles/pll_trace_" + workload_slug(args) + ".json"
                                     if trace else "labelled vertices only (closed form, lower bound)"),
                      "labelled_bytes_per_build": labelled,
-                     "pll_scanned_bytes_per_build": (float(trace["scanned_bytes"]) if trace else None),
-                     "work_note": ("sequential PLL's bytes over our tree time; unpruned trees do not read the label "
-                                   "lists counted there, so the ratio may pass 1" if tree_kernel == "team_kernel"
-                                   else None),
-                     "tree_ms_per_build": avg_tree_ms, "tree_launches": stats[-1]["tree_launches"],
-                     "ms_per_launch": per_launch_tree},
+                     "pll_scanned_bytes_per_build": (float(trace["scanned_bytes"]) if trace else None)},
         "build": {"build_s": ms_step / 1e3, "avg_label": stats[-1]["avg_label"], "labels": labels,
                   "supersteps": stats[-1]["supersteps"], "tree_ms": avg_tree_ms,
                   "commit_ms": float(np.mean([s["commit_ms"] for s in stats])),

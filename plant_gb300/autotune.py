@@ -2,20 +2,21 @@
 
 The build's speed depends on seven schedule knobs: the roots in the first
 superstep, the superstep growth factor, the label budget per superstep, the
-queue size at which a tree's queue is split into near and far parts, the
-window size and warps per tree of the first superstep's label-correcting
-trees, and the PLaNT-to-GLL phase switch ratio.  The labels never depend on them (canonical labels are unique for an
-order), and the labels of the hubs of rank < R are final once the roots below
-R are processed, so every candidate is timed on the same exact work: a prefix
-build of the roots of rank < R (``root_limit``; the whole build when
-``fraction`` is 1).  The search is coordinate descent over the knobs; the
+queue size at which a warp-built tree's queue is split into near and far
+parts, the window size and warps per tree of the block-built (label-correcting)
+trees, and the PLaNT-to-GLL phase switch ratio.  The labels never depend on
+them (canonical labels are unique for an order), and the labels of the hubs of
+rank < R are final once the roots below R are processed, so every candidate is
+timed on the same exact work: a prefix build of the roots of rank < R
+(``root_limit``; the whole build when ``fraction`` is 1).  The search is coordinate descent over the knobs; the
 winner is cached in a JSON file keyed by the graph's class, so graphs of the
 same kind skip the search.
 
 The library reads the winners too: ``write_table`` writes them as the text
 table that ``chl_build`` consults when ``autotune`` is set (options left at 0
-take the class's value).  ``tuned_schedules.txt`` beside the library ships
-the schedules measured on GB300 for the benchmark graphs' classes.
+take the class's value).  ``tuned_schedules.txt`` beside the library holds the
+classes of the two 2^20-vertex benchmark graphs with every option 0: the
+built-in defaults, which no candidate beat by more than 1% there.
 
 No reference counterpart: the reference's superstep size is the fixed label
 budget ``-s`` (shared_memory/hhl.cpp:65).
@@ -38,8 +39,8 @@ FIRST = (0, 256, 1024, 4096)      # 0: the built-in choice from graph statistics
 GROWTH = (0.0, 0.5, 1.0, 2.0)     # 0.0: built-in
 SF = (0.0, 32.0, 128.0, 1024.0)   # label budget per superstep (x n); 0.0: built-in
 QSPLIT = (0, 1, 512, 4096)        # near/far queue split size; 0: built-in, 1: off
-WTARGET = (0, 1, 256, 1024, 4096) # first-superstep window size; 0: built-in, 1: settle rounds
-WWARPS = (0, 4, 8)                # warps per first-superstep tree; 0: built-in
+WTARGET = (0, 1, 256, 1024, 4096) # window size of block-built trees; 0: built-in, 1: settle rounds
+WWARPS = (0, 4, 8)                # warps per block-built tree; 0: built-in
 PS = (0.0, 8.0, 64.0, 1024.0)     # hybrid phase switch ratio; 0.0: built-in
 KNOBS = (("first_superstep", FIRST), ("growth", GROWTH), ("sf", SF), ("queue_split", QSPLIT),
          ("window_target", WTARGET), ("window_warps", WWARPS), ("ps", PS))

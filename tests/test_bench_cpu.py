@@ -96,3 +96,27 @@ def test_reference_arm_loads_no_product_code(tmp_path):
     assert line["cpu_baseline"]["kind"] == "port" and line["e2e"]["h2d_bytes_per_step"] == 0
     assert 0.01 < line["full_build"]["estimate_over_full"] < 100   # a tiny graph: timing noise only
     assert probe == {"plant_imported": False, "libchl_mapped": False}
+
+
+def test_schedule_names_the_table_only_where_it_sets_something(P, tmp_path, monkeypatch):
+    import bench
+    g = P.Graph.grid(20, 20, seed=1)
+    path = tmp_path / "sched.txt"
+    monkeypatch.setenv("CHL_SCHEDULES", str(path))
+    path.write_text(f"# comment\n{g.graph_class()} 0 0.0 0.0 0 0 0 0.0\n")
+    assert bench.schedule_used(g) == {"class": g.graph_class(), "source": "built-in defaults"}
+    path.write_text(f"{g.graph_class()} 0 0.0 64.0 0 0 0 0.0\n")
+    got = bench.schedule_used(g)
+    assert got["source"] == "sched.txt" and got["table"]["sf"] == 64.0
+
+
+def test_roofline_is_of_traffic():
+    """The fraction of the bandwidth counts DRAM traffic; sequential PLL's
+    bytes over the trees' time stand apart (5.8 TB in 0.8 s is more than the
+    HBM moves)."""
+    import bench
+    r = bench.roofline(800.0, 1, 5.8e12, 0.224, 6786.0, "measured")
+    assert abs(r["achieved"] - 5.8e12 * 0.224 / 0.8 / 1e9) < 1e-6 and abs(r["frac"] - r["achieved"] / 6786.0) < 1e-12
+    assert r["frac"] < 1 < r["sequential_work_over_peak"]
+    r = bench.roofline(800.0, 4, 5.8e12, None, 6786.0, "measured")
+    assert r["achieved"] is None and r["frac"] is None and r["ms_per_launch"] == 200.0
