@@ -314,14 +314,15 @@ void chl_labels_free(chl_labels *l);
  * (shared_memory/labeling.hpp:56-65) over a batch, as batchLocalQuery does
  * (distributed_memory/query_funcs.hpp:23-30): out[i] = d(pairs[2i] ->
  * pairs[2i+1]), CHL_INFTY if the labels share no hub.  pairs/out are HOST
- * pointers (copied in and out on `stream`, a cudaStream_t or NULL). */
+ * pointers; the work is queued on `stream`, a cudaStream_t or NULL, through
+ * pinned host memory that the library keeps, and has ended on return. */
 int chl_query_batch(const chl_labels *l, const uint32_t *pairs, size_t k,
                     int32_t *out, void *stream);
 /* Allocation-free variant of chl_query_batch (no counterpart in the
  * reference).  For callers that cannot let a library allocate device memory:
  * processes whose HBM is already divided up by their own pool allocator, and
- * latency-critical request loops that cannot afford cudaMalloc/cudaFree and
- * their implicit synchronisation.  Same inputs, outputs and answers as
+ * latency-critical request loops that cannot afford allocations and their
+ * implicit synchronisation.  Same inputs, outputs and answers as
  * chl_query_batch, but the pairs and answers are staged through one
  * file-scope device array of CHL_NOALLOC_MAX_PAIRS pairs (12 MiB, held by
  * every GPU that loads the library until exit); larger k is rejected with

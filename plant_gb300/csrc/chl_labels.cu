@@ -768,14 +768,13 @@ extern "C" int chl_query_bench(const chl_labels *l, size_t k, uint64_t seed, int
 
 // ------------------------------------------------- allocation-free queries
 //
-// chl_query_batch stages the pairs and the answers in device memory it
-// allocates per call.  Some callers cannot let a library allocate device
-// memory: serving processes whose HBM is already carved up by their own
-// pool allocator (a cudaMalloc here would fail or fragment it), and
-// latency-critical request loops where cudaMalloc/cudaFree and their
-// implicit synchronisation are not acceptable.  chl_query_batch_noalloc
-// answers the same queries with the same kernel, staging through one
-// file-scope device array instead.
+// chl_query_batch may upload host-only labels and pin host memory for its
+// slots on a call.  Some callers cannot let a library allocate: serving
+// processes whose HBM is already carved up by their own pool allocator (a
+// cudaMalloc here would fail or fragment it), and latency-critical request
+// loops where allocations and their implicit synchronisation are not
+// acceptable.  chl_query_batch_noalloc answers the same queries with the same
+// kernel, staging through one file-scope device array instead.
 //
 // The array holds CHL_NOALLOC_MAX_PAIRS pairs (8 B) plus as many answers
 // (4 B): 12 MiB, resident on every GPU that loads this library until the
