@@ -315,7 +315,8 @@ void chl_labels_free(chl_labels *l);
  * (distributed_memory/query_funcs.hpp:23-30): out[i] = d(pairs[2i] ->
  * pairs[2i+1]), CHL_INFTY if the labels share no hub.  pairs/out are HOST
  * pointers; the work is queued on `stream`, a cudaStream_t or NULL, through
- * pinned host memory that the library keeps, and has ended on return. */
+ * pinned host memory or, for large batches, device memory that the library
+ * keeps, and has ended on return. */
 int chl_query_batch(const chl_labels *l, const uint32_t *pairs, size_t k,
                     int32_t *out, void *stream);
 /* Allocation-free variant of chl_query_batch (no counterpart in the

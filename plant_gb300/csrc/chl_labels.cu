@@ -838,7 +838,7 @@ extern "C" int chl_query_batch_noalloc(const chl_labels *l, const uint32_t *pair
     return CHL_OK;
 }
 
-// Host pairs are answered through pinned slots that the kernel reads and
+// Small batches of host pairs are answered through pinned slots that the kernel reads and
 // writes over the host link itself: no device staging and no copies to order,
 // one launch per slot, the host copies of one slot under the kernel of the
 // others.  (Device staging per call: 190 us for one pair, of which the kernel
@@ -850,6 +850,15 @@ namespace {
 constexpr size_t kSlotPairs = 32768;
 constexpr int kSlots = 4;
 constexpr size_t kManyPairs = 1u << 19;
+// Batches of six slots and more are staged whole in device memory from the
+// pool: one launch, without the ends of the slots' kernels and their reads
+// over the host link.  Pairs and ms a call through the slots and staged, alone
+// and from eight threads at once (labels of RMAT-14; of a 512-square grid):
+//     100,000  0.135 0.118, 0.069 0.085;  0.325 0.257, 0.255 0.229
+//     150,000  0.182 0.150, 0.095 0.100;  0.447 0.356, 0.348 0.307
+//     200,000  0.253 0.193, 0.130 0.118;  0.592 0.462, 0.479 0.387
+//   2,000,000  1.82  0.92,  1.28  0.68;   4.86  3.62,  4.62  3.21
+constexpr size_t kStagedPairs = 6 * kSlotPairs;
 constexpr size_t kSetsKept = 8;   // 12 MB pinned
 
 struct SlotSet {
@@ -934,6 +943,21 @@ int query_slots(const chl_labels *l, const uint32_t *pairs, size_t k, int32_t *o
     return CHL_OK;
 }
 
+int query_staged(const chl_labels *l, const uint32_t *pairs, size_t k, int32_t *out, cudaStream_t st) {
+    TmpSet t(st);
+    uint32_t *dp;
+    int32_t *dout;
+    int rc;
+    if ((rc = t.get(&dp, 2 * k)) || (rc = t.get(&dout, k))) return rc;
+    cudaError_t e = cudaMemcpyAsync(dp, pairs, k * 8, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) rc = query_launch(l, dp, k, dout, st);
+    if (e == cudaSuccess && !rc) e = cudaMemcpyAsync(out, dout, k * 4, cudaMemcpyDeviceToHost, st);
+    const cudaError_t e2 = cudaStreamSynchronize(st);
+    if (rc) return rc;
+    if (e == cudaSuccess) e = e2;
+    return e == cudaSuccess ? CHL_OK : cuda_status(e, "query copies", __FILE__, __LINE__);
+}
+
 }  // namespace
 }  // namespace chl
 
@@ -958,8 +982,11 @@ extern "C" int chl_query_batch(const chl_labels *l, const uint32_t *pairs, size_
         return CHL_ERR_INVALID;
     }
     if (k == 0) return CHL_OK;
+    int rc;
+    // (without room on the device the slots do)
+    if (k >= kStagedPairs && (rc = query_staged(l, pairs, k, out, (cudaStream_t)stream)) != CHL_ERR_OOM) return rc;
     SlotSet *s = nullptr;
-    int rc = take_slots(&s);
+    rc = take_slots(&s);
     if (rc) return rc;
     rc = query_slots(l, pairs, k, out, (cudaStream_t)stream, s);
     if (rc) {

@@ -38,6 +38,15 @@ else:
     order = np.random.default_rng(1).permutation(n).astype(np.uint32)
 want = P.build(g, order, **spec["kw"])
 got = []
+if spec["kind"] == "pairs":   # host batches without room to stage them
+    pairs = P.generate_query(400_000, n, seed=1)
+    pairs[::3] = np.minimum(pairs[::3], n - 2) | np.array([0, 1], np.uint32)
+    answers = P.query(want, pairs)
+    assert (answers < P.INFTY).any()
+    P.lib().chl_graph_release_device(g._h)
+    fake.fake_device_set(fake.fake_device_live())
+    assert np.array_equal(P.query(want, pairs), answers)
+    fake.fake_device_set(C.c_size_t(-1).value)
 for limit in spec["limits"]:
     fake.fake_device_set(limit + fake.fake_device_live())
     try:

@@ -213,3 +213,46 @@ def test_device_query_groups(P, O, more):
     want[~out_of_range] = ref.query(pairs[~out_of_range])
     assert np.array_equal(got[:k], want)
     assert (got[k:] == -7).all()
+
+
+@pytest.mark.parametrize("k", [65537, 196607, 196608, 196609, 400_003])
+def test_query_staged_batches(P, O, k):
+    """Host batches either side of the size from which they are staged whole
+    (196,608 pairs), from several threads at once on the same labels."""
+    import threading
+    g = P.Graph.rmat(10, 8, seed=2)
+    L = P.build(g, P.Order.degree(g, seed=1))
+    ref = O.OLabels.from_csr(g.get_n(), *L.export())
+    pairs = [P.generate_query(k, g.get_n(), seed=s) for s in range(4)]
+    got = [None] * 4
+
+    def ask(i):
+        for _ in range(3):
+            got[i] = P.query(L, pairs[i])
+
+    ts = [threading.Thread(target=ask, args=(i,)) for i in range(4)]
+    for x in ts:
+        x.start()
+    for x in ts:
+        x.join()
+    for p, a in zip(pairs, got):
+        assert np.array_equal(a, ref.query(p))
+
+
+def test_query_huge_batch_is_not_slower_per_pair(P):
+    """16 M pairs cost no more each than 2 M: answers past the caches made a
+    pair 1.4 times as dear while they went through the slots."""
+    import time
+    g = P.Graph.grid(12, 12, seed=1)
+    L = P.build(g, P.Order.degree(g, seed=1))
+
+    def per_pair(k):
+        pairs = P.generate_query(k, g.get_n(), seed=1)
+        best = np.inf
+        for _ in range(6):
+            t = time.perf_counter()
+            P.query(L, pairs)
+            best = min(best, time.perf_counter() - t)
+        return best / k
+
+    assert per_pair(16_000_000) < 1.2 * per_pair(2_000_000)
