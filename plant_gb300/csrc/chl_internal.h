@@ -9,6 +9,7 @@
 #include <utility>
 #include <vector>
 #include <atomic>
+#include <mutex>
 
 #include "../../include/chl.h"
 
@@ -105,12 +106,17 @@ struct NoInitAlloc : std::allocator<T> {
 struct chl_labels {
     uint32_t n = 0;
     bool sym = false;
-    mutable uint64_t *d_off = nullptr;   // nl+1 entries, nl = sym ? n : 2n
+    // The device copy and the host mirror are made on first use, by whichever
+    // call comes first: under `lazy`, each published last and whole (d_off after
+    // d_ent, host_valid after both vectors), since queries of one labeling may
+    // run at once.
+    mutable std::mutex lazy;
+    mutable std::atomic<uint64_t *> d_off{nullptr};   // nl+1 entries, nl = sym ? n : 2n
     mutable LabelEnt *d_ent = nullptr;   // uploaded lazily for imported labels
     uint64_t total = 0;              // entries stored (one side if sym)
     mutable std::vector<uint64_t> h_off;
     mutable std::vector<LabelEnt, NoInitAlloc<LabelEnt>> h_ent;
-    mutable bool host_valid = false;
+    mutable std::atomic<bool> host_valid{false};
     mutable std::atomic<bool> exported{false};   // an export went past the mirror
     chl_build_stats stats{};
     uint32_t nl() const { return sym ? n : 2 * n; }

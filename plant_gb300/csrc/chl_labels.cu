@@ -177,6 +177,8 @@ int d2h_staged(void *dst, const void *src, size_t bytes) {
 
 int labels_fetch_host(const chl_labels *l) {
     if (l->host_valid) return CHL_OK;
+    std::lock_guard<std::mutex> g(l->lazy);
+    if (l->host_valid) return CHL_OK;
     if (!l->d_off) return CHL_ERR_INVALID;
     const uint32_t nl = l->nl();
     l->h_off.resize((size_t)nl + 1);
@@ -190,21 +192,24 @@ int labels_fetch_host(const chl_labels *l) {
 
 int labels_ensure_device(const chl_labels *L) {
     if (L->d_off) return CHL_OK;
+    std::lock_guard<std::mutex> g(L->lazy);
+    if (L->d_off) return CHL_OK;
     const uint32_t nl = L->nl();
-    cudaError_t e = long_malloc(&L->d_off, ((size_t)nl + 1) * 8);
-    if (e == cudaSuccess) e = long_malloc(&L->d_ent, std::max<uint64_t>(L->total, 1) * sizeof(LabelEnt));
-    if (e == cudaSuccess)
-        e = cudaMemcpy(L->d_off, L->h_off.data(), ((size_t)nl + 1) * 8, cudaMemcpyHostToDevice);
+    uint64_t *off = nullptr;
+    LabelEnt *ent = nullptr;
+    cudaError_t e = long_malloc(&off, ((size_t)nl + 1) * 8);
+    if (e == cudaSuccess) e = long_malloc(&ent, std::max<uint64_t>(L->total, 1) * sizeof(LabelEnt));
+    if (e == cudaSuccess) e = cudaMemcpy(off, L->h_off.data(), ((size_t)nl + 1) * 8, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && L->total)
-        e = cudaMemcpy(L->d_ent, L->h_ent.data(), L->total * sizeof(LabelEnt), cudaMemcpyHostToDevice);
+        e = cudaMemcpy(ent, L->h_ent.data(), L->total * sizeof(LabelEnt), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         int rc = cuda_status(e, "label upload", __FILE__, __LINE__);
-        cudaFree(L->d_off);
-        cudaFree(L->d_ent);
-        L->d_off = nullptr;
-        L->d_ent = nullptr;
+        cudaFree(off);
+        cudaFree(ent);
         return rc;
     }
+    L->d_ent = ent;
+    L->d_off = off;   // published whole
     return CHL_OK;
 }
 

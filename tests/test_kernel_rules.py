@@ -43,3 +43,17 @@ def test_line_order_is_not_read_from_a_lane_mask():
     parse = body("chl_ingest.cu", "parse_lines(")
     tail = parse[parse.rindex("kFailFormat"):]
     assert "__shfl_xor_sync(kFull, first_a" in tail and "atomicMin(&po->first_a, first_a)" in tail
+
+
+def test_lazily_made_copies_are_published_whole():
+    """Labels read from host memory are uploaded by their first query, and
+    several queries may come first: one uploads, under a lock, and the pointer
+    that the others test is set after the last copy.  (Shown by reading: a query
+    that saw it earlier would walk memory that is not there yet.)"""
+    up = body("chl_labels.cu", "labels_ensure_device(const chl_labels *L)")
+    assert "lock_guard" in up and "&L->d_off" not in up and "&L->d_ent" not in up
+    assert up.rindex("cudaMemcpy(") < up.rindex("L->d_ent =") < up.rindex("L->d_off =")
+    down = body("chl_labels.cu", "labels_fetch_host(const chl_labels *l)")
+    assert "lock_guard" in down and down.rindex("d2h_staged(") < down.rindex("l->host_valid = true")
+    src = open(os.path.join(ROOT, "plant_gb300", "csrc", "chl_internal.h")).read()
+    assert re.search(r"std::atomic<uint64_t \*> d_off", src) and re.search(r"std::atomic<bool> host_valid", src)

@@ -256,3 +256,37 @@ def test_query_huge_batch_is_not_slower_per_pair(P):
         return best / k
 
     assert per_pair(16_000_000) < 1.2 * per_pair(2_000_000)
+
+
+def test_first_queries_and_exports_at_once(P):
+    """Labels from host memory are uploaded, and a build's host mirror is made,
+    once and whole whichever of several threads comes first."""
+    import threading
+    g = P.Graph.grid(60, 60, seed=3)
+    built = P.build(g, P.Order.degree(g, seed=1))
+    csr = built.export()
+    pairs = P.generate_query(5000, g.get_n(), seed=2)
+    want, sizes = P.query(built, pairs), built.list_sizes()
+    bad = []
+
+    def run(jobs):
+        gate = threading.Barrier(len(jobs))
+
+        def work(job):
+            gate.wait()
+            if not job():
+                bad.append(job)
+
+        ts = [threading.Thread(target=work, args=(j,)) for j in jobs]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+
+    for _ in range(5):
+        L = P.Labeling.from_csr(g.get_n(), *csr)
+        run([lambda L=L: np.array_equal(P.query(L, pairs), want)] * 12)
+        B = P.build(g, P.Order.degree(g, seed=1))
+        run([lambda B=B: all(np.array_equal(x, y) for x, y in zip(B.export(), csr))] * 4
+            + [lambda B=B: len(B.label(7, 0)[0]) == sizes.reshape(-1, 2)[7, 0]] * 4)
+    assert not bad
